@@ -59,6 +59,10 @@ struct tcw_plan {
   uint32_t *d_rect_list = nullptr, *d_exp_list = nullptr, *d_t0s = nullptr, *d_taus = nullptr;
   uint32_t n_exp = 0;
   float *d_A8 = nullptr;  // exp templates' atoms in rows of 8 floats
+  // row-chunked exp columns: segments and their sums
+  SegItem *d_segs = nullptr;
+  uint32_t n_segs = 0;
+  float *d_G = nullptr;
   uint32_t *d_counter = nullptr;  // [0] rect tiles, [1] exp tiles
   float *d_P = nullptr;
   // graph state
@@ -208,10 +212,9 @@ int prec_of(int flags) {
 }
 
 // Tiles of one template.  Rect: tn columns x tm rows per block.  Exp: tn
-// columns per block, each thread one column over `rows` rows, the block's
-// 128/tn thread rows covering consecutive row chunks; with `warp_tiles`
-// (persistent plans, whose exp kernel schedules by warp) 32 columns over
-// `rows` rows per tile.
+// columns per block over the 128 / tn next row chunks (t.e_rows rows each);
+// with `warp_tiles` (persistent plans, whose exp kernel schedules by warp) 32
+// columns over one chunk per tile.
 void tile_template(uint32_t tmpl, const TemplateDev &t, const tcw_tile_config &cfg,
                    std::vector<WorkItem> &items, std::vector<double> *cost,
                    bool warp_tiles = false) {
@@ -227,38 +230,42 @@ void tile_template(uint32_t tmpl, const TemplateDev &t, const tcw_tile_config &c
         w.n0 = n0;
         w.n1 = std::min(N_tau, n0 + tn);
         w.tn = (uint16_t)(tm / 32u);  // row groups of 32 rows (one per warp)
-        w.rows_per_lane = 0;
         items.push_back(w);
         if (cost) cost->push_back((double)(w.m1 - w.m0) * (w.n1 - w.n0));
       }
   } else {
     const uint32_t tn = warp_tiles ? 32u : cfg.exp_tn, lanes = warp_tiles ? 1u : kBlock / tn;
-    uint32_t rows = cfg.exp_rows ? cfg.exp_rows : N_t0;
-    // a lane's row chunk is a 16-bit count: longer columns become several tiles
-    rows = std::min(std::min(rows, N_t0), 65535u);
-    const uint32_t span = rows * lanes;  // rows per block
+    const uint32_t chunks = (N_t0 + t.e_hist - 1u) / t.e_hist * t.e_sub;
     for (uint32_t n0 = 0; n0 < N_tau; n0 += tn)
-      for (uint32_t m0 = 0; m0 < N_t0; m0 += span) {
+      for (uint32_t c0 = 0; c0 < chunks; c0 += lanes) {
         WorkItem w{};
         w.tmpl = tmpl;
-        w.m0 = m0;
-        w.m1 = std::min(N_t0, m0 + span);
+        w.m0 = c0;
+        w.m1 = std::min(chunks, c0 + lanes);
         w.n0 = n0;
         w.n1 = std::min(N_tau, n0 + tn);
         w.tn = (uint16_t)tn;
-        w.rows_per_lane = (uint16_t)rows;
         items.push_back(w);
         if (cost) {
           // recurrence steps: window warm-up plus the rows' atom span, per column
           double atoms_per_row = 1.0;
           if (N_t0 > 1) atoms_per_row = std::max(1.0, (double)t.g.numAtoms / N_t0);
-          double rows_here = (double)(w.m1 - w.m0);
+          const double rows_here = std::min(N_t0, t.e_rows);
           double warm = std::min((double)t.g.numAtoms, 3.0 * (double)N_tau) * lanes;
+          if (t.g_nseg) warm = std::min(warm, 2.0 * (double)(1u << t.g_shift));
           cost->push_back(((rows_here * atoms_per_row * 2.0 + warm) * 2.0 + rows_here) *
                           (w.n1 - w.n0) / 1.0);
         }
       }
   }
+}
+
+#ifndef TCW_PLAN_EXP_TILES
+#define TCW_PLAN_EXP_TILES 2
+#endif
+// Rows of a history for exp_rows of a tile configuration (0: whole columns).
+uint32_t exp_hist(uint32_t exp_rows, uint32_t N_t0) {
+  return std::min(std::min(exp_rows ? exp_rows : N_t0, N_t0), 65535u);
 }
 
 void default_plain_cfg(const TemplateDev &t, tcw_tile_config &cfg, int n_sms) {
@@ -273,10 +280,6 @@ void default_plain_cfg(const TemplateDev &t, tcw_tile_config &cfg, int n_sms) {
     cfg.rect_tn = (uint32_t)tn;
   } else {
     cfg.exp_tn = 32;
-    // rows per thread: enough chunks for parallelism, long enough to amortise
-    // each chunk's warm-up over the window
-    uint32_t rows = std::max<uint32_t>(8, (t.N_t0 + 15) / 16);
-    cfg.exp_rows = std::min(rows, t.N_t0);
   }
 }
 
@@ -521,11 +524,19 @@ static int plain_enqueue(tcw_handle *h, const float *d_atoms, uint32_t numAtoms,
                          tcw_result *d_result, int flags, char *ws, size_t ws_off) {
   TemplateDev t = make_tdev(numAtoms, TAtom, t0_data, window, N_t0, N_tau);
   tcw_tile_config cfg = h->plain_cfg;
+  const int prec = prec_of(flags);
   default_plain_cfg(t, cfg, h->n_sms);
   if (h->plain_cfg.rect_tn) cfg.rect_tn = h->plain_cfg.rect_tn;
   if (h->plain_cfg.rect_tm) cfg.rect_tm = h->plain_cfg.rect_tm;
   if (h->plain_cfg.exp_tn) cfg.exp_tn = h->plain_cfg.exp_tn;
-  if (h->plain_cfg.exp_rows) cfg.exp_rows = h->plain_cfg.exp_rows;
+  uint64_t seg_floats = 0;
+  uint32_t n_seg_items = 0;
+  if (window == TCW_WINDOW_EXP) {
+    const ExpSplit sp = plain_exp_split(numAtoms, N_t0, N_tau, h->n_sms, prec != kPrecPlain32);
+    set_split(t, sp);
+    seg_floats = sp.seg_floats(N_tau);
+    n_seg_items = (N_tau + 31u) / 32u * ((sp.nseg + kSegPerWarp - 1u) / kSegPerWarp);
+  }
   fill_cfg_defaults(cfg);
   std::vector<WorkItem> items;
   try {
@@ -554,6 +565,7 @@ static int plain_enqueue(tcw_handle *h, const float *d_atoms, uint32_t numAtoms,
   const size_t o_A8 = window == TCW_WINDOW_EXP
                           ? L.add(sizeof(float) * 8u * (size_t)numAtoms)
                           : 0;
+  const size_t o_G = L.add(sizeof(float) * seg_floats);
   const size_t o_row = post ? L.add(sizeof(double) * N_t0) : 0;
   const size_t o_col = post ? L.add(sizeof(double) * (size_t)n_chunks * N_tau) : 0;
   int rc = ensure_ws(h, L.total);
@@ -571,7 +583,6 @@ static int plain_enqueue(tcw_handle *h, const float *d_atoms, uint32_t numAtoms,
   TCW_CUDA(h, cudaEventRecord(h->stage_ev, h->stream));
   h->stage_pending = true;
 
-  const int prec = prec_of(flags);
   const TemplateDev *dT = reinterpret_cast<const TemplateDev *>(ws + o_T);
   float *dP = window == TCW_WINDOW_RECT ? reinterpret_cast<float *>(ws + o_P) : nullptr;
   Partial *dparts = reinterpret_cast<Partial *>(ws + o_parts);
@@ -582,6 +593,8 @@ static int plain_enqueue(tcw_handle *h, const float *d_atoms, uint32_t numAtoms,
   if (window == TCW_WINDOW_EXP)
     TCW_CUDA(h, launch_repack(dT, reinterpret_cast<const uint32_t *>(ws + o_list), 1, d_atoms,
                               dA8, h->stream));
+  float *dG = reinterpret_cast<float *>(ws + o_G);
+  TCW_CUDA(h, launch_exp_segments(dT, nullptr, n_seg_items, dA8, d_taus, dG, h->stream));
   MapLaunch ml{};
   ml.T = dT;
   ml.items = reinterpret_cast<const WorkItem *>(ws + o_items);
@@ -592,6 +605,7 @@ static int plain_enqueue(tcw_handle *h, const float *d_atoms, uint32_t numAtoms,
   ml.priority = h->prio_low;
   ml.atoms = d_atoms;
   ml.atoms8 = dA8;
+  ml.G = dG;
   ml.t0s = d_t0s;
   ml.taus = d_taus;
   ml.P = dP;
@@ -683,7 +697,13 @@ int tcw_map_plain_host(tcw_handle *h, const float *atoms, uint32_t numAtoms, uin
     L2.add(sizeof(WorkItem) * items_est);
     L2.add(sizeof(Partial) * items_est);
     if (window == TCW_WINDOW_RECT) L2.add(sizeof(float) * kPrefixStride * ((size_t)numAtoms + 1));
-    if (window == TCW_WINDOW_EXP) L2.add(sizeof(float) * 8u * (size_t)numAtoms);
+    if (window == TCW_WINDOW_EXP) {
+      L2.add(sizeof(float) * 8u * (size_t)numAtoms);
+      L2.add(sizeof(float) *
+             plain_exp_split(numAtoms, N_t0, N_tau, h->n_sms,
+                             prec_of(flags) != kPrecPlain32)
+                 .seg_floats(N_tau));
+    }
     L2.add(sizeof(double) * N_t0);
     L2.add(sizeof(double) * ((N_t0 + 63u) / 64u) * (size_t)N_tau);
     need_after = L2.total;
@@ -746,6 +766,22 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   std::vector<double> cost;
   std::vector<uint32_t> rect_list, exp_list;
   uint64_t p_rows = 0, a8_rows = 0, atom_rows = 0, cells = 0;
+  // Row chunks of exp columns when the caller leaves them to the library
+  // (exp_rows 0): whole columns while these fill the GPU, else as many
+  // chunks per column as bring the warp tiles to TCW_PLAN_EXP_TILES per
+  // resident warp (32 per SM), started from segment sums (a run of 96
+  // templates with maps and posteriors: whole columns 3.63 ms, 1 tile per
+  // warp 2.82, 2 tiles 2.74, 3 tiles 2.78; the 74 000 column tiles of 4096
+  // templates stay whole).
+  uint64_t exp_chunks = 1, seg_blocks = 0;
+  if (cfg.exp_rows == 0 && p->prec != kPrecPlain32) {
+    uint64_t tiles = 0;
+    for (uint32_t k = 0; k < n_templates; k++)
+      if (desc[k].window == TCW_WINDOW_EXP) tiles += ((uint64_t)desc[k].N_tau + 31u) / 32u;
+    const uint64_t want = (uint64_t)h->n_sms * 32u * TCW_PLAN_EXP_TILES;
+    if (tiles) exp_chunks = (want + tiles - 1u) / tiles;
+  }
+  std::vector<SegItem> segs;
   try {
     for (uint32_t k = 0; k < n_templates; k++) {
       const tcw_template_desc &d = desc[k];
@@ -791,6 +827,18 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
       atom_rows = std::max<uint64_t>(atom_rows, d.atom_offset + d.numAtoms);
       cells += (uint64_t)d.N_t0 * d.N_tau;
       const size_t first = items.size();
+      if (d.window == TCW_WINDOW_EXP) {
+        const uint32_t hist = exp_hist(cfg.exp_rows, d.N_t0), groups = (d.N_tau + 31u) / 32u;
+        ExpSplit sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, hist, exp_chunks);
+        if ((seg_blocks + (uint64_t)groups * sp.nseg) * kSegFloats * sizeof(float) > kSegBytesMax)
+          sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, hist, 1);
+        set_split(t, sp);
+        t.g_off = seg_blocks;
+        seg_blocks += (uint64_t)groups * sp.nseg;
+        for (uint32_t cg = 0; cg < groups; cg++)
+          for (uint32_t j = 0; j < sp.nseg; j += kSegPerWarp)
+            segs.push_back(SegItem{k, cg, j, std::min(sp.nseg, j + kSegPerWarp)});
+      }
       tile_template(k, t, cfg, items, &cost, true);
       t.part_off = (uint32_t)first;
       t.n_parts = (uint32_t)(items.size() - first);
@@ -826,6 +874,7 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   p->n_items = (uint32_t)items.size();
   p->n_rect = (uint32_t)rect_list.size();
   p->n_exp = (uint32_t)exp_list.size();
+  p->n_segs = (uint32_t)segs.size();
   p->n_cells = cells;
   p->n_atom_rows = atom_rows;
   p->p_rows = p_rows;
@@ -847,8 +896,10 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   const size_t o_elist = L.add(sizeof(uint32_t) * std::max<size_t>(1, exp_list.size()));
   const size_t o_t0 = L.add(sizeof(uint32_t) * n_t0s);
   const size_t o_tau = L.add(sizeof(uint32_t) * n_taus);
+  const size_t o_segs = L.add(sizeof(SegItem) * segs.size());
   const size_t ctl_end = L.total;
   const size_t o_parts = L.add(sizeof(Partial) * p->n_items);
+  const size_t o_G = L.add(sizeof(float) * kSegFloats * seg_blocks);
   const size_t o_P = L.add(sizeof(float) * kPrefixStride * std::max<uint64_t>(1, p_rows));
   const size_t o_A8 = L.add(sizeof(float) * 8u * std::max<uint64_t>(1, a8_rows));
   const size_t o_cnt = L.add(2 * sizeof(uint32_t));
@@ -868,6 +919,8 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   p->d_rect_list = reinterpret_cast<uint32_t *>(p->d_buf + o_list);
   p->d_exp_list = reinterpret_cast<uint32_t *>(p->d_buf + o_elist);
   p->d_A8 = reinterpret_cast<float *>(p->d_buf + o_A8);
+  p->d_segs = reinterpret_cast<SegItem *>(p->d_buf + o_segs);
+  p->d_G = reinterpret_cast<float *>(p->d_buf + o_G);
   p->d_t0s = reinterpret_cast<uint32_t *>(p->d_buf + o_t0);
   p->d_taus = reinterpret_cast<uint32_t *>(p->d_buf + o_tau);
   p->d_parts = reinterpret_cast<Partial *>(p->d_buf + o_parts);
@@ -889,6 +942,7 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
     memcpy(host.data() + o_elist, exp_list.data(), sizeof(uint32_t) * exp_list.size());
   memcpy(host.data() + o_t0, t0s, sizeof(uint32_t) * n_t0s);
   memcpy(host.data() + o_tau, taus, sizeof(uint32_t) * n_taus);
+  if (!segs.empty()) memcpy(host.data() + o_segs, segs.data(), sizeof(SegItem) * segs.size());
   cudaError_t e = cudaMemcpy(p->d_buf, host.data(), ctl_end, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && post && !post_chunks.empty())
     e = cudaMemcpy(p->d_post_chunks, post_chunks.data(), sizeof(uint2) * post_chunks.size(),
@@ -941,6 +995,7 @@ static MapLaunch plan_launch(const tcw_handle *h, const tcw_plan *p, int window,
   ml.priority = rect ? h->prio_low : h->prio_high;
   ml.atoms = d_atoms;
   ml.atoms8 = p->d_A8;
+  ml.G = p->d_G;
   ml.t0s = p->d_t0s;
   ml.taus = p->d_taus;
   ml.P = p->d_P;
@@ -968,6 +1023,8 @@ static int plan_enqueue(tcw_handle *h, tcw_plan *p, const float *d_atoms, tcw_re
   TCW_CUDA(h, cudaStreamWaitEvent(h->side_stream, h->fork_ev, 0));
   TCW_CUDA(h, launch_repack(p->d_T, p->d_exp_list, p->n_exp, d_atoms, p->d_A8, h->stream));
   if (inputs_read) TCW_CUDA(h, cudaEventRecord(inputs_read, h->stream));
+  TCW_CUDA(h, launch_exp_segments(p->d_T, p->d_segs, p->n_segs, p->d_A8, p->d_taus, p->d_G,
+                                  h->stream));
   TCW_CUDA(h, launch_prefix(p->d_T, p->d_rect_list, p->n_rect, d_atoms, p->d_P, p->prec,
                             h->side_stream));
   if (inputs_read_side) TCW_CUDA(h, cudaEventRecord(inputs_read_side, h->side_stream));
@@ -1056,6 +1113,8 @@ int tcw_plan_run_timed(tcw_handle *h, tcw_plan *p, const float *d_atoms, tcw_res
   TCW_CUDA(h, launch_prefix(p->d_T, p->d_rect_list, p->n_rect, d_atoms, p->d_P, p->prec,
                             h->stream));
   TCW_CUDA(h, launch_repack(p->d_T, p->d_exp_list, p->n_exp, d_atoms, p->d_A8, h->stream));
+  TCW_CUDA(h, launch_exp_segments(p->d_T, p->d_segs, p->n_segs, p->d_A8, p->d_taus, p->d_G,
+                                  h->stream));
   TCW_CUDA(h, cudaEventRecord(ev[1], h->stream));
   TCW_CUDA(h, launch_map(TCW_WINDOW_RECT, plan_launch(h, p, TCW_WINDOW_RECT, d_atoms, nullptr),
                          h->stream));

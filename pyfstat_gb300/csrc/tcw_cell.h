@@ -969,6 +969,17 @@ TCW_HD FF ff_axpy_ord(float x, FF r, FF E) {
   return FF{s, fadd(e, pe)};
 }
 
+// X + R*E for double-words X, R, E (R = rh + rl, nrh = -rh): a segment sum
+// joined to the window sum above it (TwoSum, whatever the operands).
+TCW_HD FF2 ff2_axpy_dw(FF2 X, F2 rh, F2 nrh, F2 rl, FF2 E) {
+  const FF2 r = ff2_axpy(X.h, rh, nrh, rl, E);
+  return FF2{r.h, add2(r.l, X.l)};
+}
+TCW_HD FF ff_axpy_dw(FF X, FF r, FF E) {
+  const FF s = ff_axpy(X.h, r, E);
+  return FF{s.h, fadd(s.l, X.l)};
+}
+
 // The scalar form of ff2_sub_scaled_x (W - p*x for the C channel).
 TCW_HD FF ff_sub_scaled_x1(FF W, FF p, float x) {
   const float a = fmul(p.h, x);
@@ -1289,6 +1300,46 @@ struct ExpColumn {
       load_row8(atoms8 + (size_t)wlo * 8u, x);
       enter(x);
     }
+  }
+
+  // The window sums as stored by exp_seg_kernel for one lane (stride 32).
+  TCW_HDM void store_sums(float *__restrict__ o) const {
+    const float v[14] = {W0.h.x, W0.h.y, W0.l.x, W0.l.y, Wc.h,   Wc.l,   W2.h.x,
+                         W2.h.y, W2.l.x, W2.l.y, W3.h.x, W3.h.y, W3.l.x, W3.l.y};
+#pragma unroll
+    for (int f = 0; f < 14; f++) o[32 * f] = v[f];
+  }
+
+  // Starts a row chunk at the window [lo, top), top - lo >= 2 segments of
+  // 2^shift atoms, from segment sums G_j = sum over the segment's atoms of
+  // x_i r^(i - j 2^shift) (exp_seg_kernel; `seg` is this lane's first value
+  // of segment 0): the atoms above the last whole segment enter one by one,
+  // then each segment below is joined by W = G_j + r^(2^shift) W.  Leaves
+  // wtop = top and wlo at the lowest joined segment (>= lo); the first row
+  // enters the rest.  Entering the whole window instead costs every chunk up
+  // to numAtoms steps.
+  TCW_HDM void warm_start(const float *__restrict__ atoms8, const Geom &g,
+                          const float *__restrict__ seg, uint32_t shift, uint32_t nseg,
+                          uint32_t lo, uint32_t top) {
+    const uint32_t j1 = (lo + (1u << shift) - 1u) >> shift;
+    const uint32_t j2 = top == g.numAtoms ? nseg : top >> shift;
+    reset_window(top);
+    if (top != g.numAtoms) enter_to(atoms8, g, j2 << shift);
+    FF R = k.r1;  // r^(2^shift) by squaring
+    for (uint32_t b = 0; b < shift; b++) R = ff_mul(R, R);
+    const FF R2 = ff_mul(R, R);
+    const F2 rh0{R2.h, R2.h}, nrh0{-R2.h, -R2.h}, rl0{R2.l, R2.l};
+    const F2 rh1{R.h, R.h}, nrh1{-R.h, -R.h}, rl1{R.l, R.l};
+    for (uint32_t j = j2; j > j1;) {
+      j--;
+      TCW_DCHECK(j < nseg);
+      const float *s = seg + (size_t)j * (14u * 32u);
+      W0 = ff2_axpy_dw(FF2{F2{s[0], s[32]}, F2{s[64], s[96]}}, rh0, nrh0, rl0, W0);
+      Wc = ff_axpy_dw(FF{s[128], s[160]}, R2, Wc);
+      W2 = ff2_axpy_dw(FF2{F2{s[192], s[224]}, F2{s[256], s[288]}}, rh1, nrh1, rl1, W2);
+      W3 = ff2_axpy_dw(FF2{F2{s[320], s[352]}, F2{s[384], s[416]}}, rh1, nrh1, rl1, W3);
+    }
+    wlo = j1 << shift;
   }
 
   // W = x + r W for one entering atom row (exp_column2's steps).

@@ -33,21 +33,105 @@ struct TemplateDev {
   uint32_t part_off, n_parts;
   uint32_t pad;
   uint64_t row_off, col_off;  // posterior row partials / column sums (plans with posteriors)
+  // exp templates whose columns are cut into row chunks: segment sums of
+  // 2^g_shift atoms (exp_seg_kernel), g_nseg segments per 32-column group
+  // (0: none), starting at float g_off * kSegFloats
+  uint64_t g_off;
+  uint32_t g_shift, g_nseg;
+  uint32_t e_hist, e_rows, e_sub;  // row chunks (ExpSplit)
+  uint32_t pad2;
 };
+// Floats of one 32-column segment sum (7 channels x hi, lo x 32 lanes).
+constexpr uint32_t kSegFloats = 14u * 32u;
+// Segments of one warp of exp_seg_kernel: amortises the column's FP64 exp.
+constexpr uint32_t kSegPerWarp = 4u;
 
-// A tile of one template: rows [m0, m1) x columns [n0, n1).  For a
-// rectangular tile the block's threads are (tn columns) x (128/tn row lanes);
-// for an exponential tile each thread runs one column over a row chunk of
-// `rows_per_lane` rows.
+// A tile of one template, columns [n0, n1).  For a rectangular tile [m0, m1)
+// are its rows and tn its groups of 32 rows; for an exponential tile they are
+// row chunks (TemplateDev::e_rows), each walked by one warp per 32 columns.
 struct WorkItem {
   uint32_t tmpl;
   uint32_t part;
   uint32_t m0, m1;
   uint32_t n0, n1;
-  uint16_t tn;            // columns per block (32, 64 or 128)
-  uint16_t rows_per_lane; // exp only: rows per thread chunk
+  uint16_t tn;            // rect: row groups; exp: columns per block (32, 64 or 128)
+  uint16_t pad16;
   uint32_t pad;
 };
+
+// Segments [j0, j1) of 32-column group cg of one exp template.
+struct SegItem {
+  uint32_t tmpl, cg, j0, j1;
+};
+
+// How an exp template's columns are cut into row chunks.  `hist` rows are one
+// history: a window's sums keep the roundings of the rows above it in the
+// same history and start afresh at the next one.  Each history is walked in
+// `sub` chunks of `rows` rows, side by side, whose starts are combined from
+// nseg segment sums of 2^shift atoms (0: every chunk enters its whole window,
+// sub is 1).
+struct ExpSplit {
+  uint32_t hist, rows, sub, shift, nseg;
+  uint32_t chunks(uint32_t N_t0) const { return (N_t0 + hist - 1u) / hist * sub; }
+  uint64_t seg_floats(uint32_t N_tau) const {
+    return (uint64_t)((N_tau + 31u) / 32u) * nseg * kSegFloats;
+  }
+};
+constexpr uint64_t kSegBytesMax = 1ull << 30;
+// Windows of fewer atoms have a history that F shows (a near-singular F
+// amplifies the roundings that Fast2Sum leaves in Fa and Fb by up to
+// 2 sqrt(1e4)): a chunk whose columns have such windows starts kRunUp tau
+// earlier, where a rounding's weight is below e^-12 and F is that of the whole
+// history (without the run-up maxF of ~2 % of the benchmark's exp templates
+// moved by up to 2e-7; with 64 atoms and 18 tau the run-up was as long as
+// the chunks: 406 against 227 us per run of 24 templates of up to 1500 atoms).
+constexpr uint32_t kShortWindow = 32;
+constexpr uint32_t kRunUp = 12;
+
+// At least `chunks` chunks per column where histories allow it (8 rows or
+// more each).  Segments of about sqrt(numAtoms) atoms: a chunk start costs up
+// to 2 x 2^shift entering steps and numAtoms / 2^shift joins.
+inline ExpSplit exp_split(uint32_t numAtoms, uint32_t N_t0, uint32_t N_tau, uint32_t hist,
+                          uint64_t chunks) {
+  ExpSplit s{hist, hist, 1, 5, 0};
+  const uint64_t n_hist = (N_t0 + hist - 1u) / hist;
+  const uint64_t sub = (chunks + n_hist - 1) / n_hist;
+  if (sub <= 1 || numAtoms < 2u * kShortWindow) return s;
+  const uint64_t rows = (hist + sub - 1) / sub;
+  s.rows = rows < 8 ? 8u : (uint32_t)rows;
+  s.sub = (hist + s.rows - 1u) / s.rows;
+  while ((4ull << (2u * s.shift)) <= numAtoms) s.shift++;
+  s.nseg = (uint32_t)(((uint64_t)numAtoms + (1u << s.shift) - 1u) >> s.shift);
+  if (s.sub <= 1 || s.seg_floats(N_tau) * sizeof(float) > kSegBytesMax)
+    return ExpSplit{hist, hist, 1, 5, 0};
+  return s;
+}
+
+// Row chunks of a single-template exp map: 16 histories per column, cut
+// further (`cut`) until there are about TCW_PLAIN_EXP_WARPS warps per
+// scheduler (one-year 8192 x 4096 map, whole call: 4 warps 908 us, 6 762 us,
+// 8 687 us, 12 709 us).
+#ifndef TCW_PLAIN_EXP_WARPS
+#define TCW_PLAIN_EXP_WARPS 8
+#endif
+inline ExpSplit plain_exp_split(uint32_t numAtoms, uint32_t N_t0, uint32_t N_tau, int n_sms,
+                                bool cut) {
+  uint32_t hist = (N_t0 + 15u) / 16u;
+  hist = hist < 8u ? 8u : hist;
+  hist = hist < N_t0 ? hist : N_t0;
+  hist = hist < 65535u ? hist : 65535u;
+  const uint64_t groups = (N_tau + 31u) / 32u;
+  const uint64_t want = (uint64_t)n_sms * 4u * TCW_PLAIN_EXP_WARPS;
+  return exp_split(numAtoms, N_t0, N_tau, hist, cut ? (want + groups - 1u) / groups : 1u);
+}
+
+inline void set_split(TemplateDev &t, const ExpSplit &sp) {
+  t.e_hist = sp.hist;
+  t.e_rows = sp.rows;
+  t.e_sub = sp.sub;
+  t.g_shift = sp.shift;
+  t.g_nseg = sp.nseg;
+}
 
 // Per-item reduction result.  s = sum over the item's cells of exp(F - maxF).
 struct Partial {
@@ -103,6 +187,12 @@ cudaError_t launch_prefix(const TemplateDev *d_T, const uint32_t *d_rect_list, u
 // Exp templates' atoms (rows of 7 floats) into rows of 8 (zero-padded).
 cudaError_t launch_repack(const TemplateDev *d_T, const uint32_t *d_exp_list, uint32_t n_exp,
                           const float *d_atoms, float *d_atoms8, cudaStream_t stream);
+// Segment sums of exp templates (the chunk starts of exp tiles are combined
+// from them): items == NULL means template 0's columns and segments, with
+// n_items = column groups x ceil(segments / kSegPerWarp).
+cudaError_t launch_exp_segments(const TemplateDev *d_T, const SegItem *d_items, uint32_t n_items,
+                                const float *d_atoms8, const uint32_t *d_taus, float *d_G,
+                                cudaStream_t stream);
 struct MapLaunch {
   const TemplateDev *T;
   const WorkItem *items;  // this window's tiles
@@ -114,6 +204,7 @@ struct MapLaunch {
   int priority;           // stream-priority value of the launch
   const float *atoms;
   const float *atoms8;    // exp tiles: atoms in 32-byte rows
+  const float *G;         // exp tiles: segment sums (NULL where no template has any)
   const uint32_t *t0s, *taus;
   const float *P;
   float *Fmn;

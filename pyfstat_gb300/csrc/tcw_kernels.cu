@@ -469,9 +469,14 @@ struct MapSink {
   float *Fmn;
   uint32_t N_tau, n;
   Red *red;
+  bool live;
+  __device__ __forceinline__ void start() {
+    red->init();
+    live = true;
+  }
   __device__ __forceinline__ void operator()(uint32_t m, float F, bool) {
     TCW_DCHECK(n < N_tau);
-    if (kWrite) Fmn[(size_t)m * N_tau + n] = F;
+    if (kWrite && live) Fmn[(size_t)m * N_tau + n] = F;
     red->add_row_desc(F, m);
   }
 };
@@ -488,18 +493,33 @@ constexpr uint32_t kExpRowTab = 128;
 
 // The row-table walk of one warp's column chunk [mb, me) (regular rows):
 // row tables of kExpRowTab rows built by the warp, then each lane's column
-// slides down them (ExpColumn).
+// slides down them (ExpColumn).  The walk starts at row ms - 1 >= me - 1: the
+// rows of [me, ms) only bring the window sums to the state that a walk from
+// further up would have.
 template <int kPrec, class Sink>
 __device__ __forceinline__ void exp_rows(const TemplateDev &t, const float *__restrict__ a8,
                                          const uint32_t *__restrict__ t0s, uint32_t mb,
-                                         uint32_t me, uint32_t tau, bool active, Sink &sink,
-                                         ExpRow *tab) {
+                                         uint32_t me, uint32_t ms, uint32_t tau, bool active,
+                                         Sink &sink, ExpRow *tab,
+                                         const float *__restrict__ seg) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t *a8u = reinterpret_cast<const uint32_t *>(a8);
   ExpColumn<kPrec == kPrecFF_F64Det, true> C;
   C.init(t.g, tau);
-  for (uint32_t ce = me; ce > mb;) {
-    const uint32_t cb = ce - mb > kExpRowTab ? ce - kExpRowTab : mb;
+  if (seg && active) {  // the walk's first window, where it is long
+    const uint32_t t0 = __ldg(t0s + ms - 1u);
+    const uint32_t lo = exp_lo(t0, t.g), d = t0 - t.g.t0_data;
+    ExpRow e;
+    e.a = fdiv(d, t.g.div);
+    e.b = d - e.a * t.g.TAtom;
+    const uint32_t top = min(max(C.top_raw(e), 1u), t.g.numAtoms);
+    if (lo < top && top - lo >= (2u << t.g_shift))
+      C.warm_start(a8, t.g, seg, t.g_shift, t.g_nseg, lo, top);
+  }
+  for (uint32_t ce = ms; ce > mb;) {
+    if (ce == me) sink.start();  // the rows of the run-up leave nothing behind
+    const uint32_t floor = ce > me ? me : mb;
+    const uint32_t cb = ce - floor > kExpRowTab ? ce - kExpRowTab : floor;
     __syncwarp();
     uint32_t t0min = 0xFFFFFFFFu;
     for (uint32_t r = lane; r < ce - cb; r += 32u) {
@@ -569,7 +589,8 @@ __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *_
                          const float *__restrict__ atoms8,
                          const uint32_t *__restrict__ t0s_all,
                          const uint32_t *__restrict__ taus_all, float *__restrict__ Fmn,
-                         Red &red, ExpRow *tab, bool warp_tile = false) {
+                         Red &red, ExpRow *tab, const float *__restrict__ G,
+                         bool warp_tile = false) {
   const uint32_t *t0s = t0s_all + t.t0_off;
   const uint32_t tn = w.tn;
   const uint32_t lane = threadIdx.x & 31u;
@@ -577,13 +598,15 @@ __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *_
   const uint32_t col = warp_tile ? lane : threadIdx.x % tn;
   const uint32_t rl = warp_tile ? 0u : threadIdx.x / tn;
   const uint32_t n = w.n0 + col;
-  const uint32_t R = w.rows_per_lane;
-  const uint32_t mb = w.m0 + rl * R;
-  if (mb >= w.m1) return;  // uniform per warp (tn >= 32)
-  const uint32_t me = min(w.m1, mb + R);
+  const uint32_t chunk = w.m0 + rl;
+  if (chunk >= w.m1) return;  // uniform per warp (tn >= 32)
+  const uint32_t h0 = chunk / t.e_sub * t.e_hist, h1 = min(t.N_t0, h0 + t.e_hist);
+  const uint32_t mb = h0 + chunk % t.e_sub * t.e_rows;
+  if (mb >= h1) return;
+  const uint32_t me = min(h1, mb + t.e_rows);
   const bool active = n < w.n1;
   const uint32_t tau = active ? __ldg(taus_all + t.tau_off + n) : 0u;
-  MapSink<kWrite> sink{kWrite ? Fmn + t.map_off : nullptr, t.N_tau, n, &red};
+  MapSink<kWrite> sink{kWrite ? Fmn + t.map_off : nullptr, t.N_tau, n, &red, true};
   if (kPrec == kPrecPlain32) {
     if (active) {
       exp_column<false, false>(atoms + t.atom_off * 7u, t.g, t0s, mb, me, tau, sink, nullptr);
@@ -593,8 +616,22 @@ __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *_
   }
   const float *a8 = atoms8 + t.a8_off * 8u;
   const uint32_t taumax = __reduce_max_sync(0xffffffffu, tau);
+  // run-up over the history above the chunk (kShortWindow, kRunUp)
+  uint32_t ms = me;
+  if (me < h1) {
+    const uint32_t taumin = __reduce_min_sync(0xffffffffu, active ? tau : 0xFFFFFFFFu);
+    if (3ull * taumin < (uint64_t)kShortWindow * t.g.TAtom) {
+      const uint64_t longest = min((uint64_t)taumax, (uint64_t)kShortWindow * t.g.TAtom / 3u + 1u);
+      const uint64_t from = __ldg(t0s + me - 1u) + kRunUp * longest + 8ull * t.g.TAtom;
+      uint32_t found = 0;
+      for (uint32_t r = me; r < h1 && !found; r += 32u) {
+        found = __ballot_sync(0xffffffffu, r + lane < h1 && __ldg(t0s + r + lane) >= from);
+        ms = found ? r + __ffs(found) : h1;
+      }
+    }
+  }
   bool reg = true;
-  for (uint32_t m = mb + lane; m < me; m += 32u)
+  for (uint32_t m = mb + lane; m < ms; m += 32u)
     reg = reg && exp_row_regular(__ldg(t0s + m), taumax, t.g);
   if (!__all_sync(0xffffffffu, reg)) {
     if (active) {
@@ -603,8 +640,69 @@ __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *_
     }
     return;
   }
-  exp_rows<kPrec>(t, a8, t0s, mb, me, tau, active, sink, tab);
+  const float *seg =
+      t.g_nseg ? G + (t.g_off + (size_t)(n >> 5) * t.g_nseg) * kSegFloats + lane : nullptr;
+  exp_rows<kPrec>(t, a8, t0s, mb, me, ms, tau, active, sink, tab, seg);
   if (active) red.row_to_index(t.N_tau, n);
+}
+
+// Segment sums of exp columns: a warp takes kSegPerWarp segments of one
+// 32-column group, each lane one column, and enters the segment's atoms into
+// an empty window (the map kernel's steps).  They let a column be cut into
+// row chunks whose first window is combined from whole segments
+// (ExpColumn::warm_start) instead of entered atom by atom, at the price of
+// one more pass over the atoms per column -- fully parallel.  Column groups
+// whose windows are shorter than two segments are never combined and are
+// skipped.  Bound by the FP32 pipe and the latency of the double-word steps:
+// 186 us for 17532 atoms x 4096 columns.  The map kernel behind it goes from
+// 3331 us (16 chunks per column, each entering up to 17532 atoms) to 440 us
+// there (one-year 8192 x 4096 map), from 645 us (whole columns, one warp per
+// 32) to 188 us for 12 templates of up to 1500 atoms and 600 x 600 cells.
+template <bool kList>
+__global__ void __launch_bounds__(128, 8)
+    exp_seg_kernel(const TemplateDev *__restrict__ T, const SegItem *__restrict__ items,
+                   uint32_t n_items, const float *__restrict__ atoms8,
+                   const uint32_t *__restrict__ taus_all, float *__restrict__ G) {
+  const uint32_t wi = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+  if (wi >= n_items) return;
+  SegItem w;
+  if (kList) {
+    w = items[wi];
+  } else {
+    const uint32_t ncg = (T[0].N_tau + 31u) >> 5;
+    w.tmpl = 0;
+    w.cg = wi % ncg;
+    w.j0 = wi / ncg * kSegPerWarp;
+    w.j1 = min(T[0].g_nseg, w.j0 + kSegPerWarp);
+  }
+  const TemplateDev t = T[w.tmpl];
+  const uint32_t n = w.cg * 32u + lane;
+  uint32_t tau = n < t.N_tau ? __ldg(taus_all + t.tau_off + n) : 0u;
+  const uint32_t taumax = __reduce_max_sync(0xffffffffu, tau);
+  // a window holds fewer than 3 tau / TAtom + 2 atoms
+  if (3ull * taumax + 2ull * t.g.TAtom < ((uint64_t)t.g.TAtom << (t.g_shift + 1u))) return;
+  if (n >= t.N_tau) tau = taumax;
+  const float *a8 = atoms8 + t.a8_off * 8u;
+  ExpColumn<false, true> C;
+  C.init(t.g, tau);
+  for (uint32_t j = w.j0; j < w.j1; j++) {
+    C.reset_window(min(t.g.numAtoms, (j + 1u) << t.g_shift));
+    C.enter_to(a8, t.g, j << t.g_shift);
+    C.store_sums(G + (t.g_off + (size_t)w.cg * t.g_nseg + j) * kSegFloats + lane);
+  }
+}
+
+cudaError_t launch_exp_segments(const TemplateDev *d_T, const SegItem *d_items, uint32_t n_items,
+                                const float *d_atoms8, const uint32_t *d_taus, float *d_G,
+                                cudaStream_t stream) {
+  if (n_items == 0) return cudaSuccess;
+  const uint32_t blocks = (n_items + 3u) / 4u;
+  if (d_items)
+    exp_seg_kernel<true><<<blocks, 128, 0, stream>>>(d_T, d_items, n_items, d_atoms8, d_taus, d_G);
+  else
+    exp_seg_kernel<false><<<blocks, 128, 0, stream>>>(d_T, d_items, n_items, d_atoms8, d_taus,
+                                                      d_G);
+  return cudaGetLastError();
 }
 
 // Minimum resident blocks per SM requested from the register allocator
@@ -637,8 +735,8 @@ __global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kWrite
                uint32_t n_items, uint32_t *__restrict__ counter, const float *__restrict__ atoms,
                const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s,
                const uint32_t *__restrict__ taus,
-               const float *__restrict__ P, float *__restrict__ Fmn,
-               Partial *__restrict__ parts) {
+               const float *__restrict__ P, const float *__restrict__ G,
+               float *__restrict__ Fmn, Partial *__restrict__ parts) {
   __shared__ uint32_t s_item;
   constexpr uint32_t kSmem = kWin == TCW_WINDOW_RECT ? (kWrite ? (kBlock / 32) * 32 * 33 : 1)
                                                      : (kBlock / 32) * kExpRowTab * 4;
@@ -695,7 +793,7 @@ __global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kWrite
       const TemplateDev t = T[w.tmpl];
       Red red;
       red.init();
-      exp_tile<kWrite, kPrec>(t, w, atoms, atoms8, t0s, taus, Fmn, red, tab, true);
+      exp_tile<kWrite, kPrec>(t, w, atoms, atoms8, t0s, taus, Fmn, red, tab, G, true);
       RedVal acc{red.mx, red.bidx, fsub(red.s, red.c)};
 #pragma unroll
       for (int d = 16; d > 0; d >>= 1) acc = red_combine(acc, shfl_down_red(acc, d));
@@ -731,7 +829,7 @@ __global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kWrite
                                4u / rg, warp / rg, s_tau + warp * 32u);
     } else
       exp_tile<kWrite, kPrec>(t, w, atoms, atoms8, t0s, taus, Fmn, red,
-                              reinterpret_cast<ExpRow *>(sm) + (threadIdx.x >> 5) * kExpRowTab);
+                              reinterpret_cast<ExpRow *>(sm) + (threadIdx.x >> 5) * kExpRowTab, G);
     block_reduce_store(red, parts + w.part);
     if (!kPersist) break;
   }
@@ -906,7 +1004,7 @@ static cudaError_t launch_map_prec(int prec, uint32_t grid, cudaStream_t s, int 
                                    const TemplateDev *T, const WorkItem *items, uint32_t n_items,
                                    uint32_t *counter, const float *atoms, const float *atoms8,
                                    const uint32_t *t0s, const uint32_t *taus, const float *P,
-                                   float *Fmn, Partial *parts) {
+                                   const float *G, float *Fmn, Partial *parts) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kBlock);
@@ -918,12 +1016,12 @@ static cudaError_t launch_map_prec(int prec, uint32_t grid, cudaStream_t s, int 
   cfg.numAttrs = 1;
   if (prec == kPrecPlain32)
     return cudaLaunchKernelEx(&cfg, map_kernel<kWin, kPersist, kWrite, kPrecPlain32>, T, items,
-                              n_items, counter, atoms, atoms8, t0s, taus, P, Fmn, parts);
+                              n_items, counter, atoms, atoms8, t0s, taus, P, G, Fmn, parts);
   if (prec == kPrecFF_F64Det)
     return cudaLaunchKernelEx(&cfg, map_kernel<kWin, kPersist, kWrite, kPrecFF_F64Det>, T, items,
-                              n_items, counter, atoms, atoms8, t0s, taus, P, Fmn, parts);
+                              n_items, counter, atoms, atoms8, t0s, taus, P, G, Fmn, parts);
   return cudaLaunchKernelEx(&cfg, map_kernel<kWin, kPersist, kWrite, kPrecFF>, T, items, n_items,
-                            counter, atoms, atoms8, t0s, taus, P, Fmn, parts);
+                            counter, atoms, atoms8, t0s, taus, P, G, Fmn, parts);
 }
 
 template <int kWin>
@@ -934,18 +1032,18 @@ static cudaError_t launch_map_win(const MapLaunch &L, cudaStream_t stream) {
     if (L.write_map)
       return launch_map_prec<kWin, true, true>(L.prec, grid, stream, L.priority, L.T, L.items,
                                                L.n_items, L.counter, L.atoms, L.atoms8, L.t0s, L.taus, L.P,
-                                               L.Fmn, L.parts);
+                                               L.G, L.Fmn, L.parts);
     return launch_map_prec<kWin, true, false>(L.prec, grid, stream, L.priority, L.T, L.items,
                                               L.n_items, L.counter, L.atoms, L.atoms8, L.t0s, L.taus, L.P,
-                                              L.Fmn, L.parts);
+                                              L.G, L.Fmn, L.parts);
   }
   if (L.write_map)
     return launch_map_prec<kWin, false, true>(L.prec, grid, stream, L.priority, L.T, L.items,
                                               L.n_items, L.counter, L.atoms, L.atoms8, L.t0s, L.taus, L.P,
-                                              L.Fmn, L.parts);
+                                              L.G, L.Fmn, L.parts);
   return launch_map_prec<kWin, false, false>(L.prec, grid, stream, L.priority, L.T, L.items,
                                              L.n_items, L.counter, L.atoms, L.atoms8, L.t0s, L.taus, L.P,
-                                             L.Fmn, L.parts);
+                                             L.G, L.Fmn, L.parts);
 }
 
 cudaError_t launch_repack(const TemplateDev *d_T, const uint32_t *d_exp_list, uint32_t n_exp,

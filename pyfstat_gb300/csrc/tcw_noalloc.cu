@@ -70,9 +70,9 @@ size_t align256(size_t x) { return (x + 255u) / 256u * 256u; }
 // are enumerated column tile outer, row tile inner, as the handle-based
 // entry point does.
 __global__ void noalloc_setup_kernel(TemplateDev t, uint32_t window, uint32_t tn,
-                                     uint32_t rows_per_tile, uint32_t rows_per_lane,
-                                     uint32_t n_mtiles, uint32_t n_items, TemplateDev *T,
-                                     uint32_t *list, WorkItem *items) {
+                                     uint32_t rows_per_tile, uint32_t n_mtiles,
+                                     uint32_t n_items, TemplateDev *T, uint32_t *list,
+                                     WorkItem *items) {
   const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
   if (i0 == 0) {
     T[0] = t;
@@ -89,10 +89,10 @@ __global__ void noalloc_setup_kernel(TemplateDev t, uint32_t window, uint32_t tn
     w.n1 = min(t.N_tau, w.n0 + tn);
     if (window == TCW_WINDOW_RECT) {
       w.tn = (uint16_t)(rows_per_tile / 32u);
-      w.rows_per_lane = 0;
-    } else {
+    } else {  // row chunks, one per warp
       w.tn = (uint16_t)tn;
-      w.rows_per_lane = (uint16_t)rows_per_lane;
+      w.m0 = mt * rows_per_tile;
+      w.m1 = w.m0 + rows_per_tile;
     }
     items[k] = w;
   }
@@ -122,50 +122,59 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
     return TCW_ERR_NO_DEVICE;
   }
 
-  // tile shapes: the same rules as the handle-based plain entry point
-  uint32_t tn, rows_per_tile, rows_per_lane = 0;
+  const int prec = (flags & TCW_FLAG_UNCOMPENSATED) ? kPrecPlain32
+                   : (flags & TCW_FLAG_FP64_DET)    ? kPrecFF_F64Det
+                                                    : kPrecFF;
+  // tile shapes and scratch layout: the same rules as the handle-based plain
+  // entry point; exp columns stay whole histories (`cut` false) where their
+  // segment sums do not fit the scratch
+  uint32_t tn = 0, rows_per_tile = 0, n_mtiles = 0, n_items = 0;
+  ExpSplit sp{};
   const uint64_t target_blocks = (uint64_t)sms * 4u;
-  if (window == TCW_WINDOW_RECT) {
-    rows_per_tile = 32;
-    const uint64_t row_tiles = (N_t0 + 31u) / 32u;
-    uint64_t c = (uint64_t)N_tau * row_tiles / (target_blocks ? target_blocks : 1);
-    tn = (uint32_t)(c < 16 ? 16 : (c > 256 ? 256 : c));
-  } else {
-    tn = 32;
-    uint32_t rows = (N_t0 + 15u) / 16u;
-    rows = rows < 8u ? 8u : rows;
-    rows_per_lane = rows < N_t0 ? rows : N_t0;
-    // a lane's row chunk is a 16-bit count: longer columns become more row
-    // tiles, as in the handle-based entry point
-    if (rows_per_lane > 65535u) rows_per_lane = 65535u;
-    rows_per_tile = rows_per_lane * (kBlock / tn);
-  }
-  const uint64_t n_mtiles = (N_t0 + rows_per_tile - 1u) / rows_per_tile;
-  const uint64_t n_ntiles = (N_tau + tn - 1u) / tn;
-  const uint64_t n_items64 = n_mtiles * n_ntiles;
-  if (n_items64 > 0x7FFFFFFFull) return TCW_ERR_OVERFLOW;
-  const uint32_t n_items = (uint32_t)n_items64;
   const uint32_t n_chunks = (N_t0 + 63u) / 64u;
-
-  // scratch layout
-  size_t off = 0;
-  const size_t o_T = off;
-  off = align256(off + sizeof(TemplateDev));
-  const size_t o_list = off;
-  off = align256(off + sizeof(uint32_t));
-  const size_t o_items = off;
-  off = align256(off + sizeof(WorkItem) * (size_t)n_items);
-  const size_t o_parts = off;
-  off = align256(off + sizeof(Partial) * (size_t)n_items);
-  const size_t o_rows = off;
-  off = align256(off + (window == TCW_WINDOW_RECT
-                            ? sizeof(float) * kPrefixStride * ((size_t)numAtoms + 1u)
-                            : sizeof(float) * 8u * (size_t)numAtoms));
-  const size_t o_row = off;
-  if (post) off = align256(off + sizeof(double) * N_t0);
-  const size_t o_col = off;
-  if (post) off = align256(off + sizeof(double) * (size_t)n_chunks * N_tau);
-  if (off > kNoallocScratchBytes) return TCW_ERR_OVERFLOW;
+  size_t o_T = 0, o_list = 0, o_items = 0, o_parts = 0, o_rows = 0, o_row = 0, o_col = 0, o_G = 0;
+  bool fits = false;
+  for (int cut = window == TCW_WINDOW_EXP && prec != kPrecPlain32 ? 1 : 0; cut >= 0 && !fits;
+       cut--) {
+    uint64_t n_mtiles64;
+    if (window == TCW_WINDOW_RECT) {
+      rows_per_tile = 32;
+      const uint64_t row_tiles = (N_t0 + 31u) / 32u;
+      uint64_t c = (uint64_t)N_tau * row_tiles / (target_blocks ? target_blocks : 1);
+      tn = (uint32_t)(c < 16 ? 16 : (c > 256 ? 256 : c));
+      n_mtiles64 = row_tiles;
+    } else {
+      tn = 32;
+      sp = plain_exp_split(numAtoms, N_t0, N_tau, sms, cut != 0);
+      rows_per_tile = kBlock / tn;  // row chunks per tile
+      n_mtiles64 = ((uint64_t)sp.chunks(N_t0) + rows_per_tile - 1u) / rows_per_tile;
+    }
+    const uint64_t n_items64 = n_mtiles64 * ((N_tau + (uint64_t)tn - 1u) / tn);
+    if (n_items64 > 0x7FFFFFFFull) continue;
+    n_mtiles = (uint32_t)n_mtiles64;
+    n_items = (uint32_t)n_items64;
+    size_t off = 0;
+    o_T = off;
+    off = align256(off + sizeof(TemplateDev));
+    o_list = off;
+    off = align256(off + sizeof(uint32_t));
+    o_items = off;
+    off = align256(off + sizeof(WorkItem) * (size_t)n_items);
+    o_parts = off;
+    off = align256(off + sizeof(Partial) * (size_t)n_items);
+    o_rows = off;
+    off = align256(off + (window == TCW_WINDOW_RECT
+                              ? sizeof(float) * kPrefixStride * ((size_t)numAtoms + 1u)
+                              : sizeof(float) * 8u * (size_t)numAtoms));
+    o_row = off;
+    if (post) off = align256(off + sizeof(double) * N_t0);
+    o_col = off;
+    if (post) off = align256(off + sizeof(double) * (size_t)n_chunks * N_tau);
+    o_G = off;
+    if (sp.nseg) off = align256(off + sizeof(float) * sp.seg_floats(N_tau));
+    fits = off <= kNoallocScratchBytes;
+  }
+  if (!fits) return TCW_ERR_OVERFLOW;
 
   unsigned char *base = nullptr;
   int rc = scratch_address(device, &base);
@@ -179,6 +188,7 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
   t.N_tau = N_tau;
   t.part_off = 0;
   t.n_parts = n_items;
+  set_split(t, sp);
   TemplateDev *dT = reinterpret_cast<TemplateDev *>(base + o_T);
   uint32_t *dlist = reinterpret_cast<uint32_t *>(base + o_list);
   WorkItem *ditems = reinterpret_cast<WorkItem *>(base + o_items);
@@ -187,16 +197,17 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
 
   const uint32_t setup_blocks = n_items / 256u + 1u < 1024u ? n_items / 256u + 1u : 1024u;
   noalloc_setup_kernel<<<setup_blocks, 256, 0, s>>>(t, (uint32_t)window, tn, rows_per_tile,
-                                                    rows_per_lane, (uint32_t)n_mtiles, n_items,
-                                                    dT, dlist, ditems);
+                                                    n_mtiles, n_items, dT, dlist, ditems);
   if (cudaGetLastError() != cudaSuccess) return TCW_ERR_CUDA;
-  const int prec = (flags & TCW_FLAG_UNCOMPENSATED) ? kPrecPlain32
-                   : (flags & TCW_FLAG_FP64_DET)    ? kPrecFF_F64Det
-                                                    : kPrecFF;
   cudaError_t e = window == TCW_WINDOW_RECT
                       ? launch_prefix(dT, dlist, 1, d_atoms, drows, prec, s)
                       : launch_repack(dT, dlist, 1, d_atoms, drows, s);
   if (e != cudaSuccess) return TCW_ERR_CUDA;
+  float *dG = reinterpret_cast<float *>(base + o_G);
+  const uint32_t n_seg_items =
+      (N_tau + 31u) / 32u * ((sp.nseg + kSegPerWarp - 1u) / kSegPerWarp);
+  if (launch_exp_segments(dT, nullptr, n_seg_items, drows, d_taus, dG, s) != cudaSuccess)
+    return TCW_ERR_CUDA;
   MapLaunch ml{};
   ml.T = dT;
   ml.items = ditems;
@@ -209,6 +220,7 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
   ml.atoms8 = window == TCW_WINDOW_EXP ? drows : nullptr;
   ml.t0s = d_t0s;
   ml.taus = d_taus;
+  ml.G = dG;
   ml.P = window == TCW_WINDOW_RECT ? drows : nullptr;
   ml.Fmn = d_Fmn;
   ml.parts = dparts;
