@@ -307,8 +307,26 @@ def plain_configs(h, dev, torch, stream, hbm, reps=200):
 # Algorithmic FP64 work per cell of the differentiable statistics: the
 # forward pass is the map's per-cell math (55 flops with an FMA as 2) in
 # FP64; the backward pass recomputes the window sums and runs their adjoint
-# (twice the forward).
+# (twice the forward).  Only cells that carry weight need it: in the forward
+# those with F within 62 of the maximum, in the backward within 42 of it
+# (the others' e^(F - max) vanishes in both sums and in every gradient).
 GRAD_FP64_FLOPS = {"forward": 55.0, "backward": 110.0}
+GRAD_WEIGHT_RANGE = {"forward": 62.0, "backward": 42.0}
+
+
+def grad_weighted_share(torch, dev, b, t):
+    """Share of one template's cells that carry weight in each pass, from its
+    FP32 map on the same grid."""
+    taus = t["tau_min"] + (t["tau_max"] - t["tau_min"]) / (t["N_tau"] - 1) * np.arange(t["N_tau"])
+    t0s = torch.from_numpy(b.t0s[:t["N_t0"]].view(np.int32)).to(dev)
+    taus = torch.from_numpy(np.rint(taus).astype(np.uint32).view(np.int32)).to(dev)
+    A = torch.from_numpy(np.ascontiguousarray(t["atoms"], np.float32)).to(dev)
+    F = torch.empty((t["N_t0"], t["N_tau"]), dtype=torch.float32, device=dev)
+    res = torch.zeros(5, dtype=torch.float64, device=dev)
+    b.handle.set_stream(torch.cuda.current_stream(dev).cuda_stream or 0x1)
+    b.handle.map_plain(A, A.shape[0], t["TAtom"], t["t0_data"], 2, t0s, t["N_t0"], taus,
+                       t["N_tau"], F, res)
+    return {k: float((F >= F.max() - r).double().mean()) for k, r in GRAD_WEIGHT_RANGE.items()}
 
 
 def grad_case(torch, dev, peaks, reps=3, n_templates=256):
@@ -344,6 +362,7 @@ def grad_case(torch, dev, peaks, reps=3, n_templates=256):
         torch.cuda.synchronize(dev)
         fwd.append(ev[0].elapsed_time(ev[1]))
         bwd.append(ev[1].elapsed_time(ev[2]))
+    share = grad_weighted_share(torch, dev, b, tl[0])
     cells = n_templates * 1024 * 1024
     out = {"workload": f"{n_templates} templates x 2000 SFTs x 2 detectors (exp), 1024 t0 x "
                        "1024 tau "
@@ -351,12 +370,14 @@ def grad_case(torch, dev, peaks, reps=3, n_templates=256):
            "cells": cells}
     for name, ms in (("forward", statistics.median(fwd)), ("backward", statistics.median(bwd))):
         cps = cells / (ms * 1e-3)
-        ach = cps * GRAD_FP64_FLOPS[name] / 1e12
+        flops = GRAD_FP64_FLOPS[name] * share[name]
+        ach = cps * flops / 1e12
         out[name] = {"ms": ms, "cells_per_s": cps,
                      "roofline": {"bound": "fp64", "achieved": ach,
                                   "peak": peaks["fp64_tflops"], "unit": "TFLOP/s",
                                   "frac": ach / peaks["fp64_tflops"],
-                                  "fp64_flops_per_cell": GRAD_FP64_FLOPS[name]}}
+                                  "fp64_flops_per_cell": flops,
+                                  "weighted_share_of_cells": share[name]}}
     return out
 
 

@@ -1135,21 +1135,75 @@ int tcw_plan_run_timed(tcw_handle *h, tcw_plan *p, const float *d_atoms, tcw_res
 // Validates descriptors, uploads descriptors, tiles and grids into the
 // handle's workspace; returns the layout of what follows them.
 struct DiffSetup {
-  size_t o_T, o_items, o_parts, o_t0, o_cnt, o_scratch, o_rlist, o_D64, o_elist, o_A8, total;
-  uint32_t n_items, n_blocks, max_rows;
-  uint32_t n_rect_items, n_rect_blocks, n_rect, n_exp;
+  size_t o_T, o_items, o_parts, o_t0, o_cnt, o_est, o_rlist, o_D64, o_elist, o_A8;
+  size_t o_cols, o_seg, o_need, o_scratch, o_cend, total;
+  uint32_t n_rect_items, n_rect_blocks, n_rect, n_exp, max_cols;
   uint64_t p_rows;
+  std::vector<DiffGroup> groups;
 };
+
+// Workspace of one group of exponential templates (adjoint sources, segment
+// sums, recurrence ends) and the most templates of one (grid y dimension).
+constexpr uint64_t kDiffGroupBytes = 1ull << 30;
+constexpr uint32_t kDiffGroupMax = 65535u;
+
+// Tiles of the exponential templates elist[y0, y1): as many row chunks per
+// column as give every resident warp (32 per SM) a tile, at least 16 rows
+// each; chunks start from segment sums of 2^shift atoms (exp_split).
+static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
+                                const std::vector<uint32_t> &elist, uint32_t y0, uint32_t y1,
+                                int pass, DiffGroup &g) {
+  uint64_t total_cg = 0;
+  for (uint32_t y = y0; y < y1; y++) total_cg += (T[elist[y]].N_tau + 31u) / 32u;
+  const uint64_t chunks = ((uint64_t)h->n_sms * 32u + total_cg - 1u) / total_cg;
+  const uint64_t seg_floats = pass ? kDiffSegFloatsV : kDiffSegFloats;
+  uint64_t seg = 0, scr = 0, cend = 0;
+  g = DiffGroup{};
+  g.y0 = y0;
+  g.ny = y1 - y0;
+  for (uint32_t y = y0; y < y1; y++) {
+    DiffTemplate &t = T[elist[y]];
+    t.n_cg = (t.N_tau + 31u) / 32u;
+    const uint64_t most = (t.N_t0 + 15u) / 16u;
+    uint64_t nc = std::max<uint64_t>(1, std::min(chunks, most));
+    t.g_shift = 5;
+    while ((4ull << (2u * t.g_shift)) <= t.g.numAtoms) t.g_shift++;
+    t.g_nseg = (uint32_t)(((uint64_t)t.g.numAtoms + (1u << t.g_shift) - 1u) >> t.g_shift);
+    if (nc > 1 && (seg + (uint64_t)t.n_cg * t.g_nseg) * seg_floats * sizeof(float) > kDiffGroupBytes)
+      nc = 1;
+    t.chunk_rows = (uint32_t)((t.N_t0 + nc - 1) / nc);
+    t.n_chunk = (t.N_t0 + t.chunk_rows - 1u) / t.chunk_rows;
+    if (t.n_chunk == 1u || t.g.numAtoms < 64u) t.g_nseg = 0;
+    t.n_aseg = (t.g.numAtoms + kDiffAtomSeg - 1u) / kDiffAtomSeg;
+    t.seg_off = seg;
+    t.scr_off = scr;
+    t.cend_off = cend;
+    seg += (uint64_t)t.n_cg * t.g_nseg;
+    scr += (uint64_t)t.n_cg * t.n_chunk * t.chunk_rows * TCW_DIFF_SLOTS * 32u;
+    cend += (uint64_t)t.n_cg * t.n_aseg;
+    g.max_cg = std::max(g.max_cg, t.n_cg);
+    g.max_atoms = std::max(g.max_atoms, t.g.numAtoms);
+    g.max_tiles = std::max(g.max_tiles, t.n_cg * t.n_chunk);
+    if (t.g_nseg)
+      g.max_segs = std::max(g.max_segs, t.n_cg * ((t.g_nseg + kSegPerWarp - 1u) / kSegPerWarp));
+    g.max_aseg = std::max(g.max_aseg, t.n_cg * t.n_aseg);
+  }
+  g.seg_floats = seg * seg_floats;
+  g.scr_floats = pass ? scr : 0;
+  g.cend_floats = pass ? cend * kDiffSegFloats : 0;
+}
 
 static int diff_prepare(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n,
                         const uint32_t *t0s, uint64_t n_t0s, int pass, DiffSetup &S) {
   if (!desc || n == 0 || !t0s) return set_err(h, TCW_ERR_INVALID_ARG, "empty template list");
-  std::vector<DiffTemplate> T(n);
-  std::vector<DiffItem> items, ritems;
+  std::vector<DiffTemplate> T;
+  std::vector<DiffItem> ritems;
   std::vector<uint32_t> rlist, elist;
-  uint32_t max_rows = 0;
-  uint64_t p_rows = 0, atom_rows = 0;
+  uint64_t p_rows = 0, atom_rows = 0, n_cols = 0, n_tiles = 0;
+  uint64_t seg_floats = 0, scr_floats = 0, cend_floats = 0;
+  uint32_t max_cols = 0;
   try {
+    T.resize(n);
     for (uint32_t k = 0; k < n; k++) {
       const tcw_diff_desc &d = desc[k];
       int rc = check_geometry(h, d.numAtoms, d.TAtom, d.t0_data, d.N_t0, d.N_tau);
@@ -1179,66 +1233,92 @@ static int diff_prepare(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n,
       t.tau_min = d.tau_min;
       t.tau_max = d.tau_max;
       t.window = rect ? (uint32_t)TCW_WINDOW_RECT : (uint32_t)TCW_WINDOW_EXP;
-      std::vector<DiffItem> &dst = rect ? ritems : items;
-      t.part_off = (uint32_t)dst.size();  // rect parts are shifted past the exp ones below
-      // exp tiles: 128 tau columns, all rows; rect tiles: 128 t0 rows, all columns
-      const uint32_t extent = rect ? d.N_t0 : d.N_tau;
-      for (uint32_t n0 = 0; n0 < extent; n0 += 128u)
-        dst.push_back(DiffItem{k, (uint32_t)dst.size(), n0, std::min(extent, n0 + 128u)});
-      t.n_parts = (uint32_t)dst.size() - t.part_off;
-      if (rect) {
+      if (rect) {  // tiles of 128 t0 rows, all columns; parts are shifted past the exp ones below
+        t.part_off = (uint32_t)ritems.size();
+        for (uint32_t m0 = 0; m0 < d.N_t0; m0 += 128u)
+          ritems.push_back(DiffItem{k, (uint32_t)ritems.size(), m0, std::min(d.N_t0, m0 + 128u)});
+        t.n_parts = (uint32_t)ritems.size() - t.part_off;
         t.p_off = p_rows;
         p_rows += (uint64_t)d.numAtoms + 1u;
         rlist.push_back(k);
       } else {
-        max_rows = std::max(max_rows, d.N_t0);
+        t.col_off = n_cols;
+        n_cols += d.N_tau;
+        max_cols = std::max(max_cols, d.N_tau);
         elist.push_back(k);
         atom_rows = std::max<uint64_t>(atom_rows, d.atom_offset + d.numAtoms);
       }
       T[k] = t;
     }
-    const uint32_t n_exp_items = (uint32_t)items.size();
-    for (DiffItem &it : ritems) it.part += n_exp_items;
-    for (uint32_t k : rlist) T[k].part_off += n_exp_items;
-    items.insert(items.end(), ritems.begin(), ritems.end());
-    S.n_rect_items = (uint32_t)ritems.size();
-    S.n_items = n_exp_items;
+    // groups of exponential templates within the workspace bound (the
+    // backward pass keeps 36 bytes per cell of a group), one template at least
+    for (uint32_t y0 = 0; y0 < elist.size();) {
+      uint32_t y1 = y0;
+      uint64_t cells = 0;
+      while (y1 < elist.size() && y1 - y0 < kDiffGroupMax) {
+        const DiffTemplate &t = T[elist[y1]];
+        const uint64_t c = (uint64_t)((t.N_tau + 31u) / 32u * 32u) * t.N_t0;
+        if (pass && y1 > y0 && (cells + c) * TCW_DIFF_SLOTS * sizeof(float) > kDiffGroupBytes)
+          break;
+        cells += c;
+        y1++;
+      }
+      DiffGroup g;
+      diff_tile_group(h, T, elist, y0, y1, pass, g);
+      S.groups.push_back(g);
+      seg_floats = std::max(seg_floats, g.seg_floats);
+      scr_floats = std::max(scr_floats, g.scr_floats);
+      cend_floats = std::max(cend_floats, g.cend_floats);
+      y0 = y1;
+    }
+    for (uint32_t k : elist) {
+      T[k].part_off = (uint32_t)n_tiles;
+      T[k].n_parts = T[k].n_cg * T[k].n_chunk;
+      n_tiles += T[k].n_parts;
+    }
+    if (n_tiles + ritems.size() > 0xFFFFFFF0ull)
+      return set_err(h, TCW_ERR_OVERFLOW, "too many tiles");
+    for (DiffItem &it : ritems) it.part += (uint32_t)n_tiles;
+    for (uint32_t k : rlist) T[k].part_off += (uint32_t)n_tiles;
   } catch (const std::bad_alloc &) {
     return set_err(h, TCW_ERR_ALLOC, "host allocation failed");
   }
-  S.max_rows = max_rows;
+  S.n_rect_items = (uint32_t)ritems.size();
   S.n_rect = (uint32_t)rlist.size();
   S.n_exp = (uint32_t)elist.size();
+  S.max_cols = max_cols;
   S.p_rows = p_rows;
-  S.n_blocks = (uint32_t)std::max<uint64_t>(
-      1, std::min<uint64_t>(S.n_items, (uint64_t)diff_blocks_per_sm(pass) * h->n_sms));
   S.n_rect_blocks = (uint32_t)std::max<uint64_t>(
       1, std::min<uint64_t>(S.n_rect_items, (uint64_t)rect_diff_blocks_per_sm(pass) * h->n_sms));
-  const size_t n_all_items = (size_t)S.n_items + S.n_rect_items;
   Layout L;
   S.o_T = L.add(sizeof(DiffTemplate) * n);
-  S.o_items = L.add(sizeof(DiffItem) * n_all_items);
+  S.o_items = L.add(sizeof(DiffItem) * ritems.size());
   S.o_t0 = L.add(sizeof(uint32_t) * n_t0s);
   S.o_cnt = L.add(2 * sizeof(uint32_t));
+  S.o_est = L.add(sizeof(uint32_t) * n);
   S.o_rlist = L.add(sizeof(uint32_t) * std::max<size_t>(1, rlist.size()));
   S.o_elist = L.add(sizeof(uint32_t) * std::max<size_t>(1, elist.size()));
   const size_t ctl = L.total;
-  S.o_parts = L.add(sizeof(DiffPartial) * n_all_items);
-  S.o_scratch = (pass == 1 && S.n_items)
-                    ? L.add(sizeof(float) * TCW_DIFF_SLOTS * 128u * (size_t)max_rows * S.n_blocks)
-                    : 0;
+  S.o_parts = L.add(sizeof(DiffPartial) * (n_tiles + ritems.size()));
+  S.o_need = L.add(sizeof(float) * n_tiles);
+  S.o_cols = L.add(sizeof(ColConsts) * n_cols);
+  S.o_seg = L.add(sizeof(float) * seg_floats);
+  S.o_scratch = L.add(sizeof(float) * scr_floats);
+  S.o_cend = L.add(sizeof(float) * cend_floats);
   S.o_D64 = pass == 1 ? L.add(sizeof(double) * 8u * std::max<uint64_t>(1, p_rows)) : 0;
   // the exponential templates' atoms in 32-byte rows, at their own row index
-  S.o_A8 = S.n_items ? L.add(sizeof(float) * 8u * std::max<uint64_t>(1, atom_rows)) : 0;
+  S.o_A8 = S.n_exp ? L.add(sizeof(float) * 8u * std::max<uint64_t>(1, atom_rows)) : 0;
   S.total = L.total;
   int rc = ensure_ws(h, S.total);
   if (rc) return rc;
   rc = ensure_stage(h, ctl);
   if (rc) return rc;
   memcpy(h->h_stage + S.o_T, T.data(), sizeof(DiffTemplate) * n);
-  memcpy(h->h_stage + S.o_items, items.data(), sizeof(DiffItem) * n_all_items);
+  if (!ritems.empty())
+    memcpy(h->h_stage + S.o_items, ritems.data(), sizeof(DiffItem) * ritems.size());
   memcpy(h->h_stage + S.o_t0, t0s, sizeof(uint32_t) * n_t0s);
   memset(h->h_stage + S.o_cnt, 0, 2 * sizeof(uint32_t));
+  memset(h->h_stage + S.o_est, 0, sizeof(uint32_t) * n);
   if (!rlist.empty()) memcpy(h->h_stage + S.o_rlist, rlist.data(), sizeof(uint32_t) * rlist.size());
   if (!elist.empty()) memcpy(h->h_stage + S.o_elist, elist.data(), sizeof(uint32_t) * elist.size());
   TCW_CUDA(h, cudaMemcpyAsync(h->d_ws, h->h_stage, ctl, cudaMemcpyHostToDevice, h->stream));
@@ -1251,24 +1331,27 @@ static DiffLaunch diff_launch(tcw_handle *h, const DiffSetup &S, const float *d_
                               double temperature) {
   DiffLaunch L{};
   L.T = reinterpret_cast<const DiffTemplate *>(h->d_ws + S.o_T);
-  L.items = reinterpret_cast<const DiffItem *>(h->d_ws + S.o_items);
-  L.n_items = S.n_items;
-  L.n_blocks = S.n_blocks;
-  L.counter = reinterpret_cast<uint32_t *>(h->d_ws + S.o_cnt);
   L.atoms = d_atoms;
   L.t0s = reinterpret_cast<const uint32_t *>(h->d_ws + S.o_t0);
   L.temp = temperature;
   L.parts = reinterpret_cast<DiffPartial *>(h->d_ws + S.o_parts);
-  L.rect_items = L.items + S.n_items;
+  L.cols = reinterpret_cast<ColConsts *>(h->d_ws + S.o_cols);
+  L.seg = reinterpret_cast<float *>(h->d_ws + S.o_seg);
+  L.need = reinterpret_cast<float *>(h->d_ws + S.o_need);
+  L.est = reinterpret_cast<uint32_t *>(h->d_ws + S.o_est);
+  L.scratch = reinterpret_cast<float *>(h->d_ws + S.o_scratch);
+  L.cend = reinterpret_cast<float *>(h->d_ws + S.o_cend);
+  L.rect_items = reinterpret_cast<const DiffItem *>(h->d_ws + S.o_items);
   L.n_rect_items = S.n_rect_items;
   L.n_rect_blocks = S.n_rect_blocks;
-  L.rect_counter = L.counter + 1;
+  L.rect_counter = reinterpret_cast<uint32_t *>(h->d_ws + S.o_cnt) + 1;
   L.rect_list = reinterpret_cast<const uint32_t *>(h->d_ws + S.o_rlist);
   L.n_rect = S.n_rect;
   L.D64 = S.o_D64 ? reinterpret_cast<double *>(h->d_ws + S.o_D64) : nullptr;
   L.atoms8 = S.o_A8 ? reinterpret_cast<float *>(h->d_ws + S.o_A8) : nullptr;
   L.exp_list = reinterpret_cast<const uint32_t *>(h->d_ws + S.o_elist);
   L.n_exp = S.n_exp;
+  L.max_cols = S.max_cols;
   return L;
 }
 
@@ -1285,7 +1368,8 @@ int tcw_map_forward(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n_templat
   rc = diff_prepare(h, desc, n_templates, t0s, n_t0s, 0, S);
   if (rc) return rc;
   DiffLaunch L = diff_launch(h, S, d_atoms, temperature);
-  TCW_CUDA(h, launch_diff(0, L, h->stream));
+  TCW_CUDA(h, launch_diff(0, L, S.groups.data(), (uint32_t)S.groups.size(), h->stream,
+                          h->side_stream, h->fork_ev, h->join_ev));
   TCW_CUDA(h, launch_diff_finalize(L.T, n_templates, L.parts, temperature, d_lnBtSG, d_softmax2F,
                                    h->stream));
   return TCW_OK;
@@ -1314,15 +1398,14 @@ int tcw_map_backward(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n_templa
   L.lnZ2 = d_softmax2F;
   L.gB = d_grad_lnBtSG;
   L.gS = d_grad_softmax2F;
-  L.scratch = reinterpret_cast<float *>(h->d_ws + S.o_scratch);
-  L.scratch_rows = S.max_rows;
   L.grad_atoms = d_grad_atoms;
   L.grad_tau = d_grad_tau;
   TCW_CUDA(h, cudaMemsetAsync(d_grad_atoms, 0, sizeof(double) * 7u * n_atom_rows, h->stream));
   TCW_CUDA(h, cudaMemsetAsync(d_grad_tau, 0, sizeof(double) * 2u * n_templates, h->stream));
   if (S.n_rect)
     TCW_CUDA(h, cudaMemsetAsync(L.D64, 0, sizeof(double) * 8u * S.p_rows, h->stream));
-  TCW_CUDA(h, launch_diff(1, L, h->stream));
+  TCW_CUDA(h, launch_diff(1, L, S.groups.data(), (uint32_t)S.groups.size(), h->stream,
+                          h->side_stream, h->fork_ev, h->join_ev));
   return TCW_OK;
 }
 

@@ -386,7 +386,9 @@ TCW_HD bool exp_window(uint32_t t0, uint32_t tau, const Geom &g, uint32_t &lo,
 // ------------------------------------------------------------ F from window sums
 // Conditioning flag of a cell whose F fell back to 2 is reported by the
 // return value of fstat_ff through the `ok` out-parameter.
-template <bool kFp64Det>
+// kWide: F of every cell that FP64 may let pass (the cut widened by 1e-3),
+// ok where it surely does (the cut narrowed by 1e-3).
+template <bool kFp64Det, bool kWide = false>
 TCW_HD float fstat_ff(FF A, FF B, FF C, FF Far, FF Fai, FF Fbr, FF Fbi, bool &ok) {
   // D = A B - C^2 with exact products of the high words
   float p = fmul(A.h, B.h);
@@ -415,8 +417,8 @@ TCW_HD float fstat_ff(FF A, FF B, FF C, FF Far, FF Fai, FF Fbr, FF Fbi, bool &ok
   float Cs = fadd(C.h, C.l);
   float disc = sqrt_approx(ffma(dAB, dAB, fmul(4.0f * Cs, Cs)));
   float t = fadd(sumAB, disc);
-  ok = (D > 0.0f) && (fmul(t, t) < fmul(4.0e4f, D));
-  if (!ok) return 2.0f;
+  ok = (D > 0.0f) && (fmul(t, t) < fmul(kWide ? 3.996e4f : 4.0e4f, D));
+  if (kWide ? !(D > 0.0f && fmul(t, t) < fmul(4.004e4f, D)) : !ok) return 2.0f;
   // G = B Fa - C Fb, real and imaginary parts
   float u, ue, v, ve;
   u = fmul(B.h, Far.h);
@@ -1124,6 +1126,23 @@ TCW_HD bool exp_row_regular(uint32_t t0, uint32_t taumax, const Geom &g) {
          (uint64_t)t0 + 3ull * (uint64_t)taumax + (uint64_t)g.half <= 0xFFFFFFFFull;
 }
 
+// A column's constants in 20 bytes, formed once per column (the FP64 exp and
+// divisions of ExpColumn::init_real take longer than a short row chunk) and
+// read by every warp that walks a part of it.
+struct ColConsts {
+  FF r1;
+  uint32_t Qp1, RmT, has_inv;
+  TCW_HDM ExpConsts consts() const {
+    ExpConsts k;
+    k.r1 = r1;
+    k.r2 = ff_mul(r1, r1);
+    k.has_inv = has_inv != 0u;
+    k.r1inv = k.has_inv ? ff_recip(r1) : FF{0.0f, 0.0f};
+    k.c1 = 0.0f;  // uncompensated variant only
+    return k;
+  }
+};
+
 // One tau column: the sliding double-word window sums of exp_column2, as
 // state carried across row-table chunks.  Every arithmetic step is the same
 // as exp_column2's, in the same order, so the results are identical; only
@@ -1136,7 +1155,7 @@ TCW_HD bool exp_row_regular(uint32_t t0, uint32_t taumax, const Geom &g) {
 // Fast2Sum steps (the map kernels); without it every step is a TwoSum, for
 // the differentiable statistics, whose FP64 F and log-sum-exps want the
 // window sums good to ~1e-14.
-template <bool kFp64Det, bool kFastSums = false>
+template <bool kFp64Det, bool kFastSums = false, bool kWide = false>
 struct ExpColumn {
   ExpConsts k;
   ExpConsts2 k2;
@@ -1176,6 +1195,17 @@ struct ExpColumn {
     reset();
   }
 
+  // A column whose constants were formed before (ColConsts).
+  TCW_HDM void init_consts(const ColConsts &c) {
+    k = c.consts();
+    k2 = exp_consts2(k);
+    Qp1 = c.Qp1;
+    RmT = c.RmT;
+    reset();
+  }
+
+  TCW_HDM ColConsts consts() const { return ColConsts{k.r1, Qp1, RmT, k.has_inv ? 1u : 0u}; }
+
   TCW_HDM void reset() {
     const F2 z{0.0f, 0.0f};
     W0 = W2 = W3 = FF2{z, z};
@@ -1193,12 +1223,16 @@ struct ExpColumn {
     return e.a + Qp1 - (v >> 31);
   }
 
+  // Row e's window end, clamped to [1, numAtoms].
+  TCW_HDM uint32_t top_of(const Geom &g, const ExpRow &e) const {
+    uint32_t top = top_raw(e);
+    top = top < 1u ? 1u : top;
+    return top < g.numAtoms ? top : g.numAtoms;
+  }
   // Moves the window to row e's: false when it holds no atom or no data
   // (F = 2), true when W0, Wc, W2, W3 hold its sums.
   TCW_HDM bool window(const float *__restrict__ atoms8, const Geom &g, const ExpRow &e) {
-    uint32_t top = top_raw(e);
-    top = top < 1u ? 1u : top;
-    top = top < g.numAtoms ? top : g.numAtoms;
+    const uint32_t top = top_of(g, e);
     if (e.lo >= top) return false;
     return slide(atoms8, g, e.lo, top, e.nz);
   }
@@ -1313,14 +1347,14 @@ struct ExpColumn {
   // Starts a row chunk at the window [lo, top), top - lo >= 2 segments of
   // 2^shift atoms, from segment sums G_j = sum over the segment's atoms of
   // x_i r^(i - j 2^shift) (exp_seg_kernel; `seg` is this lane's first value
-  // of segment 0): the atoms above the last whole segment enter one by one,
+  // of segment 0, `stride` floats lie between segments): the atoms above the last whole segment enter one by one,
   // then each segment below is joined by W = G_j + r^(2^shift) W.  Leaves
   // wtop = top and wlo at the lowest joined segment (>= lo); the first row
   // enters the rest.  Entering the whole window instead costs every chunk up
   // to numAtoms steps.
   TCW_HDM void warm_start(const float *__restrict__ atoms8, const Geom &g,
                           const float *__restrict__ seg, uint32_t shift, uint32_t nseg,
-                          uint32_t lo, uint32_t top) {
+                          uint32_t lo, uint32_t top, uint32_t stride = 14u * 32u) {
     const uint32_t j1 = (lo + (1u << shift) - 1u) >> shift;
     const uint32_t j2 = top == g.numAtoms ? nseg : top >> shift;
     reset_window(top);
@@ -1333,7 +1367,7 @@ struct ExpColumn {
     for (uint32_t j = j2; j > j1;) {
       j--;
       TCW_DCHECK(j < nseg);
-      const float *s = seg + (size_t)j * (14u * 32u);
+      const float *s = seg + (size_t)j * stride;
       W0 = ff2_axpy_dw(FF2{F2{s[0], s[32]}, F2{s[64], s[96]}}, rh0, nrh0, rl0, W0);
       Wc = ff_axpy_dw(FF{s[128], s[160]}, R2, Wc);
       W2 = ff2_axpy_dw(FF2{F2{s[192], s[224]}, F2{s[256], s[288]}}, rh1, nrh1, rl1, W2);
@@ -1425,8 +1459,9 @@ struct ExpColumn {
     const F2 s0 = add2(W0.h, W0.l), s2 = add2(W2.h, W2.l), s3 = add2(W3.h, W3.l);
     const float sc = fadd(Wc.h, Wc.l);
     if (!fstat_fast_sums(s0.x, s0.y, sc, s2.x, s2.y, s3.x, s3.y, F)) {
-      F = fstat_ff<kFp64Det>(FF{W0.h.x, W0.l.x}, FF{W0.h.y, W0.l.y}, Wc, FF{W2.h.x, W2.l.x},
-                             FF{W2.h.y, W2.l.y}, FF{W3.h.x, W3.l.x}, FF{W3.h.y, W3.l.y}, ok);
+      F = fstat_ff<kFp64Det, kWide>(FF{W0.h.x, W0.l.x}, FF{W0.h.y, W0.l.y}, Wc,
+                                    FF{W2.h.x, W2.l.x}, FF{W2.h.y, W2.l.y},
+                                    FF{W3.h.x, W3.l.x}, FF{W3.h.y, W3.l.y}, ok);
     }
     Fl = F;
     okl = ok;

@@ -18,19 +18,34 @@
 // weight is then below e^-40) the forward forms F and the log-sum-exps in
 // FP64, the backward F, dF/dW and the sources in double-word FP32:
 //
-//   diff_fwd_kernel  per tau column, rows descending: double-word window
-//            sums, FP64 log-sum-exps of F and 2F/T -> per-tile partials ->
-//            finalize per template.
-//   diff_bwd_kernel  pass B: the same walk plus the tau-derivative sums
-//            V = sum (i - lo) x r^(i - lo) (ExpColumnV); per cell the adjoint
-//            sources G_c = g dF/dW_c (g = dL/dF) go to per-block scratch (no
-//            map is kept) and g dF/dtau accumulates per column;
-//            pass C (same kernel): per column, atoms ascending, the
-//            transposed recurrence H(i) = r H(i-1) + sum_{lo(m)=i} G(m)
-//            - sum_{hi(m)+1=i} G(m) r^(L(m)) in double-word FP32 gives
-//            dL/dx(i) = H(i); each warp reduces its 32 columns per atom
-//            (recursive halving over the 7 channels) and adds the sums to
-//            the FP64 atom gradient.
+// Exponential templates are tiled by 32 tau columns x a chunk of t0 rows, one
+// warp per tile; a chunk's first window is joined from segment sums
+// (ExpColumn::warm_start), so that a single template fills the GPU.
+//
+//   diff_est_kernel  FP32 only: the tile's largest tier-1 F (`need`, infinite
+//            where a cell has none) and a lower bound of the template's
+//            maximum.  With a signal almost no tile holds a cell that carries
+//            weight, and the FP64 and adjoint work below skips whole tiles.
+//   diff_fwd_kernel  the tiles that may carry weight: double-word window
+//            sums, FP64 log-sum-exps of F and 2F/T -> partials -> finalize
+//            per template.
+//   diff_src_kernel  backward, the tiles that may carry weight: the same walk
+//            plus the tau-derivative sums V = sum (i - lo) x r^(i - lo)
+//            (ExpColumnV); per cell the adjoint sources G_c = g dF/dW_c
+//            (g = dL/dF) go to scratch (no map is kept) and g dF/dtau
+//            accumulates per column;
+//   diff_atoms_kernel  per column, atoms ascending, the transposed recurrence
+//            H(i) = r H(i-1) + sum_{lo(m)=i} G(m) - sum_{hi(m)+1=i} G(m)
+//            r^(L(m)) in double-word FP32 gives dL/dx(i) = H(i).  It is linear
+//            in H, so it runs in segments of 64 atoms side by side: a first
+//            pass leaves each segment's end from H = 0, a second one joins the
+//            ends below its segment, walks it again and adds each warp's 32
+//            columns per atom (recursive halving over the 7 channels) to the
+//            FP64 atom gradient.
+// Measured (forward + backward, 2000 atoms, 1024 x 1024 cells, signal): one
+// template 7.7-9.6 -> 1.9 ms (one block per 128 columns and all rows before),
+// 24 templates 16.4 -> 3.7 ms, 256 templates forward 14.2 -> 7.1 ms, backward
+// 38.9 -> 20.1 ms.
 // The window-sum factor e^(-k (t_lo - t0)/tau) is left out everywhere: F does
 // not depend on it, so neither do g, dF/dW (in this frame) or dF/dtau.
 //
@@ -47,6 +62,7 @@
 #include <stdint.h>
 
 #include "../../include/tcw_b200.h"
+#include "tcw_exp_walk.cuh"
 #include "tcw_internal.h"
 
 namespace tcw {
@@ -84,13 +100,17 @@ struct F64Cell {
 // sumAB + disc < 1e4 (sumAB - disc) with sumAB - disc > 0 (no division), and
 // F = N (1/D) with the one reciprocal the derivatives reuse: FP64 divisions
 // are long sequences at GB300's FP64 rate.
-__device__ __forceinline__ F64Cell fstat64(const double W[7]) {
+// `passes`: the caller knows that the test holds (a tier-1 cell, cond < 32).
+__device__ __forceinline__ F64Cell fstat64(const double W[7], bool passes = false) {
   const double A = W[0], B = W[1], C = W[2];
-  const double sumAB = A + B, diffAB = A - B;
-  const double disc = sqrt(diffAB * diffAB + 4.0 * C * C);
-  const double denom = sumAB - disc;
   F64Cell r{2.0, 0.0, false};
-  if (denom > 0.0 && sumAB + disc < 1e4 * denom) {
+  if (!passes) {
+    const double sumAB = A + B, diffAB = A - B;
+    const double disc = sqrt(diffAB * diffAB + 4.0 * C * C);
+    const double denom = sumAB - disc;
+    passes = denom > 0.0 && sumAB + disc < 1e4 * denom;
+  }
+  if (passes) {
     const double D = A * B - C * C;
     if (D > 0.0) {
       const double N = B * (W[3] * W[3] + W[4] * W[4]) + A * (W[5] * W[5] + W[6] * W[6]) -
@@ -128,15 +148,12 @@ __device__ __forceinline__ void lse_merge(double &m, double &s, double m2, doubl
   m = M;
 }
 
-// Blocks of 128 threads, one tau column each; rows of a template all in one tile.
+// Blocks of 128 threads (rectangular windows: one t0 row per thread;
+// exponential ones: one tile per warp).
 constexpr int kDiffBlock = 128;
-// Per-block scratch row of one column: G_c (c = 0..6) and r^L as a float
-// hi/lo pair, so that the removal in the transposed recurrence cancels the
-// injected term to FP64 accuracy.
-constexpr uint32_t kDiffSlots = TCW_DIFF_SLOTS;
 
 // Minimum resident blocks per SM asked of the register allocator, per pass
-// (build-time tunables; 1 leaves the allocation to ptxas).
+// of the rectangular kernel (1 leaves the allocation to ptxas).
 #ifndef TCW_DIFF_MIN_BLOCKS_FWD
 #define TCW_DIFF_MIN_BLOCKS_FWD 5
 #endif
@@ -147,181 +164,13 @@ constexpr int diff_min_blocks(int pass) {
   return pass == 0 ? TCW_DIFF_MIN_BLOCKS_FWD : TCW_DIFF_MIN_BLOCKS_BWD;
 }
 
-// ------------------------------------------------------------ exponential forward (double-word)
-
-// Forward pass of exponential windows (lnBtSG and the soft-max 2F): the
-// window sums of each tau column slide down the rows in double-word FP32
-// (ExpColumn, the map kernel's arithmetic; sums good to ~1e-14 of the
-// window's magnitude, against FP64 recurrences at GB300's 1/70 FP64 rate),
-// with the per-row quantities tabulated per warp and the real tau's window
-// end split as in ExpColumn::init_real.  F goes into the FP64 log-sum-exps:
-// a cell whose FP32 tier-1 F lies more than 62 below a lower bound of the
-// template's maximum (the column's running maximum, or the tile's largest
-// tier-1 F found by a first, FP32-only sweep) carries exp(F - max) < e^-60
-// in both sums (the soft-max's 2F/T - max is 2/T times lower still) and is
-// skipped -- the tier-1 F is good
-// to ~1.5e-6 relative and passes only for cond < 32, where the FP64 test
-// passes too; every other cell gets F in FP64 from the double-word sums
-// (the reference's formula and conditioning test, fstat64).  Rows that are
-// not regular for the tile's taus (t0 + 3 tau + TAtom/2 beyond u32, or
-// TAtom < 2) take the window end from exp_hi_real instead.
-constexpr uint32_t kDiffRowTab = 128;
-
-__global__ void __launch_bounds__(256) diff_repack_kernel(const DiffTemplate *__restrict__ T,
-                                                          const uint32_t *__restrict__ list,
-                                                          const float *__restrict__ atoms,
-                                                          float *__restrict__ atoms8) {
-  __shared__ uint32_t s_first[256];
-  const DiffTemplate t = T[list[blockIdx.x]];
-  repack_rows256(atoms + t.atom_off * 7u, reinterpret_cast<float4 *>(atoms8 + t.atom_off * 8u),
-                 t.g.numAtoms, s_first);
+// Order-preserving key of a float for atomicMax; 0 is below every key.
+__device__ __forceinline__ uint32_t float_key(float f) {
+  const uint32_t b = __float_as_uint(f);
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
-
-__device__ __forceinline__ void lse_pair_add(double &m1, double &s1, double &m2, double &s2,
-                                             double F, double temp, float &skip) {
-  lse_add(m1, s1, F);
-  lse_add(m2, s2, 2.0 * F / temp);
-  skip = (float)(m1 - 62.0);
-}
-
-__global__ void __launch_bounds__(kDiffBlock, diff_min_blocks(0))
-    diff_fwd_kernel(const DiffTemplate *__restrict__ T, const DiffItem *__restrict__ items,
-                    uint32_t n_items, uint32_t *__restrict__ counter,
-                    const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
-                    double temp, DiffPartial *__restrict__ parts) {
-  __shared__ uint32_t s_item;
-  __shared__ double sh[kDiffBlock / 32][4];
-  __shared__ __align__(16) ExpRow s_tab[kDiffBlock / 32][kDiffRowTab];
-  const uint32_t lane = threadIdx.x & 31u;
-  ExpRow *tab = s_tab[threadIdx.x >> 5];
-  for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(counter, 1u);
-    __syncthreads();
-    const uint32_t it = s_item;
-    __syncthreads();
-    if (it >= n_items) break;
-    const DiffItem w = items[it];
-    const DiffTemplate t = T[w.tmpl];
-    const uint32_t n = w.n0 + threadIdx.x;
-    const bool active = n < w.n1;
-    const uint32_t *t0s = t0s_all + t.t0_off;
-    const double tau = tau_of(t, active ? n : w.n0);
-    const float *a8 = atoms8 + t.atom_off * 8u;
-    const uint32_t *a8u = reinterpret_cast<const uint32_t *>(a8);
-    double m1 = -INFINITY, s1 = 0.0, m2 = -INFINITY, s2 = 0.0;
-    float skip = -INFINITY;
-    // the warp's largest tau, rounded up, for the regularity test
-    const uint32_t tau_up = !active ? 0u
-                            : (tau >= 4294967295.0 ? 0xFFFFFFFFu : (uint32_t)ceil(tau));
-    const uint32_t taumax = __reduce_max_sync(0xffffffffu, tau_up);
-    ExpColumn<false> C;
-    C.init_real(t.g, tau);
-    // Two sweeps down the columns: the first finds the tile's largest tier-1
-    // F (FP32 only), a lower bound of the template's maximum to within its
-    // ~1e-5 error, so that the second skips the cells 62 below it from the
-    // start instead of only below the running maximum.
-    float est = -INFINITY, skip0 = -INFINITY;
-    for (int sweep = 0; sweep < 2; sweep++) {
-      if (sweep == 1) {
-        float v = est;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, d));
-        if (lane == 0) sh[threadIdx.x >> 5][0] = (double)v;
-        __syncthreads();
-        double tile = sh[0][0];
-        for (int k = 1; k < kDiffBlock / 32; k++) tile = fmax(tile, sh[k][0]);
-        __syncthreads();
-        if (tile > -INFINITY) skip0 = (float)(tile - 1e-5 * fabs(tile) - 63.0);
-        skip = skip0;
-        C.reset();
-      }
-      for (uint32_t ce = t.N_t0; ce > 0;) {
-        const uint32_t cb = ce > kDiffRowTab ? ce - kDiffRowTab : 0u;
-        bool reg = true;
-        for (uint32_t r = lane; r < ce - cb; r += 32u)
-          reg = reg && exp_row_regular(__ldg(t0s + cb + r), taumax, t.g);
-        reg = __all_sync(0xffffffffu, reg);
-        __syncwarp();
-        for (uint32_t r = lane; r < ce - cb; r += 32u) {
-          const uint32_t t0 = __ldg(t0s + cb + r);
-          ExpRow e;
-          e.lo = exp_lo(t0, t.g);
-          e.nz = e.lo < t.g.numAtoms ? __ldg(a8u + (size_t)e.lo * 8u + 3u) : 0xFFFFFFFFu;
-          const uint32_t d = t0 - t.g.t0_data;
-          e.a = reg ? fdiv(d, t.g.div) : t0;  // irregular chunks: the generic branch reads t0
-          e.b = reg ? d - e.a * t.g.TAtom : 0u;
-          tab[r] = e;
-        }
-        __syncwarp();
-        if (active) {
-          for (uint32_t m = ce; m > cb;) {
-            m--;
-            const ExpRow e = tab[m - cb];
-            bool data;
-            if (reg) {
-              data = C.window(a8, t.g, e);
-            } else {  // the window end from the real t1 (e.a holds t0 on these rows)
-              uint32_t hi;
-              data = exp_hi_real(e.a, tau, t.g, hi) && e.lo <= hi &&
-                     C.slide(a8, t.g, e.lo, hi + 1u, e.nz);
-            }
-            double F = 2.0;
-            if (data) {
-              float F32;
-              const F2 s0 = add2(C.W0.h, C.W0.l), s2v = add2(C.W2.h, C.W2.l),
-                       s3 = add2(C.W3.h, C.W3.l);
-              const float sc = fadd(C.Wc.h, C.Wc.l);
-              const bool t1 = fstat_fast_sums(s0.x, s0.y, sc, s2v.x, s2v.y, s3.x, s3.y, F32);
-              if (sweep == 0) {
-                if (t1) est = fmaxf(est, F32);
-                continue;
-              }
-              if (t1 && F32 < skip) continue;
-              double W[7];
-              W[0] = (double)C.W0.h.x + (double)C.W0.l.x;
-              W[1] = (double)C.W0.h.y + (double)C.W0.l.y;
-              W[2] = (double)C.Wc.h + (double)C.Wc.l;
-              W[3] = (double)C.W2.h.x + (double)C.W2.l.x;
-              W[4] = (double)C.W2.h.y + (double)C.W2.l.y;
-              W[5] = (double)C.W3.h.x + (double)C.W3.l.x;
-              W[6] = (double)C.W3.h.y + (double)C.W3.l.y;
-              F = fstat64(W).F;
-            } else if (sweep == 0 || 2.0f < skip) {
-              continue;
-            }
-            lse_pair_add(m1, s1, m2, s2, F, temp, skip);
-            skip = fmaxf(skip, skip0);
-          }
-        }
-        ce = cb;
-      }
-    }
-    // block merge of the two log-sum-exp pairs (warp shuffles, then smem)
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-      const double om1 = __shfl_down_sync(0xffffffffu, m1, d);
-      const double os1 = __shfl_down_sync(0xffffffffu, s1, d);
-      const double om2 = __shfl_down_sync(0xffffffffu, m2, d);
-      const double os2 = __shfl_down_sync(0xffffffffu, s2, d);
-      lse_merge(m1, s1, om1, os1);
-      lse_merge(m2, s2, om2, os2);
-    }
-    if (lane == 0) {
-      sh[threadIdx.x >> 5][0] = m1;
-      sh[threadIdx.x >> 5][1] = s1;
-      sh[threadIdx.x >> 5][2] = m2;
-      sh[threadIdx.x >> 5][3] = s2;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int k = 1; k < kDiffBlock / 32; k++) {
-        lse_merge(m1, s1, sh[k][0], sh[k][1]);
-        lse_merge(m2, s2, sh[k][2], sh[k][3]);
-      }
-      parts[w.part] = DiffPartial{m1, s1, m2, s2};
-    }
-    __syncthreads();
-  }
+__device__ __forceinline__ float key_float(uint32_t k) {
+  return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
 }
 
 // ------------------------------------------------------------ exponential backward (double-word)
@@ -430,6 +279,7 @@ __device__ __forceinline__ FF2 ff2_add_x(FF2 E, F2 x) {
 // dW_c / dtau = k_c (TAtom / tau^2) V_c (k_c = 2 for A, B, C; 1 otherwise).
 struct ExpColumnV {
   ExpColumn<false> C;
+  __device__ __forceinline__ const ExpColumn<false> &sums() const { return C; }
   FF2 V0, V2, V3;
   FF Vc;
 
@@ -483,278 +333,988 @@ struct ExpColumnV {
     }
     return nz < top;
   }
+
+  // One lane's W and V sums of a segment (stride 32).
+  __device__ __forceinline__ void store_sums(float *__restrict__ o) const {
+    C.store_sums(o);
+    const float v[14] = {V0.h.x, V0.h.y, V0.l.x, V0.l.y, Vc.h,   Vc.l,   V2.h.x,
+                         V2.h.y, V2.l.x, V2.l.y, V3.h.x, V3.h.y, V3.l.x, V3.l.y};
+#pragma unroll
+    for (int f = 0; f < 14; f++) o[32 * (14 + f)] = v[f];
+  }
+
+  // ExpColumn::warm_start with the derivative sums: below a segment of
+  // S = 2^shift atoms, V = GV_j + r^S (V + S W) with the old W.
+  __device__ __forceinline__ void warm_start(const float *__restrict__ atoms8, const Geom &g,
+                                             const float *__restrict__ seg, uint32_t shift,
+                                             uint32_t nseg, uint32_t lo, uint32_t top,
+                                             uint32_t stride) {
+    const uint32_t j1 = (lo + (1u << shift) - 1u) >> shift;
+    const uint32_t j2 = top == g.numAtoms ? nseg : top >> shift;
+    C.reset_window(top);
+    reset_v();
+    if (top != g.numAtoms) slide(atoms8, g, j2 << shift, top, 0u);
+    FF R = C.k.r1;
+    for (uint32_t b = 0; b < shift; b++) R = ff_mul(R, R);
+    const FF R2 = ff_mul(R, R);
+    const F2 rh0{R2.h, R2.h}, nrh0{-R2.h, -R2.h}, rl0{R2.l, R2.l};
+    const F2 rh1{R.h, R.h}, nrh1{-R.h, -R.h}, rl1{R.l, R.l};
+    const float S = (float)(1u << shift);
+    const F2 S2{S, S};
+    for (uint32_t j = j2; j > j1;) {
+      j--;
+      TCW_DCHECK(j < nseg);
+      const float *s = seg + (size_t)j * stride;
+      const float *v = s + 14 * 32;
+      V0 = ff2_axpy_dw(FF2{F2{v[0], v[32]}, F2{v[64], v[96]}}, rh0, nrh0, rl0,
+                       ff2_add_dw(V0, FF2{mul2(S2, C.W0.h), mul2(S2, C.W0.l)}));
+      Vc = ff_axpy_dw(FF{v[128], v[160]}, R2, ff_add_dw(Vc, FF{S * C.Wc.h, S * C.Wc.l}));
+      V2 = ff2_axpy_dw(FF2{F2{v[192], v[224]}, F2{v[256], v[288]}}, rh1, nrh1, rl1,
+                       ff2_add_dw(V2, FF2{mul2(S2, C.W2.h), mul2(S2, C.W2.l)}));
+      V3 = ff2_axpy_dw(FF2{F2{v[320], v[352]}, F2{v[384], v[416]}}, rh1, nrh1, rl1,
+                       ff2_add_dw(V3, FF2{mul2(S2, C.W3.h), mul2(S2, C.W3.l)}));
+      C.W0 = ff2_axpy_dw(FF2{F2{s[0], s[32]}, F2{s[64], s[96]}}, rh0, nrh0, rl0, C.W0);
+      C.Wc = ff_axpy_dw(FF{s[128], s[160]}, R2, C.Wc);
+      C.W2 = ff2_axpy_dw(FF2{F2{s[192], s[224]}, F2{s[256], s[288]}}, rh1, nrh1, rl1, C.W2);
+      C.W3 = ff2_axpy_dw(FF2{F2{s[320], s[352]}, F2{s[384], s[416]}}, rh1, nrh1, rl1, C.W3);
+    }
+    C.wlo = j1 << shift;
+  }
 };
 
-// Backward pass of exponential windows.  Pass B slides W and V down each
-// tau column in double-word FP32 (ExpColumnV) with the per-row quantities
-// tabulated per warp; a cell gets F, dF/dW and its adjoint sources (in
-// double-word arithmetic, dw_fstat) only when it carries weight.  Its weight g = gB e^(F - Z1) + 2 gS e^(2F/T - Z2)
-// (Z1 = logsumexp F, Z2 = logsumexp 2F/T, from the forward outputs) is below
-// e^-40 when the FP32 tier-1 F (good to ~1e-5 of F) lies more than 42 below
-// Z1 (the lnBtSG term, gB != 0) and more than 40 T + 1 below (T/2) Z2 (the
-// soft-max term, gS != 0: its exponent is then below -80); such cells
-// contribute no sources.  Pass C (the transposed recurrence) runs in
-// double-word FP32 (FP64 recurrences: 95 ms on the differentiation workload,
-// with a per-channel butterfly reduction 67.6 ms, double-word 45.7 ms), with
-// the window ends of regular rows from the integer split.
-__global__ void __launch_bounds__(kDiffBlock, diff_min_blocks(1))
-    diff_bwd_kernel(const DiffTemplate *__restrict__ T, const DiffItem *__restrict__ items,
-                    uint32_t n_items, uint32_t *__restrict__ counter,
-                    const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
-                    double temp, const double *__restrict__ lnZ1, const double *__restrict__ lnZ2,
-                    const double *__restrict__ gB, const double *__restrict__ gS,
-                    float *__restrict__ scratch, uint32_t scratch_rows,
-                    double *__restrict__ grad_atoms, double *__restrict__ grad_tau) {
-  __shared__ uint32_t s_item;
-  __shared__ double sh[kDiffBlock / 32][8];
-  __shared__ uint32_t s_end;
-  __shared__ __align__(16) ExpRow s_tab[kDiffBlock / 32][kDiffRowTab];
-  const uint32_t lane = threadIdx.x & 31u;
-  ExpRow *tab = s_tab[threadIdx.x >> 5];
-  float *my_scratch = scratch + (size_t)blockIdx.x * scratch_rows * kDiffSlots * kDiffBlock;
-  for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(counter, 1u);
-    __syncthreads();
-    const uint32_t it = s_item;
-    __syncthreads();
-    if (it >= n_items) break;
-    const DiffItem w = items[it];
-    const DiffTemplate t = T[w.tmpl];
-    const uint32_t n = w.n0 + threadIdx.x;
-    const bool active = n < w.n1;
-    const uint32_t *t0s = t0s_all + t.t0_off;
-    const float *a8 = atoms8 + t.atom_off * 8u;
-    const uint32_t *a8u = reinterpret_cast<const uint32_t *>(a8);
-    const double tau = tau_of(t, active ? n : w.n0);
-    const double r1 = exp(-(double)t.g.TAtom / tau);
-    const double inv_r1 = r1 > 1e-280 ? 1.0 / r1 : 0.0;
-    // normalisers from the forward outputs: logsumexp F and logsumexp 2F/T
-    const double z1 = lnZ1[w.tmpl] - log(70.0 / ((double)t.N_t0 * (double)t.N_tau));
-    const double z2 = lnZ2[w.tmpl] / temp;
-    const double gb = gB[w.tmpl], gs = gS[w.tmpl];
-    const FF z1w = dw_from(z1), z2w = dw_from(z2), twoT = dw_from(2.0 / temp);
-    const float gbf = (float)gb, gsf = (float)gs;
-    FF dtw{0.0f, 0.0f};
-    // a tier-1 F below `skip` carries no weight in either sum
-    const double sk1 = gb != 0.0 ? z1 - 42.0 : INFINITY;
-    const double sk2 = gs != 0.0 ? 0.5 * temp * (z2 - 80.0) - 1.0 : INFINITY;
-    const float skip = (float)fmin(sk1, sk2);
-    const uint32_t tau_up = !active ? 0u
-                            : (tau >= 4294967295.0 ? 0xFFFFFFFFu : (uint32_t)ceil(tau));
-    const uint32_t taumax = __reduce_max_sync(0xffffffffu, tau_up);
-    ExpColumnV CV;
-    CV.C.init_real(t.g, tau);
-    CV.reset_v();
-    double dtau = 0.0, pw64 = 1.0;
-    uint32_t Lp64 = 0;
-    for (uint32_t ce = t.N_t0; ce > 0;) {
-      const uint32_t cb = ce > kDiffRowTab ? ce - kDiffRowTab : 0u;
-      bool reg = true;
-      for (uint32_t r = lane; r < ce - cb; r += 32u)
-        reg = reg && exp_row_regular(__ldg(t0s + cb + r), taumax, t.g);
-      reg = __all_sync(0xffffffffu, reg);
-      __syncwarp();
-      for (uint32_t r = lane; r < ce - cb; r += 32u) {
-        const uint32_t t0 = __ldg(t0s + cb + r);
-        ExpRow e;
-        e.lo = exp_lo(t0, t.g);
-        e.nz = e.lo < t.g.numAtoms ? __ldg(a8u + (size_t)e.lo * 8u + 3u) : 0xFFFFFFFFu;
-        const uint32_t d = t0 - t.g.t0_data;
-        e.a = reg ? fdiv(d, t.g.div) : t0;  // irregular chunks: the generic branch reads t0
-        e.b = reg ? d - e.a * t.g.TAtom : 0u;
-        tab[r] = e;
-      }
-      __syncwarp();
-      if (active) {
-        for (uint32_t m = ce; m > cb;) {
-          m--;
-          const ExpRow e = tab[m - cb];
-          uint32_t top = 0;
-          bool data = false;
-          if (reg) {
-            const uint32_t v = e.b + CV.C.RmT;
-            top = e.a + CV.C.Qp1 - (v >> 31);
-            top = top < 1u ? 1u : (top < t.g.numAtoms ? top : t.g.numAtoms);
-            data = e.lo < top && CV.slide(a8, t.g, e.lo, top, e.nz);
-          } else {
-            uint32_t hi;
-            if (exp_hi_real(e.a, tau, t.g, hi) && e.lo <= hi) {
-              top = hi + 1u;
-              data = CV.slide(a8, t.g, e.lo, top, e.nz);
-            }
-          }
-          float Gf[7] = {0, 0, 0, 0, 0, 0, 0};
-          float p1h = 0.0f, p1l = 0.0f;
-          if (data) {
-            // r^L, L = top - lo, for the removal in the transposed recurrence
-            // (FP64, one multiplication when L moves by one)
-            const uint32_t L = top - e.lo;
-            if (L != Lp64) {
-              if (L == Lp64 + 1u)
-                pw64 *= r1;
-              else if (L + 1u == Lp64 && inv_r1 > 0.0)
-                pw64 *= inv_r1;
-              else
-                pw64 = pow(r1, (double)L);
-              Lp64 = L;
-            }
-            const ExpColumn<false> &C = CV.C;
-            float F32;
-            const F2 s0 = add2(C.W0.h, C.W0.l), s2v = add2(C.W2.h, C.W2.l),
-                     s3 = add2(C.W3.h, C.W3.l);
-            const float sc = fadd(C.Wc.h, C.Wc.l);
-            const bool t1 = fstat_fast_sums(s0.x, s0.y, sc, s2v.x, s2v.y, s3.x, s3.y, F32);
-            if (!(t1 && F32 < skip)) {
-              const FF A{C.W0.h.x, C.W0.l.x}, B{C.W0.h.y, C.W0.l.y}, Cc = C.Wc;
-              const FF Far{C.W2.h.x, C.W2.l.x}, Fai{C.W2.h.y, C.W2.l.y};
-              const FF Fbr{C.W3.h.x, C.W3.l.x}, Fbi{C.W3.h.y, C.W3.l.y};
-              const DwCell fc = dw_fstat(A, B, Cc, Far, Fai, Fbr, Fbi);
-              if (fc.ok) {
-                const FF F = fc.F;
-                // exponents of the weights from double-word differences
-                const FF d1 = dw_sub(F, z1w);
-                const FF d2 = dw_sub(ff_mul(F, twoT), z2w);
-                const float g = gbf * exp2f(fadd(d1.h, d1.l) * kLog2eF) +
-                                gsf * 2.0f * exp2f(fadd(d2.h, d2.l) * kLog2eF);
-                const FF Fa2 = dw_add(ff_mul(Far, Far), ff_mul(Fai, Fai));
-                const FF re = dw_add(ff_mul(Far, Fbr), ff_mul(Fai, Fbi));
-                FF dF[7];
-                dF[0] = ff_mul(dw_sub(fc.Fb2, ff_mul(F, B)), fc.iD);
-                dF[1] = ff_mul(dw_sub(Fa2, ff_mul(F, A)), fc.iD);
-                dF[2] = dw_twice(ff_mul(dw_sub(ff_mul(F, Cc), re), fc.iD));
-                dF[3] = dw_twice(ff_mul(fc.Gre, fc.iD));
-                dF[4] = dw_twice(ff_mul(fc.Gim, fc.iD));
-                dF[5] = dw_twice(ff_mul(dw_sub(ff_mul(A, Fbr), ff_mul(Cc, Far)), fc.iD));
-                dF[6] = dw_twice(ff_mul(dw_sub(ff_mul(A, Fbi), ff_mul(Cc, Fai)), fc.iD));
-                const FF V[7] = {FF{CV.V0.h.x, CV.V0.l.x}, FF{CV.V0.h.y, CV.V0.l.y}, CV.Vc,
-                                 FF{CV.V2.h.x, CV.V2.l.x}, FF{CV.V2.h.y, CV.V2.l.y},
-                                 FF{CV.V3.h.x, CV.V3.l.x}, FF{CV.V3.h.y, CV.V3.l.y}};
-#pragma unroll
-                for (int c = 0; c < 7; c++) {
-                  const FF Gc = dw_mulf(dF[c], g);
-                  Gf[c] = fadd(Gc.h, Gc.l);
-                  const FF tv = ff_mul(Gc, V[c]);
-                  dtw = dw_add(dtw, c < 3 ? dw_twice(tv) : tv);
-                }
-                p1h = (float)pw64;
-                p1l = (float)(pw64 - (double)p1h);
-              }
-            }
-          }
-          TCW_DCHECK(m < scratch_rows);
-          float *scr = my_scratch + (size_t)m * kDiffSlots * kDiffBlock + threadIdx.x;
-#pragma unroll
-          for (int c = 0; c < 7; c++) scr[(size_t)c * kDiffBlock] = Gf[c];
-          scr[(size_t)7 * kDiffBlock] = p1h;
-          scr[(size_t)8 * kDiffBlock] = p1l;
-        }
-      }
-      ce = cb;
-    }
+// ------------------------------------------------------------ exponential tiles
 
-    // ---- pass B done for this tile: tau gradient, then pass C (ascending)
-    __syncthreads();  // scratch of all columns written
-    dtau = (double)dtw.h + (double)dtw.l;
-    const double scale = active ? (double)t.g.TAtom / (tau * tau) * dtau : 0.0;
-    const double fr = (active && t.N_tau > 1) ? (double)n / (double)(t.N_tau - 1u) : 0.0;
-    double dmax = scale * fr,
-           dmin = scale * (active && t.N_tau > 1 ? 1.0 - fr : (active ? 1.0 : 0.0));
+constexpr uint32_t kDiffRowTab = 128;
+
+__global__ void __launch_bounds__(256) diff_prep_kernel(const DiffTemplate *__restrict__ T,
+                                                        const uint32_t *__restrict__ list,
+                                                        uint32_t n_exp,
+                                                        const float *__restrict__ atoms,
+                                                        float *__restrict__ atoms8,
+                                                        ColConsts *__restrict__ cols) {
+  __shared__ uint32_t s_first[256];
+  if (blockIdx.y > 0) {  // the templates' column constants, 256 columns per block
+    for (uint32_t k = blockIdx.x; k < n_exp; k += gridDim.x) {
+      const DiffTemplate t = T[list[k]];
+      const uint32_t n = (blockIdx.y - 1u) * 256u + threadIdx.x;
+      if (n >= t.N_tau) continue;
+      ExpColumn<false> C;
+      C.init_real(t.g, tau_of(t, n));
+      cols[t.col_off + n] = C.consts();
+    }
+    return;
+  }
+  for (uint32_t k = blockIdx.x; k < n_exp; k += gridDim.x) {
+    const DiffTemplate t = T[list[k]];
+    repack_rows256(atoms + t.atom_off * 7u, reinterpret_cast<float4 *>(atoms8 + t.atom_off * 8u),
+                   t.g.numAtoms, s_first);
+    __syncthreads();
+  }
+}
+
+// One warp's share of a template: its column group, this lane's column and
+// the warp's largest tau (rounded up, for the regularity test).
+struct DiffLane {
+  DiffTemplate t;
+  uint32_t n, taumax;
+  bool active;
+  double tau;
+  const float *a8;
+  const uint32_t *t0s;
+
+  __device__ __forceinline__ void columns(const float *atoms8, const uint32_t *t0s_all,
+                                          uint32_t cg) {
+    n = cg * 32u + (threadIdx.x & 31u);
+    active = n < t.N_tau;
+    tau = tau_of(t, active ? n : cg * 32u);
+    const uint32_t up = !active ? 0u
+                        : (tau >= 4294967295.0 ? 0xFFFFFFFFu : (uint32_t)ceil(tau));
+    taumax = __reduce_max_sync(0xffffffffu, up);
+    a8 = atoms8 + t.atom_off * 8u;
+    t0s = t0s_all + t.t0_off;
+  }
+  // this lane's constants (a lane without a column takes the group's first)
+  __device__ __forceinline__ ColConsts consts(const ColConsts *__restrict__ cols) const {
+    return cols[t.col_off + (active ? n : n & ~31u)];
+  }
+};
+
+template <bool kFast, bool kWide>
+__device__ __forceinline__ const ExpColumn<false, kFast, kWide> &sums_of(
+    const ExpColumn<false, kFast, kWide> &C) {
+  return C;
+}
+__device__ __forceinline__ const ExpColumn<false> &sums_of(const ExpColumnV &C) { return C.C; }
+
+// Walks rows [mb, me) of one tile from the last one down and calls
+// cell(m, lo, top, data) for each: data says that the window [lo, top) holds
+// data and that the column holds its sums.  Rows that are not regular for
+// the group's taus (t0 + 3 tau + TAtom/2 beyond u32, or TAtom < 2) take the
+// window end from exp_hi_real.  `seg`: this lane's segment sums of the group,
+// `stride` floats apart (NULL: the first window is entered atom by atom).
+template <class Col, class Cell>
+__device__ __forceinline__ void diff_rows(const DiffLane &L, uint32_t mb, uint32_t me, Col &C,
+                                          const float *__restrict__ seg, uint32_t stride,
+                                          ExpRow *tab, Cell &&cell) {
+  const DiffTemplate &t = L.t;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t *a8u = reinterpret_cast<const uint32_t *>(L.a8);
+  if (seg && L.active) {
+    const uint32_t t0 = __ldg(L.t0s + me - 1u);
+    if (exp_row_regular(t0, L.taumax, t.g)) {
+      const uint32_t lo = exp_lo(t0, t.g), d = t0 - t.g.t0_data;
+      ExpRow e;
+      e.a = fdiv(d, t.g.div);
+      e.b = d - e.a * t.g.TAtom;
+      const uint32_t top = sums_of(C).top_of(t.g, e);
+      if (lo < top && top - lo >= (2u << t.g_shift))
+        C.warm_start(L.a8, t.g, seg, t.g_shift, t.g_nseg, lo, top, stride);
+    }
+  }
+  for (uint32_t ce = me; ce > mb;) {
+    const uint32_t cb = ce - mb > kDiffRowTab ? ce - kDiffRowTab : mb;
+    bool reg = true;
+    for (uint32_t r = lane; r < ce - cb; r += 32u)
+      reg = reg && exp_row_regular(__ldg(L.t0s + cb + r), L.taumax, t.g);
+    reg = __all_sync(0xffffffffu, reg);
+    __syncwarp();
+    for (uint32_t r = lane; r < ce - cb; r += 32u) {
+      const uint32_t t0 = __ldg(L.t0s + cb + r);
+      ExpRow e;
+      e.lo = exp_lo(t0, t.g);
+      e.nz = e.lo < t.g.numAtoms ? __ldg(a8u + (size_t)e.lo * 8u + 3u) : 0xFFFFFFFFu;
+      const uint32_t d = t0 - t.g.t0_data;
+      e.a = reg ? fdiv(d, t.g.div) : t0;  // irregular chunks: the generic branch reads t0
+      e.b = reg ? d - e.a * t.g.TAtom : 0u;
+      tab[r] = e;
+    }
+    __syncwarp();
+    if (L.active) {
+      for (uint32_t m = ce; m > cb;) {
+        m--;
+        const ExpRow e = tab[m - cb];
+        uint32_t top = 0;
+        bool data = false;
+        if (reg) {
+          top = sums_of(C).top_of(t.g, e);
+          data = e.lo < top && C.slide(L.a8, t.g, e.lo, top, e.nz);
+        } else {
+          uint32_t hi;
+          if (exp_hi_real(e.a, L.tau, t.g, hi) && e.lo <= hi) {
+            top = hi + 1u;
+            data = C.slide(L.a8, t.g, e.lo, top, e.nz);
+          }
+        }
+        cell(m, e.lo, top, data);
+      }
+    }
+    ce = cb;
+  }
+}
+
+// Tier-1 F of a column's current sums; false where it needs the test.
+__device__ __forceinline__ bool diff_tier1(const ExpColumn<false> &C, float &F32) {
+  const F2 s0 = add2(C.W0.h, C.W0.l), s2 = add2(C.W2.h, C.W2.l), s3 = add2(C.W3.h, C.W3.l);
+  const float sc = fadd(C.Wc.h, C.Wc.l);
+  return fstat_fast_sums(s0.x, s0.y, sc, s2.x, s2.y, s3.x, s3.y, F32);
+}
+
+// The largest F of every tile in FP32 (`need`, good to ~1.5e-6 relative: tier
+// 1, else tier 2 with the conditioning cut widened by 1e-3, so that no cell
+// that FP64 lets pass is missed; infinite for a NaN; at least 2 where a cell
+// has no data) and the largest F of the template's cells that surely pass
+// (`est`, a lower bound of its maximum to within 1.5e-6).  One W-only walk
+// with the map kernels' steps: on the benchmark's differentiation data
+// (maximum F 400, F within 62 of it in 4e-6 of the cells) it replaces the
+// FP64 work of 99.6 % of the tiles.
+struct EstSink {
+  float top, most;
+  __device__ __forceinline__ void start() {}
+  __device__ __forceinline__ void operator()(uint32_t, float F, bool ok) {
+    if (!(F == F)) F = INFINITY;
+    else if (ok) top = fmaxf(top, F);
+    most = fmaxf(most, F);
+  }
+};
+
+__global__ void __launch_bounds__(kDiffBlock, 8)
+    diff_est_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
+                    const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
+                    const ColConsts *__restrict__ cols, const float *__restrict__ seg,
+                    float *__restrict__ need, uint32_t *__restrict__ est) {
+  __shared__ __align__(16) ExpRow s_tab[kDiffBlock / 32][kExpRowTab];
+  DiffLane L;
+  const uint32_t k = list[blockIdx.y];
+  L.t = T[k];
+  const uint32_t tile = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+  const uint32_t cg = tile / L.t.n_chunk, mb = tile % L.t.n_chunk * L.t.chunk_rows;
+  if (cg >= L.t.n_cg) return;
+  const uint32_t me = min(L.t.N_t0, mb + L.t.chunk_rows);
+  L.columns(atoms8, t0s_all, cg);
+  ExpColumn<false, true, true> C;
+  C.init_consts(L.consts(cols));
+  const float *sg =
+      L.t.g_nseg ? seg + (L.t.seg_off + (size_t)cg * L.t.g_nseg) * kDiffSegFloats + lane : nullptr;
+  EstSink sink{-INFINITY, -INFINITY};
+  bool reg = true;
+  for (uint32_t m = mb + lane; m < me; m += 32u)
+    reg = reg && exp_row_regular(__ldg(L.t0s + m), L.taumax, L.t.g);
+  ExpRow *tab = s_tab[threadIdx.x >> 5];
+  if (__all_sync(0xffffffffu, reg)) {
+    exp_rows(C, L.t.g, L.t.g_shift, L.t.g_nseg, L.a8, L.t0s, mb, me, me, L.active, sink, tab, sg);
+  } else {
+    diff_rows(L, mb, me, C, sg, kDiffSegFloats, tab,
+              [&](uint32_t m, uint32_t, uint32_t, bool data) {
+                if (data)
+                  C.emit(m, sink);
+                else
+                  sink(m, 2.0f, false);
+              });
+  }
+  float top1 = sink.top, most = sink.most;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    top1 = fmaxf(top1, __shfl_xor_sync(0xffffffffu, top1, d));
+    most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, d));
+  }
+  if (lane == 0) {
+    need[L.t.part_off + tile] = most;
+    if (top1 > -INFINITY) atomicMax(est + k, float_key(top1));
+  }
+}
+
+// ------------------------------------------------------------ exponential forward
+
+// From the key of a template's estimated maximum: cells below `skip` carry no
+// weight in either sum, tiles that reach `hot` may hold a cell that matters
+// by itself (lnBtSG: e^-8 of the largest; the soft-max's weights fall 20 times
+// as fast).
+struct FwdBounds {
+  float skip, hot;
+  __device__ __forceinline__ explicit FwdBounds(uint32_t key) {
+    skip = hot = -INFINITY;
+    if (key) {
+      const double top = (double)key_float(key);
+      skip = (float)(top - 1e-5 * fabs(top) - 63.0);
+      hot = (float)(top - 1e-5 * fabs(top) - 8.0);
+    }
+  }
+};
+
+// FP64 log-sum-exps of F and 2F/T over the cells of one lane, then over the
+// warp.
+struct DiffLse {
+  double m1, s1, m2, s2, twoT;
+  float skip, skip0;
+  __device__ __forceinline__ DiffLse(double temp, float bound)
+      : m1(-INFINITY), s1(0.0), m2(-INFINITY), s2(0.0), twoT(2.0 / temp), skip(bound),
+        skip0(bound) {}
+  __device__ __forceinline__ void add(double F) {
+    lse_add(m1, s1, F);
+    lse_add(m2, s2, F * twoT);
+    skip = fmaxf((float)(m1 - 62.0), skip0);
+  }
+  __device__ __forceinline__ void cell(bool data, const double W[7], bool t1, float F32) {
+    if (!data) {
+      if (!(2.0f < skip)) add(2.0);
+    } else if (!(t1 && F32 < skip)) {
+      add(fstat64(W, t1).F);
+    }
+  }
+  // every lane's sums brought to the warp's maximum (one exp per sum), added
+  __device__ __forceinline__ DiffPartial merge() const {
+    double M1 = m1, M2 = m2;
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
-      dmax += __shfl_down_sync(0xffffffffu, dmax, d);
-      dmin += __shfl_down_sync(0xffffffffu, dmin, d);
+      M1 = fmax(M1, __shfl_xor_sync(0xffffffffu, M1, d));
+      M2 = fmax(M2, __shfl_xor_sync(0xffffffffu, M2, d));
     }
-    if (lane == 0) {
-      sh[threadIdx.x >> 5][0] = dmin;
-      sh[threadIdx.x >> 5][1] = dmax;
+    double S1 = s1 > 0.0 ? s1 * exp(m1 - M1) : 0.0, S2 = s2 > 0.0 ? s2 * exp(m2 - M2) : 0.0;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+      S1 += __shfl_xor_sync(0xffffffffu, S1, d);
+      S2 += __shfl_xor_sync(0xffffffffu, S2, d);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double a = 0.0, b = 0.0;
-      for (int k = 0; k < kDiffBlock / 32; k++) {
-        a += sh[k][0];
-        b += sh[k][1];
+    return DiffPartial{M1, S1, M2, S2};
+  }
+};
+
+// Forward pass of the tiles that may carry weight (lnBtSG and the soft-max
+// 2F): the window sums in double-word FP32 (ExpColumn; sums good to ~1e-14 of
+// the window's magnitude, against FP64 recurrences at GB300's 1/70 FP64
+// rate), F of the weighted cells in FP64 from them (the reference's formula
+// and conditioning test, fstat64) into FP64 log-sum-exps.  A cell whose
+// tier-1 F lies more than 62 below a lower bound of the template's maximum
+// carries exp(F - max) < e^-60 in both sums (the soft-max's 2F/T - max is 2/T
+// times lower still) and is skipped -- the tier-1 F is good to ~1.5e-6
+// relative and passes only for cond < 32, where the FP64 test passes too.
+__global__ void __launch_bounds__(kDiffBlock, 5)
+    diff_fwd_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
+                    const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
+                    const ColConsts *__restrict__ cols, const float *__restrict__ seg,
+                    const float *__restrict__ need, const uint32_t *__restrict__ est, double temp,
+                    DiffPartial *__restrict__ parts) {
+  __shared__ __align__(16) ExpRow s_tab[kDiffBlock / 32][kDiffRowTab];
+  DiffLane L;
+  const uint32_t k = list[blockIdx.y];
+  L.t = T[k];
+  const uint32_t tile = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+  const uint32_t cg = tile / L.t.n_chunk, mb = tile % L.t.n_chunk * L.t.chunk_rows;
+  if (cg >= L.t.n_cg) return;
+  DiffPartial *out = parts + L.t.part_off + tile;
+  const FwdBounds bd(est[k]);
+  const float skip0 = bd.skip, nd = need[L.t.part_off + tile];
+  if (nd < skip0) {
+    if (lane == 0) *out = DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
+    return;
+  }
+  if (!(nd < bd.hot)) return;  // diff_hot_kernel
+  const uint32_t me = min(L.t.N_t0, mb + L.t.chunk_rows);
+  L.columns(atoms8, t0s_all, cg);
+  ExpColumn<false> C;
+  C.init_consts(L.consts(cols));
+  const float *sg =
+      L.t.g_nseg ? seg + (L.t.seg_off + (size_t)cg * L.t.g_nseg) * kDiffSegFloats + lane : nullptr;
+  DiffLse lse(temp, skip0);
+  diff_rows(L, mb, me, C, sg, kDiffSegFloats, s_tab[threadIdx.x >> 5],
+            [&](uint32_t, uint32_t, uint32_t, bool data) {
+              float F32 = 0.0f;
+              const bool t1 = data && diff_tier1(C, F32);
+              double W[7] = {0, 0, 0, 0, 0, 0, 0};
+              if (data && !(t1 && F32 < lse.skip)) {
+                W[0] = (double)C.W0.h.x + (double)C.W0.l.x;
+                W[1] = (double)C.W0.h.y + (double)C.W0.l.y;
+                W[2] = (double)C.Wc.h + (double)C.Wc.l;
+                W[3] = (double)C.W2.h.x + (double)C.W2.l.x;
+                W[4] = (double)C.W2.h.y + (double)C.W2.l.y;
+                W[5] = (double)C.W3.h.x + (double)C.W3.l.x;
+                W[6] = (double)C.W3.h.y + (double)C.W3.l.y;
+              }
+              lse.cell(data, W, t1, F32);
+            });
+  const DiffPartial p = lse.merge();
+  if (lane == 0) *out = p;
+}
+
+// Whether a template's cells below `skip` carry no weight in the gradient: a
+// cell's weight g = gB e^(F - Z1) + 2 gS e^(2F/T - Z2) (Z1 = logsumexp F,
+// Z2 = logsumexp 2F/T, from the forward outputs) is below e^-40 when its
+// tier-1 F (good to ~1e-5 of F) lies more than 42 below Z1 (the lnBtSG term,
+// gB != 0) and more than 40 T + 1 below (T/2) Z2 (the soft-max term, gS != 0:
+// its exponent is then below -80).
+// `hot`: above it a single cell may carry more than e^-6 of either gradient.
+struct DiffWeights {
+  double z1, z2, gb, gs;
+  float skip, hot;
+  __device__ __forceinline__ DiffWeights(const DiffTemplate &t, uint32_t k, double temp,
+                                         const double *lnZ1, const double *lnZ2,
+                                         const double *gB, const double *gS) {
+    z1 = lnZ1[k] - log(70.0 / ((double)t.N_t0 * (double)t.N_tau));
+    z2 = lnZ2[k] / temp;
+    gb = gB[k];
+    gs = gS[k];
+    const double sk1 = gb != 0.0 ? z1 - 42.0 : INFINITY;
+    const double sk2 = gs != 0.0 ? 0.5 * temp * (z2 - 80.0) - 1.0 : INFINITY;
+    skip = (float)fmin(sk1, sk2);
+    hot = (float)fmin(gb != 0.0 ? z1 - 1e-5 * fabs(z1) - 7.0 : INFINITY,
+                      gs != 0.0 ? 0.5 * temp * (z2 - 1e-5 * fabs(z2) - 25.0) - 0.1 : INFINITY);
+  }
+};
+
+// Segment sums (exp_seg_kernel's, with TwoSum steps; kV: with the tau
+// derivatives, only for column groups that diff_src_kernel walks).
+template <bool kV>
+__global__ void __launch_bounds__(kDiffBlock)
+    diff_seg_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
+                    const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
+                    const ColConsts *__restrict__ cols, const float *__restrict__ need,
+                    double temp, const double *__restrict__ lnZ1,
+                    const double *__restrict__ lnZ2, const double *__restrict__ gB,
+                    const double *__restrict__ gS, float *__restrict__ seg) {
+  DiffLane L;
+  const uint32_t k = list[blockIdx.y];
+  L.t = T[k];
+  const uint32_t w = blockIdx.x * 4u + (threadIdx.x >> 5);
+  const uint32_t cg = w % L.t.n_cg, j0 = w / L.t.n_cg * kSegPerWarp;
+  if (j0 >= L.t.g_nseg) return;
+  if (kV) {
+    const DiffWeights w(L.t, k, temp, lnZ1, lnZ2, gB, gS);
+    const float *nd = need + L.t.part_off + (size_t)cg * L.t.n_chunk;
+    bool any = false;
+    for (uint32_t c = threadIdx.x & 31u; c < L.t.n_chunk; c += 32u)
+      any = any || (!(nd[c] < w.skip) && nd[c] < w.hot);
+    if (!__any_sync(0xffffffffu, any)) return;
+  }
+  L.columns(atoms8, t0s_all, cg);
+  const uint32_t shift = L.t.g_shift, j1 = min(L.t.g_nseg, j0 + kSegPerWarp);
+  // a window holds fewer than 3 tau / TAtom + 2 atoms: shorter ones are never joined
+  if (3ull * L.taumax + 2ull * L.t.g.TAtom < ((uint64_t)L.t.g.TAtom << (shift + 1u))) return;
+  for (uint32_t j = j0; j < j1; j++) {
+    const uint32_t lo = j << shift, top = min(L.t.g.numAtoms, (j + 1u) << shift);
+    if (kV) {
+      ExpColumnV C;
+      C.C.init_consts(L.consts(cols));
+      C.reset_v();
+      C.slide(L.a8, L.t.g, lo, top, 0u);
+      C.store_sums(seg + (L.t.seg_off + (size_t)cg * L.t.g_nseg + j) * kDiffSegFloatsV +
+                   (threadIdx.x & 31u));
+    } else {
+      ExpColumn<false> C;
+      C.init_consts(L.consts(cols));
+      C.slide(L.a8, L.t.g, lo, top, 0u);
+      C.store_sums(seg + (L.t.seg_off + (size_t)cg * L.t.g_nseg + j) * kDiffSegFloats +
+                   (threadIdx.x & 31u));
+    }
+  }
+}
+
+// The cell's gradient dL/dF dF/dW_c (Gf) from its double-word window sums in
+// double-word arithmetic, and G_c k_c V_c added to dtw; false (and Gf
+// untouched) where the conditioning test fails.
+struct DiffGrad {
+  FF z1w, z2w, twoT;
+  float gbf, gsf;
+  __device__ __forceinline__ DiffGrad(const DiffWeights &w, double temp)
+      : z1w(dw_from(w.z1)), z2w(dw_from(w.z2)), twoT(dw_from(2.0 / temp)), gbf((float)w.gb),
+        gsf((float)w.gs) {}
+  __device__ __forceinline__ bool cell(const FF W[7], const FF V[7], float Gf[7], FF &dtw) const {
+    const FF A = W[0], B = W[1], Cc = W[2], Far = W[3], Fai = W[4], Fbr = W[5], Fbi = W[6];
+    const DwCell fc = dw_fstat(A, B, Cc, Far, Fai, Fbr, Fbi);
+    if (!fc.ok) return false;
+    const FF F = fc.F;
+    // exponents of the weights from double-word differences
+    const FF d1 = dw_sub(F, z1w);
+    const FF d2 = dw_sub(ff_mul(F, twoT), z2w);
+    const float g = gbf * exp2f(fadd(d1.h, d1.l) * kLog2eF) +
+                    gsf * 2.0f * exp2f(fadd(d2.h, d2.l) * kLog2eF);
+    const FF Fa2 = dw_add(ff_mul(Far, Far), ff_mul(Fai, Fai));
+    const FF re = dw_add(ff_mul(Far, Fbr), ff_mul(Fai, Fbi));
+    FF dF[7];
+    dF[0] = ff_mul(dw_sub(fc.Fb2, ff_mul(F, B)), fc.iD);
+    dF[1] = ff_mul(dw_sub(Fa2, ff_mul(F, A)), fc.iD);
+    dF[2] = dw_twice(ff_mul(dw_sub(ff_mul(F, Cc), re), fc.iD));
+    dF[3] = dw_twice(ff_mul(fc.Gre, fc.iD));
+    dF[4] = dw_twice(ff_mul(fc.Gim, fc.iD));
+    dF[5] = dw_twice(ff_mul(dw_sub(ff_mul(A, Fbr), ff_mul(Cc, Far)), fc.iD));
+    dF[6] = dw_twice(ff_mul(dw_sub(ff_mul(A, Fbi), ff_mul(Cc, Fai)), fc.iD));
+#pragma unroll
+    for (int c = 0; c < 7; c++) {
+      const FF Gc = dw_mulf(dF[c], g);
+      Gf[c] = fadd(Gc.h, Gc.l);
+      const FF tv = ff_mul(Gc, V[c]);
+      dtw = dw_add(dtw, c < 3 ? dw_twice(tv) : tv);
+    }
+    return true;
+  }
+};
+
+// r^L, L = top - lo, for the removal in the transposed recurrence (FP64, one
+// multiplication when L moves by one), as a float pair.
+struct DiffPower {
+  double r1 = 0.0, inv_r1 = 0.0, pw = 1.0;
+  uint32_t len = 0;
+  bool init = false;
+  __device__ __forceinline__ FF at(const DiffLane &L, uint32_t n) {
+    if (!init) {
+      r1 = exp(-(double)L.t.g.TAtom / L.tau);
+      inv_r1 = r1 > 1e-280 ? 1.0 / r1 : 0.0;
+      init = true;
+    }
+    if (n != len) {
+      if (n == len + 1u) {
+        pw *= r1;
+      } else if (n + 1u == len && inv_r1 > 0.0) {
+        pw *= inv_r1;
+      } else {  // square and multiply: pow()'s chain of FP64 steps is ten times as long
+        double base = r1;
+        pw = 1.0;
+        for (uint32_t q = n; q; q >>= 1) {
+          if (q & 1u) pw *= base;
+          base *= base;
+        }
       }
-      atomicAdd(grad_tau + 2u * w.tmpl, a);
-      atomicAdd(grad_tau + 2u * w.tmpl + 1u, b);
-      s_end = 0;
+      len = n;
+    }
+    const float h = (float)pw;
+    return FF{h, (float)(pw - (double)h)};
+  }
+};
+
+__device__ __forceinline__ void add_grad_tau(const DiffLane &L, FF dtw, double *grad_tau) {
+  const double dtau = (double)dtw.h + (double)dtw.l;
+  const double scale = L.active ? (double)L.t.g.TAtom / (L.tau * L.tau) * dtau : 0.0;
+  const double fr = (L.active && L.t.N_tau > 1) ? (double)L.n / (double)(L.t.N_tau - 1u) : 0.0;
+  double dmax = scale * fr,
+         dmin = scale * (L.active && L.t.N_tau > 1 ? 1.0 - fr : (L.active ? 1.0 : 0.0));
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    dmax += __shfl_down_sync(0xffffffffu, dmax, d);
+    dmin += __shfl_down_sync(0xffffffffu, dmin, d);
+  }
+  if ((threadIdx.x & 31u) == 0) {
+    atomicAdd(grad_tau, dmin);
+    atomicAdd(grad_tau + 1, dmax);
+  }
+}
+
+// Adjoint sources of the tiles that may carry weight: W and V slide down each
+// tau column in double-word FP32 (ExpColumnV); a cell gets F, dF/dW and its
+// sources (in double-word arithmetic, dw_fstat) only when it carries weight
+// (DiffWeights).
+__global__ void __launch_bounds__(kDiffBlock)
+    diff_src_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
+                    const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
+                    const ColConsts *__restrict__ cols, const float *__restrict__ seg,
+                    const float *__restrict__ need, double temp, const double *__restrict__ lnZ1,
+                    const double *__restrict__ lnZ2, const double *__restrict__ gB,
+                    const double *__restrict__ gS, float *__restrict__ scratch,
+                    double *__restrict__ grad_tau) {
+  __shared__ __align__(16) ExpRow s_tab[kDiffBlock / 32][kDiffRowTab];
+  DiffLane L;
+  const uint32_t k = list[blockIdx.y];
+  L.t = T[k];
+  const DiffTemplate &t = L.t;
+  const uint32_t tile = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+  const uint32_t cg = tile / t.n_chunk, mb = tile % t.n_chunk * t.chunk_rows;
+  if (cg >= t.n_cg) return;
+  const DiffWeights w(t, k, temp, lnZ1, lnZ2, gB, gS);
+  const float nd = need[t.part_off + tile];
+  if (nd < w.skip) return;    // diff_atoms_kernel skips its rows
+  if (!(nd < w.hot)) return;  // diff_hot_kernel
+  const uint32_t me = min(t.N_t0, mb + t.chunk_rows);
+  L.columns(atoms8, t0s_all, cg);
+  const DiffGrad grad(w, temp);
+  DiffPower power;
+  FF dtw{0.0f, 0.0f};
+  ExpColumnV CV;
+  CV.C.init_consts(L.consts(cols));
+  CV.reset_v();
+  const float *sg =
+      t.g_nseg ? seg + (t.seg_off + (size_t)cg * t.g_nseg) * kDiffSegFloatsV + lane : nullptr;
+  float *my = scratch + t.scr_off + (size_t)tile * t.chunk_rows * (TCW_DIFF_SLOTS * 32u) + lane;
+  diff_rows(L, mb, me, CV, sg, kDiffSegFloatsV, s_tab[threadIdx.x >> 5],
+            [&](uint32_t m, uint32_t lo, uint32_t top, bool data) {
+              float Gf[7] = {0, 0, 0, 0, 0, 0, 0};
+              FF p1{0.0f, 0.0f};
+              if (data) {
+                const ExpColumn<false> &C = CV.C;
+                float F32;
+                const bool t1 = diff_tier1(C, F32);
+                if (!(t1 && F32 < w.skip)) {
+                  const FF W[7] = {FF{C.W0.h.x, C.W0.l.x}, FF{C.W0.h.y, C.W0.l.y}, C.Wc,
+                                   FF{C.W2.h.x, C.W2.l.x}, FF{C.W2.h.y, C.W2.l.y},
+                                   FF{C.W3.h.x, C.W3.l.x}, FF{C.W3.h.y, C.W3.l.y}};
+                  const FF V[7] = {FF{CV.V0.h.x, CV.V0.l.x}, FF{CV.V0.h.y, CV.V0.l.y}, CV.Vc,
+                                   FF{CV.V2.h.x, CV.V2.l.x}, FF{CV.V2.h.y, CV.V2.l.y},
+                                   FF{CV.V3.h.x, CV.V3.l.x}, FF{CV.V3.h.y, CV.V3.l.y}};
+                  if (grad.cell(W, V, Gf, dtw)) p1 = power.at(L, top - lo);
+                }
+              }
+              TCW_DCHECK(m - mb < t.chunk_rows);
+              float *scr = my + (size_t)(m - mb) * (TCW_DIFF_SLOTS * 32u);
+#pragma unroll
+              for (int c = 0; c < 7; c++) scr[32 * c] = Gf[c];
+              scr[32 * 7] = p1.h;
+              scr[32 * 8] = p1.l;
+            });
+  add_grad_tau(L, dtw, grad_tau + 2u * k);
+}
+
+// Most atoms of a template that diff_hot_kernel keeps in shared memory.
+constexpr uint32_t kHotAtoms = 7000;
+
+// The tiles whose cells matter by themselves.  Their F enters the results
+// through exponents of 20 F, where the last bits of the window sums show, so
+// their columns are walked whole from the last row down -- a tile started
+// from segment sums agrees to ~1e-14 of the sums only.  A whole walk by one
+// thread per column is a long serial chain (W, V and the removal powers of 7
+// channels: 2.4 ms for 1024 rows); here (0.6-0.9 ms, bound by the latency of
+// ~330 dependent instructions per row) a block takes 32 columns with one
+// warp per channel, whose steps are the packed pairs' bit for bit, and the
+// eighth warp evaluates the hot rows from shared memory while the others walk
+// on.  Column groups without a hot tile leave at once.
+template <bool kBack>
+__global__ void __launch_bounds__(256)
+    diff_hot_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
+                    const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
+                    const ColConsts *__restrict__ cols, const float *__restrict__ need,
+                    const uint32_t *__restrict__ est, double temp,
+                    const double *__restrict__ lnZ1, const double *__restrict__ lnZ2,
+                    const double *__restrict__ gB, const double *__restrict__ gS,
+                    float *__restrict__ scratch, double *__restrict__ grad_tau,
+                    DiffPartial *__restrict__ parts, uint32_t smem_atoms) {
+  extern __shared__ float s_x[];  // channel-major atoms, where a template's fit
+  __shared__ float2 s_pow[32][32];  // r^(2^b) of the lanes' columns
+  constexpr int kWords = kBack ? 4 : 2;
+  __shared__ __align__(16) ExpRow tab[kDiffRowTab];
+  __shared__ float s_sum[2][7][kWords][32];
+  __shared__ uint8_t s_hot[kDiffRowTab];
+  DiffLane L;
+  const uint32_t k = list[blockIdx.y], cg = blockIdx.x;
+  L.t = T[k];
+  const DiffTemplate &t = L.t;
+  if (cg >= t.n_cg) return;
+  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  const float *nd = need + t.part_off + (size_t)cg * t.n_chunk;
+  // the first and last hot chunk
+  float hot, skip;
+  if (kBack) {
+    const DiffWeights w(t, k, temp, lnZ1, lnZ2, gB, gS);
+    hot = w.hot;
+    skip = w.skip;
+  } else {
+    const FwdBounds bd(est[k]);
+    hot = bd.hot;
+    skip = bd.skip;
+  }
+  auto is_hot = [&](uint32_t c) { return !(nd[c] < skip) && !(nd[c] < hot); };
+  uint32_t c0 = 0xFFFFFFFFu;
+  for (uint32_t c = lane; c < t.n_chunk; c += 32u)
+    if (is_hot(c)) c0 = min(c0, c);
+  c0 = __reduce_min_sync(0xffffffffu, c0);
+  if (c0 == 0xFFFFFFFFu) return;  // the same in every warp
+  const uint32_t mb = c0 * t.chunk_rows;  // rows below the last hot one are not walked
+  L.columns(atoms8, t0s_all, cg);
+  const uint32_t *a8u = reinterpret_cast<const uint32_t *>(L.a8);
+  const ColConsts cc = L.consts(cols);
+  const ExpConsts kc = cc.consts();
+
+  const uint32_t N = t.g.numAtoms;
+  const bool staged = N <= smem_atoms;
+  if (staged)
+    for (uint32_t i = threadIdx.x; i < N * 8u; i += blockDim.x)
+      if ((i & 7u) != 3u) s_x[((i & 7u) - ((i & 7u) > 3u ? 1u : 0u)) * N + (i >> 3)] = __ldg(L.a8 + i);
+  if (wid == 7u) {  // ff_pow's squarings, once per column
+    FF base = kc.r1;
+    for (uint32_t b = 0; b < 32u && (1ull << b) <= N; b++) {
+      s_pow[b][lane] = make_float2(base.h, base.l);
+      base = ff_mul(base, base);
+    }
+  }
+  __syncthreads();
+
+  // this warp's channel (warps 0..6)
+  const uint32_t ch = wid < 7u ? wid : 0u;
+  const uint32_t slot = ch < 3u ? ch : ch + 1u;
+  const FF r = ch < 3u ? kc.r2 : kc.r1;
+  FF W{0.0f, 0.0f}, V{0.0f, 0.0f}, pw{1.0f, 0.0f}, pc{1.0f, 0.0f}, pv{0.0f, 0.0f};
+  uint32_t wlo = 0, wtop = 0, Lp = 0;
+  bool pinit = false;
+  auto atom = [&](uint32_t i) {  // (the index below atom 0 reads atom 0)
+    i = i < N ? i : 0u;
+    return staged ? s_x[ch * N + i] : __ldg(L.a8 + (size_t)i * 8u + slot);
+  };
+  float xl = 0.0f, xe = 0.0f;  // the atoms that leave and enter next
+  auto leave = [&]() {
+    wtop--;
+    const uint32_t ex = wtop - wlo;
+    const float x = xl;
+    xl = atom(wtop - 1u);
+    if (ex != Lp || !pinit) {  // ExpColumn::power
+      if (pinit && ex == Lp + 1u)
+        pw = ff_mul(pw, kc.r1);
+      else if (pinit && ex + 1u == Lp && kc.has_inv)
+        pw = ff_mul(pw, kc.r1inv);
+      else {
+        pw = FF{1.0f, 0.0f};  // ff_pow from the table
+        for (uint32_t q = ex; q; q &= q - 1u) {
+          const float2 f = s_pow[__ffs(q) - 1][lane];
+          pw = ff_mul(pw, FF{f.x, f.y});
+        }
+      }
+      Lp = ex;
+      pinit = true;
+      pc = ch < 3u ? ff_mul(pw, pw) : pw;  // this channel's weight, and times its exponent
+      if (kBack) pv = ff_mul(pc, FF{(float)ex, 0.0f});
+    }
+    W = ff_sub_scaled_x1(W, pc, x);
+    if (kBack) V = ff_sub_scaled_x1(V, pv, x);
+  };
+  auto enter = [&]() {
+    wlo--;
+    const float x = xe;
+    xe = atom(wlo - 1u);
+    if (kBack) V = ff_scale_dw(r, ff_add_dw(V, W));
+    W = ff_axpy(x, r, W);
+  };
+  // the evaluating warp's state
+  DiffLse lse(temp, skip);
+  FF dtw{0.0f, 0.0f};
+  DiffPower power;
+  uint32_t buf = 0;  // the half of s_sum of the next hot row
+
+  for (uint32_t ce = t.N_t0; ce > mb;) {
+    const uint32_t cb = ce - mb > kDiffRowTab ? ce - kDiffRowTab : mb;
+    bool reg = true;  // the same in every warp
+    for (uint32_t q = lane; q < ce - cb; q += 32u)
+      reg = reg && exp_row_regular(__ldg(L.t0s + cb + q), L.taumax, t.g);
+    reg = __all_sync(0xffffffffu, reg);
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < ce - cb; q += blockDim.x) {
+      const uint32_t t0 = __ldg(L.t0s + cb + q);
+      ExpRow e;
+      e.lo = exp_lo(t0, t.g);
+      e.nz = e.lo < t.g.numAtoms ? __ldg(a8u + (size_t)e.lo * 8u + 3u) : 0xFFFFFFFFu;
+      const uint32_t d = t0 - t.g.t0_data;
+      e.a = reg ? fdiv(d, t.g.div) : t0;  // irregular chunks: the generic branch reads t0
+      e.b = reg ? d - e.a * t.g.TAtom : 0u;
+      tab[q] = e;
+      s_hot[q] = is_hot((cb + q) / t.chunk_rows) ? 1 : 0;
     }
     __syncthreads();
+    for (uint32_t m = ce; m > cb;) {
+      m--;
+      const ExpRow e = tab[m - cb];
+      uint32_t top = 0;
+      bool some = false;
+      if (reg) {
+        top = e.a + cc.Qp1 - ((e.b + cc.RmT) >> 31);  // ExpColumn::top_of
+        top = top < 1u ? 1u : top;
+        top = top < t.g.numAtoms ? top : t.g.numAtoms;
+        some = e.lo < top;
+      } else {
+        uint32_t hi;
+        some = exp_hi_real(e.a, L.tau, t.g, hi) && e.lo <= hi;
+        top = some ? hi + 1u : 0u;
+      }
+      if (wid < 7u && some && L.active) {
+        if (top > wtop || e.lo > wlo || top <= wlo) {
+          wlo = wtop = top;
+          xl = xe = atom(top - 1u);
+          W = V = FF{0.0f, 0.0f};
+        }
+        if (!kBack)  // ExpColumn::slide alternates, ExpColumnV::slide does not
+          while (wtop > top && wlo > e.lo) {
+            leave();
+            enter();
+          }
+        while (wtop > top) leave();
+        while (wlo > e.lo) enter();
+      }
+      if (!s_hot[m - cb]) continue;
+      float(*sum)[kWords][32] = s_sum[buf];
+      buf ^= 1u;
+      if (wid < 7u) {
+        sum[ch][0][lane] = W.h;
+        sum[ch][1][lane] = W.l;
+        if (kBack) {
+          sum[ch][kWords - 2][lane] = V.h;
+          sum[ch][kWords - 1][lane] = V.l;
+        }
+      }
+      __syncthreads();  // the other buffer's readers are done, too
+      if (wid == 7u && L.active) {
+        const bool data = some && e.nz < top;
+        FF Wr[7];
+#pragma unroll
+        for (int c = 0; c < 7; c++) Wr[c] = FF{sum[c][0][lane], sum[c][1][lane]};
+        float F32 = 0.0f;
+        const bool t1 = data && fstat_fast(Wr, F32);
+        if (!kBack) {
+          double Wd[7] = {0, 0, 0, 0, 0, 0, 0};
+          if (data && !(t1 && F32 < lse.skip)) {
+#pragma unroll
+            for (int c = 0; c < 7; c++) Wd[c] = (double)Wr[c].h + (double)Wr[c].l;
+          }
+          lse.cell(data, Wd, t1, F32);
+        } else {
+          const DiffWeights w(t, k, temp, lnZ1, lnZ2, gB, gS);
+          float Gf[7] = {0, 0, 0, 0, 0, 0, 0};
+          FF p1{0.0f, 0.0f};
+          if (data && !(t1 && F32 < skip)) {
+            FF Vr[7];
+#pragma unroll
+            for (int c = 0; c < 7; c++)
+              Vr[c] = FF{sum[c][kWords - 2][lane], sum[c][kWords - 1][lane]};
+            const DiffGrad grad(w, temp);
+            if (grad.cell(Wr, Vr, Gf, dtw)) p1 = power.at(L, top - e.lo);
+          }
+          const uint32_t c = m / t.chunk_rows;
+          float *scr = scratch + t.scr_off +
+                       ((size_t)(cg * t.n_chunk + c) * t.chunk_rows + (m - c * t.chunk_rows)) *
+                           (TCW_DIFF_SLOTS * 32u) +
+                       lane;
+#pragma unroll
+          for (int c7 = 0; c7 < 7; c7++) scr[32 * c7] = Gf[c7];
+          scr[32 * 7] = p1.h;
+          scr[32 * 8] = p1.l;
+        }
+      }
+    }
+    ce = cb;
+  }
+  if (wid < 7u) return;
+  if (kBack) {
+    add_grad_tau(L, dtw, grad_tau + 2u * k);
+  } else {
+    // the group's hot cells are one partial, its other hot tiles' are empty
+    const DiffPartial p = lse.merge();
+    for (uint32_t c = lane; c < t.n_chunk; c += 32u)
+      if (is_hot(c))
+        parts[t.part_off + (size_t)cg * t.n_chunk + c] =
+            c == c0 ? p : DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
+  }
+}
+
+// The transposed recurrence over one 64-atom segment of one column group, in
+// double-word FP32, from the adjoint sources of the rows in the group's
+// weighted chunks.  kEnds: leaves H at the segment's end, started from zero,
+// in `cend`; else starts from the ends below and adds every atom's sum over
+// the warp's columns to the gradient.
+template <bool kEnds>
+__global__ void __launch_bounds__(kDiffBlock)
+    diff_atoms_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
+                      const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
+                      const ColConsts *__restrict__ cols, const float *__restrict__ need,
+                      double temp, const double *__restrict__ lnZ1,
+                      const double *__restrict__ lnZ2, const double *__restrict__ gB,
+                      const double *__restrict__ gS, const float *__restrict__ scratch,
+                      float *__restrict__ cend, double *__restrict__ grad_atoms) {
+  DiffLane L;
+  const uint32_t k = list[blockIdx.y];
+  L.t = T[k];
+  const DiffTemplate &t = L.t;
+  const uint32_t wi = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+  const uint32_t cg = wi / t.n_aseg, as = wi % t.n_aseg;
+  if (cg >= t.n_cg) return;
+  // the group's weighted chunks: first and last
+  uint32_t c0 = 0xFFFFFFFFu, c1 = 0;
+  {
+    const DiffWeights w(t, k, temp, lnZ1, lnZ2, gB, gS);
+    const float *nd = need + t.part_off + (size_t)cg * t.n_chunk;
+    for (uint32_t c = lane; c < t.n_chunk; c += 32u)
+      if (!(nd[c] < w.skip)) {
+        c0 = min(c0, c);
+        c1 = max(c1, c + 1u);
+      }
+    c0 = __reduce_min_sync(0xffffffffu, c0);
+    c1 = __reduce_max_sync(0xffffffffu, c1);
+    if (c0 >= c1) return;
+    L.columns(atoms8, t0s_all, cg);
+    const uint32_t rb = c0 * t.chunk_rows, re = min(t.N_t0, c1 * t.chunk_rows);
+    const uint32_t *t0s = L.t0s;
+    const ColConsts cc = L.consts(cols);
     // one past the window end of row m (the window start for empty windows:
     // removal right after injection), from the integer split on regular
     // rows, else from the real t1
     auto row_end = [&](uint32_t m) -> uint32_t {
       const uint32_t t0 = __ldg(t0s + m);
       const uint32_t lo = exp_lo(t0, t.g);
-      if (exp_row_regular(t0, taumax, t.g)) {
+      if (exp_row_regular(t0, L.taumax, t.g)) {
         const uint32_t dd = t0 - t.g.t0_data;
         const uint32_t a = fdiv(dd, t.g.div), b = dd - a * t.g.TAtom;
-        uint32_t top = a + CV.C.Qp1 - ((b + CV.C.RmT) >> 31);
+        uint32_t top = a + cc.Qp1 - ((b + cc.RmT) >> 31);
         top = top < 1u ? 1u : (top < t.g.numAtoms ? top : t.g.numAtoms);
         return lo < top ? top : lo;
       }
       uint32_t hi;
-      return (exp_hi_real(t0, tau, t.g, hi) && lo <= hi) ? hi + 1u : lo;
+      return (exp_hi_real(t0, L.tau, t.g, hi) && lo <= hi) ? hi + 1u : lo;
     };
-    // atom range of the transposed recurrence: from the first row's window
-    // start to the largest window end of the tile
-    const uint32_t i_begin = exp_lo(__ldg(t0s), t.g);
-    atomicMax(&s_end, active ? row_end(t.N_t0 - 1u) : i_begin);
-    __syncthreads();
-    const uint32_t i_end = s_end;
-    // H in double-word FP32: (A,B) and C decay with r^2, (Fa) and (Fb) with r
+    // the group's atoms: from its first weighted row's window start to the
+    // largest window end
+    const uint32_t i_begin = exp_lo(__ldg(t0s + rb), t.g);
+    const uint32_t i_end =
+        __reduce_max_sync(0xffffffffu, L.active ? row_end(re - 1u) : i_begin);
+    const uint32_t a = max(i_begin, as * kDiffAtomSeg), b = min(i_end, (as + 1u) * kDiffAtomSeg);
+    if (a >= b) return;
+    const ExpConsts kc = cc.consts();
+    const ExpConsts2 kp = exp_consts2(kc);
+    // H: (A,B) and C decay with r^2, (Fa) and (Fb) with r
     const F2 zp{0.0f, 0.0f};
     FF2 H01{zp, zp}, H34{zp, zp}, H56{zp, zp};
     FF H2{0.0f, 0.0f};
-    const ExpConsts &kc = CV.C.k;
-    const ExpConsts2 &kp = CV.C.k2;
-    uint32_t mi = 0, mr = 0;
-    uint32_t lo_next = i_begin;
-    uint32_t end_r = active ? row_end(0) : 0u;
-    const float *sc0 = my_scratch + threadIdx.x;
-    for (uint32_t i = i_begin; i < i_end; i++) {
-      if (active) {
+    float *ends = cend + (t.cend_off + (size_t)cg * t.n_aseg) * kDiffSegFloats + lane;
+    if (!kEnds) {  // H = r^len H + end, segment by segment from the first
+      const uint32_t s0 = i_begin / kDiffAtomSeg;
+      FF R = kc.r1;  // r^64
+#pragma unroll 1
+      for (int q = 0; q < 6; q++) R = ff_mul(R, R);
+      const FF R2 = ff_mul(R, R);
+      const F2 rh0{R2.h, R2.h}, nrh0{-R2.h, -R2.h}, rl0{R2.l, R2.l};
+      const F2 rh1{R.h, R.h}, nrh1{-R.h, -R.h}, rl1{R.l, R.l};
+      for (uint32_t j = s0; j < as; j++) {
+        const float *s = ends + (size_t)j * kDiffSegFloats;
+        H01 = ff2_axpy_dw(FF2{F2{s[0], s[32]}, F2{s[64], s[96]}}, rh0, nrh0, rl0, H01);
+        H2 = ff_axpy_dw(FF{s[128], s[160]}, R2, H2);
+        H34 = ff2_axpy_dw(FF2{F2{s[192], s[224]}, F2{s[256], s[288]}}, rh1, nrh1, rl1, H34);
+        H56 = ff2_axpy_dw(FF2{F2{s[320], s[352]}, F2{s[384], s[416]}}, rh1, nrh1, rl1, H56);
+      }
+    }
+    // the first row whose window starts at or after atom a, and this
+    // column's first row that ends at or after it (earlier ones are removed)
+    uint32_t mi = rb, hiw = re;
+    if (a > i_begin) {
+      while (mi < hiw) {
+        const uint32_t mid = (mi + hiw) >> 1;
+        if (exp_lo(__ldg(t0s + mid), t.g) < a) mi = mid + 1u; else hiw = mid;
+      }
+    }
+    uint32_t mr = rb;
+    hiw = re;
+    if (a > i_begin) {
+      while (mr < hiw) {
+        const uint32_t mid = (mr + hiw) >> 1;
+        if (row_end(mid) < a) mr = mid + 1u; else hiw = mid;
+      }
+    }
+    uint32_t lo_next = mi < re ? exp_lo(__ldg(t0s + mi), t.g) : 0u;
+    uint32_t end_r = mr < re ? row_end(mr) : 0u;
+    const float *scr0 = scratch + t.scr_off + lane;
+    auto sources = [&](uint32_t m) -> const float * {  // NULL: the row carries no weight
+      const uint32_t c = m / t.chunk_rows;
+      if (nd[c] < w.skip) return nullptr;
+      return scr0 + ((size_t)(cg * t.n_chunk + c) * t.chunk_rows + (m - c * t.chunk_rows)) *
+                        (TCW_DIFF_SLOTS * 32u);
+    };
+    for (uint32_t i = a; i < b; i++) {
+      if (L.active) {
         H01 = ff2_scale_dw(kp.rh[0], kp.nrh[0], kp.rl[0], H01);
         H2 = ff_scale_dw(kc.r2, H2);
         H34 = ff2_scale_dw(kp.rh[1], kp.nrh[1], kp.rl[1], H34);
         H56 = ff2_scale_dw(kp.rh[1], kp.nrh[1], kp.rl[1], H56);
-        while (mi < t.N_t0 && lo_next <= i) {
-          const float *scr = sc0 + (size_t)mi * kDiffSlots * kDiffBlock;
-          H01 = ff2_add_x(H01, F2{scr[0], scr[(size_t)1 * kDiffBlock]});
-          H2 = ff_add1(H2, scr[(size_t)2 * kDiffBlock]);
-          H34 = ff2_add_x(H34, F2{scr[(size_t)3 * kDiffBlock], scr[(size_t)4 * kDiffBlock]});
-          H56 = ff2_add_x(H56, F2{scr[(size_t)5 * kDiffBlock], scr[(size_t)6 * kDiffBlock]});
+        while (mi < re && lo_next <= i) {
+          const float *scr = sources(mi);
+          if (scr) {
+            H01 = ff2_add_x(H01, F2{scr[0], scr[32 * 1]});
+            H2 = ff_add1(H2, scr[32 * 2]);
+            H34 = ff2_add_x(H34, F2{scr[32 * 3], scr[32 * 4]});
+            H56 = ff2_add_x(H56, F2{scr[32 * 5], scr[32 * 6]});
+          }
           mi++;
-          if (mi < t.N_t0) lo_next = exp_lo(__ldg(t0s + mi), t.g);
+          if (mi < re) lo_next = exp_lo(__ldg(t0s + mi), t.g);
         }
         while (mr < mi && end_r <= i) {
-          const float *scr = sc0 + (size_t)mr * kDiffSlots * kDiffBlock;
-          const FF p1{scr[(size_t)7 * kDiffBlock], scr[(size_t)8 * kDiffBlock]};
-          const FF p2 = ff_mul(p1, p1);
-          const F2 ph0{p2.h, p2.h}, pl0{p2.l, p2.l}, nph0{-p2.h, -p2.h};
-          const F2 ph1{p1.h, p1.h}, pl1{p1.l, p1.l}, nph1{-p1.h, -p1.h};
-          H01 = ff2_sub_scaled_x(H01, ph0, nph0, pl0, F2{scr[0], scr[(size_t)1 * kDiffBlock]});
-          H2 = ff_sub_scaled_x1(H2, p2, scr[(size_t)2 * kDiffBlock]);
-          H34 = ff2_sub_scaled_x(H34, ph1, nph1, pl1,
-                                 F2{scr[(size_t)3 * kDiffBlock], scr[(size_t)4 * kDiffBlock]});
-          H56 = ff2_sub_scaled_x(H56, ph1, nph1, pl1,
-                                 F2{scr[(size_t)5 * kDiffBlock], scr[(size_t)6 * kDiffBlock]});
+          const float *scr = sources(mr);
+          if (scr) {
+            const FF p1{scr[32 * 7], scr[32 * 8]};
+            const FF p2 = ff_mul(p1, p1);
+            const F2 ph0{p2.h, p2.h}, pl0{p2.l, p2.l}, nph0{-p2.h, -p2.h};
+            const F2 ph1{p1.h, p1.h}, pl1{p1.l, p1.l}, nph1{-p1.h, -p1.h};
+            H01 = ff2_sub_scaled_x(H01, ph0, nph0, pl0, F2{scr[0], scr[32 * 1]});
+            H2 = ff_sub_scaled_x1(H2, p2, scr[32 * 2]);
+            H34 = ff2_sub_scaled_x(H34, ph1, nph1, pl1, F2{scr[32 * 3], scr[32 * 4]});
+            H56 = ff2_sub_scaled_x(H56, ph1, nph1, pl1, F2{scr[32 * 5], scr[32 * 6]});
+          }
           mr++;
-          if (mr < t.N_t0) end_r = row_end(mr);
+          if (mr < re) end_r = row_end(mr);
         }
       }
-      // reduce the warp's columns' contributions to atom i (each warp adds its
-      // own: no block barrier per atom) by recursive halving over 8 channel
-      // slots in double-word arithmetic: at each step a lane keeps half of its
-      // slots, sends the other half to its partner and adds what it receives
-      // (9 double-word additions per lane); lane L ends with channel
-      // (L >> 2) & 7 summed over the warp
+      if (kEnds) continue;
+      // reduce the warp's columns' contributions to atom i by recursive
+      // halving over 8 channel slots in double-word arithmetic: at each step a
+      // lane keeps half of its slots, sends the other half to its partner and
+      // adds what it receives (9 double-word additions per lane); lane L ends
+      // with channel (L >> 2) & 7 summed over the warp
       const bool u16 = (lane & 16u) != 0u, u8 = (lane & 8u) != 0u, u4 = (lane & 4u) != 0u;
       const FF zf{0.0f, 0.0f};
-      const FF slot[8] = {active ? FF{H01.h.x, H01.l.x} : zf, active ? FF{H01.h.y, H01.l.y} : zf,
-                          active ? H2 : zf,                    active ? FF{H34.h.x, H34.l.x} : zf,
-                          active ? FF{H34.h.y, H34.l.y} : zf, active ? FF{H56.h.x, H56.l.x} : zf,
-                          active ? FF{H56.h.y, H56.l.y} : zf, zf};
+      const FF slot[8] = {L.active ? FF{H01.h.x, H01.l.x} : zf,
+                          L.active ? FF{H01.h.y, H01.l.y} : zf,
+                          L.active ? H2 : zf,
+                          L.active ? FF{H34.h.x, H34.l.x} : zf,
+                          L.active ? FF{H34.h.y, H34.l.y} : zf,
+                          L.active ? FF{H56.h.x, H56.l.x} : zf,
+                          L.active ? FF{H56.h.y, H56.l.y} : zf,
+                          zf};
       auto xch = [&](FF send, int d) {
         return FF{__shfl_xor_sync(0xffffffffu, send.h, d), __shfl_xor_sync(0xffffffffu, send.l, d)};
       };
@@ -770,11 +1330,19 @@ __global__ void __launch_bounds__(kDiffBlock, diff_min_blocks(1))
       v = ff_add_dw(v, xch(v, 1));
       const uint32_t ch = (lane >> 2) & 7u;
       if ((lane & 3u) == 0u && ch < 7u && i < t.g.numAtoms) {
-        const double a = (double)v.h + (double)v.l;
-        if (a != 0.0) atomicAdd(grad_atoms + (t.atom_off + i) * 7u + ch, a);
+        const double x = (double)v.h + (double)v.l;
+        if (x != 0.0) atomicAdd(grad_atoms + (t.atom_off + i) * 7u + ch, x);
       }
     }
-    __syncthreads();
+    if (kEnds) {
+      // a first segment that starts inside its 64 atoms ends at the same
+      // atom as a whole one: joins decay by r^64 from end to end
+      float *o = ends + (size_t)as * kDiffSegFloats;
+      const float v[14] = {H01.h.x, H01.h.y, H01.l.x, H01.l.y, H2.h,    H2.l,    H34.h.x,
+                           H34.h.y, H34.l.x, H34.l.y, H56.h.x, H56.h.y, H56.l.x, H56.l.y};
+#pragma unroll
+      for (int f = 0; f < 14; f++) o[32 * f] = v[f];
+    }
   }
 }
 
@@ -953,35 +1521,41 @@ __global__ void __launch_bounds__(kScanBlock)
   }
 }
 
-__global__ void diff_finalize_kernel(const DiffTemplate *__restrict__ T, uint32_t n_templates,
-                                     const DiffPartial *__restrict__ parts, double temp,
-                                     double *__restrict__ lnB, double *__restrict__ soft) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per template: its partials brought to their maximum and added.
+__global__ void __launch_bounds__(128)
+    diff_finalize_kernel(const DiffTemplate *__restrict__ T, uint32_t n_templates,
+                         const DiffPartial *__restrict__ parts, double temp,
+                         double *__restrict__ lnB, double *__restrict__ soft) {
+  const uint32_t k = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
   if (k >= n_templates) return;
   const DiffTemplate t = T[k];
-  double m1 = -INFINITY, s1 = 0.0, m2 = -INFINITY, s2 = 0.0;
-  for (uint32_t p = 0; p < t.n_parts; p++) {
-    const DiffPartial q = parts[t.part_off + p];
-    lse_merge(m1, s1, q.m1, q.s1);
-    lse_merge(m2, s2, q.m2, q.s2);
+  double m1 = -INFINITY, m2 = -INFINITY, s1 = 0.0, s2 = 0.0;
+  for (uint32_t p = lane; p < t.n_parts; p += 32u) {
+    m1 = fmax(m1, parts[t.part_off + p].m1);
+    m2 = fmax(m2, parts[t.part_off + p].m2);
   }
-  lnB[k] = log(70.0 / ((double)t.N_t0 * (double)t.N_tau)) + m1 + log(s1);
-  soft[k] = temp * (m2 + log(s2));
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, d));
+    m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, d));
+  }
+  for (uint32_t p = lane; p < t.n_parts; p += 32u) {
+    const DiffPartial q = parts[t.part_off + p];
+    if (q.s1 != 0.0) s1 += q.s1 * exp(q.m1 - m1);
+    if (q.s2 != 0.0) s2 += q.s2 * exp(q.m2 - m2);
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    s1 += __shfl_xor_sync(0xffffffffu, s1, d);
+    s2 += __shfl_xor_sync(0xffffffffu, s2, d);
+  }
+  if (lane == 0) {
+    lnB[k] = log(70.0 / ((double)t.N_t0 * (double)t.N_tau)) + m1 + log(s1);
+    soft[k] = temp * (m2 + log(s2));
+  }
 }
 
 }  // namespace
-
-int diff_blocks_per_sm(int pass) {
-  int n = 0;
-  cudaError_t e = pass == 0
-                      ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, diff_fwd_kernel, kDiffBlock, 0)
-                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, diff_bwd_kernel, kDiffBlock, 0);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    n = 1;
-  }
-  return n > 0 ? n : 1;
-}
 
 int rect_diff_blocks_per_sm(int pass) {
   int n = 0;
@@ -996,20 +1570,69 @@ int rect_diff_blocks_per_sm(int pass) {
   return n > 0 ? n : 1;
 }
 
-cudaError_t launch_diff(int pass, const DiffLaunch &L, cudaStream_t stream) {
-  if (L.n_items) {
-    if (pass == 0) {
-      diff_repack_kernel<<<L.n_exp, 256, 0, stream>>>(L.T, L.exp_list, L.atoms, L.atoms8);
-      diff_fwd_kernel<<<L.n_blocks, kDiffBlock, 0, stream>>>(L.T, L.items, L.n_items, L.counter,
-                                                             L.atoms8, L.t0s, L.temp, L.parts);
-    } else {
-      diff_repack_kernel<<<L.n_exp, 256, 0, stream>>>(L.T, L.exp_list, L.atoms, L.atoms8);
-      diff_bwd_kernel<<<L.n_blocks, kDiffBlock, 0, stream>>>(
-          L.T, L.items, L.n_items, L.counter, L.atoms8, L.t0s, L.temp, L.lnZ1, L.lnZ2, L.gB,
-          L.gS, L.scratch, L.scratch_rows, L.grad_atoms, L.grad_tau);
-    }
-    const cudaError_t e = cudaGetLastError();
+// `side`: a second stream for diff_hot_kernel, whose few long blocks run beside
+// the tiles that need no whole walk; fork and join are the caller's events.
+cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, uint32_t n_groups,
+                        cudaStream_t stream, cudaStream_t side, cudaEvent_t fork,
+                        cudaEvent_t join) {
+  cudaError_t e = cudaSuccess;
+  if (L.n_exp) {
+    e = cudaFuncSetAttribute(pass == 0 ? (const void *)diff_hot_kernel<false>
+                                       : (const void *)diff_hot_kernel<true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kHotAtoms * 28u));
     if (e != cudaSuccess) return e;
+    // repacked rows (grid row 0) and column constants (one grid row per 256)
+    const dim3 prep(L.n_exp < 65535u ? L.n_exp : 65535u, 1u + (L.max_cols + 255u) / 256u);
+    diff_prep_kernel<<<prep, 256, 0, stream>>>(L.T, L.exp_list, L.n_exp, L.atoms, L.atoms8,
+                                               L.cols);
+    for (uint32_t q = 0; q < n_groups; q++) {
+      const DiffGroup &g = groups[q];
+      const uint32_t *list = L.exp_list + g.y0;
+      const dim3 tiles((g.max_tiles + 3u) / 4u, g.ny), segs((g.max_segs + 3u) / 4u, g.ny);
+      const dim3 aseg((g.max_aseg + 3u) / 4u, g.ny), hot(g.max_cg, g.ny);
+      // atoms that diff_hot_kernel stages in shared memory (28 bytes each)
+      const uint32_t smem_atoms = g.max_atoms < kHotAtoms ? g.max_atoms : kHotAtoms;
+      if (g.max_segs)
+        diff_seg_kernel<false><<<segs, kDiffBlock, 0, stream>>>(
+            L.T, list, L.atoms8, L.t0s, L.cols, nullptr, L.temp, nullptr, nullptr, nullptr,
+            nullptr, L.seg);
+      diff_est_kernel<<<tiles, kDiffBlock, 0, stream>>>(L.T, list, L.atoms8, L.t0s, L.cols, L.seg,
+                                                        L.need, L.est);
+      if ((e = cudaEventRecord(fork, stream)) != cudaSuccess ||
+          (e = cudaStreamWaitEvent(side, fork, 0)) != cudaSuccess)
+        return e;
+      if (pass == 0) {
+        diff_hot_kernel<false><<<hot, 256, (size_t)smem_atoms * 28u, side>>>(
+            L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, nullptr, nullptr, nullptr,
+            nullptr, nullptr, nullptr, L.parts, smem_atoms);
+        diff_fwd_kernel<<<tiles, kDiffBlock, 0, stream>>>(L.T, list, L.atoms8, L.t0s, L.cols,
+                                                          L.seg, L.need, L.est, L.temp, L.parts);
+      } else {
+        diff_hot_kernel<true><<<hot, 256, (size_t)smem_atoms * 28u, side>>>(
+            L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
+            L.scratch, L.grad_tau, nullptr, smem_atoms);
+        if (g.max_segs)  // (over the window sums, which nothing reads any more)
+          diff_seg_kernel<true><<<segs, kDiffBlock, 0, stream>>>(
+              L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
+              L.seg);
+        diff_src_kernel<<<tiles, kDiffBlock, 0, stream>>>(
+            L.T, list, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
+            L.scratch, L.grad_tau);
+      }
+      if ((e = cudaEventRecord(join, side)) != cudaSuccess ||
+          (e = cudaStreamWaitEvent(stream, join, 0)) != cudaSuccess)
+        return e;
+      if (pass == 1) {
+        diff_atoms_kernel<true><<<aseg, kDiffBlock, 0, stream>>>(
+            L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
+            L.scratch, L.cend, L.grad_atoms);
+        diff_atoms_kernel<false><<<aseg, kDiffBlock, 0, stream>>>(
+            L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
+            L.scratch, L.cend, L.grad_atoms);
+      }
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+    }
   }
   if (L.n_rect_items) {
     if (pass == 0) {
@@ -1020,7 +1643,7 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, cudaStream_t stream) {
       rect_diff_kernel<1><<<L.n_rect_blocks, kDiffBlock, 0, stream>>>(
           L.T, L.rect_items, L.n_rect_items, L.rect_counter, L.atoms, L.t0s, L.temp, nullptr,
           L.lnZ1, L.lnZ2, L.gB, L.gS, L.D64);
-      cudaError_t e = cudaGetLastError();
+      e = cudaGetLastError();
       if (e != cudaSuccess) return e;
       rect_diff_scan_kernel<<<L.n_rect, kScanBlock, 0, stream>>>(L.T, L.rect_list, L.D64,
                                                                  L.grad_atoms);
@@ -1034,7 +1657,7 @@ cudaError_t launch_diff_finalize(const DiffTemplate *T, uint32_t n_templates,
                                  const DiffPartial *parts, double temp, double *lnB, double *soft,
                                  cudaStream_t stream) {
   if (n_templates == 0) return cudaSuccess;
-  diff_finalize_kernel<<<(n_templates + 127u) / 128u, 128, 0, stream>>>(T, n_templates, parts,
+  diff_finalize_kernel<<<(n_templates + 3u) / 4u, 128, 0, stream>>>(T, n_templates, parts,
                                                                          temp, lnB, soft);
   return cudaGetLastError();
 }

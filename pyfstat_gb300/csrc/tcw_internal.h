@@ -221,46 +221,68 @@ cudaError_t launch_posteriors(const TemplateDev *d_T, const float *d_Fmn, void *
                               uint32_t N_tau, cudaStream_t stream);
 
 // ---------------------------------------------------------------- differentiable path
-// One template with a continuous tau grid (tcw_diff.cu); rectangular
-// templates own, in the backward pass, the difference rows of their atom
-// gradient at p_off: (numAtoms + 1) rows of 8 doubles.
+// One template with a continuous tau grid (tcw_diff.cu).  Exponential
+// templates are tiled by 32 tau columns x chunk_rows t0 rows (n_cg x n_chunk
+// tiles, tile = cg * n_chunk + chunk); rectangular templates own, in the
+// backward pass, the difference rows of their atom gradient at p_off:
+// (numAtoms + 1) rows of 8 doubles.
 struct DiffTemplate {
   uint64_t atom_off, t0_off;
   Geom g;
   uint32_t N_t0, N_tau;
   double tau_min, tau_max;
-  uint32_t part_off, n_parts;
+  uint32_t part_off, n_parts;  // partials of this template (exp: one per tile)
   uint32_t window, pad;
   uint64_t p_off;
+  uint32_t n_cg, n_chunk, chunk_rows;
+  uint32_t g_shift, g_nseg, n_aseg;  // segment sums; atom segments of the transposed recurrence
+  uint64_t col_off;   // column constants
+  uint64_t seg_off;   // segment sums, in 32-lane blocks of one segment
+  uint64_t scr_off;   // backward: adjoint sources, in floats
+  uint64_t cend_off;  // backward: recurrence ends, in 32-lane blocks
 };
-// A tile: columns [n0, n1) (at most 128) of one template, all rows.
+// A tile of rectangular windows: rows [n0, n1) (at most 128), all columns.
 struct DiffItem {
   uint32_t tmpl, part, n0, n1;
 };
-// Per-tile online log-sum-exp pairs of F and of 2F/T.
-// floats per column and t0 row in the backward pass's per-block scratch
+// Adjoint sources of one cell in the backward pass's scratch (7 channels and
+// r^L as a float pair) and atoms per segment of the transposed recurrence.
 #define TCW_DIFF_SLOTS 9u
+constexpr uint32_t kDiffAtomSeg = 64u;
+// Floats of one 32-column segment: window sums (forward), with their
+// tau derivatives (backward).
+constexpr uint32_t kDiffSegFloats = 14u * 32u;
+constexpr uint32_t kDiffSegFloatsV = 28u * 32u;
 
 struct DiffPartial {
   double m1, s1, m2, s2;
 };
+// Exponential templates [y0, y0 + ny) of exp_list with workspaces of their
+// own: a backward pass runs in groups that bound the scratch.
+struct DiffGroup {
+  uint32_t y0, ny;
+  // most column groups / tiles / segment items / atom segments of one template
+  uint32_t max_cg, max_tiles, max_segs, max_aseg, max_atoms;
+  uint64_t seg_floats, scr_floats, cend_floats;
+};
 struct DiffLaunch {
   const DiffTemplate *T;
-  const DiffItem *items;
-  uint32_t n_items, n_blocks;
-  uint32_t *counter;
   const float *atoms;
   float *atoms8;                     // exponential templates' atoms in 32-byte rows
                                      // (same row index as `atoms`), written by the launch
   const uint32_t *exp_list;          // the exponential templates' indices
-  uint32_t n_exp;
+  uint32_t n_exp, max_cols;          // their number and the largest N_tau
+  ColConsts *cols;                   // per exponential column, written by the launch
+  float *seg;                        // segment sums
+  float *need;                       // per exp tile: an upper bound of its F
+  uint32_t *est;                     // per template: key of a lower bound of max F (zeroed)
   const uint32_t *t0s;
   double temp;
   DiffPartial *parts;                // pass A output
   const double *lnZ1, *lnZ2, *gB, *gS;  // pass B inputs per template: lnBtSG, softmax2F,
                                         // dL/dlnBtSG, dL/dsoftmax2F
-  float *scratch;                    // pass B/C: n_blocks x scratch_rows x TCW_DIFF_SLOTS x 128 floats
-  uint32_t scratch_rows;
+  float *scratch;                    // backward: adjoint sources of a group's tiles
+  float *cend;                       // backward: recurrence ends of a group
   double *grad_atoms, *grad_tau;     // pass B/C outputs (accumulated; zero them first)
   // rectangular templates: their tiles (rows [n0, n1) of one template),
   // counter and persistent blocks, the list of their template indices and
@@ -273,8 +295,9 @@ struct DiffLaunch {
   double *D64;
 };
 int rect_diff_blocks_per_sm(int pass);
-int diff_blocks_per_sm(int pass);
-cudaError_t launch_diff(int pass, const DiffLaunch &L, cudaStream_t stream);
+cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, uint32_t n_groups,
+                        cudaStream_t stream, cudaStream_t side, cudaEvent_t fork,
+                        cudaEvent_t join);
 // Failed device-side debug checks per translation unit (TCW_DEBUG_CHECKS).
 unsigned int dcheck_failures_kernels();
 unsigned int dcheck_failures_diff();

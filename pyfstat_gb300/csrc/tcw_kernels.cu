@@ -24,6 +24,7 @@
 #include <stdint.h>
 
 #include "../../include/tcw_b200.h"
+#include "tcw_exp_walk.cuh"
 #include "tcw_internal.h"
 
 namespace tcw {
@@ -489,101 +490,6 @@ struct MapSink {
 // its own shared-memory slots (no block barrier) and every cell takes the
 // division-free window end of ExpColumn; otherwise the warp runs
 // exp_column2's generic index arithmetic.  Both give identical results.
-constexpr uint32_t kExpRowTab = 128;
-
-// The row-table walk of one warp's column chunk [mb, me) (regular rows):
-// row tables of kExpRowTab rows built by the warp, then each lane's column
-// slides down them (ExpColumn).  The walk starts at row ms - 1 >= me - 1: the
-// rows of [me, ms) only bring the window sums to the state that a walk from
-// further up would have.
-template <int kPrec, class Sink>
-__device__ __forceinline__ void exp_rows(const TemplateDev &t, const float *__restrict__ a8,
-                                         const uint32_t *__restrict__ t0s, uint32_t mb,
-                                         uint32_t me, uint32_t ms, uint32_t tau, bool active,
-                                         Sink &sink, ExpRow *tab,
-                                         const float *__restrict__ seg) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t *a8u = reinterpret_cast<const uint32_t *>(a8);
-  ExpColumn<kPrec == kPrecFF_F64Det, true> C;
-  C.init(t.g, tau);
-  if (seg && active) {  // the walk's first window, where it is long
-    const uint32_t t0 = __ldg(t0s + ms - 1u);
-    const uint32_t lo = exp_lo(t0, t.g), d = t0 - t.g.t0_data;
-    ExpRow e;
-    e.a = fdiv(d, t.g.div);
-    e.b = d - e.a * t.g.TAtom;
-    const uint32_t top = min(max(C.top_raw(e), 1u), t.g.numAtoms);
-    if (lo < top && top - lo >= (2u << t.g_shift))
-      C.warm_start(a8, t.g, seg, t.g_shift, t.g_nseg, lo, top);
-  }
-  for (uint32_t ce = ms; ce > mb;) {
-    if (ce == me) sink.start();  // the rows of the run-up leave nothing behind
-    const uint32_t floor = ce > me ? me : mb;
-    const uint32_t cb = ce - floor > kExpRowTab ? ce - kExpRowTab : floor;
-    __syncwarp();
-    uint32_t t0min = 0xFFFFFFFFu;
-    for (uint32_t r = lane; r < ce - cb; r += 32u) {
-      const uint32_t t0 = __ldg(t0s + cb + r);
-      t0min = min(t0min, t0);
-      ExpRow e;
-      e.lo = exp_lo(t0, t.g);
-      e.nz = e.lo < t.g.numAtoms ? __ldg(a8u + (size_t)e.lo * 8u + 3u) : 0xFFFFFFFFu;
-      const uint32_t d = t0 - t.g.t0_data;
-      e.a = fdiv(d, t.g.div);
-      e.b = d - e.a * t.g.TAtom;
-      tab[r] = e;
-    }
-    __syncwarp();
-    // the window end grows with t0: if it is clamped at numAtoms for the
-    // chunk's smallest t0, it is for every row of the chunk
-    ExpRow e0;
-    const uint32_t d0 = __reduce_min_sync(0xffffffffu, t0min) - t.g.t0_data;
-    e0.a = fdiv(d0, t.g.div);
-    e0.b = d0 - e0.a * t.g.TAtom;
-    const bool clamped = __all_sync(0xffffffffu, !active || C.top_raw(e0) >= t.g.numAtoms);
-    // window starts that never grow along the walk (t0 non-decreasing in m)
-    bool mono = true;
-    for (uint32_t r = lane; r + 1u < ce - cb; r += 32u) mono = mono && tab[r].lo <= tab[r + 1u].lo;
-    mono = __all_sync(0xffffffffu, mono);
-    if (active) {
-      if (clamped && mono) {
-        // the rows before the first window with an atom, that row, then the
-        // steady rows (row_steady's conditions hold for all of them; after
-        // the first window with data, row_steady_data's too)
-        uint32_t m = ce;
-        while (m > cb) {
-          m--;
-          const ExpRow &e = tab[m - cb];
-          C.row_clamped(a8, t.g, e, m, sink);
-          if (e.lo < t.g.numAtoms) break;
-        }
-        // once a window holds data, every later (lower-starting) one does
-        while (m > cb) {
-          m--;
-          const ExpRow &e = tab[m - cb];
-          C.row_steady(a8, t.g, e, m, sink);
-          if (e.nz < t.g.numAtoms) break;
-        }
-        while (m > cb) {
-          m--;
-          C.row_steady_data(a8, t.g, tab[m - cb], m, sink);
-        }
-      } else if (clamped) {
-        for (uint32_t m = ce; m > cb;) {
-          m--;
-          C.row_clamped(a8, t.g, tab[m - cb], m, sink);
-        }
-      } else {
-        for (uint32_t m = ce; m > cb;) {
-          m--;
-          C.row(a8, t.g, tab[m - cb], m, sink);
-        }
-      }
-    }
-    ce = cb;
-  }
-}
-
 template <bool kWrite, int kPrec>
 __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *__restrict__ atoms,
                          const float *__restrict__ atoms8,
@@ -642,7 +548,9 @@ __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *_
   }
   const float *seg =
       t.g_nseg ? G + (t.g_off + (size_t)(n >> 5) * t.g_nseg) * kSegFloats + lane : nullptr;
-  exp_rows<kPrec>(t, a8, t0s, mb, me, ms, tau, active, sink, tab, seg);
+  ExpColumn<kPrec == kPrecFF_F64Det, true> C;
+  C.init(t.g, tau);
+  exp_rows(C, t.g, t.g_shift, t.g_nseg, a8, t0s, mb, me, ms, active, sink, tab, seg);
   if (active) red.row_to_index(t.N_tau, n);
 }
 
