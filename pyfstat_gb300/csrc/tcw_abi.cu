@@ -1135,9 +1135,9 @@ int tcw_plan_run_timed(tcw_handle *h, tcw_plan *p, const float *d_atoms, tcw_res
 // Validates descriptors, uploads descriptors, tiles and grids into the
 // handle's workspace; returns the layout of what follows them.
 struct DiffSetup {
-  size_t o_T, o_items, o_parts, o_t0, o_cnt, o_est, o_rlist, o_D64, o_elist, o_A8;
+  size_t o_T, o_parts, o_t0, o_est, o_rlist, o_ident, o_RT, o_P, o_B64, o_D64, o_elist, o_A8;
   size_t o_cols, o_seg, o_need, o_scratch, o_cend, total;
-  uint32_t n_rect_items, n_rect_blocks, n_rect, n_exp, max_cols;
+  uint32_t n_rect, max_rect_tiles, max_rect_atoms, n_exp, max_cols;
   uint64_t p_rows;
   std::vector<DiffGroup> groups;
 };
@@ -1197,9 +1197,10 @@ static int diff_prepare(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n,
                         const uint32_t *t0s, uint64_t n_t0s, int pass, DiffSetup &S) {
   if (!desc || n == 0 || !t0s) return set_err(h, TCW_ERR_INVALID_ARG, "empty template list");
   std::vector<DiffTemplate> T;
-  std::vector<DiffItem> ritems;
-  std::vector<uint32_t> rlist, elist;
-  uint64_t p_rows = 0, atom_rows = 0, n_cols = 0, n_tiles = 0;
+  std::vector<TemplateDev> RT;
+  std::vector<uint32_t> rlist, elist, ident;
+  uint64_t p_rows = 0, atom_rows = 0, n_cols = 0, n_tiles = 0, b_rows = 0, row_groups = 0;
+  S.max_rect_tiles = S.max_rect_atoms = 0;
   uint64_t seg_floats = 0, scr_floats = 0, cend_floats = 0;
   uint32_t max_cols = 0;
   try {
@@ -1233,13 +1234,19 @@ static int diff_prepare(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n,
       t.tau_min = d.tau_min;
       t.tau_max = d.tau_max;
       t.window = rect ? (uint32_t)TCW_WINDOW_RECT : (uint32_t)TCW_WINDOW_EXP;
-      if (rect) {  // tiles of 128 t0 rows, all columns; parts are shifted past the exp ones below
-        t.part_off = (uint32_t)ritems.size();
-        for (uint32_t m0 = 0; m0 < d.N_t0; m0 += 128u)
-          ritems.push_back(DiffItem{k, (uint32_t)ritems.size(), m0, std::min(d.N_t0, m0 + 128u)});
-        t.n_parts = (uint32_t)ritems.size() - t.part_off;
+      if (rect) {
+        t.n_cg = (d.N_t0 + 31u) / 32u;
+        row_groups += t.n_cg;
         t.p_off = p_rows;
         p_rows += (uint64_t)d.numAtoms + 1u;
+        t.seg_off = b_rows;
+        b_rows += ((uint64_t)d.numAtoms + 31u) / 32u;
+        TemplateDev rt = make_tdev(d.numAtoms, d.TAtom, d.t0_data, TCW_WINDOW_RECT, d.N_t0, d.N_tau);
+        rt.atom_off = t.atom_off;
+        rt.p_off = t.p_off;
+        ident.push_back((uint32_t)RT.size());
+        RT.push_back(rt);
+        S.max_rect_atoms = std::max(S.max_rect_atoms, d.numAtoms);
         rlist.push_back(k);
       } else {
         t.col_off = n_cols;
@@ -1271,40 +1278,48 @@ static int diff_prepare(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n,
       cend_floats = std::max(cend_floats, g.cend_floats);
       y0 = y1;
     }
-    for (uint32_t k : elist) {
-      T[k].part_off = (uint32_t)n_tiles;
-      T[k].n_parts = T[k].n_cg * T[k].n_chunk;
-      n_tiles += T[k].n_parts;
+    // rectangular tiles: as many column chunks per row group as give every
+    // resident warp a tile, at least 16 columns each
+    const uint64_t rchunks =
+        row_groups ? ((uint64_t)h->n_sms * 32u + row_groups - 1u) / row_groups : 1u;
+    for (uint32_t k : rlist) {
+      DiffTemplate &t = T[k];
+      const uint64_t nc = std::max<uint64_t>(1, std::min<uint64_t>(rchunks, (t.N_tau + 15u) / 16u));
+      t.chunk_rows = (uint32_t)((t.N_tau + nc - 1) / nc);
+      t.n_chunk = (t.N_tau + t.chunk_rows - 1u) / t.chunk_rows;
+      S.max_rect_tiles = std::max(S.max_rect_tiles, t.n_cg * t.n_chunk);
     }
-    if (n_tiles + ritems.size() > 0xFFFFFFF0ull)
-      return set_err(h, TCW_ERR_OVERFLOW, "too many tiles");
-    for (DiffItem &it : ritems) it.part += (uint32_t)n_tiles;
-    for (uint32_t k : rlist) T[k].part_off += (uint32_t)n_tiles;
+    for (const std::vector<uint32_t> *l : {&elist, &rlist})
+      for (uint32_t k : *l) {
+        T[k].part_off = (uint32_t)n_tiles;
+        T[k].n_parts = T[k].n_cg * T[k].n_chunk;
+        n_tiles += T[k].n_parts;
+        if (n_tiles > 0xFFFFFFF0ull) return set_err(h, TCW_ERR_OVERFLOW, "too many tiles");
+      }
   } catch (const std::bad_alloc &) {
     return set_err(h, TCW_ERR_ALLOC, "host allocation failed");
   }
-  S.n_rect_items = (uint32_t)ritems.size();
   S.n_rect = (uint32_t)rlist.size();
   S.n_exp = (uint32_t)elist.size();
   S.max_cols = max_cols;
   S.p_rows = p_rows;
-  S.n_rect_blocks = (uint32_t)std::max<uint64_t>(
-      1, std::min<uint64_t>(S.n_rect_items, (uint64_t)rect_diff_blocks_per_sm(pass) * h->n_sms));
   Layout L;
   S.o_T = L.add(sizeof(DiffTemplate) * n);
-  S.o_items = L.add(sizeof(DiffItem) * ritems.size());
   S.o_t0 = L.add(sizeof(uint32_t) * n_t0s);
-  S.o_cnt = L.add(2 * sizeof(uint32_t));
   S.o_est = L.add(sizeof(uint32_t) * n);
   S.o_rlist = L.add(sizeof(uint32_t) * std::max<size_t>(1, rlist.size()));
   S.o_elist = L.add(sizeof(uint32_t) * std::max<size_t>(1, elist.size()));
+  S.o_ident = L.add(sizeof(uint32_t) * ident.size());
+  S.o_RT = L.add(sizeof(TemplateDev) * RT.size());
   const size_t ctl = L.total;
-  S.o_parts = L.add(sizeof(DiffPartial) * (n_tiles + ritems.size()));
+  S.o_parts = L.add(sizeof(DiffPartial) * n_tiles);
   S.o_need = L.add(sizeof(float) * n_tiles);
   S.o_cols = L.add(sizeof(ColConsts) * n_cols);
   S.o_seg = L.add(sizeof(float) * seg_floats);
   S.o_scratch = L.add(sizeof(float) * scr_floats);
   S.o_cend = L.add(sizeof(float) * cend_floats);
+  S.o_P = L.add(sizeof(float) * kPrefixStride * p_rows);
+  S.o_B64 = L.add(sizeof(double) * 8u * b_rows);
   S.o_D64 = pass == 1 ? L.add(sizeof(double) * 8u * std::max<uint64_t>(1, p_rows)) : 0;
   // the exponential templates' atoms in 32-byte rows, at their own row index
   S.o_A8 = S.n_exp ? L.add(sizeof(float) * 8u * std::max<uint64_t>(1, atom_rows)) : 0;
@@ -1314,12 +1329,13 @@ static int diff_prepare(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n,
   rc = ensure_stage(h, ctl);
   if (rc) return rc;
   memcpy(h->h_stage + S.o_T, T.data(), sizeof(DiffTemplate) * n);
-  if (!ritems.empty())
-    memcpy(h->h_stage + S.o_items, ritems.data(), sizeof(DiffItem) * ritems.size());
   memcpy(h->h_stage + S.o_t0, t0s, sizeof(uint32_t) * n_t0s);
-  memset(h->h_stage + S.o_cnt, 0, 2 * sizeof(uint32_t));
   memset(h->h_stage + S.o_est, 0, sizeof(uint32_t) * n);
-  if (!rlist.empty()) memcpy(h->h_stage + S.o_rlist, rlist.data(), sizeof(uint32_t) * rlist.size());
+  if (!rlist.empty()) {
+    memcpy(h->h_stage + S.o_rlist, rlist.data(), sizeof(uint32_t) * rlist.size());
+    memcpy(h->h_stage + S.o_ident, ident.data(), sizeof(uint32_t) * ident.size());
+    memcpy(h->h_stage + S.o_RT, RT.data(), sizeof(TemplateDev) * RT.size());
+  }
   if (!elist.empty()) memcpy(h->h_stage + S.o_elist, elist.data(), sizeof(uint32_t) * elist.size());
   TCW_CUDA(h, cudaMemcpyAsync(h->d_ws, h->h_stage, ctl, cudaMemcpyHostToDevice, h->stream));
   TCW_CUDA(h, cudaEventRecord(h->stage_ev, h->stream));
@@ -1341,12 +1357,14 @@ static DiffLaunch diff_launch(tcw_handle *h, const DiffSetup &S, const float *d_
   L.est = reinterpret_cast<uint32_t *>(h->d_ws + S.o_est);
   L.scratch = reinterpret_cast<float *>(h->d_ws + S.o_scratch);
   L.cend = reinterpret_cast<float *>(h->d_ws + S.o_cend);
-  L.rect_items = reinterpret_cast<const DiffItem *>(h->d_ws + S.o_items);
-  L.n_rect_items = S.n_rect_items;
-  L.n_rect_blocks = S.n_rect_blocks;
-  L.rect_counter = reinterpret_cast<uint32_t *>(h->d_ws + S.o_cnt) + 1;
   L.rect_list = reinterpret_cast<const uint32_t *>(h->d_ws + S.o_rlist);
   L.n_rect = S.n_rect;
+  L.rect_ident = reinterpret_cast<const uint32_t *>(h->d_ws + S.o_ident);
+  L.rect_T = reinterpret_cast<const TemplateDev *>(h->d_ws + S.o_RT);
+  L.max_rect_tiles = S.max_rect_tiles;
+  L.max_rect_atoms = S.max_rect_atoms;
+  L.P = reinterpret_cast<float *>(h->d_ws + S.o_P);
+  L.B64 = reinterpret_cast<double *>(h->d_ws + S.o_B64);
   L.D64 = S.o_D64 ? reinterpret_cast<double *>(h->d_ws + S.o_D64) : nullptr;
   L.atoms8 = S.o_A8 ? reinterpret_cast<float *>(h->d_ws + S.o_A8) : nullptr;
   L.exp_list = reinterpret_cast<const uint32_t *>(h->d_ws + S.o_elist);

@@ -49,14 +49,20 @@
 // The window-sum factor e^(-k (t_lo - t0)/tau) is left out everywhere: F does
 // not depend on it, so neither do g, dF/dW (in this frame) or dF/dtau.
 //
-// Rectangular windows (rect_diff_kernel): one thread per t0 row, the tau
-// columns in ascending order with FP64 running sums (the window end only
-// grows with tau, as in the reference's running sums, Rect.cu:75-91); the
-// sums of a window do not depend on tau between boundaries, so dL/dtau = 0.
-// The atom gradient is scattered as a difference array: +sum_n G(m, n) at
-// the row's start index lo(m), -G(m, n) at end(m, n) + 1 (consecutive cells
-// with the same end merged), then one prefix scan per template
-// (rect_diff_scan_kernel) gives dL/dx(i) = sum_{j <= i} D(j).
+// Rectangular windows: tiles of 32 t0 rows x a chunk of tau columns, one warp
+// per tile, one row per lane, the columns in ascending order (the window end
+// only grows with tau, as in the reference's running sums, Rect.cu:75-91).
+// rect_est_kernel bounds F per tile in FP32 from the map path's prefix rows;
+// rect_diff_kernel takes the tiles that may carry weight, with FP64 sums
+// (32-atom block sums, then single atoms) brought up to date only at cells
+// that do.  The sums of a window do not depend on tau between boundaries, so
+// dL/dtau = 0; the atom gradient is scattered as a difference array:
+// +sum_n G(m, n) at the row's start index lo(m), -G(m, n) at end(m, n) + 1
+// (consecutive cells with the same end merged), then one prefix scan per
+// template (rect_diff_scan_kernel) gives dL/dx(i) = sum_{j <= i} D(j).
+// Measured (7 templates of 1499 atoms, 777 x 611 cells, signal): forward and
+// backward 6.47 -> 0.64 ms (before, one thread per row over all columns and
+// FP64 F in every cell).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -127,42 +133,17 @@ __device__ __forceinline__ F64Cell fstat64(const double W[7], bool passes = fals
 // finite-difference checks, where FP32 rounding of the terms would show).
 // Terms below e^-60 of the running maximum are skipped: the sum is >= 1, so
 // even 1e9 of them change it by < 1e-17.
-__device__ __forceinline__ void lse_add(double &m, double &s, double v) {
+// `k`: so many terms v.
+__device__ __forceinline__ void lse_add(double &m, double &s, double v, double k = 1.0) {
   if (v > m) {
-    s = s * exp(m - v) + 1.0;
+    s = s * exp(m - v) + k;
     m = v;
   } else if (v - m > -60.0) {
-    s += exp(v - m);
+    s += k * exp(v - m);
   }
 }
 
-__device__ __forceinline__ void lse_merge(double &m, double &s, double m2, double s2) {
-  if (s2 == 0.0) return;
-  if (s == 0.0) {
-    m = m2;
-    s = s2;
-    return;
-  }
-  const double M = fmax(m, m2);
-  s = s * exp(m - M) + s2 * exp(m2 - M);
-  m = M;
-}
-
-// Blocks of 128 threads (rectangular windows: one t0 row per thread;
-// exponential ones: one tile per warp).
-constexpr int kDiffBlock = 128;
-
-// Minimum resident blocks per SM asked of the register allocator, per pass
-// of the rectangular kernel (1 leaves the allocation to ptxas).
-#ifndef TCW_DIFF_MIN_BLOCKS_FWD
-#define TCW_DIFF_MIN_BLOCKS_FWD 5
-#endif
-#ifndef TCW_DIFF_MIN_BLOCKS_BWD
-#define TCW_DIFF_MIN_BLOCKS_BWD 1
-#endif
-constexpr int diff_min_blocks(int pass) {
-  return pass == 0 ? TCW_DIFF_MIN_BLOCKS_FWD : TCW_DIFF_MIN_BLOCKS_BWD;
-}
+constexpr int kDiffBlock = 128;  // four warps, one tile each
 
 // Order-preserving key of a float for atomicMax; 0 is below every key.
 __device__ __forceinline__ uint32_t float_key(float f) {
@@ -609,9 +590,9 @@ struct DiffLse {
   __device__ __forceinline__ DiffLse(double temp, float bound)
       : m1(-INFINITY), s1(0.0), m2(-INFINITY), s2(0.0), twoT(2.0 / temp), skip(bound),
         skip0(bound) {}
-  __device__ __forceinline__ void add(double F) {
-    lse_add(m1, s1, F);
-    lse_add(m2, s2, F * twoT);
+  __device__ __forceinline__ void add(double F, double k = 1.0) {
+    lse_add(m1, s1, F, k);
+    lse_add(m2, s2, F * twoT, k);
     skip = fmaxf((float)(m1 - 62.0), skip0);
   }
   __device__ __forceinline__ void cell(bool data, const double W[7], bool t1, float F32) {
@@ -1348,13 +1329,144 @@ __global__ void __launch_bounds__(kDiffBlock)
 
 // ------------------------------------------------------------ rectangular windows
 
-// Inclusive end index of a rectangular window for a real tau (the
-// reference's i_t1, Rect.cu:54-69, with t1 = t0 + tau real); t0 >= t0_data -
-// TAtom/2 (checked on the host), so the quotient is >= -1.
-__device__ __forceinline__ uint32_t rect_end_real(uint32_t t0, double tau, const Geom &g) {
-  const double d = (double)t0 + tau - (double)g.t0_data + (double)g.half;
-  const double q = floor(d / (double)g.TAtom) - 1.0;
-  return q < 0.0 ? 0u : (q >= (double)(g.numAtoms - 1u) ? g.numAtoms - 1u : (uint32_t)q);
+// FP64 sums of aligned 32-atom blocks (8 doubles per block, 7 used).
+__global__ void __launch_bounds__(256)
+    rect_blocks_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
+                       const float *__restrict__ atoms, double *__restrict__ B64) {
+  const DiffTemplate t = T[list[blockIdx.y]];
+  const uint32_t w = blockIdx.x * 256u + threadIdx.x, b = w >> 3, c = w & 7u;
+  if (b * 32u >= t.g.numAtoms || c == 7u) return;
+  const float *x = atoms + t.atom_off * 7u + c;
+  double s = 0.0;
+  for (uint32_t i = b * 32u; i < min(t.g.numAtoms, b * 32u + 32u); i++)
+    s += (double)__ldg(x + (size_t)i * 7u);
+  B64[(t.seg_off + b) * 8u + c] = s;
+}
+
+// One warp's tile of a rectangular template: this lane's row and its window
+// starts and ends.
+struct RectLane {
+  DiffTemplate t;
+  uint32_t tile, m, nb, ne, lo;
+  bool ok;
+  double t0d;
+  const float *x;
+
+  // false: no such tile
+  __device__ __forceinline__ bool init(const DiffTemplate *T, uint32_t k, uint32_t tl,
+                                       const float *atoms, const uint32_t *t0s_all) {
+    t = T[k];
+    tile = tl;
+    const uint32_t rg = tile / t.n_chunk;
+    if (rg >= t.n_cg) return false;
+    m = rg * 32u + (threadIdx.x & 31u);
+    ok = m < t.N_t0;
+    nb = tile % t.n_chunk * t.chunk_rows;
+    ne = min(t.N_tau, nb + t.chunk_rows);
+    const uint32_t t0 = __ldg(t0s_all + t.t0_off + (ok ? m : t.N_t0 - 1u));
+    t0d = (double)t0;
+    lo = idx_start(t0, t.g);
+    x = atoms + t.atom_off * 7u;
+    return true;
+  }
+  // rect_end_real without its division: the real end's distance from the
+  // data is a sum of exact steps after t0 + tau, so its floor divided as an
+  // integer is the floor of the quotient
+  __device__ __forceinline__ uint32_t end(double tau) const {
+    const double d = t0d + tau - (double)t.g.t0_data + (double)t.g.half;
+    const uint32_t q = fdiv((uint32_t)d, t.g.div);
+    return q < 1u ? 0u : min(q - 1u, t.g.numAtoms - 1u);
+  }
+  // cell(end) for every column of the tile; all lanes call it together
+  template <class Cell>
+  __device__ __forceinline__ void columns(double *s_tau, Cell &&cell) const {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t cb = nb; cb < ne; cb += 32u) {
+      __syncwarp();
+      if (cb + lane < ne) s_tau[lane] = tau_of(t, cb + lane);
+      __syncwarp();
+      const uint32_t ce = min(ne, cb + 32u);
+      if (ok)
+        for (uint32_t n = cb; n < ce; n++) cell(end(s_tau[n - cb]));
+    }
+  }
+};
+
+// Prefix rows of a row's windows (the rectangular map kernel's): FP32 F of
+// the window [lo, e].
+struct RectPrefix {
+  const float *P;
+  float row0[16];
+  __device__ __forceinline__ void init(const RectLane &L, const float *P_all) {
+    P = P_all + L.t.p_off * kPrefixStride;
+    TCW_DCHECK(L.lo <= L.t.g.numAtoms);
+    for (int c = 0; c < 16; c++) row0[c] = __ldg(P + (size_t)L.lo * kPrefixStride + c);
+  }
+  __device__ __forceinline__ void window(uint32_t e, FF2 W[4]) const {
+    float a[16];
+    const float4 *r = reinterpret_cast<const float4 *>(P + (size_t)(e + 1u) * kPrefixStride);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const float4 v = __ldg(r + q);
+      a[4 * q] = v.x;
+      a[4 * q + 1] = v.y;
+      a[4 * q + 2] = v.z;
+      a[4 * q + 3] = v.w;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      W[q].h = sub2(F2{a[2 * q], a[2 * q + 1]}, F2{row0[2 * q], row0[2 * q + 1]});
+      W[q].l = sub2(F2{a[8 + 2 * q], a[9 + 2 * q]}, F2{row0[8 + 2 * q], row0[9 + 2 * q]});
+    }
+  }
+  __device__ __forceinline__ static bool tier1(const FF2 W[4], float &F) {
+    const F2 s0 = add2(W[0].h, W[0].l), s1 = add2(W[1].h, W[1].l);
+    const F2 s2 = add2(W[2].h, W[2].l), s3 = add2(W[3].h, W[3].l);
+    return fstat_fast_sums(s0.x, s0.y, s1.x, s1.y, s2.x, s2.y, s3.x, F);
+  }
+};
+
+// diff_est_kernel's `need` and `est` for rectangular tiles.
+__global__ void __launch_bounds__(kDiffBlock)
+    rect_est_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
+                    const float *__restrict__ atoms, const uint32_t *__restrict__ t0s_all,
+                    const float *__restrict__ P, float *__restrict__ need,
+                    uint32_t *__restrict__ est) {
+  __shared__ double s_tau[kDiffBlock / 32][32];
+  const uint32_t k = list[blockIdx.y], wid = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  RectLane L;
+  if (!L.init(T, k, blockIdx.x * 4u + wid, atoms, t0s_all)) return;
+  RectPrefix R;
+  R.init(L, P);
+  EstSink sink{-INFINITY, -INFINITY};
+  uint32_t prev = 0xFFFFFFFFu;
+  L.columns(s_tau[wid], [&](uint32_t e) {
+    if (e == prev) return;  // the same window
+    prev = e;
+    float F = 2.0f;
+    bool ok = false;
+    if (e >= L.lo) {
+      FF2 W[4];
+      R.window(e, W);
+      ok = RectPrefix::tier1(W, F);
+      if (!ok) {
+        FF w[7];
+        ff2_unpack(W, w);
+        F = fstat_ff<false, true>(w[0], w[1], w[2], w[3], w[4], w[5], w[6], ok);
+      }
+    }
+    sink(0u, F, ok);
+  });
+  float top1 = sink.top, most = sink.most;
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    top1 = fmaxf(top1, __shfl_xor_sync(0xffffffffu, top1, d));
+    most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, d));
+  }
+  if (lane == 0) {
+    need[L.t.part_off + L.tile] = most;
+    if (top1 > -INFINITY) atomicMax(est + k, float_key(top1));
+  }
 }
 
 __device__ __forceinline__ void flush_diff(double *D, uint32_t row, const double v[7], double sgn,
@@ -1365,117 +1477,121 @@ __device__ __forceinline__ void flush_diff(double *D, uint32_t row, const double
     if (v[c] != 0.0) atomicAdd(D + (size_t)row * 8u + c, sgn * v[c]);
 }
 
+// The tiles that may carry weight.  kPass 0: FP64 log-sum-exps of F and 2F/T;
+// 1: the atom gradient's difference rows.  Columns with the same window count
+// together.
 template <int kPass>
-__global__ void __launch_bounds__(kDiffBlock, diff_min_blocks(kPass))
-    rect_diff_kernel(const DiffTemplate *__restrict__ T, const DiffItem *__restrict__ items,
-                     uint32_t n_items, uint32_t *__restrict__ counter,
+__global__ void __launch_bounds__(kDiffBlock)
+    rect_diff_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
                      const float *__restrict__ atoms, const uint32_t *__restrict__ t0s_all,
+                     const float *__restrict__ P, const double *__restrict__ B64,
+                     const float *__restrict__ need, const uint32_t *__restrict__ est,
                      double temp, DiffPartial *__restrict__ parts,
                      const double *__restrict__ lnZ1, const double *__restrict__ lnZ2,
                      const double *__restrict__ gB, const double *__restrict__ gS,
                      double *__restrict__ D64) {
-  __shared__ uint32_t s_item;
-  __shared__ double sh[kDiffBlock / 32][4];
-  for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(counter, 1u);
-    __syncthreads();
-    const uint32_t it = s_item;
-    __syncthreads();
-    if (it >= n_items) break;
-    const DiffItem w = items[it];
-    const DiffTemplate t = T[w.tmpl];
-    const uint32_t m = w.n0 + threadIdx.x;  // this thread's t0 row
-    const bool active = m < w.n1;
-    double m1 = -INFINITY, s1 = 0.0, m2 = -INFINITY, s2 = 0.0;
-    double z1 = 0.0, z2 = 0.0, gb = 0.0, gs = 0.0;
-    if (kPass == 1) {
-      z1 = lnZ1[w.tmpl] - log(70.0 / ((double)t.N_t0 * (double)t.N_tau));
-      z2 = lnZ2[w.tmpl] / temp;
-      gb = gB[w.tmpl];
-      gs = gS[w.tmpl];
-    }
-    if (active) {
-      const float *x = atoms + t.atom_off * 7u;
-      double *D = kPass == 1 ? D64 + t.p_off * 8u : nullptr;
-      const uint32_t t0 = __ldg(t0s_all + t.t0_off + m);
-      const uint32_t lo = idx_start(t0, t.g);
-      double S[7] = {0, 0, 0, 0, 0, 0, 0};
-      double R[7] = {0, 0, 0, 0, 0, 0, 0}, acc[7] = {0, 0, 0, 0, 0, 0, 0};
-      uint32_t next = lo, acc_end = 0xFFFFFFFFu;
-      for (uint32_t n = 0; n < t.N_tau; n++) {
-        const uint32_t end = rect_end_real(t0, tau_of(t, n), t.g);
-        for (; next <= end; next++) {
-          TCW_DCHECK(next < t.g.numAtoms);
-#pragma unroll
-          for (int c = 0; c < 7; c++) S[c] += (double)__ldg(x + (size_t)next * 7u + c);
-        }
-        F64Cell fc{2.0, 0.0, false};
-        if (end >= lo) fc = fstat64(S);
-        const double F = fc.F;
-        if (kPass == 0) {
-          lse_add(m1, s1, F);
-          lse_add(m2, s2, 2.0 * F / temp);
-        } else if (fc.ok) {
-          // dL/dF of this cell (FP32 exponentials: relative 1e-7 on a gradient
-          // term; cells far below the maxima get exactly 0 and are skipped)
-          const double g = gb * (double)exp2f((float)(F - z1) * kLog2eF) +
-                           gs * 2.0 * (double)exp2f((float)(2.0 * F / temp - z2) * kLog2eF);
-          if (g == 0.0) continue;
-          const double A = S[0], B = S[1], C = S[2], iD = fc.iD;
-          const double Fa2 = S[3] * S[3] + S[4] * S[4], Fb2 = S[5] * S[5] + S[6] * S[6];
-          const double re = S[3] * S[5] + S[4] * S[6];
-          double G[7];
-          G[0] = (Fb2 - F * B) * iD;
-          G[1] = (Fa2 - F * A) * iD;
-          G[2] = (2.0 * F * C - 2.0 * re) * iD;
-          G[3] = 2.0 * (B * S[3] - C * S[5]) * iD;
-          G[4] = 2.0 * (B * S[4] - C * S[6]) * iD;
-          G[5] = 2.0 * (A * S[5] - C * S[3]) * iD;
-          G[6] = 2.0 * (A * S[6] - C * S[4]) * iD;
-          if (end != acc_end) {
-            if (acc_end != 0xFFFFFFFFu) flush_diff(D, acc_end + 1u, acc, -1.0, t.g.numAtoms);
-#pragma unroll
-            for (int c = 0; c < 7; c++) acc[c] = 0.0;
-            acc_end = end;
-          }
-#pragma unroll
-          for (int c = 0; c < 7; c++) {
-            acc[c] += g * G[c];
-            R[c] += g * G[c];
-          }
-        }
-      }
-      if (kPass == 1) {
-        if (acc_end != 0xFFFFFFFFu) flush_diff(D, acc_end + 1u, acc, -1.0, t.g.numAtoms);
-        flush_diff(D, lo, R, 1.0, t.g.numAtoms);
-      }
-    }
+  __shared__ double s_tau[kDiffBlock / 32][32];
+  const uint32_t k = list[blockIdx.y], wid = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  RectLane L;
+  if (!L.init(T, k, blockIdx.x * 4u + wid, atoms, t0s_all)) return;
+  const DiffTemplate &t = L.t;
+  DiffPartial *out = kPass == 0 ? parts + t.part_off + L.tile : nullptr;
+  double z1 = 0.0, z2 = 0.0, gb = 0.0, gs = 0.0;
+  float skip0;
+  if (kPass == 0) {
+    skip0 = FwdBounds(est[k]).skip;
+  } else {  // a cell whose weights are below e^-62 in both sums has no gradient
+    z1 = lnZ1[k] - log(70.0 / ((double)t.N_t0 * (double)t.N_tau));
+    z2 = lnZ2[k] / temp;
+    gb = gB[k];
+    gs = gS[k];
+    skip0 = (float)fmin(gb != 0.0 ? z1 - 1e-5 * fabs(z1) - 63.0 : INFINITY,
+                        gs != 0.0 ? 0.5 * temp * (z2 - 1e-5 * fabs(z2) - 62.0) - 1.0 : INFINITY);
+  }
+  if (need[t.part_off + L.tile] < skip0) {
+    if (kPass == 0 && lane == 0) *out = DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
+    return;
+  }
+  RectPrefix R;
+  R.init(L, P);
+  const double *B = B64 + t.seg_off * 8u;
+  double *D = kPass == 1 ? D64 + t.p_off * 8u : nullptr;
+  DiffLse lse(temp, skip0);
+  double S[7] = {0, 0, 0, 0, 0, 0, 0}, Rs[7] = {0, 0, 0, 0, 0, 0, 0};
+  uint32_t next = L.lo, prev = 0xFFFFFFFFu, count = 0;
+  bool weighs = false;   // the current window carries weight
+  F64Cell fc{2.0, 0.0, false};
+  // the columns of the current window, all at once
+  auto finish = [&]() {
+    if (!weighs || count == 0u) return;
     if (kPass == 0) {
+      lse.add(fc.F, (double)count);
+    } else {
+      // dL/dF of the cells (FP32 exponentials: relative 1e-7 on a gradient term)
+      const double F = fc.F;
+      double g = gb * (double)exp2f((float)(F - z1) * kLog2eF) +
+                 gs * 2.0 * (double)exp2f((float)(2.0 * F / temp - z2) * kLog2eF);
+      if (g == 0.0) return;
+      g *= (double)count;
+      const double A = S[0], B2 = S[1], C = S[2], iD = fc.iD;
+      const double Fa2 = S[3] * S[3] + S[4] * S[4], Fb2 = S[5] * S[5] + S[6] * S[6];
+      const double re = S[3] * S[5] + S[4] * S[6];
+      double G[7];
+      G[0] = (Fb2 - F * B2) * iD;
+      G[1] = (Fa2 - F * A) * iD;
+      G[2] = (2.0 * F * C - 2.0 * re) * iD;
+      G[3] = 2.0 * (B2 * S[3] - C * S[5]) * iD;
+      G[4] = 2.0 * (B2 * S[4] - C * S[6]) * iD;
+      G[5] = 2.0 * (A * S[5] - C * S[3]) * iD;
+      G[6] = 2.0 * (A * S[6] - C * S[4]) * iD;
 #pragma unroll
-      for (int d = 16; d > 0; d >>= 1) {
-        const double om1 = __shfl_down_sync(0xffffffffu, m1, d);
-        const double os1 = __shfl_down_sync(0xffffffffu, s1, d);
-        const double om2 = __shfl_down_sync(0xffffffffu, m2, d);
-        const double os2 = __shfl_down_sync(0xffffffffu, s2, d);
-        lse_merge(m1, s1, om1, os1);
-        lse_merge(m2, s2, om2, os2);
+      for (int c = 0; c < 7; c++) {
+        G[c] *= g;
+        Rs[c] += G[c];
       }
-      if ((threadIdx.x & 31u) == 0) {
-        sh[threadIdx.x >> 5][0] = m1;
-        sh[threadIdx.x >> 5][1] = s1;
-        sh[threadIdx.x >> 5][2] = m2;
-        sh[threadIdx.x >> 5][3] = s2;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        for (int k = 1; k < kDiffBlock / 32; k++) {
-          lse_merge(m1, s1, sh[k][0], sh[k][1]);
-          lse_merge(m2, s2, sh[k][2], sh[k][3]);
-        }
-        parts[w.part] = DiffPartial{m1, s1, m2, s2};
-      }
-      __syncthreads();
+      flush_diff(D, prev + 1u, G, -1.0, t.g.numAtoms);
     }
+  };
+  L.columns(s_tau[wid], [&](uint32_t e) {
+    if (e == prev) {
+      count++;
+      return;
+    }
+    finish();
+    prev = e;
+    count = 1u;
+    if (e < L.lo) {  // no atoms: F = 2, no gradient
+      fc = F64Cell{2.0, 0.0, false};
+      weighs = kPass == 0 && !(2.0f < lse.skip);
+      return;
+    }
+    FF2 W[4];
+    float F32 = 0.0f;
+    R.window(e, W);
+    const bool t1 = RectPrefix::tier1(W, F32);
+    weighs = !(t1 && F32 < lse.skip);
+    if (!weighs) return;
+    while (next <= e) {
+      TCW_DCHECK(next < t.g.numAtoms);
+      if ((next & 31u) == 0u && next + 31u <= e) {
+#pragma unroll
+        for (int c = 0; c < 7; c++) S[c] += __ldg(B + (size_t)(next >> 5) * 8u + c);
+        next += 32u;
+      } else {
+#pragma unroll
+        for (int c = 0; c < 7; c++) S[c] += (double)__ldg(L.x + (size_t)next * 7u + c);
+        next++;
+      }
+    }
+    fc = fstat64(S, t1);
+    if (kPass == 1 && !fc.ok) weighs = false;
+  });
+  if (L.ok) finish();
+  if (kPass == 0) {
+    const DiffPartial p = lse.merge();
+    if (lane == 0) *out = p;
+  } else if (L.ok) {
+    flush_diff(D, L.lo, Rs, 1.0, t.g.numAtoms);
   }
 }
 
@@ -1487,9 +1603,9 @@ constexpr int kScanBlock = 256;
 __global__ void __launch_bounds__(kScanBlock)
     rect_diff_scan_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
                           const double *__restrict__ D64, double *__restrict__ grad_atoms) {
-  __shared__ double sh[kScanBlock][7];
+  __shared__ double sh[kScanBlock / 32][7];
   const DiffTemplate t = T[list[blockIdx.x]];
-  const uint32_t n = t.g.numAtoms;
+  const uint32_t n = t.g.numAtoms, lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
   const double *D = D64 + t.p_off * 8u;
   const uint32_t chunk = (n + kScanBlock - 1u) / kScanBlock;
   const uint32_t a0 = min(n, threadIdx.x * chunk), a1 = min(n, a0 + chunk);
@@ -1497,21 +1613,24 @@ __global__ void __launch_bounds__(kScanBlock)
   for (uint32_t i = a0; i < a1; i++)
 #pragma unroll
     for (int c = 0; c < 7; c++) s[c] += D[(size_t)i * 8u + c];
-#pragma unroll
-  for (int c = 0; c < 7; c++) sh[threadIdx.x][c] = s[c];
-  __syncthreads();
-  if (threadIdx.x < 7u) {
-    double run = 0.0;
-    for (int k = 0; k < kScanBlock; k++) {
-      const double v = sh[k][threadIdx.x];
-      sh[k][threadIdx.x] = run;
-      run += v;
-    }
-  }
-  __syncthreads();
+  // exclusive scan of the chunk sums: within the warp, then over the warps
   double run[7];
 #pragma unroll
-  for (int c = 0; c < 7; c++) run[c] = sh[threadIdx.x][c];
+  for (int c = 0; c < 7; c++) {
+    double v = s[c];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const double o = __shfl_up_sync(0xffffffffu, v, d);
+      if (lane >= (uint32_t)d) v += o;
+    }
+    if (lane == 31u) sh[wid][c] = v;
+    const double ex = __shfl_up_sync(0xffffffffu, v, 1);
+    run[c] = lane ? ex : 0.0;
+  }
+  __syncthreads();
+  for (uint32_t w = 0; w < wid; w++)
+#pragma unroll
+    for (int c = 0; c < 7; c++) run[c] += sh[w][c];
   for (uint32_t i = a0; i < a1; i++) {
 #pragma unroll
     for (int c = 0; c < 7; c++) {
@@ -1556,19 +1675,6 @@ __global__ void __launch_bounds__(128)
 }
 
 }  // namespace
-
-int rect_diff_blocks_per_sm(int pass) {
-  int n = 0;
-  cudaError_t e =
-      pass == 0
-          ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rect_diff_kernel<0>, kDiffBlock, 0)
-          : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rect_diff_kernel<1>, kDiffBlock, 0);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    n = 1;
-  }
-  return n > 0 ? n : 1;
-}
 
 // `side`: a second stream for diff_hot_kernel, whose few long blocks run beside
 // the tiles that need no whole walk; fork and join are the caller's events.
@@ -1634,21 +1740,30 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
       if (e != cudaSuccess) return e;
     }
   }
-  if (L.n_rect_items) {
-    if (pass == 0) {
-      rect_diff_kernel<0><<<L.n_rect_blocks, kDiffBlock, 0, stream>>>(
-          L.T, L.rect_items, L.n_rect_items, L.rect_counter, L.atoms, L.t0s, L.temp, L.parts,
-          nullptr, nullptr, nullptr, nullptr, nullptr);
-    } else {
-      rect_diff_kernel<1><<<L.n_rect_blocks, kDiffBlock, 0, stream>>>(
-          L.T, L.rect_items, L.n_rect_items, L.rect_counter, L.atoms, L.t0s, L.temp, nullptr,
-          L.lnZ1, L.lnZ2, L.gB, L.gS, L.D64);
-      e = cudaGetLastError();
+  for (uint32_t y0 = 0; y0 < L.n_rect; y0 += 65535u) {
+    const uint32_t ny = L.n_rect - y0 < 65535u ? L.n_rect - y0 : 65535u;
+    const uint32_t *list = L.rect_list + y0;
+    const dim3 tiles((L.max_rect_tiles + 3u) / 4u, ny);
+    const dim3 blocks((L.max_rect_atoms + 1023u) / 1024u, ny);  // 32 blocks of 32 atoms each
+    if (y0 == 0) {
+      e = launch_prefix(L.rect_T, L.rect_ident, L.n_rect, L.atoms, L.P, kPrecFF, stream);
       if (e != cudaSuccess) return e;
-      rect_diff_scan_kernel<<<L.n_rect, kScanBlock, 0, stream>>>(L.T, L.rect_list, L.D64,
-                                                                 L.grad_atoms);
     }
-    return cudaGetLastError();
+    rect_blocks_kernel<<<blocks, 256, 0, stream>>>(L.T, list, L.atoms, L.B64);
+    rect_est_kernel<<<tiles, kDiffBlock, 0, stream>>>(L.T, list, L.atoms, L.t0s, L.P, L.need,
+                                                      L.est);
+    if (pass == 0) {
+      rect_diff_kernel<0><<<tiles, kDiffBlock, 0, stream>>>(
+          L.T, list, L.atoms, L.t0s, L.P, L.B64, L.need, L.est, L.temp, L.parts, nullptr, nullptr,
+          nullptr, nullptr, nullptr);
+    } else {
+      rect_diff_kernel<1><<<tiles, kDiffBlock, 0, stream>>>(
+          L.T, list, L.atoms, L.t0s, L.P, L.B64, L.need, L.est, L.temp, nullptr, L.lnZ1, L.lnZ2,
+          L.gB, L.gS, L.D64);
+      rect_diff_scan_kernel<<<ny, kScanBlock, 0, stream>>>(L.T, list, L.D64, L.grad_atoms);
+    }
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }

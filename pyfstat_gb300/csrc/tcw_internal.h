@@ -223,15 +223,16 @@ cudaError_t launch_posteriors(const TemplateDev *d_T, const float *d_Fmn, void *
 // ---------------------------------------------------------------- differentiable path
 // One template with a continuous tau grid (tcw_diff.cu).  Exponential
 // templates are tiled by 32 tau columns x chunk_rows t0 rows (n_cg x n_chunk
-// tiles, tile = cg * n_chunk + chunk); rectangular templates own, in the
-// backward pass, the difference rows of their atom gradient at p_off:
-// (numAtoms + 1) rows of 8 doubles.
+// tiles, tile = cg * n_chunk + chunk), rectangular ones by 32 t0 rows x
+// chunk_rows tau columns (n_cg row groups, n_chunk column chunks); these own
+// (numAtoms + 1) prefix rows at p_off, as many difference rows of their atom
+// gradient in the backward pass, and FP64 block sums at seg_off.
 struct DiffTemplate {
   uint64_t atom_off, t0_off;
   Geom g;
   uint32_t N_t0, N_tau;
   double tau_min, tau_max;
-  uint32_t part_off, n_parts;  // partials of this template (exp: one per tile)
+  uint32_t part_off, n_parts;  // this template's tiles (need, partials)
   uint32_t window, pad;
   uint64_t p_off;
   uint32_t n_cg, n_chunk, chunk_rows;
@@ -240,10 +241,6 @@ struct DiffTemplate {
   uint64_t seg_off;   // segment sums, in 32-lane blocks of one segment
   uint64_t scr_off;   // backward: adjoint sources, in floats
   uint64_t cend_off;  // backward: recurrence ends, in 32-lane blocks
-};
-// A tile of rectangular windows: rows [n0, n1) (at most 128), all columns.
-struct DiffItem {
-  uint32_t tmpl, part, n0, n1;
 };
 // Adjoint sources of one cell in the backward pass's scratch (7 channels and
 // r^L as a float pair) and atoms per segment of the transposed recurrence.
@@ -284,17 +281,16 @@ struct DiffLaunch {
   float *scratch;                    // backward: adjoint sources of a group's tiles
   float *cend;                       // backward: recurrence ends of a group
   double *grad_atoms, *grad_tau;     // pass B/C outputs (accumulated; zero them first)
-  // rectangular templates: their tiles (rows [n0, n1) of one template),
-  // counter and persistent blocks, the list of their template indices and
-  // (backward) the difference rows of the atom gradient (zeroed by the caller)
-  const DiffItem *rect_items;
-  uint32_t n_rect_items, n_rect_blocks;
-  uint32_t *rect_counter;
-  const uint32_t *rect_list;
-  uint32_t n_rect;
-  double *D64;
+  // rectangular templates: the list of their indices, their geometry for the
+  // prefix kernel (rect_ident counts 0, 1, ...) with the prefix rows it fills,
+  // FP64 32-atom block sums and (backward) the difference rows of the atom
+  // gradient (zeroed by the caller)
+  const uint32_t *rect_list, *rect_ident;
+  uint32_t n_rect, max_rect_tiles, max_rect_atoms;
+  const TemplateDev *rect_T;
+  float *P;
+  double *B64, *D64;
 };
-int rect_diff_blocks_per_sm(int pass);
 cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, uint32_t n_groups,
                         cudaStream_t stream, cudaStream_t side, cudaEvent_t fork,
                         cudaEvent_t join);
