@@ -57,11 +57,12 @@ struct tcw_plan {
   WorkItem *d_items = nullptr;
   Partial *d_parts = nullptr;
   uint32_t *d_rect_list = nullptr, *d_exp_list = nullptr, *d_t0s = nullptr, *d_taus = nullptr;
-  uint32_t n_exp = 0;
+  uint32_t n_exp = 0, max_exp_atoms = 0;
   float *d_A8 = nullptr;  // exp templates' atoms in rows of 8 floats
   // row-chunked exp columns: segments and their sums
   SegItem *d_segs = nullptr;
   uint32_t n_segs = 0;
+  bool exp_chunks = false;  // some columns are cut within a history
   float *d_G = nullptr;
   uint32_t *d_counter = nullptr;  // [0] rect tiles, [1] exp tiles
   float *d_P = nullptr;
@@ -260,8 +261,11 @@ void tile_template(uint32_t tmpl, const TemplateDev &t, const tcw_tile_config &c
   }
 }
 
-#ifndef TCW_PLAN_EXP_TILES
-#define TCW_PLAN_EXP_TILES 2
+#ifndef TCW_PLAN_RECT_WARPS
+#define TCW_PLAN_RECT_WARPS 10
+#endif
+#ifndef TCW_PLAN_EXP_WARPS
+#define TCW_PLAN_EXP_WARPS 8
 #endif
 // Rows of a history for exp_rows of a tile configuration (0: whole columns).
 uint32_t exp_hist(uint32_t exp_rows, uint32_t N_t0) {
@@ -530,12 +534,14 @@ static int plain_enqueue(tcw_handle *h, const float *d_atoms, uint32_t numAtoms,
   if (h->plain_cfg.rect_tm) cfg.rect_tm = h->plain_cfg.rect_tm;
   if (h->plain_cfg.exp_tn) cfg.exp_tn = h->plain_cfg.exp_tn;
   uint64_t seg_floats = 0;
-  uint32_t n_seg_items = 0;
+  uint32_t n_seg_items = 0, seg_per = 1;
   if (window == TCW_WINDOW_EXP) {
     const ExpSplit sp = plain_exp_split(numAtoms, N_t0, N_tau, h->n_sms, prec != kPrecPlain32);
     set_split(t, sp);
     seg_floats = sp.seg_floats(N_tau);
-    n_seg_items = (N_tau + 31u) / 32u * ((sp.nseg + kSegPerWarp - 1u) / kSegPerWarp);
+    const uint32_t groups = (N_tau + 31u) / 32u;
+    seg_per = segs_per_warp((uint64_t)groups * sp.nseg, h->n_sms);
+    n_seg_items = groups * ((sp.nseg + seg_per - 1u) / seg_per);
   }
   fill_cfg_defaults(cfg);
   std::vector<WorkItem> items;
@@ -591,10 +597,11 @@ static int plain_enqueue(tcw_handle *h, const float *d_atoms, uint32_t numAtoms,
                               dP, prec, h->stream));
   float *dA8 = window == TCW_WINDOW_EXP ? reinterpret_cast<float *>(ws + o_A8) : nullptr;
   if (window == TCW_WINDOW_EXP)
-    TCW_CUDA(h, launch_repack(dT, reinterpret_cast<const uint32_t *>(ws + o_list), 1, d_atoms,
-                              dA8, h->stream));
+    TCW_CUDA(h, launch_repack(dT, reinterpret_cast<const uint32_t *>(ws + o_list), 1, numAtoms,
+                              d_atoms, dA8, h->stream));
   float *dG = reinterpret_cast<float *>(ws + o_G);
-  TCW_CUDA(h, launch_exp_segments(dT, nullptr, n_seg_items, dA8, d_taus, dG, h->stream));
+  TCW_CUDA(h, launch_exp_segments(dT, nullptr, n_seg_items, seg_per, dA8, d_taus, dG,
+                                  h->stream));
   MapLaunch ml{};
   ml.T = dT;
   ml.items = reinterpret_cast<const WorkItem *>(ws + o_items);
@@ -767,19 +774,37 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   std::vector<uint32_t> rect_list, exp_list;
   uint64_t p_rows = 0, a8_rows = 0, atom_rows = 0, cells = 0;
   // Row chunks of exp columns when the caller leaves them to the library
-  // (exp_rows 0): whole columns while these fill the GPU, else as many
-  // chunks per column as bring the warp tiles to TCW_PLAN_EXP_TILES per
-  // resident warp (32 per SM), started from segment sums (a run of 96
-  // templates with maps and posteriors: whole columns 3.63 ms, 1 tile per
-  // warp 2.82, 2 tiles 2.74, 3 tiles 2.78; the 74 000 column tiles of 4096
-  // templates stay whole).
+  // (exp_rows 0): whole columns while these are half of TCW_PLAN_EXP_WARPS per
+  // scheduler or more (a lone warp is bound by its own latency, eight share the
+  // issue slots), else as many chunks per column as bring the warp tiles there,
+  // started from segment sums.  Whole / cut, per run: 96 templates with maps
+  // and posteriors 3.55 / 2.76 ms, 300 templates 2.11 / 1.17, 24 templates
+  // 0.67 / 0.23; 1143 templates of up to 900 x 900 cells (9000 column tiles)
+  // 1.57 / 2.04.  3 or 5 warps leave the 96 and the 300 templates whole, 12 is
+  // no faster.
   uint64_t exp_chunks = 1, seg_blocks = 0;
   if (cfg.exp_rows == 0 && p->prec != kPrecPlain32) {
     uint64_t tiles = 0;
     for (uint32_t k = 0; k < n_templates; k++)
       if (desc[k].window == TCW_WINDOW_EXP) tiles += ((uint64_t)desc[k].N_tau + 31u) / 32u;
-    const uint64_t want = (uint64_t)h->n_sms * 32u * TCW_PLAN_EXP_TILES;
-    if (tiles) exp_chunks = (want + tiles - 1u) / tiles;
+    const uint64_t want = (uint64_t)h->n_sms * 4u * TCW_PLAN_EXP_WARPS;
+    if (tiles && 2u * tiles <= want) exp_chunks = (want + tiles - 1u) / tiles;
+  }
+  // Rect tiles when the caller leaves them to the library: 128 x 128 while
+  // these give every scheduler TCW_PLAN_RECT_WARPS warps' worth of tiles, else
+  // 32 rows x as many columns (32..128) as do (rect map kernel of 24
+  // templates: 182 -> 38 us).
+  tcw_tile_config rcfg = cfg;
+  if (!cfg_in || (cfg_in->rect_tn == 0 && cfg_in->rect_tm == 0)) {
+    uint64_t rect_cells = 0;
+    for (uint32_t k = 0; k < n_templates; k++)
+      if (desc[k].window == TCW_WINDOW_RECT) rect_cells += (uint64_t)desc[k].N_t0 * desc[k].N_tau;
+    const uint64_t per = rect_cells / ((uint64_t)h->n_sms * 4u * TCW_PLAN_RECT_WARPS);
+    if (per < (uint64_t)cfg.rect_tn * cfg.rect_tm) {
+      rcfg.rect_tm = 32;
+      rcfg.rect_tn =
+          (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>(128, per / 32u / 32u * 32u));
+    }
   }
   std::vector<SegItem> segs;
   try {
@@ -823,6 +848,7 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
         t.a8_off = a8_rows;
         a8_rows += d.numAtoms;
         exp_list.push_back(k);
+        p->max_exp_atoms = std::max(p->max_exp_atoms, d.numAtoms);
       }
       atom_rows = std::max<uint64_t>(atom_rows, d.atom_offset + d.numAtoms);
       cells += (uint64_t)d.N_t0 * d.N_tau;
@@ -833,18 +859,21 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
         if ((seg_blocks + (uint64_t)groups * sp.nseg) * kSegFloats * sizeof(float) > kSegBytesMax)
           sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, hist, 1);
         set_split(t, sp);
+        p->exp_chunks = p->exp_chunks || sp.sub > 1u;
         t.g_off = seg_blocks;
         seg_blocks += (uint64_t)groups * sp.nseg;
-        for (uint32_t cg = 0; cg < groups; cg++)
-          for (uint32_t j = 0; j < sp.nseg; j += kSegPerWarp)
-            segs.push_back(SegItem{k, cg, j, std::min(sp.nseg, j + kSegPerWarp)});
       }
-      tile_template(k, t, cfg, items, &cost, true);
+      tile_template(k, t, rcfg, items, &cost, true);
       t.part_off = (uint32_t)first;
       t.n_parts = (uint32_t)(items.size() - first);
       for (size_t i = first; i < items.size(); i++) items[i].part = (uint32_t)i;
       T[k] = t;
     }
+    const uint32_t per = segs_per_warp(seg_blocks, h->n_sms);
+    for (uint32_t k : exp_list)
+      for (uint32_t cg = 0; cg < (T[k].N_tau + 31u) / 32u; cg++)
+        for (uint32_t j = 0; j < T[k].g_nseg; j += per)
+          segs.push_back(SegItem{k, cg, j, std::min(T[k].g_nseg, j + per)});
     // two queues (rect tiles, then exp tiles), each in longest-processing-time
     // order: most expensive tiles first
     std::vector<uint32_t> order(items.size());
@@ -879,9 +908,9 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   p->n_atom_rows = atom_rows;
   p->p_rows = p_rows;
   {
-    const uint32_t br = (uint32_t)std::min<int>(map_blocks_per_sm(TCW_WINDOW_RECT, p->prec),
+    const uint32_t br = (uint32_t)std::min<int>(map_blocks_per_sm(TCW_WINDOW_RECT, p->prec, false),
                                                 (int)cfg.blocks_per_sm);
-    const uint32_t be = (uint32_t)std::min<int>(map_blocks_per_sm(TCW_WINDOW_EXP, p->prec),
+    const uint32_t be = (uint32_t)std::min<int>(map_blocks_per_sm(TCW_WINDOW_EXP, p->prec, p->exp_chunks),
                                                 (int)cfg.blocks_per_sm);
     p->n_blocks_rect = (uint32_t)std::max<uint64_t>(
         1, std::min<uint64_t>(p->n_items_rect, (uint64_t)br * h->n_sms));
@@ -990,6 +1019,7 @@ static MapLaunch plan_launch(const tcw_handle *h, const tcw_plan *p, int window,
   ml.counter = p->d_counter + (rect ? 0 : 1);
   ml.n_blocks = rect ? p->n_blocks_rect : p->n_blocks_exp;
   ml.persistent = true;
+  ml.chunks = p->exp_chunks;
   ml.write_map = d_maps != nullptr;
   ml.prec = p->prec;
   ml.priority = rect ? h->prio_low : h->prio_high;
@@ -1021,9 +1051,10 @@ static int plan_enqueue(tcw_handle *h, tcw_plan *p, const float *d_atoms, tcw_re
   // tile queue runs dry (its tail).
   TCW_CUDA(h, cudaEventRecord(h->fork_ev, h->stream));
   TCW_CUDA(h, cudaStreamWaitEvent(h->side_stream, h->fork_ev, 0));
-  TCW_CUDA(h, launch_repack(p->d_T, p->d_exp_list, p->n_exp, d_atoms, p->d_A8, h->stream));
+  TCW_CUDA(h, launch_repack(p->d_T, p->d_exp_list, p->n_exp, p->max_exp_atoms, d_atoms, p->d_A8,
+                            h->stream));
   if (inputs_read) TCW_CUDA(h, cudaEventRecord(inputs_read, h->stream));
-  TCW_CUDA(h, launch_exp_segments(p->d_T, p->d_segs, p->n_segs, p->d_A8, p->d_taus, p->d_G,
+  TCW_CUDA(h, launch_exp_segments(p->d_T, p->d_segs, p->n_segs, 0, p->d_A8, p->d_taus, p->d_G,
                                   h->stream));
   TCW_CUDA(h, launch_prefix(p->d_T, p->d_rect_list, p->n_rect, d_atoms, p->d_P, p->prec,
                             h->side_stream));
@@ -1112,8 +1143,9 @@ int tcw_plan_run_timed(tcw_handle *h, tcw_plan *p, const float *d_atoms, tcw_res
   TCW_CUDA(h, cudaEventRecord(ev[0], h->stream));
   TCW_CUDA(h, launch_prefix(p->d_T, p->d_rect_list, p->n_rect, d_atoms, p->d_P, p->prec,
                             h->stream));
-  TCW_CUDA(h, launch_repack(p->d_T, p->d_exp_list, p->n_exp, d_atoms, p->d_A8, h->stream));
-  TCW_CUDA(h, launch_exp_segments(p->d_T, p->d_segs, p->n_segs, p->d_A8, p->d_taus, p->d_G,
+  TCW_CUDA(h, launch_repack(p->d_T, p->d_exp_list, p->n_exp, p->max_exp_atoms, d_atoms, p->d_A8,
+                            h->stream));
+  TCW_CUDA(h, launch_exp_segments(p->d_T, p->d_segs, p->n_segs, 0, p->d_A8, p->d_taus, p->d_G,
                                   h->stream));
   TCW_CUDA(h, cudaEventRecord(ev[1], h->stream));
   TCW_CUDA(h, launch_map(TCW_WINDOW_RECT, plan_launch(h, p, TCW_WINDOW_RECT, d_atoms, nullptr),
@@ -1185,9 +1217,10 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     g.max_atoms = std::max(g.max_atoms, t.g.numAtoms);
     g.max_tiles = std::max(g.max_tiles, t.n_cg * t.n_chunk);
     if (t.g_nseg)
-      g.max_segs = std::max(g.max_segs, t.n_cg * ((t.g_nseg + kSegPerWarp - 1u) / kSegPerWarp));
+      g.max_segs = std::max(g.max_segs, t.n_cg * t.g_nseg);
     g.max_aseg = std::max(g.max_aseg, t.n_cg * t.n_aseg);
   }
+  g.seg_per = segs_per_warp(seg, h->n_sms);
   g.seg_floats = seg * seg_floats;
   g.scr_floats = pass ? scr : 0;
   g.cend_floats = pass ? cend * kDiffSegFloats : 0;

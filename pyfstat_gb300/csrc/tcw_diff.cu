@@ -367,30 +367,25 @@ struct ExpColumnV {
 
 constexpr uint32_t kDiffRowTab = 128;
 
+// Grid y: the template; the first `n_atom_blocks` blocks of x repack its atoms
+// (256 each), the others form its column constants (256 each).
 __global__ void __launch_bounds__(256) diff_prep_kernel(const DiffTemplate *__restrict__ T,
                                                         const uint32_t *__restrict__ list,
-                                                        uint32_t n_exp,
+                                                        uint32_t n_atom_blocks,
                                                         const float *__restrict__ atoms,
                                                         float *__restrict__ atoms8,
                                                         ColConsts *__restrict__ cols) {
-  __shared__ uint32_t s_first[256];
-  if (blockIdx.y > 0) {  // the templates' column constants, 256 columns per block
-    for (uint32_t k = blockIdx.x; k < n_exp; k += gridDim.x) {
-      const DiffTemplate t = T[list[k]];
-      const uint32_t n = (blockIdx.y - 1u) * 256u + threadIdx.x;
-      if (n >= t.N_tau) continue;
-      ExpColumn<false> C;
-      C.init_real(t.g, tau_of(t, n));
-      cols[t.col_off + n] = C.consts();
-    }
+  const DiffTemplate t = T[list[blockIdx.y]];
+  if (blockIdx.x < n_atom_blocks) {
+    repack_rows(atoms + t.atom_off * 7u, reinterpret_cast<float4 *>(atoms8 + t.atom_off * 8u),
+                t.g.numAtoms, blockIdx.x * 256u);
     return;
   }
-  for (uint32_t k = blockIdx.x; k < n_exp; k += gridDim.x) {
-    const DiffTemplate t = T[list[k]];
-    repack_rows256(atoms + t.atom_off * 7u, reinterpret_cast<float4 *>(atoms8 + t.atom_off * 8u),
-                   t.g.numAtoms, s_first);
-    __syncthreads();
-  }
+  const uint32_t n = (blockIdx.x - n_atom_blocks) * 256u + threadIdx.x;
+  if (n >= t.N_tau) return;
+  ExpColumn<false> C;
+  C.init_real(t.g, tau_of(t, n));
+  cols[t.col_off + n] = C.consts();
 }
 
 // One warp's share of a template: its column group, this lane's column and
@@ -510,7 +505,6 @@ __device__ __forceinline__ bool diff_tier1(const ExpColumn<false> &C, float &F32
 // FP64 work of 99.6 % of the tiles.
 struct EstSink {
   float top, most;
-  __device__ __forceinline__ void start() {}
   __device__ __forceinline__ void operator()(uint32_t, float F, bool ok) {
     if (!(F == F)) F = INFINITY;
     else if (ok) top = fmaxf(top, F);
@@ -542,7 +536,7 @@ __global__ void __launch_bounds__(kDiffBlock, 8)
     reg = reg && exp_row_regular(__ldg(L.t0s + m), L.taumax, L.t.g);
   ExpRow *tab = s_tab[threadIdx.x >> 5];
   if (__all_sync(0xffffffffu, reg)) {
-    exp_rows(C, L.t.g, L.t.g_shift, L.t.g_nseg, L.a8, L.t0s, mb, me, me, L.active, sink, tab, sg);
+    exp_rows<true, false>(C, L.t.g, L.t.g_shift, L.t.g_nseg, L.a8, L.t0s, mb, me, me, L.active, sink, tab, sg);
   } else {
     diff_rows(L, mb, me, C, sg, kDiffSegFloats, tab,
               [&](uint32_t m, uint32_t, uint32_t, bool data) {
@@ -711,12 +705,12 @@ __global__ void __launch_bounds__(kDiffBlock)
                     const ColConsts *__restrict__ cols, const float *__restrict__ need,
                     double temp, const double *__restrict__ lnZ1,
                     const double *__restrict__ lnZ2, const double *__restrict__ gB,
-                    const double *__restrict__ gS, float *__restrict__ seg) {
+                    const double *__restrict__ gS, uint32_t per, float *__restrict__ seg) {
   DiffLane L;
   const uint32_t k = list[blockIdx.y];
   L.t = T[k];
   const uint32_t w = blockIdx.x * 4u + (threadIdx.x >> 5);
-  const uint32_t cg = w % L.t.n_cg, j0 = w / L.t.n_cg * kSegPerWarp;
+  const uint32_t cg = w % L.t.n_cg, j0 = w / L.t.n_cg * per;
   if (j0 >= L.t.g_nseg) return;
   if (kV) {
     const DiffWeights w(L.t, k, temp, lnZ1, lnZ2, gB, gS);
@@ -727,7 +721,7 @@ __global__ void __launch_bounds__(kDiffBlock)
     if (!__any_sync(0xffffffffu, any)) return;
   }
   L.columns(atoms8, t0s_all, cg);
-  const uint32_t shift = L.t.g_shift, j1 = min(L.t.g_nseg, j0 + kSegPerWarp);
+  const uint32_t shift = L.t.g_shift, j1 = min(L.t.g_nseg, j0 + per);
   // a window holds fewer than 3 tau / TAtom + 2 atoms: shorter ones are never joined
   if (3ull * L.taumax + 2ull * L.t.g.TAtom < ((uint64_t)L.t.g.TAtom << (shift + 1u))) return;
   for (uint32_t j = j0; j < j1; j++) {
@@ -1687,10 +1681,6 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
                                        : (const void *)diff_hot_kernel<true>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kHotAtoms * 28u));
     if (e != cudaSuccess) return e;
-    // repacked rows (grid row 0) and column constants (one grid row per 256)
-    const dim3 prep(L.n_exp < 65535u ? L.n_exp : 65535u, 1u + (L.max_cols + 255u) / 256u);
-    diff_prep_kernel<<<prep, 256, 0, stream>>>(L.T, L.exp_list, L.n_exp, L.atoms, L.atoms8,
-                                               L.cols);
     for (uint32_t q = 0; q < n_groups; q++) {
       const DiffGroup &g = groups[q];
       const uint32_t *list = L.exp_list + g.y0;
@@ -1698,10 +1688,13 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
       const dim3 aseg((g.max_aseg + 3u) / 4u, g.ny), hot(g.max_cg, g.ny);
       // atoms that diff_hot_kernel stages in shared memory (28 bytes each)
       const uint32_t smem_atoms = g.max_atoms < kHotAtoms ? g.max_atoms : kHotAtoms;
+      const uint32_t atom_blocks = (g.max_atoms + 255u) / 256u;
+      diff_prep_kernel<<<dim3(atom_blocks + (L.max_cols + 255u) / 256u, g.ny), 256, 0, stream>>>(
+          L.T, list, atom_blocks, L.atoms, L.atoms8, L.cols);
       if (g.max_segs)
         diff_seg_kernel<false><<<segs, kDiffBlock, 0, stream>>>(
             L.T, list, L.atoms8, L.t0s, L.cols, nullptr, L.temp, nullptr, nullptr, nullptr,
-            nullptr, L.seg);
+            nullptr, g.seg_per, L.seg);
       diff_est_kernel<<<tiles, kDiffBlock, 0, stream>>>(L.T, list, L.atoms8, L.t0s, L.cols, L.seg,
                                                         L.need, L.est);
       if ((e = cudaEventRecord(fork, stream)) != cudaSuccess ||
@@ -1720,7 +1713,7 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
         if (g.max_segs)  // (over the window sums, which nothing reads any more)
           diff_seg_kernel<true><<<segs, kDiffBlock, 0, stream>>>(
               L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
-              L.seg);
+              g.seg_per, L.seg);
         diff_src_kernel<<<tiles, kDiffBlock, 0, stream>>>(
             L.T, list, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
             L.scratch, L.grad_tau);

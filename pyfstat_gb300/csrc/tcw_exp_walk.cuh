@@ -13,9 +13,10 @@ constexpr uint32_t kExpRowTab = 128;
 // The row-table walk of one warp's column chunk [mb, me) (regular rows):
 // row tables of kExpRowTab rows built by the warp, then each lane's column
 // slides down them (ExpColumn).  The walk starts at row ms - 1 >= me - 1: the
-// rows of [me, ms) only bring the window sums to the state that a walk from
-// further up would have.
-template <class Column, class Sink>
+// rows of [me, ms) bring the window sums to the state that a walk from further
+// up would have, without an F.  kSegs, kRunUpRows: whether the
+// walk may start from segment sums and above me.
+template <bool kSegs, bool kRunUpRows, class Column, class Sink>
 __device__ __forceinline__ void exp_rows(Column &C, const Geom &g, uint32_t shift, uint32_t nseg,
                                          const float *__restrict__ a8,
                                          const uint32_t *__restrict__ t0s, uint32_t mb,
@@ -23,7 +24,7 @@ __device__ __forceinline__ void exp_rows(Column &C, const Geom &g, uint32_t shif
                                          ExpRow *tab, const float *__restrict__ seg) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t *a8u = reinterpret_cast<const uint32_t *>(a8);
-  if (seg && active) {  // the walk's first window, where it is long
+  if (kSegs && seg && active) {  // the walk's first window, where it is long
     const uint32_t t0 = __ldg(t0s + ms - 1u);
     const uint32_t lo = exp_lo(t0, g), d = t0 - g.t0_data;
     ExpRow e;
@@ -33,10 +34,21 @@ __device__ __forceinline__ void exp_rows(Column &C, const Geom &g, uint32_t shif
     if (lo < top && top - lo >= (2u << shift))
       C.warm_start(a8, g, seg, shift, nseg, lo, top);
   }
-  for (uint32_t ce = ms; ce > mb;) {
-    if (ce == me) sink.start();  // the rows of the run-up leave nothing behind
-    const uint32_t floor = ce > me ? me : mb;
-    const uint32_t cb = ce - floor > kExpRowTab ? ce - kExpRowTab : floor;
+  // the run-up moves the window only
+  if (kRunUpRows && active) {
+    for (uint32_t m = ms; m > me;) {
+      m--;
+      const uint32_t t0 = __ldg(t0s + m), d = t0 - g.t0_data;
+      ExpRow e;
+      e.lo = exp_lo(t0, g);
+      e.nz = 0u;
+      e.a = fdiv(d, g.div);
+      e.b = d - e.a * g.TAtom;
+      C.window(a8, g, e);
+    }
+  }
+  for (uint32_t ce = me; ce > mb;) {
+    const uint32_t cb = ce - mb > kExpRowTab ? ce - kExpRowTab : mb;
     __syncwarp();
     uint32_t t0min = 0xFFFFFFFFu;
     for (uint32_t r = lane; r < ce - cb; r += 32u) {

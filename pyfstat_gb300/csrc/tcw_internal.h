@@ -43,8 +43,13 @@ struct TemplateDev {
 };
 // Floats of one 32-column segment sum (7 channels x hi, lo x 32 lanes).
 constexpr uint32_t kSegFloats = 14u * 32u;
-// Segments of one warp of exp_seg_kernel: amortises the column's FP64 exp.
-constexpr uint32_t kSegPerWarp = 4u;
+// Segments of one warp of exp_seg_kernel: up to 4 amortise the column's FP64
+// exp, fewer where that leaves resident warps (32 per SM) without one (480
+// atoms x 512 columns: 4 per warp 22.8 us; 24 templates: 24 -> 16 us).
+inline uint32_t segs_per_warp(uint64_t segments, int n_sms) {
+  const uint64_t per = segments / ((uint64_t)n_sms * 32u);
+  return per < 1 ? 1u : (per > 4 ? 4u : (uint32_t)per);
+}
 
 // A tile of one template, columns [n0, n1).  For a rectangular tile [m0, m1)
 // are its rows and tn its groups of 32 rows; for an exponential tile they are
@@ -142,41 +147,55 @@ struct Partial {
 };
 
 #if defined(__CUDACC__)
-// One template's atoms (rows of 7 floats, x) into 32-byte rows
-// [a2 b2 ab nz Fa_re Fa_im Fb_re Fb_im] (o), by one block of 256 threads;
-// nz (as u32 bits) is the lowest atom index >= i with a2 or b2 non-zero
-// (0xFFFFFFFF: none).  Each thread owns a contiguous chunk of atoms and walks
-// it backwards, starting from the first non-zero atom of the chunks above it.
-__device__ __forceinline__ void repack_rows256(const float *__restrict__ x,
-                                               float4 *__restrict__ o, uint32_t N,
-                                               uint32_t *s_first) {
-  const uint32_t tid = threadIdx.x;
-  const uint32_t chunk = (N + 255u) / 256u;
-  const uint32_t i0 = min(N, tid * chunk), i1 = min(N, i0 + chunk);
-  uint32_t first = 0xFFFFFFFFu;
-  for (uint32_t i = i0; i < i1; i++) {
-    const float *r = x + (size_t)i * 7u;
-    if (__ldg(r) != 0.0f || __ldg(r + 1) != 0.0f) {
-      first = i;
-      break;
-    }
-  }
-  s_first[tid] = first;
+// 256 of one template's atoms from i0 on (rows of 7 floats, x) into 32-byte
+// rows [a2 b2 ab nz Fa_re Fa_im Fb_re Fb_im] (o), by a block of 256 threads,
+// one atom each; nz (as u32 bits) is the lowest atom index >= i with a2 or b2
+// non-zero (0xFFFFFFFF: none), from the warps' ballots and, past the block's
+// atoms, a search upwards 256 at a time (one step unless a gap is that long).
+// (One block walking all atoms: 46 us for 17532 atoms.)
+__device__ __forceinline__ void repack_rows(const float *__restrict__ x, float4 *__restrict__ o,
+                                            uint32_t N, uint32_t i0) {
+  __shared__ uint32_t s_mask[8];
+  if (i0 >= N) return;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5, i = i0 + tid;
+  float r[7] = {0, 0, 0, 0, 0, 0, 0};
+  if (i < N)
+    for (int c = 0; c < 7; c++) r[c] = __ldg(x + (size_t)i * 7u + c);
+  const uint32_t mine = __ballot_sync(0xffffffffu, r[0] != 0.0f || r[1] != 0.0f);
+  if (lane == 0) s_mask[wid] = mine;
   __syncthreads();
   uint32_t nz = 0xFFFFFFFFu;
-  for (uint32_t k = tid + 1u; k < 256u; k++) {
-    if (s_first[k] != 0xFFFFFFFFu) {
-      nz = s_first[k];
-      break;
+  const uint32_t here = mine >> lane;
+  if (here) {
+    nz = i + __ffs(here) - 1u;
+  } else {
+    for (uint32_t w = wid + 1u; w < 8u; w++)
+      if (s_mask[w]) {
+        nz = i0 + w * 32u + __ffs(s_mask[w]) - 1u;
+        break;
+      }
+  }
+  // the lanes without one look above the block (all threads take part)
+  bool search = __syncthreads_or(i < N && nz == 0xFFFFFFFFu) != 0;
+  for (uint32_t base = i0 + 256u; search && base < N; base += 256u) {
+    const uint32_t j = base + tid;
+    const bool hit = j < N && (__ldg(x + (size_t)j * 7u) != 0.0f ||
+                               __ldg(x + (size_t)j * 7u + 1) != 0.0f);
+    const uint32_t m = __ballot_sync(0xffffffffu, hit);
+    if (lane == 0) s_mask[wid] = m;
+    if (__syncthreads_or(hit)) {
+      if (nz == 0xFFFFFFFFu)
+        for (uint32_t w = 0; w < 8u; w++)
+          if (s_mask[w]) {
+            nz = base + w * 32u + __ffs(s_mask[w]) - 1u;
+            break;
+          }
+      search = false;
     }
   }
-  for (uint32_t i = i1; i > i0;) {
-    i--;
-    const float *r = x + (size_t)i * 7u;
-    const float a2 = __ldg(r), b2 = __ldg(r + 1);
-    if (a2 != 0.0f || b2 != 0.0f) nz = i;
-    o[2u * i] = make_float4(a2, b2, __ldg(r + 2), __uint_as_float(nz));
-    o[2u * i + 1u] = make_float4(__ldg(r + 3), __ldg(r + 4), __ldg(r + 5), __ldg(r + 6));
+  if (i < N) {
+    o[2u * i] = make_float4(r[0], r[1], r[2], __uint_as_float(nz));
+    o[2u * i + 1u] = make_float4(r[3], r[4], r[5], r[6]);
   }
 }
 #endif
@@ -184,14 +203,16 @@ __device__ __forceinline__ void repack_rows256(const float *__restrict__ x,
 // Launchers (tcw_kernels.cu).  All asynchronous on `stream`.
 cudaError_t launch_prefix(const TemplateDev *d_T, const uint32_t *d_rect_list, uint32_t n_rect,
                           const float *d_atoms, float *d_P, int prec, cudaStream_t stream);
-// Exp templates' atoms (rows of 7 floats) into rows of 8 (zero-padded).
+// Exp templates' atoms (rows of 7 floats) into rows of 8 (repack_rows);
+// max_atoms: the most atoms of one of them.
 cudaError_t launch_repack(const TemplateDev *d_T, const uint32_t *d_exp_list, uint32_t n_exp,
-                          const float *d_atoms, float *d_atoms8, cudaStream_t stream);
+                          uint32_t max_atoms, const float *d_atoms, float *d_atoms8,
+                          cudaStream_t stream);
 // Segment sums of exp templates (the chunk starts of exp tiles are combined
 // from them): items == NULL means template 0's columns and segments, with
-// n_items = column groups x ceil(segments / kSegPerWarp).
+// n_items = column groups x ceil(segments / per).
 cudaError_t launch_exp_segments(const TemplateDev *d_T, const SegItem *d_items, uint32_t n_items,
-                                const float *d_atoms8, const uint32_t *d_taus, float *d_G,
+                                uint32_t per, const float *d_atoms8, const uint32_t *d_taus, float *d_G,
                                 cudaStream_t stream);
 struct MapLaunch {
   const TemplateDev *T;
@@ -200,6 +221,7 @@ struct MapLaunch {
   uint32_t *counter;      // persistent launches: tile counter, zeroed before
   uint32_t n_blocks;      // persistent grid size
   bool persistent, write_map;
+  bool chunks;            // persistent exp launches: some columns are cut (e_sub > 1)
   int prec;
   int priority;           // stream-priority value of the launch
   const float *atoms;
@@ -212,7 +234,7 @@ struct MapLaunch {
 };
 cudaError_t launch_map(int window, const MapLaunch &L, cudaStream_t stream);
 // Resident blocks per SM of the persistent (map-less) kernel of a window.
-int map_blocks_per_sm(int window, int prec);
+int map_blocks_per_sm(int window, int prec, bool chunks);
 
 cudaError_t launch_finalize(const TemplateDev *d_T, uint32_t n_templates, const Partial *d_parts,
                             void *d_results, cudaStream_t stream);
@@ -258,8 +280,9 @@ struct DiffPartial {
 // own: a backward pass runs in groups that bound the scratch.
 struct DiffGroup {
   uint32_t y0, ny;
-  // most column groups / tiles / segment items / atom segments of one template
+  // most column groups / tiles / segments / atom segments / atoms of one template
   uint32_t max_cg, max_tiles, max_segs, max_aseg, max_atoms;
+  uint32_t seg_per;  // segments per warp
   uint64_t seg_floats, scr_floats, cend_floats;
 };
 struct DiffLaunch {

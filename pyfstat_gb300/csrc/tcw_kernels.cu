@@ -59,14 +59,14 @@ __device__ __forceinline__ void ld_row16(const float *p, float r[16]) {
 
 // ------------------------------------------------------------------ repack
 
+// One block per 256 atoms of a template (grid y: the template).
 __global__ void __launch_bounds__(256) repack_kernel(const TemplateDev *__restrict__ T,
                                                      const uint32_t *__restrict__ exp_list,
                                                      const float *__restrict__ atoms,
                                                      float *__restrict__ A8) {
-  __shared__ uint32_t s_first[256];
-  const TemplateDev t = T[exp_list[blockIdx.x]];
-  repack_rows256(atoms + t.atom_off * 7u, reinterpret_cast<float4 *>(A8 + t.a8_off * 8u),
-                 t.g.numAtoms, s_first);
+  const TemplateDev t = T[exp_list[blockIdx.y]];
+  repack_rows(atoms + t.atom_off * 7u, reinterpret_cast<float4 *>(A8 + t.a8_off * 8u),
+              t.g.numAtoms, blockIdx.x * 256u);
 }
 
 // ------------------------------------------------------------------ prefix
@@ -160,6 +160,112 @@ __global__ void __launch_bounds__(256) prefix_kernel(const TemplateDev *__restri
     for (int c = 0; c < 7; c++) {
       float v = __ldg(x + (size_t)i * 7u + c);
       loc[c] = kComp ? ff_add1(loc[c], v) : FF{fadd(loc[c].h, v), 0.0f};
+    }
+  }
+  if (i0 < N && i1 == N) write_row(N);
+}
+
+// prefix_kernel for few templates: a cluster of eight blocks per template.
+// Rank b takes the 32 chunks of prefix_kernel's warp b, eight threads per
+// chunk (one channel each, the eighth writes the pads), so that its chains
+// run 1792 wide instead of 256 and its loads and row writes are whole
+// sectors; one warp per channel scans the block's chunk sums as that warp
+// did, and the ranks exchange their totals through distributed shared memory:
+// the same sums in the same order, bit for bit.  Bound by the chunks' serial
+// double-word sums (numAtoms / 256 steps, twice).  17532 atoms: 107 -> 19 us,
+// 480 atoms: 8.3 -> 3.3 us.
+constexpr uint32_t kPrefixCluster = 8;
+
+template <bool kComp>
+__global__ void __launch_bounds__(256)
+    prefix_cluster_kernel(const TemplateDev *__restrict__ T,
+                          const uint32_t *__restrict__ rect_list,
+                          const float *__restrict__ atoms, float *__restrict__ P) {
+  __shared__ FF s_sum[7][32];     // chunk sums, then their offsets in the block
+  __shared__ float s_abs[7][32];
+  __shared__ float s_tot[kPrefixCluster][7][3];  // every rank's total (h, l) and sum |x|
+  const uint32_t rank = blockIdx.x % kPrefixCluster;  // = rank in the cluster
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  const TemplateDev t = T[rect_list[blockIdx.x / kPrefixCluster]];
+  const uint32_t N = t.g.numAtoms;
+  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  const uint32_t ci = threadIdx.x >> 3, c = threadIdx.x & 7u;
+  const float *x = atoms + t.atom_off * 7u + c;
+  const uint32_t chunk = (N + 255u) / 256u;
+  const uint32_t i0 = min(N, (rank * 32u + ci) * chunk), i1 = min(N, i0 + chunk);
+  FF loc = ff_zero();
+  if (c < 7u) {
+    float sabs = 0.0f;
+#pragma unroll 8
+    for (uint32_t i = i0; i < i1; i++) {
+      const float v = __ldg(x + (size_t)i * 7u);
+      loc = kComp ? ff_add1(loc, v) : FF{fadd(loc.h, v), 0.0f};
+      sabs += fabsf(v);
+    }
+    s_sum[c][ci] = loc;
+    s_abs[c][ci] = sabs;
+  }
+  __syncthreads();
+  // every rank runs before its shared memory is written to
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  if (wid < 7u) {
+    FF v = s_sum[wid][lane];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      FF o = shfl_up_ff(v, d);
+      if (lane >= (uint32_t)d) v = kComp ? ff_add(o, v) : FF{fadd(o.h, v.h), 0.0f};
+    }
+    FF ex = shfl_up_ff(v, 1);
+    if (lane == 0) ex = ff_zero();
+    s_sum[wid][lane] = ex;
+    float a = s_abs[wid][lane];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) a += __shfl_xor_sync(0xffffffffu, a, d);
+    // lane r < 8 leaves the totals in rank r's shared memory
+    const float th = __shfl_sync(0xffffffffu, v.h, 31), tl = __shfl_sync(0xffffffffu, v.l, 31);
+    if (lane < kPrefixCluster) {
+      const uint32_t own = (uint32_t)__cvta_generic_to_shared(&s_tot[rank][wid][0]);
+      uint32_t far;
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(own), "r"(lane));
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(far), "f"(th) : "memory");
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(far + 4u), "f"(tl) : "memory");
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(far + 8u), "f"(a) : "memory");
+    }
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  float *out = P + t.p_off * kPrefixStride;
+  float Q = 1.0f, invQ = 1.0f;
+  if (c < 7u) {
+    FF off = ff_zero();
+    for (uint32_t w = 0; w < rank; w++) {
+      const FF tw{s_tot[w][c][0], s_tot[w][c][1]};
+      off = kComp ? ff_add(off, tw) : FF{fadd(off.h, tw.h), 0.0f};
+    }
+    const FF ex = s_sum[c][ci];
+    loc = kComp ? ff_add(off, ex) : FF{fadd(off.h, ex.h), 0.0f};
+    float S = 0.0f;
+    for (uint32_t w = 0; w < kPrefixCluster; w++) S += s_tot[w][c][2];
+    Q = prefix_quantum(S);
+    invQ = 1.0f / Q;
+  }
+  auto write_row = [&](uint32_t j) {
+    float h = 0.0f, l = 0.0f;
+    if (c < 7u) {
+      if (kComp)
+        quantise_prefix(loc.h, loc.l, Q, invQ, h, l);
+      else
+        h = loc.h;
+    }
+    out[(size_t)j * kPrefixStride + c] = h;
+    out[(size_t)j * kPrefixStride + 8u + c] = l;
+  };
+#pragma unroll 8
+  for (uint32_t i = i0; i < i1; i++) {
+    write_row(i);
+    if (c < 7u) {
+      const float v = __ldg(x + (size_t)i * 7u);
+      loc = kComp ? ff_add1(loc, v) : FF{fadd(loc.h, v), 0.0f};
     }
   }
   if (i0 < N && i1 == N) write_row(N);
@@ -470,14 +576,9 @@ struct MapSink {
   float *Fmn;
   uint32_t N_tau, n;
   Red *red;
-  bool live;
-  __device__ __forceinline__ void start() {
-    red->init();
-    live = true;
-  }
   __device__ __forceinline__ void operator()(uint32_t m, float F, bool) {
     TCW_DCHECK(n < N_tau);
-    if (kWrite && live) Fmn[(size_t)m * N_tau + n] = F;
+    if (kWrite) Fmn[(size_t)m * N_tau + n] = F;
     red->add_row_desc(F, m);
   }
 };
@@ -490,7 +591,7 @@ struct MapSink {
 // its own shared-memory slots (no block barrier) and every cell takes the
 // division-free window end of ExpColumn; otherwise the warp runs
 // exp_column2's generic index arithmetic.  Both give identical results.
-template <bool kWrite, int kPrec>
+template <bool kWrite, int kPrec, bool kChunks>
 __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *__restrict__ atoms,
                          const float *__restrict__ atoms8,
                          const uint32_t *__restrict__ t0s_all,
@@ -512,7 +613,7 @@ __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *_
   const uint32_t me = min(h1, mb + t.e_rows);
   const bool active = n < w.n1;
   const uint32_t tau = active ? __ldg(taus_all + t.tau_off + n) : 0u;
-  MapSink<kWrite> sink{kWrite ? Fmn + t.map_off : nullptr, t.N_tau, n, &red, true};
+  MapSink<kWrite> sink{kWrite ? Fmn + t.map_off : nullptr, t.N_tau, n, &red};
   if (kPrec == kPrecPlain32) {
     if (active) {
       exp_column<false, false>(atoms + t.atom_off * 7u, t.g, t0s, mb, me, tau, sink, nullptr);
@@ -524,7 +625,7 @@ __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *_
   const uint32_t taumax = __reduce_max_sync(0xffffffffu, tau);
   // run-up over the history above the chunk (kShortWindow, kRunUp)
   uint32_t ms = me;
-  if (me < h1) {
+  if (kChunks && me < h1) {
     const uint32_t taumin = __reduce_min_sync(0xffffffffu, active ? tau : 0xFFFFFFFFu);
     if (3ull * taumin < (uint64_t)kShortWindow * t.g.TAtom) {
       const uint64_t longest = min((uint64_t)taumax, (uint64_t)kShortWindow * t.g.TAtom / 3u + 1u);
@@ -550,11 +651,11 @@ __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *_
       t.g_nseg ? G + (t.g_off + (size_t)(n >> 5) * t.g_nseg) * kSegFloats + lane : nullptr;
   ExpColumn<kPrec == kPrecFF_F64Det, true> C;
   C.init(t.g, tau);
-  exp_rows(C, t.g, t.g_shift, t.g_nseg, a8, t0s, mb, me, ms, active, sink, tab, seg);
+  exp_rows<kChunks, kChunks>(C, t.g, t.g_shift, t.g_nseg, a8, t0s, mb, me, ms, active, sink, tab, seg);
   if (active) red.row_to_index(t.N_tau, n);
 }
 
-// Segment sums of exp columns: a warp takes kSegPerWarp segments of one
+// Segment sums of exp columns: a warp takes `per` segments of one
 // 32-column group, each lane one column, and enters the segment's atoms into
 // an empty window (the map kernel's steps).  They let a column be cut into
 // row chunks whose first window is combined from whole segments
@@ -569,7 +670,7 @@ __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *_
 template <bool kList>
 __global__ void __launch_bounds__(128, 8)
     exp_seg_kernel(const TemplateDev *__restrict__ T, const SegItem *__restrict__ items,
-                   uint32_t n_items, const float *__restrict__ atoms8,
+                   uint32_t n_items, uint32_t per, const float *__restrict__ atoms8,
                    const uint32_t *__restrict__ taus_all, float *__restrict__ G) {
   const uint32_t wi = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
   if (wi >= n_items) return;
@@ -580,8 +681,8 @@ __global__ void __launch_bounds__(128, 8)
     const uint32_t ncg = (T[0].N_tau + 31u) >> 5;
     w.tmpl = 0;
     w.cg = wi % ncg;
-    w.j0 = wi / ncg * kSegPerWarp;
-    w.j1 = min(T[0].g_nseg, w.j0 + kSegPerWarp);
+    w.j0 = wi / ncg * per;
+    w.j1 = min(T[0].g_nseg, w.j0 + per);
   }
   const TemplateDev t = T[w.tmpl];
   const uint32_t n = w.cg * 32u + lane;
@@ -601,15 +702,16 @@ __global__ void __launch_bounds__(128, 8)
 }
 
 cudaError_t launch_exp_segments(const TemplateDev *d_T, const SegItem *d_items, uint32_t n_items,
-                                const float *d_atoms8, const uint32_t *d_taus, float *d_G,
-                                cudaStream_t stream) {
+                                uint32_t per, const float *d_atoms8, const uint32_t *d_taus,
+                                float *d_G, cudaStream_t stream) {
   if (n_items == 0) return cudaSuccess;
   const uint32_t blocks = (n_items + 3u) / 4u;
   if (d_items)
-    exp_seg_kernel<true><<<blocks, 128, 0, stream>>>(d_T, d_items, n_items, d_atoms8, d_taus, d_G);
+    exp_seg_kernel<true><<<blocks, 128, 0, stream>>>(d_T, d_items, n_items, per, d_atoms8, d_taus,
+                                                     d_G);
   else
-    exp_seg_kernel<false><<<blocks, 128, 0, stream>>>(d_T, d_items, n_items, d_atoms8, d_taus,
-                                                      d_G);
+    exp_seg_kernel<false><<<blocks, 128, 0, stream>>>(d_T, d_items, n_items, per, d_atoms8,
+                                                      d_taus, d_G);
   return cudaGetLastError();
 }
 
@@ -630,15 +732,25 @@ cudaError_t launch_exp_segments(const TemplateDev *d_T, const SegItem *d_items, 
 #define TCW_EXP_MIN_BLOCKS_OTHER 5
 #endif
 
-template <int kWin, bool kPersist, bool kWrite>
+// Launches whose columns are cut are small: registers matter more than
+// occupancy (24 templates 210 / 189 / 182 us at 8 / 6 / 5 blocks, 96 templates
+// with maps 2.67 / 2.57 / 2.61 ms).
+#ifndef TCW_EXP_MIN_BLOCKS_CHUNKS
+#define TCW_EXP_MIN_BLOCKS_CHUNKS 6
+#endif
+
+template <int kWin, bool kPersist, bool kChunks>
 constexpr int map_min_blocks() {
   return kWin == TCW_WINDOW_RECT ? TCW_RECT_MIN_BLOCKS
-         : kPersist ? TCW_EXP_MIN_BLOCKS
-                                 : TCW_EXP_MIN_BLOCKS_OTHER;
+         : !kPersist             ? TCW_EXP_MIN_BLOCKS_OTHER
+         : kChunks               ? TCW_EXP_MIN_BLOCKS_CHUNKS
+                                 : TCW_EXP_MIN_BLOCKS;
 }
 
-template <int kWin, bool kPersist, bool kWrite, int kPrec>
-__global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kWrite>()))
+// kChunks (exponential windows): columns may be cut into row chunks within a
+// history (TemplateDev::e_sub > 1).
+template <int kWin, bool kPersist, bool kWrite, int kPrec, bool kChunks>
+__global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kChunks>()))
     map_kernel(const TemplateDev *__restrict__ T, const WorkItem *__restrict__ items,
                uint32_t n_items, uint32_t *__restrict__ counter, const float *__restrict__ atoms,
                const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s,
@@ -701,7 +813,7 @@ __global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kWrite
       const TemplateDev t = T[w.tmpl];
       Red red;
       red.init();
-      exp_tile<kWrite, kPrec>(t, w, atoms, atoms8, t0s, taus, Fmn, red, tab, G, true);
+      exp_tile<kWrite, kPrec, kChunks>(t, w, atoms, atoms8, t0s, taus, Fmn, red, tab, G, true);
       RedVal acc{red.mx, red.bidx, fsub(red.s, red.c)};
 #pragma unroll
       for (int d = 16; d > 0; d >>= 1) acc = red_combine(acc, shfl_down_red(acc, d));
@@ -736,7 +848,7 @@ __global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kWrite
                                reinterpret_cast<float *>(sm) + warp * (32 * 33), warp % rg,
                                4u / rg, warp / rg, s_tau + warp * 32u);
     } else
-      exp_tile<kWrite, kPrec>(t, w, atoms, atoms8, t0s, taus, Fmn, red,
+      exp_tile<kWrite, kPrec, kChunks>(t, w, atoms, atoms8, t0s, taus, Fmn, red,
                               reinterpret_cast<ExpRow *>(sm) + (threadIdx.x >> 5) * kExpRowTab, G);
     block_reduce_store(red, parts + w.part);
     if (!kPersist) break;
@@ -897,9 +1009,31 @@ __global__ void __launch_bounds__(1024) posterior_argmax_kernel(const double *__
 
 // ------------------------------------------------------------------ launchers
 
+// Templates up to which a prefix scan takes a cluster each (8 x 148 blocks
+// fill the GPU); more run one block each, which costs no redundant scans.
+constexpr uint32_t kPrefixFew = 152;
+
 cudaError_t launch_prefix(const TemplateDev *d_T, const uint32_t *d_rect_list, uint32_t n_rect,
                           const float *d_atoms, float *d_P, int prec, cudaStream_t stream) {
   if (n_rect == 0) return cudaSuccess;
+  if (n_rect <= kPrefixFew) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(n_rect * kPrefixCluster);
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kPrefixCluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return prec == kPrecPlain32
+               ? cudaLaunchKernelEx(&cfg, prefix_cluster_kernel<false>, d_T, d_rect_list, d_atoms,
+                                    d_P)
+               : cudaLaunchKernelEx(&cfg, prefix_cluster_kernel<true>, d_T, d_rect_list, d_atoms,
+                                    d_P);
+  }
   if (prec == kPrecPlain32)
     prefix_kernel<false><<<n_rect, 256, 0, stream>>>(d_T, d_rect_list, d_atoms, d_P);
   else
@@ -907,7 +1041,7 @@ cudaError_t launch_prefix(const TemplateDev *d_T, const uint32_t *d_rect_list, u
   return cudaGetLastError();
 }
 
-template <int kWin, bool kPersist, bool kWrite>
+template <int kWin, bool kPersist, bool kWrite, bool kChunks>
 static cudaError_t launch_map_prec(int prec, uint32_t grid, cudaStream_t s, int priority,
                                    const TemplateDev *T, const WorkItem *items, uint32_t n_items,
                                    uint32_t *counter, const float *atoms, const float *atoms8,
@@ -923,41 +1057,41 @@ static cudaError_t launch_map_prec(int prec, uint32_t grid, cudaStream_t s, int 
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   if (prec == kPrecPlain32)
-    return cudaLaunchKernelEx(&cfg, map_kernel<kWin, kPersist, kWrite, kPrecPlain32>, T, items,
-                              n_items, counter, atoms, atoms8, t0s, taus, P, G, Fmn, parts);
+    return cudaLaunchKernelEx(&cfg, map_kernel<kWin, kPersist, kWrite, kPrecPlain32, false>, T,
+                              items, n_items, counter, atoms, atoms8, t0s, taus, P, G, Fmn, parts);
   if (prec == kPrecFF_F64Det)
-    return cudaLaunchKernelEx(&cfg, map_kernel<kWin, kPersist, kWrite, kPrecFF_F64Det>, T, items,
-                              n_items, counter, atoms, atoms8, t0s, taus, P, G, Fmn, parts);
-  return cudaLaunchKernelEx(&cfg, map_kernel<kWin, kPersist, kWrite, kPrecFF>, T, items, n_items,
-                            counter, atoms, atoms8, t0s, taus, P, G, Fmn, parts);
+    return cudaLaunchKernelEx(&cfg, map_kernel<kWin, kPersist, kWrite, kPrecFF_F64Det, kChunks>, T,
+                              items, n_items, counter, atoms, atoms8, t0s, taus, P, G, Fmn, parts);
+  return cudaLaunchKernelEx(&cfg, map_kernel<kWin, kPersist, kWrite, kPrecFF, kChunks>, T, items,
+                            n_items, counter, atoms, atoms8, t0s, taus, P, G, Fmn, parts);
 }
 
 template <int kWin>
 static cudaError_t launch_map_win(const MapLaunch &L, cudaStream_t stream) {
   if (L.n_items == 0) return cudaSuccess;
   const uint32_t grid = L.persistent ? L.n_blocks : L.n_items;
-  if (L.persistent) {
-    if (L.write_map)
-      return launch_map_prec<kWin, true, true>(L.prec, grid, stream, L.priority, L.T, L.items,
-                                               L.n_items, L.counter, L.atoms, L.atoms8, L.t0s, L.taus, L.P,
-                                               L.G, L.Fmn, L.parts);
-    return launch_map_prec<kWin, true, false>(L.prec, grid, stream, L.priority, L.T, L.items,
-                                              L.n_items, L.counter, L.atoms, L.atoms8, L.t0s, L.taus, L.P,
-                                              L.G, L.Fmn, L.parts);
-  }
-  if (L.write_map)
-    return launch_map_prec<kWin, false, true>(L.prec, grid, stream, L.priority, L.T, L.items,
-                                              L.n_items, L.counter, L.atoms, L.atoms8, L.t0s, L.taus, L.P,
-                                              L.G, L.Fmn, L.parts);
-  return launch_map_prec<kWin, false, false>(L.prec, grid, stream, L.priority, L.T, L.items,
-                                             L.n_items, L.counter, L.atoms, L.atoms8, L.t0s, L.taus, L.P,
-                                             L.G, L.Fmn, L.parts);
+  constexpr bool kExp = kWin == TCW_WINDOW_EXP;
+  auto launch = [&](auto fn) {
+    return fn(L.prec, grid, stream, L.priority, L.T, L.items, L.n_items, L.counter, L.atoms,
+              L.atoms8, L.t0s, L.taus, L.P, L.G, L.Fmn, L.parts);
+  };
+  if (!L.persistent)
+    return L.write_map ? launch(launch_map_prec<kWin, false, true, kExp>)
+                       : launch(launch_map_prec<kWin, false, false, kExp>);
+  if (kExp && L.chunks)
+    return L.write_map ? launch(launch_map_prec<kWin, true, true, kExp>)
+                       : launch(launch_map_prec<kWin, true, false, kExp>);
+  return L.write_map ? launch(launch_map_prec<kWin, true, true, false>)
+                     : launch(launch_map_prec<kWin, true, false, false>);
 }
 
 cudaError_t launch_repack(const TemplateDev *d_T, const uint32_t *d_exp_list, uint32_t n_exp,
-                          const float *d_atoms, float *d_atoms8, cudaStream_t stream) {
-  if (n_exp == 0) return cudaSuccess;
-  repack_kernel<<<n_exp, 256, 0, stream>>>(d_T, d_exp_list, d_atoms, d_atoms8);
+                          uint32_t max_atoms, const float *d_atoms, float *d_atoms8,
+                          cudaStream_t stream) {
+  for (uint32_t y0 = 0; y0 < n_exp; y0 += 65535u) {
+    const dim3 grid((max_atoms + 255u) / 256u, n_exp - y0 < 65535u ? n_exp - y0 : 65535u);
+    repack_kernel<<<grid, 256, 0, stream>>>(d_T, d_exp_list + y0, d_atoms, d_atoms8);
+  }
   return cudaGetLastError();
 }
 
@@ -968,19 +1102,19 @@ cudaError_t launch_map(int window, const MapLaunch &L, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-template <int kWin>
+template <int kWin, bool kChunks>
 static int blocks_per_sm_win(int prec) {
   int n = 0;
   cudaError_t e;
   if (prec == kPrecPlain32)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &n, map_kernel<kWin, true, false, kPrecPlain32>, kBlock, 0);
+        &n, map_kernel<kWin, true, false, kPrecPlain32, false>, kBlock, 0);
   else if (prec == kPrecFF_F64Det)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &n, map_kernel<kWin, true, false, kPrecFF_F64Det>, kBlock, 0);
+        &n, map_kernel<kWin, true, false, kPrecFF_F64Det, kChunks>, kBlock, 0);
   else
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, map_kernel<kWin, true, false, kPrecFF>,
-                                                      kBlock, 0);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &n, map_kernel<kWin, true, false, kPrecFF, kChunks>, kBlock, 0);
   if (e != cudaSuccess) {
     cudaGetLastError();
     n = 1;
@@ -989,9 +1123,10 @@ static int blocks_per_sm_win(int prec) {
 }
 
 // Resident blocks per SM of the persistent (map-less) kernel of a window.
-int map_blocks_per_sm(int window, int prec) {
-  return window == TCW_WINDOW_RECT ? blocks_per_sm_win<TCW_WINDOW_RECT>(prec)
-                                   : blocks_per_sm_win<TCW_WINDOW_EXP>(prec);
+int map_blocks_per_sm(int window, int prec, bool chunks) {
+  return window == TCW_WINDOW_RECT ? blocks_per_sm_win<TCW_WINDOW_RECT, false>(prec)
+         : chunks                  ? blocks_per_sm_win<TCW_WINDOW_EXP, true>(prec)
+                                   : blocks_per_sm_win<TCW_WINDOW_EXP, false>(prec);
 }
 
 // One template, one block: the partials of a large single-template call (up

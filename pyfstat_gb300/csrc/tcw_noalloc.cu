@@ -201,12 +201,13 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
   if (cudaGetLastError() != cudaSuccess) return TCW_ERR_CUDA;
   cudaError_t e = window == TCW_WINDOW_RECT
                       ? launch_prefix(dT, dlist, 1, d_atoms, drows, prec, s)
-                      : launch_repack(dT, dlist, 1, d_atoms, drows, s);
+                      : launch_repack(dT, dlist, 1, numAtoms, d_atoms, drows, s);
   if (e != cudaSuccess) return TCW_ERR_CUDA;
   float *dG = reinterpret_cast<float *>(base + o_G);
-  const uint32_t n_seg_items =
-      (N_tau + 31u) / 32u * ((sp.nseg + kSegPerWarp - 1u) / kSegPerWarp);
-  if (launch_exp_segments(dT, nullptr, n_seg_items, drows, d_taus, dG, s) != cudaSuccess)
+  const uint32_t groups = (N_tau + 31u) / 32u;
+  const uint32_t per = segs_per_warp((uint64_t)groups * sp.nseg, sms);
+  const uint32_t n_seg_items = groups * ((sp.nseg + per - 1u) / per);
+  if (launch_exp_segments(dT, nullptr, n_seg_items, per, drows, d_taus, dG, s) != cudaSuccess)
     return TCW_ERR_CUDA;
   MapLaunch ml{};
   ml.T = dT;
