@@ -76,11 +76,8 @@ struct tcw_plan {
   float *d_atoms_in = nullptr;
   tcw_result *d_res_out = nullptr;
   float *d_maps_out = nullptr;  // maps of tcw_plan_run_maps_host (n_cells floats)
-  // posterior plans: column chunks and the row / column sums
-  uint2 *d_post_chunks = nullptr;
-  uint32_t n_post_chunks = 0;
-  float *d_rowpart = nullptr;
-  double *d_colsum = nullptr;
+  // posterior plans: chunks and the row / column sums
+  PostLayout post{};
 };
 
 namespace {
@@ -558,7 +555,8 @@ static int plain_enqueue(tcw_handle *h, const float *d_atoms, uint32_t numAtoms,
   t.map_off = 0;
 
   const bool post = (flags & TCW_FLAG_POSTERIORS) != 0;
-  const uint32_t n_chunks = (N_t0 + 63u) / 64u;
+  const uint32_t prows = post_rows((uint64_t)N_t0 * N_tau, h->n_sms);
+  const uint32_t n_rc = (N_t0 + prows - 1u) / prows, n_cc = (N_tau + 1023u) / 1024u;
   Layout L;
   L.total = ws_off;
   const size_t o_T = L.add(sizeof(TemplateDev));
@@ -572,8 +570,9 @@ static int plain_enqueue(tcw_handle *h, const float *d_atoms, uint32_t numAtoms,
                           ? L.add(sizeof(float) * 8u * (size_t)numAtoms)
                           : 0;
   const size_t o_G = L.add(sizeof(float) * seg_floats);
-  const size_t o_row = post ? L.add(sizeof(double) * N_t0) : 0;
-  const size_t o_col = post ? L.add(sizeof(double) * (size_t)n_chunks * N_tau) : 0;
+  const size_t o_row = post ? L.add(sizeof(double) * (size_t)N_t0 * n_cc) : 0;
+  const size_t o_col = post ? L.add(sizeof(double) * (size_t)n_rc * N_tau) : 0;
+  const size_t o_pp = post ? L.add(sizeof(PostPart) * 2u * kPostParts + sizeof(uint32_t)) : 0;
   int rc = ensure_ws(h, L.total);
   if (rc) return rc;
   ws = h->d_ws;  // the workspace may have moved
@@ -620,10 +619,14 @@ static int plain_enqueue(tcw_handle *h, const float *d_atoms, uint32_t numAtoms,
   ml.parts = dparts;
   TCW_CUDA(h, launch_map(window, ml, h->stream));
   TCW_CUDA(h, launch_finalize(dT, 1, dparts, d_result, h->stream));
-  if (post)
-    TCW_CUDA(h, launch_posteriors(dT, d_Fmn, d_result, reinterpret_cast<double *>(ws + o_row),
-                                  reinterpret_cast<double *>(ws + o_col), N_t0, N_tau,
-                                  h->stream));
+  if (post) {
+    PostPart *pp = reinterpret_cast<PostPart *>(ws + o_pp);
+    const PostLayout pl{prows, 1024u, n_rc * n_cc, nullptr,
+                        reinterpret_cast<double *>(ws + o_row),
+                        reinterpret_cast<double *>(ws + o_col), pp,
+                        reinterpret_cast<uint32_t *>(pp + 2u * kPostParts)};
+    TCW_CUDA(h, launch_posteriors(dT, 1, pl, d_Fmn, d_result, h->stream));
+  }
   return TCW_OK;
 }
 
@@ -711,8 +714,9 @@ int tcw_map_plain_host(tcw_handle *h, const float *atoms, uint32_t numAtoms, uin
                              prec_of(flags) != kPrecPlain32)
                  .seg_floats(N_tau));
     }
-    L2.add(sizeof(double) * N_t0);
-    L2.add(sizeof(double) * ((N_t0 + 63u) / 64u) * (size_t)N_tau);
+    L2.add(sizeof(double) * (size_t)N_t0 * ((N_tau + 1023u) / 1024u));
+    L2.add(sizeof(double) * ((N_t0 + 15u) / 16u) * (size_t)N_tau);
+    L2.add(sizeof(PostPart) * 2u * kPostParts + sizeof(uint32_t));
     need_after = L2.total;
   }
   if (need_after > h->ws_cap) {
@@ -767,7 +771,7 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   p->n_templates = n_templates;
   p->cfg = cfg;
   std::vector<uint2> post_chunks;
-  uint64_t post_rows = 0, post_cols = 0;
+  uint64_t post_row_sums = 0, post_col_sums = 0;
   std::vector<TemplateDev> T(n_templates);
   std::vector<WorkItem> items;
   std::vector<double> cost;
@@ -807,6 +811,12 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
     }
   }
   std::vector<SegItem> segs;
+  {
+    uint64_t all = 0;
+    for (uint32_t k = 0; k < n_templates; k++) all += (uint64_t)desc[k].N_t0 * desc[k].N_tau;
+    p->post.rows = post_rows(all, h->n_sms);
+    p->post.cols = 1024u;
+  }
   try {
     for (uint32_t k = 0; k < n_templates; k++) {
       const tcw_template_desc &d = desc[k];
@@ -834,12 +844,15 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
       t.t0_off = d.t0_offset;
       t.tau_off = d.tau_offset;
       t.map_off = cells;  // maps of tcw_plan_run_maps: templates in descriptor order
-      t.row_off = post_rows;  // row partials: N_t0 per column chunk
-      t.col_off = post_cols;
-      post_rows += (uint64_t)d.N_t0 * ((d.N_tau + kPostCols - 1u) / kPostCols);
-      post_cols += d.N_tau;
-      if (flags & TCW_FLAG_POSTERIORS)
-        for (uint32_t n0 = 0; n0 < d.N_tau; n0 += kPostCols) post_chunks.push_back(make_uint2(k, n0));
+      t.row_off = post_row_sums;
+      t.col_off = post_col_sums;
+      if (flags & TCW_FLAG_POSTERIORS) {
+        const uint32_t n_cc = (d.N_tau + 1023u) / 1024u;
+        const uint32_t n_rc = (d.N_t0 + p->post.rows - 1u) / p->post.rows;
+        post_row_sums += (uint64_t)d.N_t0 * n_cc;
+        post_col_sums += (uint64_t)d.N_tau * n_rc;
+        for (uint32_t c = 0; c < n_cc * n_rc; c++) post_chunks.push_back(make_uint2(k, c));
+      }
       if (d.window == TCW_WINDOW_RECT) {
         t.p_off = p_rows;
         p_rows += (uint64_t)d.numAtoms + 1u;
@@ -934,8 +947,10 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   const size_t o_cnt = L.add(2 * sizeof(uint32_t));
   const bool post = (flags & TCW_FLAG_POSTERIORS) != 0;
   const size_t o_chunks = post ? L.add(sizeof(uint2) * std::max<size_t>(1, post_chunks.size())) : 0;
-  const size_t o_rowsum = post ? L.add(sizeof(float) * std::max<uint64_t>(1, post_rows)) : 0;
-  const size_t o_colsum = post ? L.add(sizeof(double) * std::max<uint64_t>(1, post_cols)) : 0;
+  const size_t o_rowsum = post ? L.add(sizeof(double) * post_row_sums) : 0;
+  const size_t o_colsum = post ? L.add(sizeof(double) * post_col_sums) : 0;
+  const size_t o_pp = post ? L.add(sizeof(PostPart) * 2u * kPostParts * (size_t)n_templates) : 0;
+  const size_t o_ticket = post ? L.add(sizeof(uint32_t) * n_templates) : 0;
   void *buf = nullptr;
   rc = ws_alloc(h, &buf, L.total);
   if (rc) {
@@ -956,10 +971,12 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   p->d_P = reinterpret_cast<float *>(p->d_buf + o_P);
   p->d_counter = reinterpret_cast<uint32_t *>(p->d_buf + o_cnt);
   if (post) {
-    p->d_post_chunks = reinterpret_cast<uint2 *>(p->d_buf + o_chunks);
-    p->n_post_chunks = (uint32_t)post_chunks.size();
-    p->d_rowpart = reinterpret_cast<float *>(p->d_buf + o_rowsum);
-    p->d_colsum = reinterpret_cast<double *>(p->d_buf + o_colsum);
+    p->post.chunks = reinterpret_cast<const uint2 *>(p->d_buf + o_chunks);
+    p->post.n_chunks = (uint32_t)post_chunks.size();
+    p->post.rowsum = reinterpret_cast<double *>(p->d_buf + o_rowsum);
+    p->post.colsum = reinterpret_cast<double *>(p->d_buf + o_colsum);
+    p->post.parts = reinterpret_cast<PostPart *>(p->d_buf + o_pp);
+    p->post.ticket = reinterpret_cast<uint32_t *>(p->d_buf + o_ticket);
   }
   // control data: a synchronous copy (plans are built once)
   std::vector<char> host(ctl_end, 0);
@@ -974,7 +991,7 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   if (!segs.empty()) memcpy(host.data() + o_segs, segs.data(), sizeof(SegItem) * segs.size());
   cudaError_t e = cudaMemcpy(p->d_buf, host.data(), ctl_end, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && post && !post_chunks.empty())
-    e = cudaMemcpy(p->d_post_chunks, post_chunks.data(), sizeof(uint2) * post_chunks.size(),
+    e = cudaMemcpy(p->d_buf + o_chunks, post_chunks.data(), sizeof(uint2) * post_chunks.size(),
                    cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cudaFree(p->d_buf);
@@ -1067,8 +1084,7 @@ static int plan_enqueue(tcw_handle *h, tcw_plan *p, const float *d_atoms, tcw_re
   TCW_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_ev, 0));
   TCW_CUDA(h, launch_finalize(p->d_T, p->n_templates, p->d_parts, d_results, h->stream));
   if (d_maps && (p->flags & TCW_FLAG_POSTERIORS))
-    TCW_CUDA(h, launch_plan_posteriors(p->d_T, p->n_templates, p->d_post_chunks, p->n_post_chunks,
-                                       d_maps, d_results, p->d_rowpart, p->d_colsum, h->stream));
+    TCW_CUDA(h, launch_posteriors(p->d_T, p->n_templates, p->post, d_maps, d_results, h->stream));
   return TCW_OK;
 }
 

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "../../include/tcw_b200.h"
 #include "tcw_cell.h"
 
 namespace tcw {
@@ -32,7 +33,7 @@ struct TemplateDev {
   uint32_t N_t0, N_tau;
   uint32_t part_off, n_parts;
   uint32_t pad;
-  uint64_t row_off, col_off;  // posterior row partials / column sums (plans with posteriors)
+  uint64_t row_off, col_off;  // posterior row and column sums (PostLayout)
   // exp templates whose columns are cut into row chunks: segment sums of
   // 2^g_shift atoms (exp_seg_kernel), g_nseg segments per 32-column group
   // (0: none), starting at float g_off * kSegFloats
@@ -238,9 +239,39 @@ int map_blocks_per_sm(int window, int prec, bool chunks);
 
 cudaError_t launch_finalize(const TemplateDev *d_T, uint32_t n_templates, const Partial *d_parts,
                             void *d_results, cudaStream_t stream);
-cudaError_t launch_posteriors(const TemplateDev *d_T, const float *d_Fmn, void *d_result,
-                              double *d_rowsum, double *d_colsum, uint32_t N_t0,
-                              uint32_t N_tau, cudaStream_t stream);
+// Posterior indices of templates whose maps were written: blocks of `rows`
+// t0 rows x `cols` columns (a multiple of 1024) leave row sums per column
+// chunk (rowsum + row_off + chunk * N_t0) and column sums per row chunk
+// (colsum + col_off + chunk * N_tau); up to kPostParts blocks per template and
+// direction then leave their first maximum in `parts`.
+constexpr uint32_t kPostParts = 32;
+struct PostPart {
+  double v;
+  int64_t i;
+};
+struct PostLayout {
+  uint32_t rows, cols, n_chunks;
+  const uint2 *chunks;  // (template, chunk); NULL: template 0's chunks
+  double *rowsum, *colsum;
+  PostPart *parts;      // 2 kPostParts per template
+  uint32_t *ticket;     // one per template
+};
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+inline uint32_t post_part_entries(uint32_t n) {
+  const uint32_t e = (n + kPostParts - 1u) / kPostParts;
+  return e < 256u ? 256u : e;
+}
+// Rows per block for maps of `cells` cells in all: 256, fewer where that
+// leaves fewer than 8 blocks per SM, 16 at least.
+inline uint32_t post_rows(uint64_t cells, int n_sms) {
+  uint32_t rows = 256;
+  while (rows > 16u && cells / ((uint64_t)rows * 1024u) < (uint64_t)n_sms * 8u) rows >>= 1;
+  return rows;
+}
+cudaError_t launch_posteriors(const TemplateDev *d_T, uint32_t n_templates, const PostLayout &L,
+                              const float *d_maps, tcw_result *d_results, cudaStream_t stream);
 
 // ---------------------------------------------------------------- differentiable path
 // One template with a continuous tau grid (tcw_diff.cu).  Exponential
@@ -322,16 +353,6 @@ unsigned int dcheck_failures_kernels();
 unsigned int dcheck_failures_diff();
 unsigned int dcheck_failures_f64();
 unsigned int dcheck_failures_noalloc();
-// Posterior indices of every template of a plan from its written maps:
-// per column chunk (template, first column; kPostCols columns) one block
-// reads its part of the map once and stores its row partials
-// (d_rowpart + row_off + chunk * N_t0), then one warp per template takes
-// the argmaxes.
-constexpr uint32_t kPostCols = 1024;
-cudaError_t launch_plan_posteriors(const TemplateDev *d_T, uint32_t n_templates,
-                                   const uint2 *d_chunks, uint32_t n_chunks, const float *d_maps,
-                                   tcw_result *d_results, float *d_rowpart, double *d_colsum,
-                                   cudaStream_t stream);
 // Full-FP64 direct-summation map of rows rows[0..n_rows) (all rows when rows
 // is NULL) into F[r * N_tau + n]; cond optional.
 cudaError_t launch_map_f64(int window, const float *atoms, const Geom &g, const uint32_t *t0s,

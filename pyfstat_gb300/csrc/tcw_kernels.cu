@@ -15,9 +15,9 @@
 //                    load per recurrence step)
 //   finalize_kernel  per template, merges the tile partials in a fixed order:
 //                    maxF, argmax, lnBtSG in FP64.
-//   posterior kernels  row / column sums of exp(F - maxF) over a written map and
-//                    their argmax (t0 / tau max-posterior bins): one template
-//                    (plain path) or every template of a plan
+//   posterior kernels  row / column sums of exp(F - maxF) over written maps and
+//                    their argmax (t0 / tau max-posterior bins), for one
+//                    template or every template of a plan
 //                    (post_sums_kernel, post_argmax_kernel).
 // No tensor cores: nothing on this path is a dense contraction.
 #include <math.h>
@@ -903,110 +903,6 @@ __global__ void __launch_bounds__(128) finalize_kernel(const TemplateDev *__rest
   }
 }
 
-// ------------------------------------------------------------------ posteriors
-
-constexpr uint32_t kColChunk = 64;
-
-__global__ void __launch_bounds__(256) rowsum_kernel(const float *__restrict__ Fmn,
-                                                     const tcw_result *__restrict__ res,
-                                                     uint32_t N_tau, double *__restrict__ rowsum) {
-  const float maxF = res->maxF;
-  const float *row = Fmn + (size_t)blockIdx.x * N_tau;
-  float s = 0.0f, c = 0.0f;
-  for (uint32_t n = threadIdx.x; n < N_tau; n += blockDim.x) {
-    float y = fsub(exp2f((row[n] - maxF) * kLog2e), c);
-    float t = fadd(s, y);
-    c = fsub(fsub(t, s), y);
-    s = t;
-  }
-  double v = (double)s - (double)c;
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-  __shared__ double sh[8];
-  if ((threadIdx.x & 31u) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double tot = 0.0;
-    for (int w = 0; w < 8; w++) tot += sh[w];
-    rowsum[blockIdx.x] = tot;
-  }
-}
-
-__global__ void __launch_bounds__(128) colsum_kernel(const float *__restrict__ Fmn,
-                                                     const tcw_result *__restrict__ res,
-                                                     uint32_t N_t0, uint32_t N_tau,
-                                                     double *__restrict__ colpart) {
-  const uint32_t n = blockIdx.x * 128u + threadIdx.x;
-  if (n >= N_tau) return;
-  const float maxF = res->maxF;
-  const uint32_t m0 = blockIdx.y * kColChunk, m1 = min(N_t0, m0 + kColChunk);
-  float s = 0.0f, c = 0.0f;
-  for (uint32_t m = m0; m < m1; m++) {
-    float y = fsub(exp2f((Fmn[(size_t)m * N_tau + n] - maxF) * kLog2e), c);
-    float t = fadd(s, y);
-    c = fsub(fsub(t, s), y);
-    s = t;
-  }
-  colpart[(size_t)blockIdx.y * N_tau + n] = (double)s - (double)c;
-}
-
-// First-occurrence argmax of the row sums and of the chunked column sums.
-__global__ void __launch_bounds__(1024) posterior_argmax_kernel(const double *__restrict__ rowsum,
-                                                                const double *__restrict__ colpart,
-                                                                uint32_t N_t0, uint32_t N_tau,
-                                                                uint32_t n_chunks,
-                                                                tcw_result *__restrict__ res) {
-  __shared__ double sv[32];
-  __shared__ int64_t si[32];
-  for (int pass = 0; pass < 2; pass++) {
-    const uint32_t N = pass == 0 ? N_t0 : N_tau;
-    double best = -1.0;
-    int64_t bidx = INT64_MAX;
-    for (uint32_t k = threadIdx.x; k < N; k += blockDim.x) {
-      double v;
-      if (pass == 0) {
-        v = rowsum[k];
-      } else {
-        v = 0.0;
-        for (uint32_t ch = 0; ch < n_chunks; ch++) v += colpart[(size_t)ch * N_tau + k];
-      }
-      if (v > best) {  // k increases within a thread: keeps the first
-        best = v;
-        bidx = k;
-      }
-    }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-      double ob = __shfl_xor_sync(0xffffffffu, best, d);
-      int64_t oi = __shfl_xor_sync(0xffffffffu, bidx, d);
-      if (ob > best || (ob == best && oi < bidx)) {
-        best = ob;
-        bidx = oi;
-      }
-    }
-    if ((threadIdx.x & 31u) == 0) {
-      sv[threadIdx.x >> 5] = best;
-      si[threadIdx.x >> 5] = bidx;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      best = sv[0];
-      bidx = si[0];
-      for (uint32_t w = 1; w < blockDim.x / 32u; w++) {
-        if (sv[w] > best || (sv[w] == best && si[w] < bidx)) {
-          best = sv[w];
-          bidx = si[w];
-        }
-      }
-      if (pass == 0)
-        res->t0_mp_idx = bidx;
-      else
-        res->tau_mp_idx = bidx;
-    }
-    __syncthreads();
-  }
-}
-
 // ------------------------------------------------------------------ launchers
 
 // Templates up to which a prefix scan takes a cluster each (8 x 148 blocks
@@ -1129,16 +1025,16 @@ int map_blocks_per_sm(int window, int prec, bool chunks) {
                                    : blocks_per_sm_win<TCW_WINDOW_EXP, false>(prec);
 }
 
-// One template, one block: the partials of a large single-template call (up
-// to thousands of tiles) merged by 256 threads; warps' results combined in
-// warp order.
-__global__ void __launch_bounds__(256) finalize_one_kernel(const TemplateDev *__restrict__ T,
-                                                           const Partial *__restrict__ parts,
-                                                           tcw_result *__restrict__ results) {
+// One block per template where there are few (up to thousands of tiles
+// each): its partials merged by 256 threads, warps' results combined in warp
+// order.
+__global__ void __launch_bounds__(256) finalize_block_kernel(const TemplateDev *__restrict__ T,
+                                                             const Partial *__restrict__ parts,
+                                                             tcw_result *__restrict__ results) {
   __shared__ float s_best[8];
   __shared__ int64_t s_bidx[8];
   __shared__ double s_sum[8];
-  const TemplateDev t = T[0];
+  const TemplateDev t = T[blockIdx.x];
   const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
   float best = -INFINITY;
   int64_t bidx = INT64_MAX;
@@ -1189,165 +1085,201 @@ __global__ void __launch_bounds__(256) finalize_one_kernel(const TemplateDev *__
     r.t0_mp_idx = -1;
     r.tau_mp_idx = -1;
     r.status = 0;
-    results[0] = r;
+    results[blockIdx.x] = r;
   }
 }
 
 cudaError_t launch_finalize(const TemplateDev *d_T, uint32_t n_templates, const Partial *d_parts,
                             void *d_results, cudaStream_t stream) {
   if (n_templates == 0) return cudaSuccess;
-  if (n_templates == 1)
-    finalize_one_kernel<<<1, 256, 0, stream>>>(d_T, d_parts,
-                                               reinterpret_cast<tcw_result *>(d_results));
+  if (n_templates <= 1024)  // (a warp each: 38 us for 3 templates of 2100 x 1581 cells)
+    finalize_block_kernel<<<n_templates, 256, 0, stream>>>(
+        d_T, d_parts, reinterpret_cast<tcw_result *>(d_results));
   else
     finalize_kernel<<<(n_templates + 3u) / 4u, 128, 0, stream>>>(
         d_T, n_templates, d_parts, reinterpret_cast<tcw_result *>(d_results));
   return cudaGetLastError();
 }
 
-// Batched posteriors of a plan whose maps were written (tcw:219-287): the
-// row and column sums of exp(F - maxF) in one read of the maps.  A block
-// owns kPostCols columns of one template: each thread sums its four
-// adjacent columns down the rows (FP32, Kahan); the block's row sums (the
-// thread's four terms, warp shuffles, then shared memory) are stored per
-// column chunk and summed in FP64 by the argmax kernel (no global atomics).
-constexpr uint32_t kPostRowTile = 1024;
-constexpr uint32_t kPostThreads = 256;  // kPostCols / 4: four adjacent columns per thread
+// Posteriors of written maps (tcw:219-287): the row and column sums of
+// exp(F - maxF) in one read of the maps, then their first argmaxes.
+//
+// post_sums_kernel: a block takes `rows` t0 rows x `cols` columns of one
+// template (the whole of it in 1024-column strips); its threads walk four rows
+// at a time over four columns each, 256 apart (whole-line loads).  Column sums
+// are FP32 with Kahan compensation per thread, row sums double-words added
+// over the warp by recursive halving (six steps for four rows) and over the
+// block's warps in order: no atomics.  Bound by issue (~16 instructions per
+// cell) and the map's read: 137e6 cells of 96 templates 924 -> 225 us (2.4
+// TB/s; before, one block per template and 1024 columns walked all rows).
+// post_argmax_kernel: per template up to kPostParts blocks each for rows and
+// columns add the chunks' sums in FP64 and leave their first maximum; the
+// template's last block picks among them in index order (same maps: 68 ->
+// 33 us with one warp per template before).
+constexpr uint32_t kPostThreads = 256;
+constexpr uint32_t kPostCols = 1024;
+constexpr uint32_t kPostMaxRows = 256;
 
 __global__ void __launch_bounds__(kPostThreads) post_sums_kernel(
-    const TemplateDev *__restrict__ T, const uint2 *__restrict__ chunks,
-    const float *__restrict__ maps, const tcw_result *__restrict__ results,
-    float *__restrict__ rowpart, double *__restrict__ colsum) {
-  __shared__ float srow[kPostRowTile];
-  const uint2 ch = chunks[blockIdx.x];
+    const TemplateDev *__restrict__ T, const uint2 *__restrict__ chunks, uint32_t rows,
+    uint32_t cols, const float *__restrict__ maps, const tcw_result *__restrict__ results,
+    double *__restrict__ rowsum, double *__restrict__ colsum, uint32_t *__restrict__ ticket) {
+  __shared__ float2 srow[kPostThreads / 32][kPostMaxRows];
+  uint2 ch;  // template, chunk within it (column chunk fastest)
+  if (chunks)
+    ch = chunks[blockIdx.x];
+  else
+    ch = make_uint2(0u, blockIdx.x);
   const TemplateDev t = T[ch.x];
+  const uint32_t n_cc = (t.N_tau + cols - 1u) / cols;
+  const uint32_t cc = ch.y % n_cc, rc = ch.y / n_cc;
+  const uint32_t m0 = rc * rows, m1 = min(t.N_t0, m0 + rows);
+  const uint32_t nb = cc * cols, ne = min(t.N_tau, nb + cols);
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
+  if (ch.y == 0u && tid == 0u) ticket[ch.x] = 0u;
   const float maxF = results[ch.x].maxF;
   const float *F = maps + t.map_off;
-  const uint32_t n0 = ch.y + 4u * threadIdx.x;  // this thread's first column
-  const uint32_t lane = threadIdx.x & 31u;
-  float *rp = rowpart + t.row_off + (size_t)(ch.y / kPostCols) * t.N_t0;  // this chunk's rows
-  float cs[4] = {0, 0, 0, 0}, cc[4] = {0, 0, 0, 0};
-  for (uint32_t m0 = 0; m0 < t.N_t0; m0 += kPostRowTile) {
-    const uint32_t m1 = min(t.N_t0, m0 + kPostRowTile);
-    for (uint32_t k = threadIdx.x; k < kPostRowTile; k += kPostThreads) srow[k] = 0.0f;
-    __syncthreads();
-    // four rows per step: independent loads and shuffle chains
+  for (uint32_t k = lane; k < m1 - m0; k += 32u) srow[wid][k] = make_float2(0.0f, 0.0f);
+  __syncwarp();
+  for (uint32_t n0 = nb + tid; n0 - tid < ne; n0 += kPostCols) {
+    float cs[4] = {0, 0, 0, 0}, cc4[4] = {0, 0, 0, 0};
     for (uint32_t m = m0; m < m1; m += 4u) {
-      float w[4];
+      FF w[4];
 #pragma unroll
       for (int q = 0; q < 4; q++) {
-        const uint32_t mq = m + q;
-        const float *row = F + (size_t)mq * t.N_tau;
+        const float *row = F + (size_t)(m + q) * t.N_tau;
         float e[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++)
-          e[j] = (mq < m1 && n0 + j < t.N_tau) ? ex2_approx((row[n0 + j] - maxF) * kLog2e) : 0.0f;
+        for (int j = 0; j < 4; j++) {
+          const uint32_t n = n0 + 256u * j;
+          e[j] = (m + q < m1 && n < ne) ? ex2_approx((__ldg(row + n) - maxF) * kLog2e) : 0.0f;
+        }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-          const float y = fsub(e[j], cc[j]);
+          const float y = fsub(e[j], cc4[j]);
           const float u = fadd(cs[j], y);
-          cc[j] = fsub(fsub(u, cs[j]), y);
+          cc4[j] = fsub(fsub(u, cs[j]), y);
           cs[j] = u;
         }
-        w[q] = fadd(fadd(e[0], e[1]), fadd(e[2], e[3]));
+        w[q] = ff_add1(ff_add1(ff_add1(FF{e[0], 0.0f}, e[1]), e[2]), e[3]);
       }
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) w[q] += __shfl_xor_sync(0xffffffffu, w[q], d);
+      // four rows over 32 lanes: a lane keeps half of its rows per step
+      auto xch = [&](FF v, int d) {
+        return FF{__shfl_xor_sync(0xffffffffu, v.h, d), __shfl_xor_sync(0xffffffffu, v.l, d)};
+      };
+      const bool u16 = (lane & 16u) != 0u, u8 = (lane & 8u) != 0u;
+      const FF a0 = ff_add(u16 ? w[2] : w[0], xch(u16 ? w[0] : w[2], 16));
+      const FF a1 = ff_add(u16 ? w[3] : w[1], xch(u16 ? w[1] : w[3], 16));
+      FF v = ff_add(u8 ? a1 : a0, xch(u8 ? a0 : a1, 8));
+      v = ff_add(v, xch(v, 4));
+      v = ff_add(v, xch(v, 2));
+      v = ff_add(v, xch(v, 1));
+      const uint32_t r = m - m0 + (u16 ? 2u : 0u) + (u8 ? 1u : 0u);
+      if ((lane & 7u) == 0u && r < m1 - m0) {
+        const float2 o = srow[wid][r];
+        const FF s = ff_add(FF{o.x, o.y}, v);
+        srow[wid][r] = make_float2(s.h, s.l);
       }
-      if (lane == 0) {
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-          if (m + q < m1 && w[q] != 0.0f) atomicAdd(&srow[m + q - m0], w[q]);
-      }
+      __syncwarp();
     }
-    __syncthreads();
-    for (uint32_t k = threadIdx.x; k < m1 - m0; k += kPostThreads) rp[m0 + k] = srow[k];
-    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (n0 + 256u * j < ne)
+        colsum[t.col_off + (size_t)rc * t.N_tau + n0 + 256u * j] =
+            (double)cs[j] - (double)cc4[j];
   }
+  __syncthreads();
+  for (uint32_t k = tid; k < m1 - m0; k += kPostThreads) {
+    double s = 0.0;
 #pragma unroll
-  for (int j = 0; j < 4; j++)
-    if (n0 + j < t.N_tau) colsum[t.col_off + n0 + j] = (double)cs[j] - (double)cc[j];
-}
-
-// One warp per template: first-occurrence argmax of its row sums (the
-// column chunks' partials summed in FP64) and of its column sums.
-__global__ void __launch_bounds__(128) post_argmax_kernel(const TemplateDev *__restrict__ T,
-                                                          uint32_t n_templates,
-                                                          const float *__restrict__ rowpart,
-                                                          const double *__restrict__ colsum,
-                                                          tcw_result *__restrict__ results) {
-  const uint32_t tmpl = blockIdx.x * 4u + (threadIdx.x >> 5);
-  const uint32_t lane = threadIdx.x & 31u;
-  if (tmpl >= n_templates) return;
-  const TemplateDev t = T[tmpl];
-  int64_t out[2];
-  for (int pass = 0; pass < 2; pass++) {
-    const uint32_t N = pass == 0 ? t.N_t0 : t.N_tau;
-    const uint32_t n_chunks = (t.N_tau + kPostCols - 1u) / kPostCols;
-    double best = -1.0;
-    int64_t bidx = INT64_MAX;
-    for (uint32_t k = lane; k < N; k += 32u) {
-      double x;
-      if (pass == 0) {
-        x = 0.0;
-        for (uint32_t c = 0; c < n_chunks; c++) x += (double)rowpart[t.row_off + (size_t)c * N + k];
-      } else {
-        x = colsum[t.col_off + k];
-      }
-      if (x > best) {  // k increases within a lane: keeps the first
-        best = x;
-        bidx = k;
-      }
-    }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-      const double ob = __shfl_xor_sync(0xffffffffu, best, d);
-      const int64_t oi = __shfl_xor_sync(0xffffffffu, bidx, d);
-      if (ob > best || (ob == best && oi < bidx)) {
-        best = ob;
-        bidx = oi;
-      }
-    }
-    out[pass] = bidx == INT64_MAX ? -1 : bidx;
-  }
-  if (lane == 0) {
-    results[tmpl].t0_mp_idx = out[0];
-    results[tmpl].tau_mp_idx = out[1];
+    for (uint32_t w = 0; w < kPostThreads / 32u; w++)
+      s += (double)srow[w][k].x + (double)srow[w][k].y;
+    rowsum[t.row_off + (size_t)cc * t.N_t0 + m0 + k] = s;
   }
 }
 
-cudaError_t launch_plan_posteriors(const TemplateDev *d_T, uint32_t n_templates,
-                                   const uint2 *d_chunks, uint32_t n_chunks, const float *d_maps,
-                                   tcw_result *d_results, float *d_rowpart, double *d_colsum,
-                                   cudaStream_t stream) {
-  if (n_chunks) {
-    post_sums_kernel<<<n_chunks, kPostThreads, 0, stream>>>(d_T, d_chunks, d_maps, d_results,
-                                                            d_rowpart, d_colsum);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+struct PostBest {
+  double v;
+  int64_t i;
+};
+__device__ __forceinline__ PostBest post_better(PostBest a, PostBest b) {
+  return b.v > a.v || (b.v == a.v && b.i < a.i) ? b : a;
+}
+__device__ __forceinline__ PostBest post_block_best(PostBest best, PostBest *sh) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    PostBest o;
+    o.v = __shfl_xor_sync(0xffffffffu, best.v, d);
+    o.i = __shfl_xor_sync(0xffffffffu, best.i, d);
+    best = post_better(best, o);
   }
-  post_argmax_kernel<<<(n_templates + 3u) / 4u, 128, 0, stream>>>(d_T, n_templates, d_rowpart,
-                                                                  d_colsum, d_results);
-  return cudaGetLastError();
+  if ((threadIdx.x & 31u) == 0) sh[threadIdx.x >> 5] = best;
+  __syncthreads();
+  best = sh[0];
+  for (uint32_t w = 1; w < kPostThreads / 32u; w++) best = post_better(best, sh[w]);
+  return best;
 }
 
-cudaError_t launch_posteriors(const TemplateDev *d_T, const float *d_Fmn, void *d_result,
-                              double *d_rowsum, double *d_colsum, uint32_t N_t0,
-                              uint32_t N_tau, cudaStream_t stream) {
-  (void)d_T;
-  tcw_result *res = reinterpret_cast<tcw_result *>(d_result);
-  rowsum_kernel<<<N_t0, 256, 0, stream>>>(d_Fmn, res, N_tau, d_rowsum);
-  cudaError_t e = cudaGetLastError();
+__global__ void __launch_bounds__(kPostThreads) post_argmax_kernel(
+    const TemplateDev *__restrict__ T, uint32_t rows, uint32_t cols,
+    const double *__restrict__ rowsum, const double *__restrict__ colsum,
+    PostPart *__restrict__ parts, uint32_t *__restrict__ ticket,
+    tcw_result *__restrict__ results) {
+  __shared__ PostBest sh[kPostThreads / 32];
+  __shared__ uint32_t s_last;
+  const uint32_t k = blockIdx.y;
+  const TemplateDev t = T[k];
+  const uint32_t e_row = post_part_entries(t.N_t0), e_col = post_part_entries(t.N_tau);
+  const uint32_t p_row = (t.N_t0 + e_row - 1u) / e_row, p_col = (t.N_tau + e_col - 1u) / e_col;
+  const uint32_t n_parts = p_row + p_col, part = blockIdx.x;
+  if (part >= n_parts) return;
+  const bool is_row = part < p_row;
+  const uint32_t N = is_row ? t.N_t0 : t.N_tau, e = is_row ? e_row : e_col;
+  const uint32_t i0 = (is_row ? part : part - p_row) * e, i1 = min(N, i0 + e);
+  const uint32_t n_sum = is_row ? (t.N_tau + cols - 1u) / cols : (t.N_t0 + rows - 1u) / rows;
+  const double *S = is_row ? rowsum + t.row_off : colsum + t.col_off;
+  PostBest best{-1.0, INT64_MAX};
+  for (uint32_t i = i0 + threadIdx.x; i < i1; i += kPostThreads) {
+    double v = 0.0;
+#pragma unroll 4
+    for (uint32_t c = 0; c < n_sum; c++) v += S[(size_t)c * N + i];
+    if (v > best.v) best = PostBest{v, (int64_t)i};  // i increases: keeps the first
+  }
+  best = post_block_best(best, sh);
+  PostPart *mine = parts + (size_t)k * (2u * kPostParts);
+  if (threadIdx.x == 0) {
+    mine[is_row ? part : kPostParts + part - p_row] = PostPart{best.v, best.i};
+    __threadfence();
+    s_last = atomicAdd(ticket + k, 1u) == n_parts - 1u ? 1u : 0u;
+  }
+  __syncthreads();
+  if (!s_last || threadIdx.x >= 2u) return;
+  __threadfence();
+  // thread 0 the rows' parts, thread 1 the columns'
+  const uint32_t n = threadIdx.x == 0 ? p_row : p_col;
+  const volatile PostPart *v = mine + threadIdx.x * kPostParts;
+  PostBest b{-1.0, INT64_MAX};
+  for (uint32_t q = 0; q < n; q++) b = post_better(b, PostBest{v[q].v, v[q].i});
+  const int64_t idx = b.i == INT64_MAX ? -1 : b.i;
+  if (threadIdx.x == 0)
+    results[k].t0_mp_idx = idx;
+  else
+    results[k].tau_mp_idx = idx;
+}
+
+cudaError_t launch_posteriors(const TemplateDev *d_T, uint32_t n_templates, const PostLayout &L,
+                              const float *d_maps, tcw_result *d_results, cudaStream_t stream) {
+  if (L.n_chunks == 0 || n_templates == 0) return cudaSuccess;
+  post_sums_kernel<<<L.n_chunks, kPostThreads, 0, stream>>>(
+      d_T, L.chunks, L.rows, L.cols, d_maps, d_results, L.rowsum, L.colsum, L.ticket);
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  const uint32_t n_chunks = (N_t0 + kColChunk - 1u) / kColChunk;
-  dim3 grid((N_tau + 127u) / 128u, n_chunks);
-  colsum_kernel<<<grid, 128, 0, stream>>>(d_Fmn, res, N_t0, N_tau, d_colsum);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  posterior_argmax_kernel<<<1, 1024, 0, stream>>>(d_rowsum, d_colsum, N_t0, N_tau, n_chunks,
-                                                  res);
+  for (uint32_t y0 = 0; y0 < n_templates; y0 += 65535u) {
+    const uint32_t ny = n_templates - y0 < 65535u ? n_templates - y0 : 65535u;
+    post_argmax_kernel<<<dim3(2u * kPostParts, ny), kPostThreads, 0, stream>>>(
+        d_T + y0, L.rows, L.cols, L.rowsum, L.colsum, L.parts + (size_t)y0 * 2u * kPostParts,
+        L.ticket + y0, d_results + y0);
+  }
   return cudaGetLastError();
 }
 

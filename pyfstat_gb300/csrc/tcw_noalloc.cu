@@ -42,23 +42,29 @@ constexpr size_t kNoallocScratchBytes = TCW_NOALLOC_SCRATCH_BYTES;
 constexpr int kMaxDevices = 64;
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocScratchBytes];
+// the posterior argmax's partial maxima and ticket, apart from the scratch
+__device__ PostPart g_noalloc_post[2u * kPostParts + 1u];
 
 std::mutex g_scratch_mu;
 void *g_scratch_ptr[kMaxDevices] = {nullptr};
+void *g_post_ptr[kMaxDevices] = {nullptr};
 
-// Device address of the scratch array on the current device (cached).
-int scratch_address(int device, unsigned char **out) {
+// Device addresses of the two arrays on the current device (cached).
+int scratch_address(int device, unsigned char **out, PostPart **post) {
   if (device < 0 || device >= kMaxDevices) return TCW_ERR_NO_DEVICE;
   std::lock_guard<std::mutex> lock(g_scratch_mu);
   if (!g_scratch_ptr[device]) {
-    void *p = nullptr;
+    void *p = nullptr, *q = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-    if (e != cudaSuccess || !p) {
+    if (e == cudaSuccess) e = cudaGetSymbolAddress(&q, g_noalloc_post);
+    if (e != cudaSuccess || !p || !q) {
       cudaGetLastError();
       return TCW_ERR_CUDA;
     }
+    g_post_ptr[device] = q;
     g_scratch_ptr[device] = p;
   }
+  *post = static_cast<PostPart *>(g_post_ptr[device]);
   *out = static_cast<unsigned char *>(g_scratch_ptr[device]);
   return TCW_OK;
 }
@@ -177,7 +183,8 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
   if (!fits) return TCW_ERR_OVERFLOW;
 
   unsigned char *base = nullptr;
-  int rc = scratch_address(device, &base);
+  PostPart *pp = nullptr;
+  int rc = scratch_address(device, &base, &pp);
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
@@ -227,10 +234,14 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
   ml.parts = dparts;
   if (launch_map(window, ml, s) != cudaSuccess) return TCW_ERR_CUDA;
   if (launch_finalize(dT, 1, dparts, d_result, s) != cudaSuccess) return TCW_ERR_CUDA;
-  if (post && launch_posteriors(dT, d_Fmn, d_result, reinterpret_cast<double *>(base + o_row),
-                                reinterpret_cast<double *>(base + o_col), N_t0, N_tau,
-                                s) != cudaSuccess)
-    return TCW_ERR_CUDA;
+  if (post) {
+    // one column chunk per row chunk of 64 rows: the documented scratch
+    const PostLayout pl{64u, (N_tau + 1023u) / 1024u * 1024u, n_chunks, nullptr,
+                        reinterpret_cast<double *>(base + o_row),
+                        reinterpret_cast<double *>(base + o_col), pp,
+                        reinterpret_cast<uint32_t *>(pp + 2u * kPostParts)};
+    if (launch_posteriors(dT, 1, pl, d_Fmn, d_result, s) != cudaSuccess) return TCW_ERR_CUDA;
+  }
   return TCW_OK;
 }
 
