@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -40,7 +41,6 @@ struct tcw_handle {
   cudaEvent_t stage_ev = nullptr;
   bool stage_pending = false;
   int fail_alloc_countdown = 0;
-  tcw_tile_config plain_cfg{};
   char err[512] = {0};
 };
 
@@ -209,13 +209,10 @@ int prec_of(int flags) {
   return kPrecFF;
 }
 
-// Tiles of one template.  Rect: tn columns x tm rows per block.  Exp: tn
-// columns per block over the 128 / tn next row chunks (t.e_rows rows each);
-// with `warp_tiles` (persistent plans, whose exp kernel schedules by warp) 32
-// columns over one chunk per tile.
+// A plan's tiles of one template.  Rect: tn columns x tm rows.  Exp: 32 columns
+// x one row chunk (t.e_rows rows).
 void tile_template(uint32_t tmpl, const TemplateDev &t, const tcw_tile_config &cfg,
-                   std::vector<WorkItem> &items, std::vector<double> *cost,
-                   bool warp_tiles = false) {
+                   std::vector<WorkItem> &items, std::vector<double> &cost) {
   const uint32_t N_t0 = t.N_t0, N_tau = t.N_tau;
   if (t.window == TCW_WINDOW_RECT) {
     const uint32_t tn = cfg.rect_tn, tm = cfg.rect_tm;
@@ -229,31 +226,28 @@ void tile_template(uint32_t tmpl, const TemplateDev &t, const tcw_tile_config &c
         w.n1 = std::min(N_tau, n0 + tn);
         w.tn = (uint16_t)(tm / 32u);  // row groups of 32 rows (one per warp)
         items.push_back(w);
-        if (cost) cost->push_back((double)(w.m1 - w.m0) * (w.n1 - w.n0));
+        cost.push_back((double)(w.m1 - w.m0) * (w.n1 - w.n0));
       }
   } else {
-    const uint32_t tn = warp_tiles ? 32u : cfg.exp_tn, lanes = warp_tiles ? 1u : kBlock / tn;
     const uint32_t chunks = (N_t0 + t.e_hist - 1u) / t.e_hist * t.e_sub;
-    for (uint32_t n0 = 0; n0 < N_tau; n0 += tn)
-      for (uint32_t c0 = 0; c0 < chunks; c0 += lanes) {
+    for (uint32_t n0 = 0; n0 < N_tau; n0 += 32u)
+      for (uint32_t c = 0; c < chunks; c++) {
         WorkItem w{};
         w.tmpl = tmpl;
-        w.m0 = c0;
-        w.m1 = std::min(chunks, c0 + lanes);
+        w.m0 = c;
+        w.m1 = c + 1u;
         w.n0 = n0;
-        w.n1 = std::min(N_tau, n0 + tn);
-        w.tn = (uint16_t)tn;
+        w.n1 = std::min(N_tau, n0 + 32u);
+        w.tn = 32;
         items.push_back(w);
-        if (cost) {
-          // recurrence steps: window warm-up plus the rows' atom span, per column
-          double atoms_per_row = 1.0;
-          if (N_t0 > 1) atoms_per_row = std::max(1.0, (double)t.g.numAtoms / N_t0);
-          const double rows_here = std::min(N_t0, t.e_rows);
-          double warm = std::min((double)t.g.numAtoms, 3.0 * (double)N_tau) * lanes;
-          if (t.g_nseg) warm = std::min(warm, 2.0 * (double)(1u << t.g_shift));
-          cost->push_back(((rows_here * atoms_per_row * 2.0 + warm) * 2.0 + rows_here) *
-                          (w.n1 - w.n0) / 1.0);
-        }
+        // recurrence steps: window warm-up plus the rows' atom span, per column
+        double atoms_per_row = 1.0;
+        if (N_t0 > 1) atoms_per_row = std::max(1.0, (double)t.g.numAtoms / N_t0);
+        const double rows_here = std::min(N_t0, t.e_rows);
+        double warm = std::min((double)t.g.numAtoms, 3.0 * (double)N_tau);
+        if (t.g_nseg) warm = std::min(warm, 2.0 * (double)(1u << t.g_shift));
+        cost.push_back(((rows_here * atoms_per_row * 2.0 + warm) * 2.0 + rows_here) *
+                       (w.n1 - w.n0));
       }
   }
 }
@@ -267,21 +261,6 @@ void tile_template(uint32_t tmpl, const TemplateDev &t, const tcw_tile_config &c
 // Rows of a history for exp_rows of a tile configuration (0: whole columns).
 uint32_t exp_hist(uint32_t exp_rows, uint32_t N_t0) {
   return std::min(std::min(exp_rows ? exp_rows : N_t0, N_t0), 65535u);
-}
-
-void default_plain_cfg(const TemplateDev &t, tcw_tile_config &cfg, int n_sms) {
-  const uint64_t target_blocks = (uint64_t)n_sms * 4u;
-  if (t.window == TCW_WINDOW_RECT) {
-    // 32-row tiles; columns per tile so that the grid has ~4 blocks per SM,
-    // at least 4 columns per warp and at most 256
-    cfg.rect_tm = 32;
-    const uint64_t row_tiles = (t.N_t0 + 31u) / 32u;
-    uint64_t tn = (uint64_t)t.N_tau * row_tiles / std::max<uint64_t>(1, target_blocks);
-    tn = std::max<uint64_t>(16, std::min<uint64_t>(256, tn));
-    cfg.rect_tn = (uint32_t)tn;
-  } else {
-    cfg.exp_tn = 32;
-  }
 }
 
 void fill_cfg_defaults(tcw_tile_config &c) {
@@ -298,6 +277,7 @@ TemplateDev make_tdev(uint32_t numAtoms, uint32_t TAtom, uint32_t t0_data, int w
   t.window = (uint32_t)window;
   t.N_t0 = N_t0;
   t.N_tau = N_tau;
+  t.ln_prior = log(70.0 / ((double)N_t0 * (double)N_tau));
   return t;
 }
 
@@ -519,113 +499,102 @@ int tcw_debug_fail_alloc(tcw_handle *h, int n) {
 
 // ---------------------------------------------------------------- plain map
 
-static int plain_enqueue(tcw_handle *h, const float *d_atoms, uint32_t numAtoms, uint32_t TAtom,
-                         uint32_t t0_data, int window, const uint32_t *d_t0s, uint32_t N_t0,
-                         const uint32_t *d_taus, uint32_t N_tau, float *d_Fmn,
-                         tcw_result *d_result, int flags, char *ws, size_t ws_off) {
-  TemplateDev t = make_tdev(numAtoms, TAtom, t0_data, window, N_t0, N_tau);
-  tcw_tile_config cfg = h->plain_cfg;
-  const int prec = prec_of(flags);
-  default_plain_cfg(t, cfg, h->n_sms);
-  if (h->plain_cfg.rect_tn) cfg.rect_tn = h->plain_cfg.rect_tn;
-  if (h->plain_cfg.rect_tm) cfg.rect_tm = h->plain_cfg.rect_tm;
-  if (h->plain_cfg.exp_tn) cfg.exp_tn = h->plain_cfg.exp_tn;
+// Inputs of a host-buffer map that go through page-locked staging.
+constexpr size_t kStagedInputs = 1u << 20;
+
+// Descriptor and workspace of one single-template map behind `off` bytes.
+struct PlainLayout {
+  TemplateDev t;
+  uint32_t n_items, n_seg_items, seg_per, post_rows, post_chunks;
+  size_t o_T, o_parts, o_rows, o_G, o_row, o_col, o_pp, total;
+};
+
+static int plain_layout(tcw_handle *h, uint32_t numAtoms, uint32_t TAtom, uint32_t t0_data,
+                        int window, uint32_t N_t0, uint32_t N_tau, int flags, size_t off,
+                        PlainLayout &P) {
+  TemplateDev &t = P.t;
+  t = make_tdev(numAtoms, TAtom, t0_data, window, N_t0, N_tau);
   uint64_t seg_floats = 0;
-  uint32_t n_seg_items = 0, seg_per = 1;
+  P.n_seg_items = 0;
+  P.seg_per = 1;
   if (window == TCW_WINDOW_EXP) {
-    const ExpSplit sp = plain_exp_split(numAtoms, N_t0, N_tau, h->n_sms, prec != kPrecPlain32);
+    const ExpSplit sp =
+        plain_exp_split(numAtoms, N_t0, N_tau, h->n_sms, prec_of(flags) != kPrecPlain32);
     set_split(t, sp);
     seg_floats = sp.seg_floats(N_tau);
     const uint32_t groups = (N_tau + 31u) / 32u;
-    seg_per = segs_per_warp((uint64_t)groups * sp.nseg, h->n_sms);
-    n_seg_items = groups * ((sp.nseg + seg_per - 1u) / seg_per);
+    P.seg_per = segs_per_warp((uint64_t)groups * sp.nseg, h->n_sms);
+    P.n_seg_items = groups * ((sp.nseg + P.seg_per - 1u) / P.seg_per);
   }
-  fill_cfg_defaults(cfg);
-  std::vector<WorkItem> items;
-  try {
-    tile_template(0, t, cfg, items, nullptr);
-  } catch (const std::bad_alloc &) {
-    return set_err(h, TCW_ERR_ALLOC, "host allocation of the tile list failed");
-  }
-  const uint32_t n_items = (uint32_t)items.size();
-  for (uint32_t k = 0; k < n_items; k++) items[k].part = k;
-  t.part_off = 0;
-  t.n_parts = n_items;
-  t.p_off = 0;
-  t.map_off = 0;
-
+  const uint64_t tiles = plain_tiles(t, h->n_sms);
+  if (tiles > 0x7FFFFFFFull) return set_err(h, TCW_ERR_OVERFLOW, "too many tiles");
+  P.n_items = t.n_parts = (uint32_t)tiles;
   const bool post = (flags & TCW_FLAG_POSTERIORS) != 0;
-  const uint32_t prows = post_rows((uint64_t)N_t0 * N_tau, h->n_sms);
-  const uint32_t n_rc = (N_t0 + prows - 1u) / prows, n_cc = (N_tau + 1023u) / 1024u;
+  P.post_rows = post_rows((uint64_t)N_t0 * N_tau, h->n_sms);
+  const uint32_t n_rc = (N_t0 + P.post_rows - 1u) / P.post_rows, n_cc = (N_tau + 1023u) / 1024u;
+  P.post_chunks = n_rc * n_cc;
   Layout L;
-  L.total = ws_off;
-  const size_t o_T = L.add(sizeof(TemplateDev));
-  const size_t o_list = L.add(sizeof(uint32_t));  // {0}: the one template
-  const size_t o_items = L.add(sizeof(WorkItem) * n_items);
-  const size_t o_parts = L.add(sizeof(Partial) * n_items);
-  const size_t o_P = window == TCW_WINDOW_RECT
-                         ? L.add(sizeof(float) * kPrefixStride * ((size_t)numAtoms + 1))
-                         : 0;
-  const size_t o_A8 = window == TCW_WINDOW_EXP
-                          ? L.add(sizeof(float) * 8u * (size_t)numAtoms)
-                          : 0;
-  const size_t o_G = L.add(sizeof(float) * seg_floats);
-  const size_t o_row = post ? L.add(sizeof(double) * (size_t)N_t0 * n_cc) : 0;
-  const size_t o_col = post ? L.add(sizeof(double) * (size_t)n_rc * N_tau) : 0;
-  const size_t o_pp = post ? L.add(sizeof(PostPart) * 2u * kPostParts + sizeof(uint32_t)) : 0;
-  int rc = ensure_ws(h, L.total);
-  if (rc) return rc;
-  ws = h->d_ws;  // the workspace may have moved
-  const size_t ctl_bytes = o_parts - o_T;
-  rc = ensure_stage(h, ctl_bytes);
-  if (rc) return rc;
-  char *st = h->h_stage;
-  memcpy(st, &t, sizeof(t));
-  uint32_t zero = 0;
-  memcpy(st + (o_list - o_T), &zero, sizeof(zero));
-  memcpy(st + (o_items - o_T), items.data(), sizeof(WorkItem) * n_items);
-  TCW_CUDA(h, cudaMemcpyAsync(ws + o_T, st, ctl_bytes, cudaMemcpyHostToDevice, h->stream));
-  TCW_CUDA(h, cudaEventRecord(h->stage_ev, h->stream));
-  h->stage_pending = true;
+  L.total = off;
+  P.o_T = L.add(sizeof(TemplateDev));
+  P.o_parts = L.add(sizeof(Partial) * P.n_items);
+  P.o_rows = L.add(window == TCW_WINDOW_RECT
+                       ? sizeof(float) * kPrefixStride * ((size_t)numAtoms + 1)
+                       : sizeof(float) * 8u * (size_t)numAtoms);
+  P.o_G = L.add(sizeof(float) * seg_floats);
+  P.o_row = post ? L.add(sizeof(double) * (size_t)N_t0 * n_cc) : 0;
+  P.o_col = post ? L.add(sizeof(double) * (size_t)n_rc * N_tau) : 0;
+  P.o_pp = post ? L.add(sizeof(PostPart) * 2u * kPostParts + sizeof(uint32_t)) : 0;
+  P.total = L.total;
+  return TCW_OK;
+}
 
-  const TemplateDev *dT = reinterpret_cast<const TemplateDev *>(ws + o_T);
-  float *dP = window == TCW_WINDOW_RECT ? reinterpret_cast<float *>(ws + o_P) : nullptr;
-  Partial *dparts = reinterpret_cast<Partial *>(ws + o_parts);
-  if (window == TCW_WINDOW_RECT)
-    TCW_CUDA(h, launch_prefix(dT, reinterpret_cast<const uint32_t *>(ws + o_list), 1, d_atoms,
-                              dP, prec, h->stream));
-  float *dA8 = window == TCW_WINDOW_EXP ? reinterpret_cast<float *>(ws + o_A8) : nullptr;
-  if (window == TCW_WINDOW_EXP)
-    TCW_CUDA(h, launch_repack(dT, reinterpret_cast<const uint32_t *>(ws + o_list), 1, numAtoms,
-                              d_atoms, dA8, h->stream));
-  float *dG = reinterpret_cast<float *>(ws + o_G);
-  TCW_CUDA(h, launch_exp_segments(dT, nullptr, n_seg_items, seg_per, dA8, d_taus, dG,
+// One map: prepare (prefix or repacked rows, the descriptor), exp segment sums,
+// map tiles, finalize, posteriors -- a chain of programmatic dependent
+// launches that needs nothing from the host but their arguments.  `ws_off`:
+// the workspace's first bytes are the caller's.
+static int plain_enqueue(tcw_handle *h, const float *d_atoms, uint32_t numAtoms, uint32_t TAtom,
+                         uint32_t t0_data, int window, const uint32_t *d_t0s, uint32_t N_t0,
+                         const uint32_t *d_taus, uint32_t N_tau, float *d_Fmn,
+                         tcw_result *d_result, int flags, size_t ws_off) {
+  PlainLayout L;
+  int rc = plain_layout(h, numAtoms, TAtom, t0_data, window, N_t0, N_tau, flags, ws_off, L);
+  if (rc) return rc;
+  rc = ensure_ws(h, L.total);
+  if (rc) return rc;
+  char *ws = h->d_ws;
+  const int prec = prec_of(flags);
+  const bool rect = window == TCW_WINDOW_RECT;
+  TemplateDev *dT = reinterpret_cast<TemplateDev *>(ws + L.o_T);
+  float *drows = reinterpret_cast<float *>(ws + L.o_rows);
+  Partial *dparts = reinterpret_cast<Partial *>(ws + L.o_parts);
+  TCW_CUDA(h, launch_prepare_one(L.t, dT, d_atoms, drows, prec, h->stream));
+  float *dG = reinterpret_cast<float *>(ws + L.o_G);
+  TCW_CUDA(h, launch_exp_segments(dT, nullptr, L.n_seg_items, L.seg_per, drows, d_taus, dG,
                                   h->stream));
   MapLaunch ml{};
   ml.T = dT;
-  ml.items = reinterpret_cast<const WorkItem *>(ws + o_items);
-  ml.n_items = n_items;
+  ml.n_items = L.n_items;
   ml.persistent = false;
+  ml.chained = plain_map_chained(L.n_seg_items, numAtoms, h->n_sms);
   ml.write_map = d_Fmn != nullptr;
   ml.prec = prec;
-  ml.priority = h->prio_low;
   ml.atoms = d_atoms;
-  ml.atoms8 = dA8;
+  ml.atoms8 = rect ? nullptr : drows;
   ml.G = dG;
   ml.t0s = d_t0s;
   ml.taus = d_taus;
-  ml.P = dP;
+  ml.P = rect ? drows : nullptr;
   ml.Fmn = d_Fmn;
   ml.parts = dparts;
   TCW_CUDA(h, launch_map(window, ml, h->stream));
-  TCW_CUDA(h, launch_finalize(dT, 1, dparts, d_result, h->stream));
-  if (post) {
-    PostPart *pp = reinterpret_cast<PostPart *>(ws + o_pp);
-    const PostLayout pl{prows, 1024u, n_rc * n_cc, nullptr,
-                        reinterpret_cast<double *>(ws + o_row),
-                        reinterpret_cast<double *>(ws + o_col), pp,
+  TCW_CUDA(h, launch_finalize(dT, 1, dparts, d_result, true, h->stream));
+  if (flags & TCW_FLAG_POSTERIORS) {
+    PostPart *pp = reinterpret_cast<PostPart *>(ws + L.o_pp);
+    const PostLayout pl{L.post_rows, 1024u, L.post_chunks, nullptr,
+                        reinterpret_cast<double *>(ws + L.o_row),
+                        reinterpret_cast<double *>(ws + L.o_col), pp,
                         reinterpret_cast<uint32_t *>(pp + 2u * kPostParts)};
-    TCW_CUDA(h, launch_posteriors(dT, 1, pl, d_Fmn, d_result, h->stream));
+    TCW_CUDA(h, launch_posteriors(dT, 1, pl, d_Fmn, d_result, true, h->stream));
   }
   return TCW_OK;
 }
@@ -649,7 +618,7 @@ int tcw_map_plain(tcw_handle *h, const float *d_atoms, uint32_t numAtoms, uint32
   rc = set_device(h);
   if (rc) return rc;
   return plain_enqueue(h, d_atoms, numAtoms, TAtom, t0_data, window, d_t0s, N_t0, d_taus, N_tau,
-                       d_Fmn, d_result, flags, h->d_ws, 0);
+                       d_Fmn, d_result, flags, 0);
 }
 
 int tcw_map_plain_host(tcw_handle *h, const float *atoms, uint32_t numAtoms, uint32_t TAtom,
@@ -679,71 +648,60 @@ int tcw_map_plain_host(tcw_handle *h, const float *atoms, uint32_t numAtoms, uin
   if (rc) return rc;
   rc = set_device(h);
   if (rc) return rc;
+  // Workspace: the inputs (atoms, t0s, taus) back to back, the result record,
+  // the map, then plain_enqueue's own.  The inputs go up in one copy from
+  // page-locked staging (three pageable copies cost the caller ~10 us each)
+  // where they are small; the record comes back through staging, too.
   const bool want_map = Fmn != nullptr || (flags & TCW_FLAG_POSTERIORS);
+  const size_t b_atoms = sizeof(float) * 7u * (size_t)numAtoms, b_t0 = sizeof(uint32_t) * N_t0,
+               b_tau = sizeof(uint32_t) * N_tau;
   Layout L;
-  const size_t o_atoms = L.add(sizeof(float) * 7u * (size_t)numAtoms);
-  const size_t o_t0 = L.add(sizeof(uint32_t) * N_t0);
-  const size_t o_tau = L.add(sizeof(uint32_t) * N_tau);
-  const size_t o_map = want_map ? L.add(sizeof(float) * (size_t)N_t0 * N_tau) : 0;
+  const size_t o_atoms = L.add(b_atoms);
+  const size_t o_t0 = L.add(b_t0);
+  const size_t o_tau = L.add(b_tau);
+  const size_t in_bytes = L.total;
   const size_t o_res = L.add(sizeof(tcw_result));
-  rc = ensure_ws(h, L.total + (1 << 20));
+  const size_t o_map = want_map ? L.add(sizeof(float) * (size_t)N_t0 * N_tau) : 0;
+  PlainLayout P;
+  rc = plain_layout(h, numAtoms, TAtom, t0_data, window, N_t0, N_tau, flags, L.total, P);
+  if (rc) return rc;
+  rc = ensure_ws(h, P.total);
+  if (rc) return rc;
+  const bool staged = in_bytes <= kStagedInputs;
+  const size_t s_res = align_up(staged ? in_bytes : 0, 64);
+  rc = ensure_stage(h, s_res + sizeof(tcw_result));
   if (rc) return rc;
   char *ws = h->d_ws;
-  TCW_CUDA(h, cudaMemcpyAsync(ws + o_atoms, atoms, sizeof(float) * 7u * (size_t)numAtoms,
-                              cudaMemcpyHostToDevice, h->stream));
-  TCW_CUDA(h, cudaMemcpyAsync(ws + o_t0, t0s, sizeof(uint32_t) * N_t0, cudaMemcpyHostToDevice,
-                              h->stream));
-  TCW_CUDA(h, cudaMemcpyAsync(ws + o_tau, taus, sizeof(uint32_t) * N_tau, cudaMemcpyHostToDevice,
-                              h->stream));
-  // the plain enqueue places its own buffers after ours; growing the
-  // workspace there would move these inputs, so reserve generously first
-  size_t need_after = 0;
-  {
-    Layout L2;
-    L2.total = L.total;
-    L2.add(sizeof(TemplateDev));
-    L2.add(sizeof(uint32_t));
-    uint64_t items_est = (uint64_t)N_t0 * ((N_tau + 31u) / 32u) + 16u;
-    L2.add(sizeof(WorkItem) * items_est);
-    L2.add(sizeof(Partial) * items_est);
-    if (window == TCW_WINDOW_RECT) L2.add(sizeof(float) * kPrefixStride * ((size_t)numAtoms + 1));
-    if (window == TCW_WINDOW_EXP) {
-      L2.add(sizeof(float) * 8u * (size_t)numAtoms);
-      L2.add(sizeof(float) *
-             plain_exp_split(numAtoms, N_t0, N_tau, h->n_sms,
-                             prec_of(flags) != kPrecPlain32)
-                 .seg_floats(N_tau));
-    }
-    L2.add(sizeof(double) * (size_t)N_t0 * ((N_tau + 1023u) / 1024u));
-    L2.add(sizeof(double) * ((N_t0 + 15u) / 16u) * (size_t)N_tau);
-    L2.add(sizeof(PostPart) * 2u * kPostParts + sizeof(uint32_t));
-    need_after = L2.total;
-  }
-  if (need_after > h->ws_cap) {
-    // grow now (synchronises) and redo the input copies into the new buffer
-    rc = ensure_ws(h, need_after);
-    if (rc) return rc;
-    ws = h->d_ws;
-    TCW_CUDA(h, cudaMemcpyAsync(ws + o_atoms, atoms, sizeof(float) * 7u * (size_t)numAtoms,
-                                cudaMemcpyHostToDevice, h->stream));
-    TCW_CUDA(h, cudaMemcpyAsync(ws + o_t0, t0s, sizeof(uint32_t) * N_t0, cudaMemcpyHostToDevice,
-                                h->stream));
-    TCW_CUDA(h, cudaMemcpyAsync(ws + o_tau, taus, sizeof(uint32_t) * N_tau,
-                                cudaMemcpyHostToDevice, h->stream));
+  if (staged) {
+    memcpy(h->h_stage + o_atoms, atoms, b_atoms);
+    memcpy(h->h_stage + o_t0, t0s, b_t0);
+    memcpy(h->h_stage + o_tau, taus, b_tau);
+    TCW_CUDA(h, cudaMemcpyAsync(ws, h->h_stage, in_bytes, cudaMemcpyHostToDevice, h->stream));
+  } else {
+    TCW_CUDA(h, cudaMemcpyAsync(ws + o_atoms, atoms, b_atoms, cudaMemcpyHostToDevice, h->stream));
+    TCW_CUDA(h, cudaMemcpyAsync(ws + o_t0, t0s, b_t0, cudaMemcpyHostToDevice, h->stream));
+    TCW_CUDA(h, cudaMemcpyAsync(ws + o_tau, taus, b_tau, cudaMemcpyHostToDevice, h->stream));
   }
   float *dmap = want_map ? reinterpret_cast<float *>(ws + o_map) : nullptr;
   tcw_result *dres = reinterpret_cast<tcw_result *>(ws + o_res);
   rc = plain_enqueue(h, reinterpret_cast<const float *>(ws + o_atoms), numAtoms, TAtom, t0_data,
                      window, reinterpret_cast<const uint32_t *>(ws + o_t0), N_t0,
-                     reinterpret_cast<const uint32_t *>(ws + o_tau), N_tau, dmap, dres, flags, ws,
+                     reinterpret_cast<const uint32_t *>(ws + o_tau), N_tau, dmap, dres, flags,
                      L.total);
+  // on any error below the stream is drained first: the staging and the
+  // caller's buffers must not be in use when this returns
+  if (rc == TCW_OK) {
+    cudaError_t e = cudaMemcpyAsync(h->h_stage + s_res, dres, sizeof(tcw_result),
+                                    cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess && Fmn)
+      e = cudaMemcpyAsync(Fmn, dmap, sizeof(float) * (size_t)N_t0 * N_tau,
+                          cudaMemcpyDeviceToHost, h->stream);
+    if (e != cudaSuccess) rc = cuda_err(h, e, "result download");
+  }
+  const cudaError_t es = cudaStreamSynchronize(h->stream);
   if (rc) return rc;
-  if (Fmn)
-    TCW_CUDA(h, cudaMemcpyAsync(Fmn, dmap, sizeof(float) * (size_t)N_t0 * N_tau,
-                                cudaMemcpyDeviceToHost, h->stream));
-  TCW_CUDA(h, cudaMemcpyAsync(result, dres, sizeof(tcw_result), cudaMemcpyDeviceToHost,
-                              h->stream));
-  TCW_CUDA(h, cudaStreamSynchronize(h->stream));
+  if (es != cudaSuccess) return cuda_err(h, es, "cudaStreamSynchronize");
+  memcpy(result, h->h_stage + s_res, sizeof(tcw_result));
   return TCW_OK;
 }
 
@@ -872,11 +830,11 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
         if ((seg_blocks + (uint64_t)groups * sp.nseg) * kSegFloats * sizeof(float) > kSegBytesMax)
           sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, hist, 1);
         set_split(t, sp);
-        p->exp_chunks = p->exp_chunks || sp.sub > 1u;
+        p->exp_chunks = p->exp_chunks || sp.sub > 1u || sp.nseg > 0u;
         t.g_off = seg_blocks;
         seg_blocks += (uint64_t)groups * sp.nseg;
       }
-      tile_template(k, t, rcfg, items, &cost, true);
+      tile_template(k, t, rcfg, items, cost);
       t.part_off = (uint32_t)first;
       t.n_parts = (uint32_t)(items.size() - first);
       for (size_t i = first; i < items.size(); i++) items[i].part = (uint32_t)i;
@@ -1082,9 +1040,11 @@ static int plan_enqueue(tcw_handle *h, tcw_plan *p, const float *d_atoms, tcw_re
                          h->side_stream));
   TCW_CUDA(h, cudaEventRecord(h->join_ev, h->side_stream));
   TCW_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_ev, 0));
-  TCW_CUDA(h, launch_finalize(p->d_T, p->n_templates, p->d_parts, d_results, h->stream));
+  TCW_CUDA(h, launch_finalize(p->d_T, p->n_templates, p->d_parts, d_results, false,
+                              h->stream));
   if (d_maps && (p->flags & TCW_FLAG_POSTERIORS))
-    TCW_CUDA(h, launch_posteriors(p->d_T, p->n_templates, p->post, d_maps, d_results, h->stream));
+    TCW_CUDA(h, launch_posteriors(p->d_T, p->n_templates, p->post, d_maps, d_results, false,
+                                  h->stream));
   return TCW_OK;
 }
 
@@ -1170,7 +1130,8 @@ int tcw_plan_run_timed(tcw_handle *h, tcw_plan *p, const float *d_atoms, tcw_res
   TCW_CUDA(h, launch_map(TCW_WINDOW_EXP, plan_launch(h, p, TCW_WINDOW_EXP, d_atoms, nullptr),
                          h->stream));
   TCW_CUDA(h, cudaEventRecord(ev[3], h->stream));
-  TCW_CUDA(h, launch_finalize(p->d_T, p->n_templates, p->d_parts, d_results, h->stream));
+  TCW_CUDA(h, launch_finalize(p->d_T, p->n_templates, p->d_parts, d_results, false,
+                              h->stream));
   TCW_CUDA(h, cudaEventRecord(ev[4], h->stream));
   TCW_CUDA(h, cudaEventSynchronize(ev[4]));
   for (int i = 0; i < 4; i++) TCW_CUDA(h, cudaEventElapsedTime(&ms[i], ev[i], ev[i + 1]));

@@ -40,7 +40,10 @@ struct TemplateDev {
   uint64_t g_off;
   uint32_t g_shift, g_nseg;
   uint32_t e_hist, e_rows, e_sub;  // row chunks (ExpSplit)
-  uint32_t pad2;
+  // single-template launches: tiles of tile_tn columns x tile_tm rows (rect)
+  // or row chunks (exp), row tiles fastest (plain_tile)
+  uint32_t tile_tn, tile_tm, tile_rows;  // tile_rows: row tiles per column tile
+  double ln_prior;                 // ln(70 / (N_t0 N_tau))
 };
 // Floats of one 32-column segment sum (7 channels x hi, lo x 32 lanes).
 constexpr uint32_t kSegFloats = 14u * 32u;
@@ -74,8 +77,8 @@ struct SegItem {
 // history: a window's sums keep the roundings of the rows above it in the
 // same history and start afresh at the next one.  Each history is walked in
 // `sub` chunks of `rows` rows, side by side, whose starts are combined from
-// nseg segment sums of 2^shift atoms (0: every chunk enters its whole window,
-// sub is 1).
+// nseg segment sums of 2^shift atoms (0: every chunk enters its whole window
+// atom by atom, sub is 1).
 struct ExpSplit {
   uint32_t hist, rows, sub, shift, nseg;
   uint32_t chunks(uint32_t N_t0) const { return (N_t0 + hist - 1u) / hist * sub; }
@@ -102,13 +105,13 @@ inline ExpSplit exp_split(uint32_t numAtoms, uint32_t N_t0, uint32_t N_tau, uint
   ExpSplit s{hist, hist, 1, 5, 0};
   const uint64_t n_hist = (N_t0 + hist - 1u) / hist;
   const uint64_t sub = (chunks + n_hist - 1) / n_hist;
-  if (sub <= 1 || numAtoms < 2u * kShortWindow) return s;
+  if (chunks <= 1 || numAtoms < 2u * kShortWindow) return s;
   const uint64_t rows = (hist + sub - 1) / sub;
   s.rows = rows < 8 ? 8u : (uint32_t)rows;
   s.sub = (hist + s.rows - 1u) / s.rows;
   while ((4ull << (2u * s.shift)) <= numAtoms) s.shift++;
   s.nseg = (uint32_t)(((uint64_t)numAtoms + (1u << s.shift) - 1u) >> s.shift);
-  if (s.sub <= 1 || s.seg_floats(N_tau) * sizeof(float) > kSegBytesMax)
+  if (n_hist * s.sub <= 1 || s.seg_floats(N_tau) * sizeof(float) > kSegBytesMax)
     return ExpSplit{hist, hist, 1, 5, 0};
   return s;
 }
@@ -129,6 +132,36 @@ inline ExpSplit plain_exp_split(uint32_t numAtoms, uint32_t N_t0, uint32_t N_tau
   const uint64_t groups = (N_tau + 31u) / 32u;
   const uint64_t want = (uint64_t)n_sms * 4u * TCW_PLAIN_EXP_WARPS;
   return exp_split(numAtoms, N_t0, N_tau, hist, cut ? (want + groups - 1u) / groups : 1u);
+}
+
+// Whether a single map's tiles are launched as the dependent of the kernel
+// before (prepare or segment sums): where that one leaves most of the GPU
+// idle.  Tiles that arrive while thousands of segment blocks still run settle
+// on the SMs that happen to be free (one-year exp map 650 -> 760 us); behind
+// the eight blocks of a prefix scan they save the launch (one-year rect map
+// 250 -> 233 us, 480 x 480 53 -> 29 us per call with the other launches).
+inline bool plain_map_chained(uint32_t n_seg_items, uint32_t numAtoms, int n_sms) {
+  const uint32_t before = n_seg_items ? (n_seg_items + 3u) / 4u : (numAtoms + 255u) / 256u;
+  return before <= (uint32_t)n_sms;
+}
+
+// Tiles of a single-template map (tile_tn, tile_tm, tile_rows); the number of
+// tiles, each one block.  Rect: 32 rows x as many columns as give ~4 blocks per
+// SM, 16 to 256 (at least 4 per warp).  Exp: 32 columns x 4 row chunks (a warp
+// each), t.e_* set.
+inline uint64_t plain_tiles(TemplateDev &t, int n_sms) {
+  if (t.window == 1u) {
+    t.tile_tm = 32;
+    t.tile_rows = (t.N_t0 + 31u) / 32u;
+    const uint64_t c = (uint64_t)t.N_tau * t.tile_rows / ((uint64_t)n_sms * 4u);
+    t.tile_tn = (uint32_t)(c < 16 ? 16 : (c > 256 ? 256 : c));
+  } else {
+    t.tile_tn = 32;
+    t.tile_tm = kBlock / 32;
+    const uint32_t chunks = (t.N_t0 + t.e_hist - 1u) / t.e_hist * t.e_sub;
+    t.tile_rows = (chunks + t.tile_tm - 1u) / t.tile_tm;
+  }
+  return (uint64_t)t.tile_rows * (((uint64_t)t.N_tau + t.tile_tn - 1u) / t.tile_tn);
 }
 
 inline void set_split(TemplateDev &t, const ExpSplit &sp) {
@@ -204,6 +237,11 @@ __device__ __forceinline__ void repack_rows(const float *__restrict__ x, float4 
 // Launchers (tcw_kernels.cu).  All asynchronous on `stream`.
 cudaError_t launch_prefix(const TemplateDev *d_T, const uint32_t *d_rect_list, uint32_t n_rect,
                           const float *d_atoms, float *d_P, int prec, cudaStream_t stream);
+// The first kernel of a single-template map: prefix rows (rect) or repacked
+// rows (exp) of `t`, which it leaves at d_T for the launches that follow (no
+// control data is uploaded).
+cudaError_t launch_prepare_one(const TemplateDev &t, TemplateDev *d_T, const float *d_atoms,
+                               float *d_rows, int prec, cudaStream_t stream);
 // Exp templates' atoms (rows of 7 floats) into rows of 8 (repack_rows);
 // max_atoms: the most atoms of one of them.
 cudaError_t launch_repack(const TemplateDev *d_T, const uint32_t *d_exp_list, uint32_t n_exp,
@@ -217,14 +255,15 @@ cudaError_t launch_exp_segments(const TemplateDev *d_T, const SegItem *d_items, 
                                 cudaStream_t stream);
 struct MapLaunch {
   const TemplateDev *T;
-  const WorkItem *items;  // this window's tiles
+  const WorkItem *items;  // this window's tiles (persistent launches)
   uint32_t n_items;
   uint32_t *counter;      // persistent launches: tile counter, zeroed before
   uint32_t n_blocks;      // persistent grid size
   bool persistent, write_map;
   bool chunks;            // persistent exp launches: some columns are cut (e_sub > 1)
   int prec;
-  int priority;           // stream-priority value of the launch
+  int priority;           // stream-priority value of a persistent launch
+  bool chained;           // single maps: programmatic dependent of the launch before
   const float *atoms;
   const float *atoms8;    // exp tiles: atoms in 32-byte rows
   const float *G;         // exp tiles: segment sums (NULL where no template has any)
@@ -237,8 +276,10 @@ cudaError_t launch_map(int window, const MapLaunch &L, cudaStream_t stream);
 // Resident blocks per SM of the persistent (map-less) kernel of a window.
 int map_blocks_per_sm(int window, int prec, bool chunks);
 
+// `chained` (finalize, posteriors): part of a single map's chain of programmatic
+// dependent launches.
 cudaError_t launch_finalize(const TemplateDev *d_T, uint32_t n_templates, const Partial *d_parts,
-                            void *d_results, cudaStream_t stream);
+                            void *d_results, bool chained, cudaStream_t stream);
 // Posterior indices of templates whose maps were written: blocks of `rows`
 // t0 rows x `cols` columns (a multiple of 1024) leave row sums per column
 // chunk (rowsum + row_off + chunk * N_t0) and column sums per row chunk
@@ -246,8 +287,7 @@ cudaError_t launch_finalize(const TemplateDev *d_T, uint32_t n_templates, const 
 // direction then leave their first maximum in `parts`.
 constexpr uint32_t kPostParts = 32;
 struct PostPart {
-  double v;
-  int64_t i;
+  int64_t v, i;  // the sum's key (its bits: sums are >= 0) and index
 };
 struct PostLayout {
   uint32_t rows, cols, n_chunks;
@@ -271,7 +311,8 @@ inline uint32_t post_rows(uint64_t cells, int n_sms) {
   return rows;
 }
 cudaError_t launch_posteriors(const TemplateDev *d_T, uint32_t n_templates, const PostLayout &L,
-                              const float *d_maps, tcw_result *d_results, cudaStream_t stream);
+                              const float *d_maps, tcw_result *d_results, bool chained,
+                              cudaStream_t stream);
 
 // ---------------------------------------------------------------- differentiable path
 // One template with a continuous tau grid (tcw_diff.cu).  Exponential

@@ -45,6 +45,15 @@ __device__ __forceinline__ FF shfl_up_ff(FF v, int d) {
   return FF{__shfl_up_sync(0xffffffffu, v.h, d), __shfl_up_sync(0xffffffffu, v.l, d)};
 }
 
+// Programmatic dependent launch (the chain of small kernels of one map): a
+// kernel's blocks may start while the kernel before it still runs and wait
+// here until it has finished and its writes are visible; both are no-ops in
+// launches without the attribute.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // One 64-byte prefix row as two 256-bit loads (each lane's request covers
 // whole 32-byte sectors).
 __device__ __forceinline__ void ld_row16(const float *p, float r[16]) {
@@ -65,6 +74,17 @@ __global__ void __launch_bounds__(256) repack_kernel(const TemplateDev *__restri
                                                      const float *__restrict__ atoms,
                                                      float *__restrict__ A8) {
   const TemplateDev t = T[exp_list[blockIdx.y]];
+  repack_rows(atoms + t.atom_off * 7u, reinterpret_cast<float4 *>(A8 + t.a8_off * 8u),
+              t.g.numAtoms, blockIdx.x * 256u);
+}
+
+// One template given by value, left at T for the launches that follow.
+__global__ void __launch_bounds__(256) repack_one_kernel(const __grid_constant__ TemplateDev t,
+                                                         TemplateDev *__restrict__ T,
+                                                         const float *__restrict__ atoms,
+                                                         float *__restrict__ A8) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (blockIdx.x == 0 && threadIdx.x == 0) *T = t;
   repack_rows(atoms + t.atom_off * 7u, reinterpret_cast<float4 *>(A8 + t.a8_off * 8u),
               t.g.numAtoms, blockIdx.x * 256u);
 }
@@ -177,16 +197,13 @@ __global__ void __launch_bounds__(256) prefix_kernel(const TemplateDev *__restri
 constexpr uint32_t kPrefixCluster = 8;
 
 template <bool kComp>
-__global__ void __launch_bounds__(256)
-    prefix_cluster_kernel(const TemplateDev *__restrict__ T,
-                          const uint32_t *__restrict__ rect_list,
-                          const float *__restrict__ atoms, float *__restrict__ P) {
+__device__ __forceinline__ void prefix_cluster(const TemplateDev &t, uint32_t rank,
+                                               const float *__restrict__ atoms,
+                                               float *__restrict__ P) {
   __shared__ FF s_sum[7][32];     // chunk sums, then their offsets in the block
   __shared__ float s_abs[7][32];
   __shared__ float s_tot[kPrefixCluster][7][3];  // every rank's total (h, l) and sum |x|
-  const uint32_t rank = blockIdx.x % kPrefixCluster;  // = rank in the cluster
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-  const TemplateDev t = T[rect_list[blockIdx.x / kPrefixCluster]];
   const uint32_t N = t.g.numAtoms;
   const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
   const uint32_t ci = threadIdx.x >> 3, c = threadIdx.x & 7u;
@@ -269,6 +286,25 @@ __global__ void __launch_bounds__(256)
     }
   }
   if (i0 < N && i1 == N) write_row(N);
+}
+
+template <bool kComp>
+__global__ void __launch_bounds__(256)
+    prefix_cluster_kernel(const TemplateDev *__restrict__ T,
+                          const uint32_t *__restrict__ rect_list,
+                          const float *__restrict__ atoms, float *__restrict__ P) {
+  const TemplateDev t = T[rect_list[blockIdx.x / kPrefixCluster]];
+  prefix_cluster<kComp>(t, blockIdx.x % kPrefixCluster, atoms, P);
+}
+
+// One template given by value, left at T for the launches that follow.
+template <bool kComp>
+__global__ void __launch_bounds__(256)
+    prefix_one_kernel(const __grid_constant__ TemplateDev t, TemplateDev *__restrict__ T,
+                      const float *__restrict__ atoms, float *__restrict__ P) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (blockIdx.x == 0 && threadIdx.x == 0) *T = t;
+  prefix_cluster<kComp>(t, blockIdx.x, atoms, P);
 }
 
 // ------------------------------------------------------------------ reductions
@@ -673,6 +709,7 @@ __global__ void __launch_bounds__(128, 8)
                    uint32_t n_items, uint32_t per, const float *__restrict__ atoms8,
                    const uint32_t *__restrict__ taus_all, float *__restrict__ G) {
   const uint32_t wi = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+  pdl_begin();
   if (wi >= n_items) return;
   SegItem w;
   if (kList) {
@@ -699,20 +736,6 @@ __global__ void __launch_bounds__(128, 8)
     C.enter_to(a8, t.g, j << t.g_shift);
     C.store_sums(G + (t.g_off + (size_t)w.cg * t.g_nseg + j) * kSegFloats + lane);
   }
-}
-
-cudaError_t launch_exp_segments(const TemplateDev *d_T, const SegItem *d_items, uint32_t n_items,
-                                uint32_t per, const float *d_atoms8, const uint32_t *d_taus,
-                                float *d_G, cudaStream_t stream) {
-  if (n_items == 0) return cudaSuccess;
-  const uint32_t blocks = (n_items + 3u) / 4u;
-  if (d_items)
-    exp_seg_kernel<true><<<blocks, 128, 0, stream>>>(d_T, d_items, n_items, per, d_atoms8, d_taus,
-                                                     d_G);
-  else
-    exp_seg_kernel<false><<<blocks, 128, 0, stream>>>(d_T, d_items, n_items, per, d_atoms8,
-                                                      d_taus, d_G);
-  return cudaGetLastError();
 }
 
 // Minimum resident blocks per SM requested from the register allocator
@@ -757,7 +780,6 @@ __global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kChunk
                const uint32_t *__restrict__ taus,
                const float *__restrict__ P, const float *__restrict__ G,
                float *__restrict__ Fmn, Partial *__restrict__ parts) {
-  __shared__ uint32_t s_item;
   constexpr uint32_t kSmem = kWin == TCW_WINDOW_RECT ? (kWrite ? (kBlock / 32) * 32 * 33 : 1)
                                                      : (kBlock / 32) * kExpRowTab * 4;
   __shared__ __align__(16) uint32_t sm[kSmem];
@@ -829,30 +851,34 @@ __global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kChunk
     }
     return;
   }
-  uint32_t it = blockIdx.x;
-  for (;;) {
-    if (kPersist) {
-      if (threadIdx.x == 0) s_item = atomicAdd(counter, 1u);
-      __syncthreads();
-      it = s_item;
-      __syncthreads();
-    }
-    if (it >= n_items) break;
-    const WorkItem w = items[it];
-    const TemplateDev t = T[w.tmpl];
-    Red red;
-    red.init();
-    if (kWin == TCW_WINDOW_RECT) {
-      const uint32_t warp = threadIdx.x >> 5, rg = w.tn;
-      rect_tile<kWrite, kPrec>(t, w, t0s, taus, P, Fmn, red,
-                               reinterpret_cast<float *>(sm) + warp * (32 * 33), warp % rg,
-                               4u / rg, warp / rg, s_tau + warp * 32u);
-    } else
-      exp_tile<kWrite, kPrec, kChunks>(t, w, atoms, atoms8, t0s, taus, Fmn, red,
-                              reinterpret_cast<ExpRow *>(sm) + (threadIdx.x >> 5) * kExpRowTab, G);
-    block_reduce_store(red, parts + w.part);
-    if (!kPersist) break;
+  if (kPersist) return;
+  // one tile of template 0 per block
+  pdl_begin();
+  const TemplateDev t = T[0];
+  WorkItem w;
+  w.tmpl = 0;
+  w.part = blockIdx.x;
+  const uint32_t nt = blockIdx.x / t.tile_rows, mt = blockIdx.x - nt * t.tile_rows;
+  w.n0 = nt * t.tile_tn;
+  w.n1 = min(t.N_tau, w.n0 + t.tile_tn);
+  w.m0 = mt * t.tile_tm;
+  Red red;
+  red.init();
+  if (kWin == TCW_WINDOW_RECT) {
+    w.m1 = min(t.N_t0, w.m0 + t.tile_tm);
+    w.tn = (uint16_t)(t.tile_tm / 32u);  // row groups of 32 rows (one per warp)
+    const uint32_t warp = threadIdx.x >> 5, rg = w.tn;
+    rect_tile<kWrite, kPrec>(t, w, t0s, taus, P, Fmn, red,
+                             reinterpret_cast<float *>(sm) + warp * (32 * 33), warp % rg, 4u / rg,
+                             warp / rg, s_tau + warp * 32u);
+  } else {
+    w.m1 = w.m0 + t.tile_tm;
+    w.tn = (uint16_t)t.tile_tn;
+    exp_tile<kWrite, kPrec, kChunks>(
+        t, w, atoms, atoms8, t0s, taus, Fmn, red,
+        reinterpret_cast<ExpRow *>(sm) + (threadIdx.x >> 5) * kExpRowTab, G);
   }
+  block_reduce_store(red, parts + w.part);
 }
 
 // ------------------------------------------------------------------ finalize
@@ -864,6 +890,7 @@ __global__ void __launch_bounds__(128) finalize_kernel(const TemplateDev *__rest
                                                        tcw_result *__restrict__ results) {
   const uint32_t tmpl = blockIdx.x * 4u + (threadIdx.x >> 5);
   const uint32_t lane = threadIdx.x & 31u;
+  pdl_begin();
   if (tmpl >= n_templates) return;
   const TemplateDev t = T[tmpl];
   float best = -INFINITY;
@@ -895,7 +922,7 @@ __global__ void __launch_bounds__(128) finalize_kernel(const TemplateDev *__rest
     tcw_result r;
     r.maxF = best;
     r.argmax = bidx;
-    r.lnBtSG = log(70.0 / ((double)t.N_t0 * (double)t.N_tau)) + (double)best + log(S);
+    r.lnBtSG = t.ln_prior + (double)best + log(S);
     r.t0_mp_idx = -1;
     r.tau_mp_idx = -1;
     r.status = 0;
@@ -904,6 +931,35 @@ __global__ void __launch_bounds__(128) finalize_kernel(const TemplateDev *__rest
 }
 
 // ------------------------------------------------------------------ launchers
+
+// Launches `kernel`; `pdl`: as the programmatic dependent of the kernel before
+// it in the stream (which must be one of the same chain).
+template <class... KArgs, class... Args>
+static cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block,
+                                 cudaStream_t stream, bool pdl, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+cudaError_t launch_exp_segments(const TemplateDev *d_T, const SegItem *d_items, uint32_t n_items,
+                                uint32_t per, const float *d_atoms8, const uint32_t *d_taus,
+                                float *d_G, cudaStream_t stream) {
+  if (n_items == 0) return cudaSuccess;
+  const uint32_t blocks = (n_items + 3u) / 4u;
+  if (d_items)
+    return launch_kernel(exp_seg_kernel<true>, blocks, 128, stream, false, d_T, d_items, n_items,
+                         per, d_atoms8, d_taus, d_G);
+  return launch_kernel(exp_seg_kernel<false>, blocks, 128, stream, true, d_T, d_items, n_items,
+                       per, d_atoms8, d_taus, d_G);
+}
 
 // Templates up to which a prefix scan takes a cluster each (8 x 148 blocks
 // fill the GPU); more run one block each, which costs no redundant scans.
@@ -937,8 +993,30 @@ cudaError_t launch_prefix(const TemplateDev *d_T, const uint32_t *d_rect_list, u
   return cudaGetLastError();
 }
 
+cudaError_t launch_prepare_one(const TemplateDev &t, TemplateDev *d_T, const float *d_atoms,
+                               float *d_rows, int prec, cudaStream_t stream) {
+  if (t.window != TCW_WINDOW_RECT)
+    return launch_kernel(repack_one_kernel, (t.g.numAtoms + 255u) / 256u, 256, stream, false, t,
+                         d_T, d_atoms, d_rows);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kPrefixCluster);
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kPrefixCluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return prec == kPrecPlain32
+             ? cudaLaunchKernelEx(&cfg, prefix_one_kernel<false>, t, d_T, d_atoms, d_rows)
+             : cudaLaunchKernelEx(&cfg, prefix_one_kernel<true>, t, d_T, d_atoms, d_rows);
+}
+
 template <int kWin, bool kPersist, bool kWrite, bool kChunks>
 static cudaError_t launch_map_prec(int prec, uint32_t grid, cudaStream_t s, int priority,
+                                   bool chained,
                                    const TemplateDev *T, const WorkItem *items, uint32_t n_items,
                                    uint32_t *counter, const float *atoms, const float *atoms8,
                                    const uint32_t *t0s, const uint32_t *taus, const float *P,
@@ -948,10 +1026,15 @@ static cudaError_t launch_map_prec(int prec, uint32_t grid, cudaStream_t s, int 
   cfg.blockDim = dim3(kBlock);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributePriority;
-  attr[0].val.priority = priority;
+  if (kPersist) {
+    attr[0].id = cudaLaunchAttributePriority;
+    attr[0].val.priority = priority;
+  } else {
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = kPersist || chained ? 1 : 0;
   if (prec == kPrecPlain32)
     return cudaLaunchKernelEx(&cfg, map_kernel<kWin, kPersist, kWrite, kPrecPlain32, false>, T,
                               items, n_items, counter, atoms, atoms8, t0s, taus, P, G, Fmn, parts);
@@ -968,7 +1051,7 @@ static cudaError_t launch_map_win(const MapLaunch &L, cudaStream_t stream) {
   const uint32_t grid = L.persistent ? L.n_blocks : L.n_items;
   constexpr bool kExp = kWin == TCW_WINDOW_EXP;
   auto launch = [&](auto fn) {
-    return fn(L.prec, grid, stream, L.priority, L.T, L.items, L.n_items, L.counter, L.atoms,
+    return fn(L.prec, grid, stream, L.priority, L.chained, L.T, L.items, L.n_items, L.counter, L.atoms,
               L.atoms8, L.t0s, L.taus, L.P, L.G, L.Fmn, L.parts);
   };
   if (!L.persistent)
@@ -1034,6 +1117,7 @@ __global__ void __launch_bounds__(256) finalize_block_kernel(const TemplateDev *
   __shared__ float s_best[8];
   __shared__ int64_t s_bidx[8];
   __shared__ double s_sum[8];
+  pdl_begin();
   const TemplateDev t = T[blockIdx.x];
   const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
   float best = -INFINITY;
@@ -1081,7 +1165,7 @@ __global__ void __launch_bounds__(256) finalize_block_kernel(const TemplateDev *
     tcw_result r;
     r.maxF = best;
     r.argmax = bidx;
-    r.lnBtSG = log(70.0 / ((double)t.N_t0 * (double)t.N_tau)) + (double)best + log(S);
+    r.lnBtSG = t.ln_prior + (double)best + log(S);
     r.t0_mp_idx = -1;
     r.tau_mp_idx = -1;
     r.status = 0;
@@ -1090,15 +1174,13 @@ __global__ void __launch_bounds__(256) finalize_block_kernel(const TemplateDev *
 }
 
 cudaError_t launch_finalize(const TemplateDev *d_T, uint32_t n_templates, const Partial *d_parts,
-                            void *d_results, cudaStream_t stream) {
+                            void *d_results, bool chained, cudaStream_t stream) {
   if (n_templates == 0) return cudaSuccess;
   if (n_templates <= 1024)  // (a warp each: 38 us for 3 templates of 2100 x 1581 cells)
-    finalize_block_kernel<<<n_templates, 256, 0, stream>>>(
-        d_T, d_parts, reinterpret_cast<tcw_result *>(d_results));
-  else
-    finalize_kernel<<<(n_templates + 3u) / 4u, 128, 0, stream>>>(
-        d_T, n_templates, d_parts, reinterpret_cast<tcw_result *>(d_results));
-  return cudaGetLastError();
+    return launch_kernel(finalize_block_kernel, n_templates, 256, stream, chained, d_T, d_parts,
+                         reinterpret_cast<tcw_result *>(d_results));
+  return launch_kernel(finalize_kernel, (n_templates + 3u) / 4u, 128, stream, chained, d_T,
+                       n_templates, d_parts, reinterpret_cast<tcw_result *>(d_results));
 }
 
 // Posteriors of written maps (tcw:219-287): the row and column sums of
@@ -1125,6 +1207,7 @@ __global__ void __launch_bounds__(kPostThreads) post_sums_kernel(
     uint32_t cols, const float *__restrict__ maps, const tcw_result *__restrict__ results,
     double *__restrict__ rowsum, double *__restrict__ colsum, uint32_t *__restrict__ ticket) {
   __shared__ float2 srow[kPostThreads / 32][kPostMaxRows];
+  pdl_begin();
   uint2 ch;  // template, chunk within it (column chunk fastest)
   if (chunks)
     ch = chunks[blockIdx.x];
@@ -1198,10 +1281,16 @@ __global__ void __launch_bounds__(kPostThreads) post_sums_kernel(
   }
 }
 
+// A sum as an integer of the same order (sums are >= 0; a NaN is below all),
+// so that no FP64 comparison stands in the chains.
 struct PostBest {
-  double v;
+  int64_t v;
   int64_t i;
 };
+__device__ __forceinline__ int64_t post_key(double x) {
+  const int64_t k = __double_as_longlong(x);
+  return (uint64_t)k > 0x7FF0000000000000ull ? -1 : k;
+}
 __device__ __forceinline__ PostBest post_better(PostBest a, PostBest b) {
   return b.v > a.v || (b.v == a.v && b.i < a.i) ? b : a;
 }
@@ -1227,6 +1316,7 @@ __global__ void __launch_bounds__(kPostThreads) post_argmax_kernel(
     tcw_result *__restrict__ results) {
   __shared__ PostBest sh[kPostThreads / 32];
   __shared__ uint32_t s_last;
+  pdl_begin();
   const uint32_t k = blockIdx.y;
   const TemplateDev t = T[k];
   const uint32_t e_row = post_part_entries(t.N_t0), e_col = post_part_entries(t.N_tau);
@@ -1238,12 +1328,16 @@ __global__ void __launch_bounds__(kPostThreads) post_argmax_kernel(
   const uint32_t i0 = (is_row ? part : part - p_row) * e, i1 = min(N, i0 + e);
   const uint32_t n_sum = is_row ? (t.N_tau + cols - 1u) / cols : (t.N_t0 + rows - 1u) / rows;
   const double *S = is_row ? rowsum + t.row_off : colsum + t.col_off;
-  PostBest best{-1.0, INT64_MAX};
+  PostBest best{-1, INT64_MAX};
   for (uint32_t i = i0 + threadIdx.x; i < i1; i += kPostThreads) {
-    double v = 0.0;
-#pragma unroll 4
-    for (uint32_t c = 0; c < n_sum; c++) v += S[(size_t)c * N + i];
-    if (v > best.v) best = PostBest{v, (int64_t)i};  // i increases: keeps the first
+    double v[4] = {0.0, 0.0, 0.0, 0.0};  // four chains: FP64 additions are slow to return
+    uint32_t c = 0;
+    for (; c + 4u <= n_sum; c += 4u)
+#pragma unroll
+      for (uint32_t q = 0; q < 4u; q++) v[q] += S[(size_t)(c + q) * N + i];
+    for (; c < n_sum; c++) v[0] += S[(size_t)c * N + i];
+    const int64_t key = post_key((v[0] + v[1]) + (v[2] + v[3]));
+    if (key > best.v) best = PostBest{key, (int64_t)i};  // i increases: keeps the first
   }
   best = post_block_best(best, sh);
   PostPart *mine = parts + (size_t)k * (2u * kPostParts);
@@ -1258,7 +1352,7 @@ __global__ void __launch_bounds__(kPostThreads) post_argmax_kernel(
   // thread 0 the rows' parts, thread 1 the columns'
   const uint32_t n = threadIdx.x == 0 ? p_row : p_col;
   const volatile PostPart *v = mine + threadIdx.x * kPostParts;
-  PostBest b{-1.0, INT64_MAX};
+  PostBest b{-1, INT64_MAX};
   for (uint32_t q = 0; q < n; q++) b = post_better(b, PostBest{v[q].v, v[q].i});
   const int64_t idx = b.i == INT64_MAX ? -1 : b.i;
   if (threadIdx.x == 0)
@@ -1268,19 +1362,21 @@ __global__ void __launch_bounds__(kPostThreads) post_argmax_kernel(
 }
 
 cudaError_t launch_posteriors(const TemplateDev *d_T, uint32_t n_templates, const PostLayout &L,
-                              const float *d_maps, tcw_result *d_results, cudaStream_t stream) {
+                              const float *d_maps, tcw_result *d_results, bool chained,
+                              cudaStream_t stream) {
   if (L.n_chunks == 0 || n_templates == 0) return cudaSuccess;
-  post_sums_kernel<<<L.n_chunks, kPostThreads, 0, stream>>>(
-      d_T, L.chunks, L.rows, L.cols, d_maps, d_results, L.rowsum, L.colsum, L.ticket);
-  const cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_kernel(post_sums_kernel, L.n_chunks, kPostThreads, stream, chained, d_T,
+                                L.chunks, L.rows, L.cols, d_maps, d_results, L.rowsum, L.colsum,
+                                L.ticket);
   if (e != cudaSuccess) return e;
   for (uint32_t y0 = 0; y0 < n_templates; y0 += 65535u) {
     const uint32_t ny = n_templates - y0 < 65535u ? n_templates - y0 : 65535u;
-    post_argmax_kernel<<<dim3(2u * kPostParts, ny), kPostThreads, 0, stream>>>(
-        d_T + y0, L.rows, L.cols, L.rowsum, L.colsum, L.parts + (size_t)y0 * 2u * kPostParts,
-        L.ticket + y0, d_results + y0);
+    e = launch_kernel(post_argmax_kernel, dim3(2u * kPostParts, ny), kPostThreads, stream,
+                      chained && y0 == 0, d_T + y0, L.rows, L.cols, L.rowsum, L.colsum,
+                      L.parts + (size_t)y0 * 2u * kPostParts, L.ticket + y0, d_results + y0);
+    if (e != cudaSuccess) return e;
   }
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 }  // namespace tcw

@@ -24,11 +24,12 @@
 // device share the array and it keeps the last call's contents, so calls
 // whose work overlaps on the GPU (different streams, or threads racing to the
 // same stream) corrupt each other's scratch: serialise them.  Everything a
-// call reads from the array it has written earlier in the same call (tile
-// list and descriptor by a set-up kernel, prefix or atom rows, partials), so
-// no clearing is needed between calls.
+// call reads from the array it has written earlier in the same call
+// (descriptor, prefix or atom rows, partials), so no clearing is needed
+// between calls.
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <mutex>
 
 #include "../../include/tcw_b200.h"
@@ -71,39 +72,6 @@ int scratch_address(int device, unsigned char **out, PostPart **post) {
 
 size_t align256(size_t x) { return (x + 255u) / 256u * 256u; }
 
-// Writes the template descriptor, the one-entry template list and the tile
-// list into the scratch array (so nothing is copied from the host).  Tiles
-// are enumerated column tile outer, row tile inner, as the handle-based
-// entry point does.
-__global__ void noalloc_setup_kernel(TemplateDev t, uint32_t window, uint32_t tn,
-                                     uint32_t rows_per_tile, uint32_t n_mtiles,
-                                     uint32_t n_items, TemplateDev *T, uint32_t *list,
-                                     WorkItem *items) {
-  const uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i0 == 0) {
-    T[0] = t;
-    list[0] = 0;
-  }
-  for (uint32_t k = i0; k < n_items; k += gridDim.x * blockDim.x) {
-    const uint32_t nt = k / n_mtiles, mt = k % n_mtiles;
-    WorkItem w{};
-    w.tmpl = 0;
-    w.part = k;
-    w.m0 = mt * rows_per_tile;
-    w.m1 = min(t.N_t0, w.m0 + rows_per_tile);
-    w.n0 = nt * tn;
-    w.n1 = min(t.N_tau, w.n0 + tn);
-    if (window == TCW_WINDOW_RECT) {
-      w.tn = (uint16_t)(rows_per_tile / 32u);
-    } else {  // row chunks, one per warp
-      w.tn = (uint16_t)tn;
-      w.m0 = mt * rows_per_tile;
-      w.m1 = w.m0 + rows_per_tile;
-    }
-    items[k] = w;
-  }
-}
-
 }  // namespace
 
 extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_t numAtoms,
@@ -134,40 +102,29 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
   // tile shapes and scratch layout: the same rules as the handle-based plain
   // entry point; exp columns stay whole histories (`cut` false) where their
   // segment sums do not fit the scratch
-  uint32_t tn = 0, rows_per_tile = 0, n_mtiles = 0, n_items = 0;
+  TemplateDev t{};
+  t.g = make_geom(numAtoms, TAtom, t0_data);
+  t.window = (uint32_t)window;
+  t.N_t0 = N_t0;
+  t.N_tau = N_tau;
+  t.ln_prior = log(70.0 / ((double)N_t0 * (double)N_tau));
   ExpSplit sp{};
-  const uint64_t target_blocks = (uint64_t)sms * 4u;
   const uint32_t n_chunks = (N_t0 + 63u) / 64u;
-  size_t o_T = 0, o_list = 0, o_items = 0, o_parts = 0, o_rows = 0, o_row = 0, o_col = 0, o_G = 0;
-  bool fits = false;
-  for (int cut = window == TCW_WINDOW_EXP && prec != kPrecPlain32 ? 1 : 0; cut >= 0 && !fits;
-       cut--) {
-    uint64_t n_mtiles64;
-    if (window == TCW_WINDOW_RECT) {
-      rows_per_tile = 32;
-      const uint64_t row_tiles = (N_t0 + 31u) / 32u;
-      uint64_t c = (uint64_t)N_tau * row_tiles / (target_blocks ? target_blocks : 1);
-      tn = (uint32_t)(c < 16 ? 16 : (c > 256 ? 256 : c));
-      n_mtiles64 = row_tiles;
-    } else {
-      tn = 32;
-      sp = plain_exp_split(numAtoms, N_t0, N_tau, sms, cut != 0);
-      rows_per_tile = kBlock / tn;  // row chunks per tile
-      n_mtiles64 = ((uint64_t)sp.chunks(N_t0) + rows_per_tile - 1u) / rows_per_tile;
+  size_t o_T = 0, o_parts = 0, o_rows = 0, o_row = 0, o_col = 0, o_G = 0;
+  auto layout = [&](bool cut, bool documented) {
+    if (window == TCW_WINDOW_EXP) {
+      sp = plain_exp_split(numAtoms, N_t0, N_tau, sms, cut);
+      set_split(t, sp);
     }
-    const uint64_t n_items64 = n_mtiles64 * ((N_tau + (uint64_t)tn - 1u) / tn);
-    if (n_items64 > 0x7FFFFFFFull) continue;
-    n_mtiles = (uint32_t)n_mtiles64;
-    n_items = (uint32_t)n_items64;
+    const uint64_t tiles = plain_tiles(t, sms);
+    if (tiles > 0x7FFFFFFFull) return false;
+    t.n_parts = (uint32_t)tiles;
     size_t off = 0;
     o_T = off;
     off = align256(off + sizeof(TemplateDev));
-    o_list = off;
-    off = align256(off + sizeof(uint32_t));
-    o_items = off;
-    off = align256(off + sizeof(WorkItem) * (size_t)n_items);
+    if (documented) off += 256u + align256(sizeof(WorkItem) * (size_t)tiles);
     o_parts = off;
-    off = align256(off + sizeof(Partial) * (size_t)n_items);
+    off = align256(off + sizeof(Partial) * (size_t)tiles);
     o_rows = off;
     off = align256(off + (window == TCW_WINDOW_RECT
                               ? sizeof(float) * kPrefixStride * ((size_t)numAtoms + 1u)
@@ -178,9 +135,13 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
     if (post) off = align256(off + sizeof(double) * (size_t)n_chunks * N_tau);
     o_G = off;
     if (sp.nseg) off = align256(off + sizeof(float) * sp.seg_floats(N_tau));
-    fits = off <= kNoallocScratchBytes;
-  }
-  if (!fits) return TCW_ERR_OVERFLOW;
+    return off <= kNoallocScratchBytes;
+  };
+  // admitted by the documented sizes (with a tile list, whole histories); what
+  // they admit fits without the list
+  if (!layout(false, true)) return TCW_ERR_OVERFLOW;
+  const bool cut = window == TCW_WINDOW_EXP && prec != kPrecPlain32;
+  if (!layout(cut, false)) layout(false, false);
 
   unsigned char *base = nullptr;
   PostPart *pp = nullptr;
@@ -188,28 +149,10 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
   if (rc) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
-  TemplateDev t{};
-  t.g = make_geom(numAtoms, TAtom, t0_data);
-  t.window = (uint32_t)window;
-  t.N_t0 = N_t0;
-  t.N_tau = N_tau;
-  t.part_off = 0;
-  t.n_parts = n_items;
-  set_split(t, sp);
   TemplateDev *dT = reinterpret_cast<TemplateDev *>(base + o_T);
-  uint32_t *dlist = reinterpret_cast<uint32_t *>(base + o_list);
-  WorkItem *ditems = reinterpret_cast<WorkItem *>(base + o_items);
   Partial *dparts = reinterpret_cast<Partial *>(base + o_parts);
   float *drows = reinterpret_cast<float *>(base + o_rows);
-
-  const uint32_t setup_blocks = n_items / 256u + 1u < 1024u ? n_items / 256u + 1u : 1024u;
-  noalloc_setup_kernel<<<setup_blocks, 256, 0, s>>>(t, (uint32_t)window, tn, rows_per_tile,
-                                                    n_mtiles, n_items, dT, dlist, ditems);
-  if (cudaGetLastError() != cudaSuccess) return TCW_ERR_CUDA;
-  cudaError_t e = window == TCW_WINDOW_RECT
-                      ? launch_prefix(dT, dlist, 1, d_atoms, drows, prec, s)
-                      : launch_repack(dT, dlist, 1, numAtoms, d_atoms, drows, s);
-  if (e != cudaSuccess) return TCW_ERR_CUDA;
+  if (launch_prepare_one(t, dT, d_atoms, drows, prec, s) != cudaSuccess) return TCW_ERR_CUDA;
   float *dG = reinterpret_cast<float *>(base + o_G);
   const uint32_t groups = (N_tau + 31u) / 32u;
   const uint32_t per = segs_per_warp((uint64_t)groups * sp.nseg, sms);
@@ -218,12 +161,11 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
     return TCW_ERR_CUDA;
   MapLaunch ml{};
   ml.T = dT;
-  ml.items = ditems;
-  ml.n_items = n_items;
+  ml.n_items = t.n_parts;
   ml.persistent = false;
+  ml.chained = plain_map_chained(n_seg_items, numAtoms, sms);
   ml.write_map = d_Fmn != nullptr;
   ml.prec = prec;
-  ml.priority = 0;
   ml.atoms = d_atoms;
   ml.atoms8 = window == TCW_WINDOW_EXP ? drows : nullptr;
   ml.t0s = d_t0s;
@@ -233,14 +175,14 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
   ml.Fmn = d_Fmn;
   ml.parts = dparts;
   if (launch_map(window, ml, s) != cudaSuccess) return TCW_ERR_CUDA;
-  if (launch_finalize(dT, 1, dparts, d_result, s) != cudaSuccess) return TCW_ERR_CUDA;
+  if (launch_finalize(dT, 1, dparts, d_result, true, s) != cudaSuccess) return TCW_ERR_CUDA;
   if (post) {
     // one column chunk per row chunk of 64 rows: the documented scratch
     const PostLayout pl{64u, (N_tau + 1023u) / 1024u * 1024u, n_chunks, nullptr,
                         reinterpret_cast<double *>(base + o_row),
                         reinterpret_cast<double *>(base + o_col), pp,
                         reinterpret_cast<uint32_t *>(pp + 2u * kPostParts)};
-    if (launch_posteriors(dT, 1, pl, d_Fmn, d_result, s) != cudaSuccess) return TCW_ERR_CUDA;
+    if (launch_posteriors(dT, 1, pl, d_Fmn, d_result, true, s) != cudaSuccess) return TCW_ERR_CUDA;
   }
   return TCW_OK;
 }
