@@ -163,3 +163,27 @@ def test_gpu_memory_debug_log_never_fails_the_call(caplog):
     with caplog.at_level(logging.DEBUG, logger=tcw.logger.name):
         tcw._print_GPU_memory_MB("Initial", 0)
     assert any("Initial GPU memory" in r.getMessage() for r in caplog.records)
+
+
+@pytest.mark.parametrize("order", ["gapless", "gaps", "repeated", "unordered"])
+def test_merge_adds_the_same_bits_whatever_the_bins_look_like(order):
+    """Every way in which the merge adds a detector's atoms (as a slice, by
+    index, one by one) is the FP32 sum of np.add.at, bit for bit."""
+    rng = np.random.default_rng(5)
+    bins = {"gapless": np.arange(40), "gaps": np.flatnonzero(rng.random(40) < 0.7),
+            "repeated": np.sort(rng.integers(0, 40, 60)), "unordered": rng.permutation(40)}[order]
+    ends = (np.zeros(1, np.int64), bins, np.full(1, 39))
+    multi, expect = [], np.zeros((40, 7), np.float32)
+    for X in range(2):
+        idx = np.concatenate(ends) if X == 0 else bins
+        m = rng.normal(0, 1, (idx.shape[0], 7)).astype(np.float32)
+        m[0] = -0.0
+        m[-1, 0] = np.nan
+        np.add.at(expect, idx, m)
+        multi.append(A.FstatAtomVector(700000000 + 1800 * idx, m[:, 0], m[:, 1], m[:, 2],
+                                       m[:, 3] + 1j * m[:, 4], m[:, 5] + 1j * m[:, 6], 1800))
+    t0, M = A.merge_multi_atoms_binned(A.MultiFstatAtomVector(multi), 1800)
+    assert t0 == 700000000
+    assert M.shape == (40, 7)
+    assert np.array_equal(M, expect, equal_nan=True)
+    assert np.array_equal(np.signbit(M), np.signbit(expect))
