@@ -749,6 +749,7 @@ __global__ void __launch_bounds__(kDiffBlock)
 struct DiffGrad {
   FF z1w, z2w, twoT;
   float gbf, gsf;
+  DiffGrad() = default;
   __device__ __forceinline__ DiffGrad(const DiffWeights &w, double temp)
       : z1w(dw_from(w.z1)), z2w(dw_from(w.z2)), twoT(dw_from(2.0 / temp)), gbf((float)w.gb),
         gsf((float)w.gs) {}
@@ -897,19 +898,38 @@ __global__ void __launch_bounds__(kDiffBlock)
 
 // Most atoms of a template that diff_hot_kernel keeps in shared memory.
 constexpr uint32_t kHotAtoms = 7000;
+// Its evaluating warps, and the rows of each half of its ring of window sums.
+constexpr uint32_t kHotEval = 2;
+constexpr uint32_t kHotThreads = (7u + kHotEval) * 32u;
+
+// Barriers of diff_hot_kernel: all its warps, when a half of the ring is full;
+// the seven walking warps.
+__device__ __forceinline__ void hot_ring_sync() {
+  asm volatile("barrier.sync 1, %0;" ::"r"(kHotThreads) : "memory");
+}
+__device__ __forceinline__ void hot_walk_sync() {
+  asm volatile("barrier.sync 2, %0;" ::"r"(7u * 32u) : "memory");
+}
 
 // The tiles whose cells matter by themselves.  Their F enters the results
 // through exponents of 20 F, where the last bits of the window sums show, so
 // their columns are walked whole from the last row down -- a tile started
 // from segment sums agrees to ~1e-14 of the sums only.  A whole walk by one
 // thread per column is a long serial chain (W, V and the removal powers of 7
-// channels: 2.4 ms for 1024 rows); here (0.6-0.9 ms, bound by the latency of
-// ~330 dependent instructions per row) a block takes 32 columns with one
-// warp per channel, whose steps are the packed pairs' bit for bit, and the
-// eighth warp evaluates the hot rows from shared memory while the others walk
+// channels: 2.4 ms for 1024 rows); here a block takes 32 columns with one
+// warp per channel, whose steps are the packed pairs' bit for bit, and two
+// more warps evaluate the hot rows from shared memory while the others walk
 // on.  Column groups without a hot tile leave at once.
+// Bound by the latency of each walking warp's own dependent instructions
+// (~1000 cycles per row of 2 atoms), so: the loops hold no evaluation code,
+// the next removal power is prepared beside the present sums, and a block may
+// use all the registers (96 by the compiler's own choice cost 30 %).  Forward
+// / backward of one 1024 x 1024 template 756 / 816 -> 517 / 577 us against one
+// evaluating warp and powers in the chain, of 24 templates 1096 / 972 -> 650 /
+// 757 (73 pairs of hot rows in a group: evaluating one takes as long as
+// walking two, one warp alone 870 / 947, three as two).
 template <bool kBack>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kHotThreads, 1)
     diff_hot_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
                     const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
                     const ColConsts *__restrict__ cols, const float *__restrict__ need,
@@ -922,7 +942,14 @@ __global__ void __launch_bounds__(256)
   __shared__ float2 s_pow[32][32];  // r^(2^b) of the lanes' columns
   constexpr int kWords = kBack ? 4 : 2;
   __shared__ __align__(16) ExpRow tab[kDiffRowTab];
-  __shared__ float s_sum[2][7][kWords][32];
+  struct HotRow {
+    ExpRow e;
+    uint32_t m;
+    bool reg;
+  };
+  __shared__ float s_sum[2][kHotEval][7][kWords][32];
+  __shared__ HotRow s_row[2][kHotEval];
+  __shared__ DiffPartial s_part[kHotEval];
   __shared__ uint8_t s_hot[kDiffRowTab];
   DiffLane L;
   const uint32_t k = list[blockIdx.y], cg = blockIdx.x;
@@ -933,10 +960,12 @@ __global__ void __launch_bounds__(256)
   const float *nd = need + t.part_off + (size_t)cg * t.n_chunk;
   // the first and last hot chunk
   float hot, skip;
+  DiffGrad grad;
   if (kBack) {
     const DiffWeights w(t, k, temp, lnZ1, lnZ2, gB, gS);
     hot = w.hot;
     skip = w.skip;
+    grad = DiffGrad(w, temp);
   } else {
     const FwdBounds bd(est[k]);
     hot = bd.hot;
@@ -972,163 +1001,230 @@ __global__ void __launch_bounds__(256)
   const uint32_t ch = wid < 7u ? wid : 0u;
   const uint32_t slot = ch < 3u ? ch : ch + 1u;
   const FF r = ch < 3u ? kc.r2 : kc.r1;
-  FF W{0.0f, 0.0f}, V{0.0f, 0.0f}, pw{1.0f, 0.0f}, pc{1.0f, 0.0f}, pv{0.0f, 0.0f};
+  FF W{0.0f, 0.0f}, V{0.0f, 0.0f}, pw{1.0f, 0.0f};
   uint32_t wlo = 0, wtop = 0, Lp = 0;
   bool pinit = false;
+  // this channel's atoms, in shared memory or not: one generic load, no branch
+  const float *xp = staged ? s_x + ch * N : L.a8 + slot;
+  const uint32_t xs = staged ? 1u : 8u;
   auto atom = [&](uint32_t i) {  // (the index below atom 0 reads atom 0)
-    i = i < N ? i : 0u;
-    return staged ? s_x[ch * N + i] : __ldg(L.a8 + (size_t)i * 8u + slot);
+    return xp[(size_t)(i < N ? i : 0u) * xs];
   };
   float xl = 0.0f, xe = 0.0f;  // the atoms that leave and enter next
-  auto leave = [&]() {
-    wtop--;
-    const uint32_t ex = wtop - wlo;
-    const float x = xl;
-    xl = atom(wtop - 1u);
-    if (ex != Lp || !pinit) {  // ExpColumn::power
-      if (pinit && ex == Lp + 1u)
-        pw = ff_mul(pw, kc.r1);
-      else if (pinit && ex + 1u == Lp && kc.has_inv)
-        pw = ff_mul(pw, kc.r1inv);
-      else {
-        pw = FF{1.0f, 0.0f};  // ff_pow from the table
-        for (uint32_t q = ex; q; q &= q - 1u) {
-          const float2 f = s_pow[__ffs(q) - 1][lane];
-          pw = ff_mul(pw, FF{f.x, f.y});
-        }
+  // A lone warp waits for every instruction's result, so what counts is the
+  // longest dependent chain of a step: the next leaving atom's power is
+  // prepared beside the sums of the present step, and taken over (pw, Lp)
+  // only when an atom leaves.
+  FF np{1.0f, 0.0f}, pc{1.0f, 0.0f}, pv{0.0f, 0.0f};
+  uint32_t ex = 0;
+  auto prepare = [&]() {  // ExpColumn::power
+    ex = wtop - 1u - wlo;
+    const bool same = ex == Lp, up = ex == Lp + 1u, down = ex + 1u == Lp && kc.has_inv;
+    const FF step = ff_mul(pw, up ? kc.r1 : kc.r1inv);
+    np = up || down ? step : pw;
+    FF sq = ff_mul(np, np);
+    if (!(pinit && (same || up || down)) && wtop > wlo) {
+      np = FF{1.0f, 0.0f};  // ff_pow from the table
+      for (uint32_t q = ex; q; q &= q - 1u) {
+        const float2 f = s_pow[__ffs(q) - 1][lane];
+        np = ff_mul(np, FF{f.x, f.y});
       }
-      Lp = ex;
-      pinit = true;
-      pc = ch < 3u ? ff_mul(pw, pw) : pw;  // this channel's weight, and times its exponent
-      if (kBack) pv = ff_mul(pc, FF{(float)ex, 0.0f});
+      sq = ff_mul(np, np);
     }
-    W = ff_sub_scaled_x1(W, pc, x);
-    if (kBack) V = ff_sub_scaled_x1(V, pv, x);
+    pc = ch < 3u ? sq : np;  // this channel's weight, and times its exponent
+    if (kBack) pv = ff_mul(pc, FF{(float)ex, 0.0f});
   };
-  auto enter = [&]() {
-    wlo--;
-    const float x = xe;
+  auto leave = [&](bool on) {
+    const FF w = ff_sub_scaled_x1(W, pc, xl);
+    if (kBack) {
+      const FF v = ff_sub_scaled_x1(V, pv, xl);
+      V = on ? v : V;
+    }
+    W = on ? w : W;
+    pw = on ? np : pw;
+    Lp = on ? ex : Lp;
+    pinit = pinit || on;
+    wtop -= on ? 1u : 0u;
+    xl = atom(wtop - 1u);
+  };
+  auto enter = [&](bool on) {
+    if (kBack) {
+      const FF v = ff_scale_dw(r, ff_add_dw(V, W));
+      V = on ? v : V;
+    }
+    const FF w = ff_axpy(xe, r, W);
+    W = on ? w : W;
+    wlo -= on ? 1u : 0u;
     xe = atom(wlo - 1u);
-    if (kBack) V = ff_scale_dw(r, ff_add_dw(V, W));
-    W = ff_axpy(x, r, W);
   };
-  // the evaluating warp's state
+  // an evaluating warp's state
   DiffLse lse(temp, skip);
   FF dtw{0.0f, 0.0f};
   DiffPower power;
-  uint32_t buf = 0;  // the half of s_sum of the next hot row
+  uint32_t half = 0, fill = 0;  // the ring's half that is being filled, its rows so far
 
-  for (uint32_t ce = t.N_t0; ce > mb;) {
-    const uint32_t cb = ce - mb > kDiffRowTab ? ce - kDiffRowTab : mb;
-    bool reg = true;  // the same in every warp
-    for (uint32_t q = lane; q < ce - cb; q += 32u)
-      reg = reg && exp_row_regular(__ldg(L.t0s + cb + q), L.taumax, t.g);
-    reg = __all_sync(0xffffffffu, reg);
-    __syncthreads();
-    for (uint32_t q = threadIdx.x; q < ce - cb; q += blockDim.x) {
-      const uint32_t t0 = __ldg(L.t0s + cb + q);
-      ExpRow e;
-      e.lo = exp_lo(t0, t.g);
-      e.nz = e.lo < t.g.numAtoms ? __ldg(a8u + (size_t)e.lo * 8u + 3u) : 0xFFFFFFFFu;
-      const uint32_t d = t0 - t.g.t0_data;
-      e.a = reg ? fdiv(d, t.g.div) : t0;  // irregular chunks: the generic branch reads t0
-      e.b = reg ? d - e.a * t.g.TAtom : 0u;
-      tab[q] = e;
-      s_hot[q] = is_hot((cb + q) / t.chunk_rows) ? 1 : 0;
+  auto window = [&](const ExpRow &e, bool reg, uint32_t &top) {
+    if (reg) {
+      top = e.a + cc.Qp1 - ((e.b + cc.RmT) >> 31);  // ExpColumn::top_of
+      top = top < 1u ? 1u : top;
+      top = top < t.g.numAtoms ? top : t.g.numAtoms;
+      return e.lo < top;
     }
-    __syncthreads();
-    for (uint32_t m = ce; m > cb;) {
-      m--;
-      const ExpRow e = tab[m - cb];
-      uint32_t top = 0;
-      bool some = false;
-      if (reg) {
-        top = e.a + cc.Qp1 - ((e.b + cc.RmT) >> 31);  // ExpColumn::top_of
-        top = top < 1u ? 1u : top;
-        top = top < t.g.numAtoms ? top : t.g.numAtoms;
-        some = e.lo < top;
-      } else {
-        uint32_t hi;
-        some = exp_hi_real(e.a, L.tau, t.g, hi) && e.lo <= hi;
-        top = some ? hi + 1u : 0u;
+    uint32_t hi;
+    const bool some = exp_hi_real(e.a, L.tau, t.g, hi) && e.lo <= hi;
+    top = some ? hi + 1u : 0u;
+    return some;
+  };
+  // row `wid - 7` of the half that was filled before the last barrier
+  auto evaluate = [&](uint32_t filled, uint32_t rows) {
+    const uint32_t q = wid - 7u;
+    if (wid < 7u || q >= rows || !L.active) return;
+    const HotRow row = s_row[filled][q];
+    float(*sum)[kWords][32] = s_sum[filled][q];
+    uint32_t top;
+    const bool data = window(row.e, row.reg, top) && row.e.nz < top;
+    FF Wr[7];
+#pragma unroll
+    for (int c = 0; c < 7; c++) Wr[c] = FF{sum[c][0][lane], sum[c][1][lane]};
+    float F32 = 0.0f;
+    const bool t1 = data && fstat_fast(Wr, F32);
+    if (!kBack) {
+      double Wd[7] = {0, 0, 0, 0, 0, 0, 0};
+      if (data && !(t1 && F32 < lse.skip)) {
+#pragma unroll
+        for (int c = 0; c < 7; c++) Wd[c] = (double)Wr[c].h + (double)Wr[c].l;
       }
-      if (wid < 7u && some && L.active) {
-        if (top > wtop || e.lo > wlo || top <= wlo) {
-          wlo = wtop = top;
-          xl = xe = atom(top - 1u);
-          W = V = FF{0.0f, 0.0f};
-        }
-        if (!kBack)  // ExpColumn::slide alternates, ExpColumnV::slide does not
-          while (wtop > top && wlo > e.lo) {
-            leave();
-            enter();
+      lse.cell(data, Wd, t1, F32);
+    } else {
+      float Gf[7] = {0, 0, 0, 0, 0, 0, 0};
+      FF p1{0.0f, 0.0f};
+      if (data && !(t1 && F32 < skip)) {
+        FF Vr[7];
+#pragma unroll
+        for (int c = 0; c < 7; c++)
+          Vr[c] = FF{sum[c][kWords - 2][lane], sum[c][kWords - 1][lane]};
+        if (grad.cell(Wr, Vr, Gf, dtw)) p1 = power.at(L, top - row.e.lo);
+      }
+      const uint32_t c = row.m / t.chunk_rows;
+      float *scr = scratch + t.scr_off +
+                   ((size_t)(cg * t.n_chunk + c) * t.chunk_rows + (row.m - c * t.chunk_rows)) *
+                       (TCW_DIFF_SLOTS * 32u) +
+                   lane;
+#pragma unroll
+      for (int c7 = 0; c7 < 7; c7++) scr[32 * c7] = Gf[c7];
+      scr[32 * 7] = p1.h;
+      scr[32 * 8] = p1.l;
+    }
+  };
+
+  if (wid >= 7u) {  // the evaluating warps: a barrier for every half that is filled
+    uint32_t rows = 0;  // hot rows, all of them at or above mb
+    for (uint32_t c = lane; c < t.n_chunk; c += 32u)
+      if (is_hot(c)) rows += min(t.N_t0, (c + 1u) * t.chunk_rows) - c * t.chunk_rows;
+    rows = __reduce_add_sync(0xffffffffu, rows);
+    for (; rows; half ^= 1u) {
+      const uint32_t n = min(rows, kHotEval);
+      hot_ring_sync();
+      evaluate(half, n);
+      rows -= n;
+    }
+  } else {
+    for (uint32_t ce = t.N_t0; ce > mb;) {
+      const uint32_t cb = ce - mb > kDiffRowTab ? ce - kDiffRowTab : mb;
+      bool reg = true;  // the same in every warp
+      for (uint32_t q = lane; q < ce - cb; q += 32u)
+        reg = reg && exp_row_regular(__ldg(L.t0s + cb + q), L.taumax, t.g);
+      reg = __all_sync(0xffffffffu, reg);
+      hot_walk_sync();
+      for (uint32_t q = threadIdx.x; q < ce - cb; q += 7u * 32u) {
+        const uint32_t t0 = __ldg(L.t0s + cb + q);
+        ExpRow e;
+        e.lo = exp_lo(t0, t.g);
+        e.nz = e.lo < t.g.numAtoms ? __ldg(a8u + (size_t)e.lo * 8u + 3u) : 0xFFFFFFFFu;
+        const uint32_t d = t0 - t.g.t0_data;
+        e.a = reg ? fdiv(d, t.g.div) : t0;  // irregular chunks: the generic branch reads t0
+        e.b = reg ? d - e.a * t.g.TAtom : 0u;
+        tab[q] = e;
+        s_hot[q] = is_hot((cb + q) / t.chunk_rows) ? 1 : 0;
+      }
+      hot_walk_sync();
+#pragma unroll 1
+      for (uint32_t m = ce; m > cb;) {
+        m--;
+        const ExpRow e = tab[m - cb];
+        const bool hot_row = s_hot[m - cb];
+        uint32_t top;
+        if (window(e, reg, top) && L.active) {
+          if (top > wtop || e.lo > wlo || top <= wlo) {
+            wlo = wtop = top;
+            xl = xe = atom(top - 1u);
+            W = V = FF{0.0f, 0.0f};
           }
-        while (wtop > top) leave();
-        while (wlo > e.lo) enter();
-      }
-      if (!s_hot[m - cb]) continue;
-      float(*sum)[kWords][32] = s_sum[buf];
-      buf ^= 1u;
-      if (wid < 7u) {
+          // ExpColumn::slide alternates, ExpColumnV::slide does not
+          const uint32_t nl = wtop - top;
+          if (kBack) {
+#pragma unroll 1
+            for (uint32_t j = 0; j < nl; j++) {
+              leave(true);
+              prepare();
+            }
+          } else {
+            const uint32_t ne = wlo - e.lo, n = max(nl, min(ne, nl + 2u));
+#pragma unroll 1
+            for (uint32_t j = 0; j < n; j++) {
+              leave(j < nl);
+              enter(j < ne);
+              prepare();
+            }
+          }
+          if (wlo > e.lo) {
+#pragma unroll 1
+            while (wlo > e.lo) enter(true);
+            prepare();
+          }
+        }
+        if (!hot_row) continue;
+        float(*sum)[kWords][32] = s_sum[half][fill];
         sum[ch][0][lane] = W.h;
         sum[ch][1][lane] = W.l;
         if (kBack) {
           sum[ch][kWords - 2][lane] = V.h;
           sum[ch][kWords - 1][lane] = V.l;
         }
+        if (threadIdx.x == 0) s_row[half][fill] = HotRow{e, m, reg};
+        if (++fill < kHotEval) continue;
+        hot_ring_sync();  // (the readers of the other half are done, too)
+        half ^= 1u;
+        fill = 0;
       }
-      __syncthreads();  // the other buffer's readers are done, too
-      if (wid == 7u && L.active) {
-        const bool data = some && e.nz < top;
-        FF Wr[7];
-#pragma unroll
-        for (int c = 0; c < 7; c++) Wr[c] = FF{sum[c][0][lane], sum[c][1][lane]};
-        float F32 = 0.0f;
-        const bool t1 = data && fstat_fast(Wr, F32);
-        if (!kBack) {
-          double Wd[7] = {0, 0, 0, 0, 0, 0, 0};
-          if (data && !(t1 && F32 < lse.skip)) {
-#pragma unroll
-            for (int c = 0; c < 7; c++) Wd[c] = (double)Wr[c].h + (double)Wr[c].l;
-          }
-          lse.cell(data, Wd, t1, F32);
-        } else {
-          const DiffWeights w(t, k, temp, lnZ1, lnZ2, gB, gS);
-          float Gf[7] = {0, 0, 0, 0, 0, 0, 0};
-          FF p1{0.0f, 0.0f};
-          if (data && !(t1 && F32 < skip)) {
-            FF Vr[7];
-#pragma unroll
-            for (int c = 0; c < 7; c++)
-              Vr[c] = FF{sum[c][kWords - 2][lane], sum[c][kWords - 1][lane]};
-            const DiffGrad grad(w, temp);
-            if (grad.cell(Wr, Vr, Gf, dtw)) p1 = power.at(L, top - e.lo);
-          }
-          const uint32_t c = m / t.chunk_rows;
-          float *scr = scratch + t.scr_off +
-                       ((size_t)(cg * t.n_chunk + c) * t.chunk_rows + (m - c * t.chunk_rows)) *
-                           (TCW_DIFF_SLOTS * 32u) +
-                       lane;
-#pragma unroll
-          for (int c7 = 0; c7 < 7; c7++) scr[32 * c7] = Gf[c7];
-          scr[32 * 7] = p1.h;
-          scr[32 * 8] = p1.l;
-        }
-      }
+      ce = cb;
     }
-    ce = cb;
+    if (fill) hot_ring_sync();
   }
-  if (wid < 7u) return;
   if (kBack) {
-    add_grad_tau(L, dtw, grad_tau + 2u * k);
-  } else {
-    // the group's hot cells are one partial, its other hot tiles' are empty
-    const DiffPartial p = lse.merge();
-    for (uint32_t c = lane; c < t.n_chunk; c += 32u)
-      if (is_hot(c))
-        parts[t.part_off + (size_t)cg * t.n_chunk + c] =
-            c == c0 ? p : DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
+    if (wid >= 7u) add_grad_tau(L, dtw, grad_tau + 2u * k);
+    return;
   }
+  // the group's hot cells are one partial, its other hot tiles' are empty
+  if (wid >= 7u) {
+    const DiffPartial p = lse.merge();
+    if (lane == 0) s_part[wid - 7u] = p;
+  }
+  __syncthreads();
+  if (wid != 7u) return;
+  DiffPartial sum{-INFINITY, 0.0, -INFINITY, 0.0};
+  for (uint32_t q = 0; q < kHotEval; q++) {
+    sum.m1 = fmax(sum.m1, s_part[q].m1);
+    sum.m2 = fmax(sum.m2, s_part[q].m2);
+  }
+  for (uint32_t q = 0; q < kHotEval; q++) {
+    if (s_part[q].s1 != 0.0) sum.s1 += s_part[q].s1 * exp(s_part[q].m1 - sum.m1);
+    if (s_part[q].s2 != 0.0) sum.s2 += s_part[q].s2 * exp(s_part[q].m2 - sum.m2);
+  }
+  for (uint32_t c = lane; c < t.n_chunk; c += 32u)
+    if (is_hot(c))
+      parts[t.part_off + (size_t)cg * t.n_chunk + c] =
+          c == c0 ? sum : DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
 }
 
 // The transposed recurrence over one 64-atom segment of one column group, in
@@ -1701,13 +1797,13 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
           (e = cudaStreamWaitEvent(side, fork, 0)) != cudaSuccess)
         return e;
       if (pass == 0) {
-        diff_hot_kernel<false><<<hot, 256, (size_t)smem_atoms * 28u, side>>>(
+        diff_hot_kernel<false><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
             L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, nullptr, nullptr, nullptr,
             nullptr, nullptr, nullptr, L.parts, smem_atoms);
         diff_fwd_kernel<<<tiles, kDiffBlock, 0, stream>>>(L.T, list, L.atoms8, L.t0s, L.cols,
                                                           L.seg, L.need, L.est, L.temp, L.parts);
       } else {
-        diff_hot_kernel<true><<<hot, 256, (size_t)smem_atoms * 28u, side>>>(
+        diff_hot_kernel<true><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
             L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
             L.scratch, L.grad_tau, nullptr, smem_atoms);
         if (g.max_segs)  // (over the window sums, which nothing reads any more)
