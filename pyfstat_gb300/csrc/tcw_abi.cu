@@ -1157,14 +1157,18 @@ constexpr uint64_t kDiffGroupBytes = 1ull << 30;
 constexpr uint32_t kDiffGroupMax = 65535u;
 
 // Tiles of the exponential templates elist[y0, y1): as many row chunks per
-// column as give every resident warp (32 per SM) a tile, at least 16 rows
-// each; chunks start from segment sums of 2^shift atoms (exp_split).
+// column as give every resident warp (32 per SM) four tiles, at least 16 rows
+// each; chunks start from segment sums of 2^shift atoms (exp_split).  Four
+// rather than one: the tiles that carry weight are few, and the kernels that
+// walk them last as long as their longest tile (24 templates 3.19 -> 2.99 ms,
+// 100 5.4 -> 5.0, 600 17.8 -> 12.9; two 2.98 / 5.1 / 14.3, eight 3.1: the
+// estimate starts too many chunks).
 static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
                                 const std::vector<uint32_t> &elist, uint32_t y0, uint32_t y1,
                                 int pass, DiffGroup &g) {
   uint64_t total_cg = 0;
   for (uint32_t y = y0; y < y1; y++) total_cg += (T[elist[y]].N_tau + 31u) / 32u;
-  const uint64_t chunks = ((uint64_t)h->n_sms * 32u + total_cg - 1u) / total_cg;
+  const uint64_t chunks = ((uint64_t)h->n_sms * 128u + total_cg - 1u) / total_cg;
   const uint64_t seg_floats = pass ? kDiffSegFloatsV : kDiffSegFloats;
   uint64_t seg = 0, scr = 0, cend = 0;
   g = DiffGroup{};

@@ -43,9 +43,8 @@
 //            columns per atom (recursive halving over the 7 channels) to the
 //            FP64 atom gradient.
 // Measured (forward + backward, 2000 atoms, 1024 x 1024 cells, signal): one
-// template 7.7-9.6 -> 1.9 ms (one block per 128 columns and all rows before),
-// 24 templates 16.4 -> 3.7 ms, 256 templates forward 14.2 -> 7.1 ms, backward
-// 38.9 -> 20.1 ms.
+// template 7.7-9.6 -> 1.6 ms (one block per 128 columns and all rows before),
+// 24 templates 16.5 -> 3.0 ms, 256 templates 53 -> 24 ms.
 // The window-sum factor e^(-k (t_lo - t0)/tau) is left out everywhere: F does
 // not depend on it, so neither do g, dF/dW (in this frame) or dF/dtau.
 //
@@ -1730,37 +1729,51 @@ __global__ void __launch_bounds__(kScanBlock)
   }
 }
 
-// One warp per template: its partials brought to their maximum and added.
-__global__ void __launch_bounds__(128)
-    diff_finalize_kernel(const DiffTemplate *__restrict__ T, uint32_t n_templates,
-                         const DiffPartial *__restrict__ parts, double temp,
-                         double *__restrict__ lnB, double *__restrict__ soft) {
-  const uint32_t k = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
-  if (k >= n_templates) return;
+// One block per template: its partials brought to their maximum and added
+// (one warp: 33 us for the 2048 partials of a lone template, now 8).
+__global__ void __launch_bounds__(256)
+    diff_finalize_kernel(const DiffTemplate *__restrict__ T, const DiffPartial *__restrict__ parts,
+                         double temp, double *__restrict__ lnB, double *__restrict__ soft) {
+  __shared__ DiffPartial sh[8];
+  const uint32_t k = blockIdx.x, lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
   const DiffTemplate t = T[k];
-  double m1 = -INFINITY, m2 = -INFINITY, s1 = 0.0, s2 = 0.0;
-  for (uint32_t p = lane; p < t.n_parts; p += 32u) {
-    m1 = fmax(m1, parts[t.part_off + p].m1);
-    m2 = fmax(m2, parts[t.part_off + p].m2);
+  DiffPartial a{-INFINITY, 0.0, -INFINITY, 0.0};
+  for (uint32_t p = threadIdx.x; p < t.n_parts; p += 256u) {
+    a.m1 = fmax(a.m1, parts[t.part_off + p].m1);
+    a.m2 = fmax(a.m2, parts[t.part_off + p].m2);
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
-    m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, d));
-    m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, d));
+    a.m1 = fmax(a.m1, __shfl_xor_sync(0xffffffffu, a.m1, d));
+    a.m2 = fmax(a.m2, __shfl_xor_sync(0xffffffffu, a.m2, d));
   }
-  for (uint32_t p = lane; p < t.n_parts; p += 32u) {
+  if (lane == 0) sh[wid] = a;
+  __syncthreads();
+  for (int w = 0; w < 8; w++) {
+    a.m1 = fmax(a.m1, sh[w].m1);
+    a.m2 = fmax(a.m2, sh[w].m2);
+  }
+  for (uint32_t p = threadIdx.x; p < t.n_parts; p += 256u) {
     const DiffPartial q = parts[t.part_off + p];
-    if (q.s1 != 0.0) s1 += q.s1 * exp(q.m1 - m1);
-    if (q.s2 != 0.0) s2 += q.s2 * exp(q.m2 - m2);
+    if (q.s1 != 0.0) a.s1 += q.s1 * exp(q.m1 - a.m1);
+    if (q.s2 != 0.0) a.s2 += q.s2 * exp(q.m2 - a.m2);
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
-    s1 += __shfl_xor_sync(0xffffffffu, s1, d);
-    s2 += __shfl_xor_sync(0xffffffffu, s2, d);
+    a.s1 += __shfl_xor_sync(0xffffffffu, a.s1, d);
+    a.s2 += __shfl_xor_sync(0xffffffffu, a.s2, d);
   }
-  if (lane == 0) {
-    lnB[k] = log(70.0 / ((double)t.N_t0 * (double)t.N_tau)) + m1 + log(s1);
-    soft[k] = temp * (m2 + log(s2));
+  __syncthreads();  // every thread has read the maxima
+  if (lane == 0) sh[wid] = a;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s1 = 0.0, s2 = 0.0;
+    for (int w = 0; w < 8; w++) {
+      s1 += sh[w].s1;
+      s2 += sh[w].s2;
+    }
+    lnB[k] = log(70.0 / ((double)t.N_t0 * (double)t.N_tau)) + a.m1 + log(s1);
+    soft[k] = temp * (a.m2 + log(s2));
   }
 }
 
@@ -1861,8 +1874,7 @@ cudaError_t launch_diff_finalize(const DiffTemplate *T, uint32_t n_templates,
                                  const DiffPartial *parts, double temp, double *lnB, double *soft,
                                  cudaStream_t stream) {
   if (n_templates == 0) return cudaSuccess;
-  diff_finalize_kernel<<<(n_templates + 3u) / 4u, 128, 0, stream>>>(T, n_templates, parts,
-                                                                         temp, lnB, soft);
+  diff_finalize_kernel<<<n_templates, 256, 0, stream>>>(T, parts, temp, lnB, soft);
   return cudaGetLastError();
 }
 

@@ -961,7 +961,7 @@ cudaError_t launch_exp_segments(const TemplateDev *d_T, const SegItem *d_items, 
                        per, d_atoms8, d_taus, d_G);
 }
 
-// Templates up to which a prefix scan takes a cluster each (8 x 148 blocks
+// Templates up to which a prefix scan takes a cluster each (8 x 152 blocks
 // fill the GPU); more run one block each, which costs no redundant scans.
 constexpr uint32_t kPrefixFew = 152;
 
