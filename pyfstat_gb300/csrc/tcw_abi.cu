@@ -209,10 +209,32 @@ int prec_of(int flags) {
   return kPrecFF;
 }
 
+// Time of an exp column in recurrence steps (one atom entering or leaving its
+// window): a row's F and table entry take that of kExpRowSteps, and of
+// kExpShortRowSteps where windows are so short that F is often near-singular
+// and evaluated in double-word FP32 (kShortWindow).  Chunks of equal steps
+// rather than equally many per column: with one weight per row the rows of the
+// shortest windows were left running when the other warps had ended (35 % of
+// the time; 96 templates with maps 1.82 -> 1.55 ms; weights of 3 / 6 / 10 for
+// the short windows' rows 1.81 / 1.63 / 1.56).
+constexpr double kExpRowSteps = 3.0, kExpShortRowSteps = 10.0;
+
+// The steps of `rows` rows from row m0 on (starts spread over the data) of the
+// column group that starts with duration tau: the atoms that enter, those that
+// leave while the window ends before the data do, and the rows.
+double exp_steps(double atoms, uint32_t TAtom, uint32_t N_t0, uint32_t tau, uint32_t m0,
+                 uint32_t rows) {
+  const double window = 3.0 * tau / TAtom, per_row = atoms / N_t0, enter = per_row * rows;
+  const double leave = std::min(enter, std::max(0.0, atoms - window - per_row * m0));
+  return enter + leave + rows * (window < kShortWindow ? kExpShortRowSteps : kExpRowSteps);
+}
+
 // A plan's tiles of one template.  Rect: tn columns x tm rows.  Exp: 32 columns
-// x one row chunk (t.e_rows rows).
+// x a row chunk of about `chunk_steps` steps where the template has segment
+// sums to start one from (8 rows or more), else a history.
 void tile_template(uint32_t tmpl, const TemplateDev &t, const tcw_tile_config &cfg,
-                   std::vector<WorkItem> &items, std::vector<double> &cost) {
+                   const uint32_t *taus, double chunk_steps, std::vector<WorkItem> &items,
+                   std::vector<double> &cost) {
   const uint32_t N_t0 = t.N_t0, N_tau = t.N_tau;
   if (t.window == TCW_WINDOW_RECT) {
     const uint32_t tn = cfg.rect_tn, tm = cfg.rect_tm;
@@ -229,26 +251,34 @@ void tile_template(uint32_t tmpl, const TemplateDev &t, const tcw_tile_config &c
         cost.push_back((double)(w.m1 - w.m0) * (w.n1 - w.n0));
       }
   } else {
-    const uint32_t chunks = (N_t0 + t.e_hist - 1u) / t.e_hist * t.e_sub;
-    for (uint32_t n0 = 0; n0 < N_tau; n0 += 32u)
-      for (uint32_t c = 0; c < chunks; c++) {
-        WorkItem w{};
-        w.tmpl = tmpl;
-        w.m0 = c;
-        w.m1 = c + 1u;
-        w.n0 = n0;
-        w.n1 = std::min(N_tau, n0 + 32u);
-        w.tn = 32;
-        items.push_back(w);
-        // recurrence steps: window warm-up plus the rows' atom span, per column
-        double atoms_per_row = 1.0;
-        if (N_t0 > 1) atoms_per_row = std::max(1.0, (double)t.g.numAtoms / N_t0);
-        const double rows_here = std::min(N_t0, t.e_rows);
-        double warm = std::min((double)t.g.numAtoms, 3.0 * (double)N_tau);
-        if (t.g_nseg) warm = std::min(warm, 2.0 * (double)(1u << t.g_shift));
-        cost.push_back(((rows_here * atoms_per_row * 2.0 + warm) * 2.0 + rows_here) *
-                       (w.n1 - w.n0));
+    const double atoms = (double)t.g.numAtoms;
+    for (uint32_t n0 = 0; n0 < N_tau; n0 += 32u) {
+      uint32_t rows = t.e_hist;
+      double run_up = 0.0;  // rows of a chunk's run-up
+      if (t.g_nseg) {
+        const double n = exp_steps(atoms, t.g.TAtom, N_t0, taus[n0], 0, N_t0) / chunk_steps;
+        const double tau = taus[std::min(N_tau, n0 + 32u) - 1u] / (double)t.g.TAtom;
+        if (3.0 * taus[n0] < (double)kShortWindow * t.g.TAtom)
+          run_up = kRunUp * std::min(tau, kShortWindow / 3.0) * N_t0 / atoms;
+        rows = std::min(rows, (uint32_t)std::max(8.0, ceil(N_t0 / std::max(1.0, ceil(n)))));
       }
+      for (uint32_t h0 = 0; h0 < N_t0; h0 += t.e_hist)
+        for (uint32_t m0 = h0, h1 = std::min(N_t0, h0 + t.e_hist); m0 < h1; m0 += rows) {
+          WorkItem w{};
+          w.tmpl = tmpl;
+          w.m0 = m0;
+          w.m1 = std::min(h1, m0 + rows);
+          w.n0 = n0;
+          w.n1 = std::min(N_tau, n0 + 32u);
+          w.tn = 32;
+          items.push_back(w);
+          // the first window, atom by atom or from segment sums
+          double warm = std::min(atoms - atoms * w.m1 / N_t0, 3.0 * taus[n0] / t.g.TAtom);
+          if (t.g_nseg) warm = std::min(warm, 2.0 * ((1u << t.g_shift) + (double)t.g_nseg));
+          if (w.m1 < h1) warm += run_up;
+          cost.push_back(warm + exp_steps(atoms, t.g.TAtom, N_t0, taus[n0], m0, w.m1 - m0));
+        }
+    }
   }
 }
 
@@ -738,19 +768,26 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   // Row chunks of exp columns when the caller leaves them to the library
   // (exp_rows 0): whole columns while these are half of TCW_PLAN_EXP_WARPS per
   // scheduler or more (a lone warp is bound by its own latency, eight share the
-  // issue slots), else as many chunks per column as bring the warp tiles there,
-  // started from segment sums.  Whole / cut, per run: 96 templates with maps
-  // and posteriors 3.55 / 2.76 ms, 300 templates 2.11 / 1.17, 24 templates
-  // 0.67 / 0.23; 1143 templates of up to 900 x 900 cells (9000 column tiles)
-  // 1.57 / 2.04.  3 or 5 warps leave the 96 and the 300 templates whole, 12 is
-  // no faster.
-  uint64_t exp_chunks = 1, seg_blocks = 0;
+  // issue slots), else cut into chunks of equal steps that bring the warp tiles
+  // there, started from segment sums.  Whole / cut, per run: 96 templates with
+  // maps and posteriors 3.55 / 1.55 ms, 300 templates of up to 3000 atoms and
+  // 300 x 300 cells 0.93 / 0.50, 24 templates 0.67 / 0.18; 1143 templates of up
+  // to 900 x 900 cells (9000 column tiles) 1.57 / 2.04 with equally many chunks
+  // per column.  6 or 12 warps are no faster (1.66 and 1.64 ms, 0.51 and 0.51).
+  uint64_t seg_blocks = 0;
+  double chunk_steps = 0.0;  // 0: whole columns
   if (cfg.exp_rows == 0 && p->prec != kPrecPlain32) {
     uint64_t tiles = 0;
-    for (uint32_t k = 0; k < n_templates; k++)
-      if (desc[k].window == TCW_WINDOW_EXP) tiles += ((uint64_t)desc[k].N_tau + 31u) / 32u;
+    double steps = 0.0;
+    for (uint32_t k = 0; k < n_templates; k++) {
+      const tcw_template_desc &d = desc[k];
+      if (d.window != TCW_WINDOW_EXP || d.tau_offset + d.N_tau > n_taus) continue;
+      tiles += ((uint64_t)d.N_tau + 31u) / 32u;
+      for (uint32_t n0 = 0; n0 < d.N_tau; n0 += 32u)
+        steps += exp_steps(d.numAtoms, d.TAtom, d.N_t0, taus[d.tau_offset + n0], 0, d.N_t0);
+    }
     const uint64_t want = (uint64_t)h->n_sms * 4u * TCW_PLAN_EXP_WARPS;
-    if (tiles && 2u * tiles <= want) exp_chunks = (want + tiles - 1u) / tiles;
+    if (tiles && 2u * tiles <= want) chunk_steps = steps / (double)want;
   }
   // Rect tiles when the caller leaves them to the library: 128 x 128 while
   // these give every scheduler TCW_PLAN_RECT_WARPS warps' worth of tiles, else
@@ -826,7 +863,11 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
       const size_t first = items.size();
       if (d.window == TCW_WINDOW_EXP) {
         const uint32_t hist = exp_hist(cfg.exp_rows, d.N_t0), groups = (d.N_tau + 31u) / 32u;
-        ExpSplit sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, hist, exp_chunks);
+        // cut where the shortest windows' columns hold more than a chunk
+        const bool cut = chunk_steps > 0.0 &&
+                         exp_steps(d.numAtoms, d.TAtom, d.N_t0, taus[d.tau_offset], 0, d.N_t0) >
+                             chunk_steps;
+        ExpSplit sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, hist, cut ? 2 : 1);
         if ((seg_blocks + (uint64_t)groups * sp.nseg) * kSegFloats * sizeof(float) > kSegBytesMax)
           sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, hist, 1);
         set_split(t, sp);
@@ -834,7 +875,7 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
         t.g_off = seg_blocks;
         seg_blocks += (uint64_t)groups * sp.nseg;
       }
-      tile_template(k, t, rcfg, items, cost);
+      tile_template(k, t, rcfg, taus + d.tau_offset, chunk_steps, items, cost);
       t.part_off = (uint32_t)first;
       t.n_parts = (uint32_t)(items.size() - first);
       for (size_t i = first; i < items.size(); i++) items[i].part = (uint32_t)i;

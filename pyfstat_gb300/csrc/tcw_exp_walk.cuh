@@ -34,17 +34,29 @@ __device__ __forceinline__ void exp_rows(Column &C, const Geom &g, uint32_t shif
     if (lo < top && top - lo >= (2u << shift))
       C.warm_start(a8, g, seg, shift, nseg, lo, top);
   }
-  // the run-up moves the window only
-  if (kRunUpRows && active) {
-    for (uint32_t m = ms; m > me;) {
-      m--;
-      const uint32_t t0 = __ldg(t0s + m), d = t0 - g.t0_data;
-      ExpRow e;
-      e.lo = exp_lo(t0, g);
-      e.nz = 0u;
-      e.a = fdiv(d, g.div);
-      e.b = d - e.a * g.TAtom;
-      C.window(a8, g, e);
+  // the run-up moves the window only (tables as below: rows much finer than
+  // the atoms make it hundreds of rows, whose loads and divisions one after the
+  // other took longer than the chunk)
+  if (kRunUpRows) {
+    for (uint32_t ce = ms; ce > me;) {
+      const uint32_t cb = ce - me > kExpRowTab ? ce - kExpRowTab : me;
+      __syncwarp();
+      for (uint32_t r = lane; r < ce - cb; r += 32u) {
+        const uint32_t t0 = __ldg(t0s + cb + r), d = t0 - g.t0_data;
+        ExpRow e;
+        e.lo = exp_lo(t0, g);
+        e.nz = 0u;
+        e.a = fdiv(d, g.div);
+        e.b = d - e.a * g.TAtom;
+        tab[r] = e;
+      }
+      __syncwarp();
+      if (active)
+        for (uint32_t m = ce; m > cb;) {
+          m--;
+          C.window(a8, g, tab[m - cb]);
+        }
+      ce = cb;
     }
   }
   for (uint32_t ce = me; ce > mb;) {

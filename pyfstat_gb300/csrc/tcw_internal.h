@@ -55,15 +55,15 @@ inline uint32_t segs_per_warp(uint64_t segments, int n_sms) {
   return per < 1 ? 1u : (per > 4 ? 4u : (uint32_t)per);
 }
 
-// A tile of one template, columns [n0, n1).  For a rectangular tile [m0, m1)
-// are its rows and tn its groups of 32 rows; for an exponential tile they are
-// row chunks (TemplateDev::e_rows), each walked by one warp per 32 columns.
+// A tile of one template, rows [m0, m1) x columns [n0, n1).  Rectangular: tn
+// groups of 32 rows.  Exponential: 32 columns, walked by one warp (within one
+// history).
 struct WorkItem {
   uint32_t tmpl;
   uint32_t part;
   uint32_t m0, m1;
   uint32_t n0, n1;
-  uint16_t tn;            // rect: row groups; exp: columns per block (32, 64 or 128)
+  uint16_t tn;            // rect: row groups; exp: columns (32)
   uint16_t pad16;
   uint32_t pad;
 };

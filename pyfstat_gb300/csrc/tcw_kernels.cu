@@ -641,12 +641,20 @@ __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *_
   const uint32_t col = warp_tile ? lane : threadIdx.x % tn;
   const uint32_t rl = warp_tile ? 0u : threadIdx.x / tn;
   const uint32_t n = w.n0 + col;
-  const uint32_t chunk = w.m0 + rl;
-  if (chunk >= w.m1) return;  // uniform per warp (tn >= 32)
-  const uint32_t h0 = chunk / t.e_sub * t.e_hist, h1 = min(t.N_t0, h0 + t.e_hist);
-  const uint32_t mb = h0 + chunk % t.e_sub * t.e_rows;
-  if (mb >= h1) return;
-  const uint32_t me = min(h1, mb + t.e_rows);
+  // the rows [mb, me) of the history that ends at h1: a warp tile's own, or
+  // chunk m0 + rl of a single map (uniform per warp, tn >= 32)
+  uint32_t mb = w.m0, me = w.m1, h1;
+  if (warp_tile) {
+    h1 = min(t.N_t0, mb / t.e_hist * t.e_hist + t.e_hist);
+  } else {
+    const uint32_t chunk = w.m0 + rl;
+    if (chunk >= w.m1) return;
+    const uint32_t h0 = chunk / t.e_sub * t.e_hist;
+    h1 = min(t.N_t0, h0 + t.e_hist);
+    mb = h0 + chunk % t.e_sub * t.e_rows;
+    if (mb >= h1) return;
+    me = min(h1, mb + t.e_rows);
+  }
   const bool active = n < w.n1;
   const uint32_t tau = active ? __ldg(taus_all + t.tau_off + n) : 0u;
   MapSink<kWrite> sink{kWrite ? Fmn + t.map_off : nullptr, t.N_tau, n, &red};

@@ -59,3 +59,12 @@ def test_chunked_columns_match_the_oracle_and_whole_columns(oracle, case, shuffl
     assert np.array_equal(fused["argmax"], res["argmax"])
     for b in (batch, whole):
         b.close()
+
+
+# rows much finer than the atoms: run-ups of a chunk's short windows over
+# several row tables (128 rows), chunks of different lengths side by side
+@pytest.mark.parametrize("case", [(217, 1754, 70, 222, 1800, 331, 0.1),
+                                  (100, 129, 33, 900, 1800, 60, 0.0),
+                                  (64, 2600, 40, 44, 600, 97, 0.2)])
+def test_chunks_of_rows_finer_than_the_atoms(oracle, case):
+    test_chunked_columns_match_the_oracle_and_whole_columns(oracle, case, False)
