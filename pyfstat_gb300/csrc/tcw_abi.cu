@@ -219,15 +219,20 @@ int prec_of(int flags) {
 // the short windows' rows 1.81 / 1.63 / 1.56).
 constexpr double kExpRowSteps = 3.0, kExpShortRowSteps = 10.0;
 
-// The steps of `rows` rows from row m0 on (starts spread over the data) of the
-// column group that starts with duration tau: the atoms that enter, those that
-// leave while the window ends before the data do, and the rows.
-double exp_steps(double atoms, uint32_t TAtom, uint32_t N_t0, uint32_t tau, uint32_t m0,
-                 uint32_t rows) {
-  const double window = 3.0 * tau / TAtom, per_row = atoms / N_t0, enter = per_row * rows;
-  const double leave = std::min(enter, std::max(0.0, atoms - window - per_row * m0));
-  return enter + leave + rows * (window < kShortWindow ? kExpShortRowSteps : kExpRowSteps);
-}
+// The columns of one 32-column group, whose first duration is tau.
+struct ExpGroupSteps {
+  double atoms, window, per_row, row;
+  ExpGroupSteps(double n_atoms, uint32_t TAtom, uint32_t N_t0, uint32_t tau)
+      : atoms(n_atoms), window(3.0 * tau / TAtom), per_row(n_atoms / N_t0),
+        row(window < kShortWindow ? kExpShortRowSteps : kExpRowSteps) {}
+  // Steps of `rows` rows from row m0 on (starts spread over the data): the
+  // atoms that enter, those that leave while the window ends before the data
+  // do, and the rows.
+  double rows(uint32_t m0, uint32_t n) const {
+    const double enter = per_row * n;
+    return enter + std::min(enter, std::max(0.0, atoms - window - per_row * m0)) + row * n;
+  }
+};
 
 // A plan's tiles of one template.  Rect: tn columns x tm rows.  Exp: 32 columns
 // x a row chunk of about `chunk_steps` steps where the template has segment
@@ -255,8 +260,11 @@ void tile_template(uint32_t tmpl, const TemplateDev &t, const tcw_tile_config &c
     for (uint32_t n0 = 0; n0 < N_tau; n0 += 32u) {
       uint32_t rows = t.e_hist;
       double run_up = 0.0;  // rows of a chunk's run-up
+      const ExpGroupSteps steps(atoms, t.g.TAtom, N_t0, taus[n0]);
+      double start = 0.0;  // most steps of a chunk's first window
       if (t.g_nseg) {
-        const double n = exp_steps(atoms, t.g.TAtom, N_t0, taus[n0], 0, N_t0) / chunk_steps;
+        start = std::min(steps.window, 2.0 * ((1u << t.g_shift) + (double)t.g_nseg));
+        const double n = steps.rows(0, N_t0) / chunk_steps;
         const double tau = taus[std::min(N_tau, n0 + 32u) - 1u] / (double)t.g.TAtom;
         if (3.0 * taus[n0] < (double)kShortWindow * t.g.TAtom)
           run_up = kRunUp * std::min(tau, kShortWindow / 3.0) * N_t0 / atoms;
@@ -272,11 +280,16 @@ void tile_template(uint32_t tmpl, const TemplateDev &t, const tcw_tile_config &c
           w.n1 = std::min(N_tau, n0 + 32u);
           w.tn = 32;
           items.push_back(w);
-          // the first window, atom by atom or from segment sums
-          double warm = std::min(atoms - atoms * w.m1 / N_t0, 3.0 * taus[n0] / t.g.TAtom);
-          if (t.g_nseg) warm = std::min(warm, 2.0 * ((1u << t.g_shift) + (double)t.g_nseg));
-          if (w.m1 < h1) warm += run_up;
-          cost.push_back(warm + exp_steps(atoms, t.g.TAtom, N_t0, taus[n0], m0, w.m1 - m0));
+          // Whole columns: one cost for all of a template's groups, so that
+          // they stay neighbours in the queue and the warps of an SM read the
+          // same atoms (ordered by each group's own steps, 1000 templates of up
+          // to 600 x 600 cells take 3.45 ms for 2.30).
+          if (!t.g_nseg)
+            cost.push_back((w.m1 - m0) * (4.0 * std::max(1.0, steps.per_row) + 1.0) +
+                           2.0 * std::min(atoms, 3.0 * N_tau));
+          else
+            cost.push_back(std::min(start, atoms - steps.per_row * w.m1) +
+                           (w.m1 < h1 ? run_up : 0.0) + steps.rows(m0, w.m1 - m0));
         }
     }
   }
@@ -749,7 +762,7 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   tcw_tile_config cfg{};
   if (cfg_in) cfg = *cfg_in;
   fill_cfg_defaults(cfg);
-  cfg.exp_tn = 32;  // plans run 32-column warp tiles (tile_template's warp_tiles)
+  cfg.exp_tn = 32;  // plans run 32-column warp tiles (tile_template)
 
   tcw_plan *p = new (std::nothrow) tcw_plan();
   if (!p) return TCW_ERR_ALLOC;
@@ -784,7 +797,7 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
       if (d.window != TCW_WINDOW_EXP || d.tau_offset + d.N_tau > n_taus) continue;
       tiles += ((uint64_t)d.N_tau + 31u) / 32u;
       for (uint32_t n0 = 0; n0 < d.N_tau; n0 += 32u)
-        steps += exp_steps(d.numAtoms, d.TAtom, d.N_t0, taus[d.tau_offset + n0], 0, d.N_t0);
+        steps += ExpGroupSteps(d.numAtoms, d.TAtom, d.N_t0, taus[d.tau_offset + n0]).rows(0, d.N_t0);
     }
     const uint64_t want = (uint64_t)h->n_sms * 4u * TCW_PLAN_EXP_WARPS;
     if (tiles && 2u * tiles <= want) chunk_steps = steps / (double)want;
@@ -865,8 +878,8 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
         const uint32_t hist = exp_hist(cfg.exp_rows, d.N_t0), groups = (d.N_tau + 31u) / 32u;
         // cut where the shortest windows' columns hold more than a chunk
         const bool cut = chunk_steps > 0.0 &&
-                         exp_steps(d.numAtoms, d.TAtom, d.N_t0, taus[d.tau_offset], 0, d.N_t0) >
-                             chunk_steps;
+                         ExpGroupSteps(d.numAtoms, d.TAtom, d.N_t0, taus[d.tau_offset])
+                                 .rows(0, d.N_t0) > chunk_steps;
         ExpSplit sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, hist, cut ? 2 : 1);
         if ((seg_blocks + (uint64_t)groups * sp.nseg) * kSegFloats * sizeof(float) > kSegBytesMax)
           sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, hist, 1);
@@ -887,20 +900,24 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
         for (uint32_t j = 0; j < T[k].g_nseg; j += per)
           segs.push_back(SegItem{k, cg, j, std::min(T[k].g_nseg, j + per)});
     // two queues (rect tiles, then exp tiles), each in longest-processing-time
-    // order: most expensive tiles first
-    std::vector<uint32_t> order(items.size());
-    for (size_t i = 0; i < order.size(); i++) order[i] = (uint32_t)i;
-    auto is_rect = [&](uint32_t i) { return T[items[i].tmpl].window == TCW_WINDOW_RECT; };
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
-      if (is_rect(a) != is_rect(b)) return is_rect(a);
-      return cost[a] > cost[b];
-    });
-    std::vector<WorkItem> sorted(items.size());
-    uint32_t nr = 0;
-    for (size_t i = 0; i < order.size(); i++) {
-      sorted[i] = items[order[i]];
-      if (is_rect(order[i])) nr++;
+    // order to within 1 % (a counting sort by the cost's exponent and upper
+    // mantissa bits)
+    auto bucket = [&](size_t i) {
+      const float c = (float)cost[i];
+      uint32_t bits;
+      memcpy(&bits, &c, sizeof bits);
+      return (T[items[i].tmpl].window == TCW_WINDOW_RECT ? 0u : 0x8000u) + 0x7FFFu - (bits >> 16);
+    };
+    std::vector<uint32_t> at(0x10001u, 0u);
+    std::vector<uint16_t> key(items.size());
+    for (size_t i = 0; i < items.size(); i++) {
+      key[i] = (uint16_t)bucket(i);
+      at[key[i] + 1u]++;
     }
+    for (uint32_t b = 0; b < 0x10000u; b++) at[b + 1u] += at[b];
+    const uint32_t nr = at[0x8000u];
+    std::vector<WorkItem> sorted(items.size());
+    for (size_t i = 0; i < items.size(); i++) sorted[at[key[i]]++] = items[i];
     items.swap(sorted);
     p->n_items_rect = nr;
     p->n_items_exp = (uint32_t)items.size() - nr;

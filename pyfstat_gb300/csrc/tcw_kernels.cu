@@ -627,25 +627,27 @@ struct MapSink {
 // its own shared-memory slots (no block barrier) and every cell takes the
 // division-free window end of ExpColumn; otherwise the warp runs
 // exp_column2's generic index arithmetic.  Both give identical results.
-template <bool kWrite, int kPrec, bool kChunks>
+template <bool kWrite, int kPrec, bool kChunks, bool kWarp>
 __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *__restrict__ atoms,
                          const float *__restrict__ atoms8,
                          const uint32_t *__restrict__ t0s_all,
                          const uint32_t *__restrict__ taus_all, float *__restrict__ Fmn,
-                         Red &red, ExpRow *tab, const float *__restrict__ G,
-                         bool warp_tile = false) {
+                         Red &red, ExpRow *tab, const float *__restrict__ G) {
   const uint32_t *t0s = t0s_all + t.t0_off;
   const uint32_t tn = w.tn;
   const uint32_t lane = threadIdx.x & 31u;
   // a warp tile (persistent launches) is 32 columns over all the tile's rows
-  const uint32_t col = warp_tile ? lane : threadIdx.x % tn;
-  const uint32_t rl = warp_tile ? 0u : threadIdx.x / tn;
+  const uint32_t col = kWarp ? lane : threadIdx.x % tn;
+  const uint32_t rl = kWarp ? 0u : threadIdx.x / tn;
   const uint32_t n = w.n0 + col;
   // the rows [mb, me) of the history that ends at h1: a warp tile's own, or
   // chunk m0 + rl of a single map (uniform per warp, tn >= 32)
-  uint32_t mb = w.m0, me = w.m1, h1;
-  if (warp_tile) {
-    h1 = min(t.N_t0, mb / t.e_hist * t.e_hist + t.e_hist);
+  uint32_t mb = w.m0, me = w.m1, h1 = me;
+  if (kWarp) {
+    // (holds for every tile; with the exit the register allocator spills 48
+    // bytes of the whole-column kernel, without it 80)
+    if (mb >= t.N_t0) return;
+    if (kChunks) h1 = min(t.N_t0, mb / t.e_hist * t.e_hist + t.e_hist);
   } else {
     const uint32_t chunk = w.m0 + rl;
     if (chunk >= w.m1) return;
@@ -843,7 +845,7 @@ __global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kChunk
       const TemplateDev t = T[w.tmpl];
       Red red;
       red.init();
-      exp_tile<kWrite, kPrec, kChunks>(t, w, atoms, atoms8, t0s, taus, Fmn, red, tab, G, true);
+      exp_tile<kWrite, kPrec, kChunks, true>(t, w, atoms, atoms8, t0s, taus, Fmn, red, tab, G);
       RedVal acc{red.mx, red.bidx, fsub(red.s, red.c)};
 #pragma unroll
       for (int d = 16; d > 0; d >>= 1) acc = red_combine(acc, shfl_down_red(acc, d));
@@ -882,7 +884,7 @@ __global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kChunk
   } else {
     w.m1 = w.m0 + t.tile_tm;
     w.tn = (uint16_t)t.tile_tn;
-    exp_tile<kWrite, kPrec, kChunks>(
+    exp_tile<kWrite, kPrec, kChunks, false>(
         t, w, atoms, atoms8, t0s, taus, Fmn, red,
         reinterpret_cast<ExpRow *>(sm) + (threadIdx.x >> 5) * kExpRowTab, G);
   }
@@ -969,9 +971,12 @@ cudaError_t launch_exp_segments(const TemplateDev *d_T, const SegItem *d_items, 
                        per, d_atoms8, d_taus, d_G);
 }
 
-// Templates up to which a prefix scan takes a cluster each (8 x 152 blocks
-// fill the GPU); more run one block each, which costs no redundant scans.
-constexpr uint32_t kPrefixFew = 152;
+// Templates up to which a prefix scan takes a cluster each; more run one block
+// each, which costs no redundant scans.  Above 152 the scans run beside the exp
+// map kernel, where a lone block's chain of scans is what the rect tiles wait
+// for (one block / cluster per template, whole run: 172 templates 1.28 / 1.25
+// ms, 500 2.35 / 2.22, 570 1.81 / 1.78, 700 0.295 / 0.303).
+constexpr uint32_t kPrefixFew = 600;
 
 cudaError_t launch_prefix(const TemplateDev *d_T, const uint32_t *d_rect_list, uint32_t n_rect,
                           const float *d_atoms, float *d_P, int prec, cudaStream_t stream) {
