@@ -779,14 +779,16 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   std::vector<uint32_t> rect_list, exp_list;
   uint64_t p_rows = 0, a8_rows = 0, atom_rows = 0, cells = 0;
   // Row chunks of exp columns when the caller leaves them to the library
-  // (exp_rows 0): whole columns while these are half of TCW_PLAN_EXP_WARPS per
-  // scheduler or more (a lone warp is bound by its own latency, eight share the
-  // issue slots), else cut into chunks of equal steps that bring the warp tiles
-  // there, started from segment sums.  Whole / cut, per run: 96 templates with
-  // maps and posteriors 3.55 / 1.55 ms, 300 templates of up to 3000 atoms and
-  // 300 x 300 cells 0.93 / 0.50, 24 templates 0.67 / 0.18; 1143 templates of up
-  // to 900 x 900 cells (9000 column tiles) 1.57 / 2.04 with equally many chunks
-  // per column.  6 or 12 warps are no faster (1.66 and 1.64 ms, 0.51 and 0.51).
+  // (exp_rows 0): whole columns where these give TCW_PLAN_EXP_WARPS warps per
+  // scheduler a tile and a third more (a lone warp is bound by its own latency,
+  // eight share the issue slots, and one wave of whole columns lasts as long
+  // as its longest), else cut into chunks of equal steps that bring the warp
+  // tiles there, started from segment sums.  Whole / cut, per run: 96 templates
+  // with maps and posteriors 3.55 / 1.55 ms, 24 templates 0.67 / 0.18, 298 of
+  // up to 2985 atoms and 1292 x 1292 cells (3300 column tiles) 2.33 / 1.44, 840
+  // of up to 2500 and 700 x 700 (5200) 1.90 / 1.70, 330 of up to 3500 and 2000
+  // x 2000 (5900) 3.05 / 2.99; 678 of up to 1132 and 1322 x 1322 (7900) 1.62 /
+  // 1.85.  6 or 12 warps are no faster (96 templates 1.66 and 1.64 ms).
   uint64_t seg_blocks = 0;
   double chunk_steps = 0.0;  // 0: whole columns
   if (cfg.exp_rows == 0 && p->prec != kPrecPlain32) {
@@ -800,7 +802,7 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
         steps += ExpGroupSteps(d.numAtoms, d.TAtom, d.N_t0, taus[d.tau_offset + n0]).rows(0, d.N_t0);
     }
     const uint64_t want = (uint64_t)h->n_sms * 4u * TCW_PLAN_EXP_WARPS;
-    if (tiles && 2u * tiles <= want) chunk_steps = steps / (double)want;
+    if (tiles && 3u * tiles <= 4u * want) chunk_steps = steps / (double)want;
   }
   // Rect tiles when the caller leaves them to the library: 128 x 128 while
   // these give every scheduler TCW_PLAN_RECT_WARPS warps' worth of tiles, else
