@@ -420,7 +420,7 @@ def cpu_model():
 
 # Sources whose compiled code the map-kernel profiles describe; each committed
 # summary records their hash ("kernel_source_sha16 = ...") at capture time.
-KERNEL_SOURCES = ("tcw_kernels.cu", "tcw_cell.h", "tcw_internal.h")
+KERNEL_SOURCES = ("tcw_kernels.cu", "tcw_cell.h", "tcw_exp_walk.cuh", "tcw_internal.h")
 
 
 def kernel_source_hash():
@@ -461,7 +461,8 @@ def traffic_per_launch(kernel):
 
 def launches_per_step(n_rect, n_exp):
     """Kernels one plan step launches: prefix (rect templates), repack and
-    map (exp templates), map (rect templates), finalize."""
+    map (exp templates), map (rect templates), finalize (the workload's plans
+    walk whole columns: no segment sums)."""
     return (2 if n_rect else 0) + (2 if n_exp else 0) + 1
 
 

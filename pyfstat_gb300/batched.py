@@ -9,7 +9,9 @@ template, maxF (2F = 2 maxF), the flat argmax and lnBtSG (FP64), without
 writing any map.  A run is one CUDA graph of five launches on two branches:
 (repack -> persistent exponential-window map kernel) and (prefix ->
 persistent rectangular-window map kernel), joined by a finalize kernel
-(plus the posterior kernels when maps are written).
+(plus the segment sums before the exponential kernel in plans small enough
+to cut its columns into row chunks, and the posterior kernels when maps are
+written).
 """
 
 import numpy as np

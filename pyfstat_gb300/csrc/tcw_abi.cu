@@ -897,6 +897,10 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
       T[k] = t;
     }
     const uint32_t per = segs_per_warp(seg_blocks, h->n_sms);
+    size_t n_segs = 0;
+    for (uint32_t k : exp_list)
+      n_segs += (size_t)((T[k].N_tau + 31u) / 32u) * ((T[k].g_nseg + per - 1u) / per);
+    segs.reserve(n_segs);
     for (uint32_t k : exp_list)
       for (uint32_t cg = 0; cg < (T[k].N_tau + 31u) / 32u; cg++)
         for (uint32_t j = 0; j < T[k].g_nseg; j += per)
@@ -997,7 +1001,7 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
     p->post.ticket = reinterpret_cast<uint32_t *>(p->d_buf + o_ticket);
   }
   // control data: a synchronous copy (plans are built once)
-  std::vector<char> host(ctl_end, 0);
+  std::vector<char> host(ctl_end);
   memcpy(host.data() + o_T, T.data(), sizeof(TemplateDev) * n_templates);
   memcpy(host.data() + o_items, items.data(), sizeof(WorkItem) * p->n_items);
   if (!rect_list.empty())
