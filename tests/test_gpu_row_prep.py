@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("nsft", [1, 7, 255, 256, 257, 511, 2049, 5000])
 def test_prefix_cluster_gives_the_block_kernels_bits(nsft):
-    """153 rectangular templates take one block each, a single one a cluster:
+    """601 rectangular templates take one block each, a single one a cluster:
     the maps are the same bit for bit."""
     from pyfstat_gb300.batched import TransientMapBatch
 
@@ -20,12 +20,12 @@ def test_prefix_cluster_gives_the_block_kernels_bits(nsft):
     t0s = (t0_data + max(1, nsft // 40) * 1800 * np.arange(33)).astype(np.uint32)
     taus = (1800 + max(1, nsft // 30) * 1800 * np.arange(35)).astype(np.uint32)
     t = dict(window=1, atoms=A, TAtom=1800, t0_data=t0_data, t0s=t0s, taus=taus)
-    many = TransientMapBatch([t] * 153)
+    many = TransientMapBatch([t] * 601)
     _, maps = many.plan.run_maps_host(many.atoms)
     one, _ = many.handle.map_plain_host(A, 1800, t0_data, 1, t0s, taus)
-    maps = maps.reshape(153, 33, 35).view(np.uint32)
+    maps = maps.reshape(601, 33, 35).view(np.uint32)
     assert np.array_equal(maps[0], one.view(np.uint32))
-    assert np.array_equal(maps[152], maps[0])
+    assert np.array_equal(maps[600], maps[0])
     many.close()
 
 
