@@ -559,17 +559,24 @@ __global__ void __launch_bounds__(kDiffBlock, 8)
 
 // ------------------------------------------------------------ exponential forward
 
+// A cell so far below the largest F weighs less than e^-62 in both sums:
+// e^(F - max) in lnBtSG, e^(2 (F - max) / T) in the soft-max, whose weights
+// fall slower than lnBtSG's above T = 2.
+__device__ __forceinline__ double no_weight_below(double temp) {
+  return 62.0 * fmax(1.0, 0.5 * temp);
+}
+
 // From the key of a template's estimated maximum: cells below `skip` carry no
-// weight in either sum, tiles that reach `hot` may hold a cell that matters
-// by itself (lnBtSG: e^-8 of the largest; the soft-max's weights fall 20 times
-// as fast).
+// weight in either sum, tiles that reach `hot` may hold a cell whose last bits
+// show (lnBtSG: e^-8 of the largest; the soft-max multiplies them by 2/T,
+// where this is large its weights fall as much faster).
 struct FwdBounds {
   float skip, hot;
-  __device__ __forceinline__ explicit FwdBounds(uint32_t key) {
+  __device__ __forceinline__ FwdBounds(uint32_t key, double temp) {
     skip = hot = -INFINITY;
     if (key) {
       const double top = (double)key_float(key);
-      skip = (float)(top - 1e-5 * fabs(top) - 63.0);
+      skip = (float)(top - 1e-5 * fabs(top) - no_weight_below(temp) - 1.0);
       hot = (float)(top - 1e-5 * fabs(top) - 8.0);
     }
   }
@@ -578,15 +585,15 @@ struct FwdBounds {
 // FP64 log-sum-exps of F and 2F/T over the cells of one lane, then over the
 // warp.
 struct DiffLse {
-  double m1, s1, m2, s2, twoT;
+  double m1, s1, m2, s2, twoT, far;
   float skip, skip0;
   __device__ __forceinline__ DiffLse(double temp, float bound)
-      : m1(-INFINITY), s1(0.0), m2(-INFINITY), s2(0.0), twoT(2.0 / temp), skip(bound),
-        skip0(bound) {}
+      : m1(-INFINITY), s1(0.0), m2(-INFINITY), s2(0.0), twoT(2.0 / temp),
+        far(no_weight_below(temp)), skip(bound), skip0(bound) {}
   __device__ __forceinline__ void add(double F, double k = 1.0) {
     lse_add(m1, s1, F, k);
     lse_add(m2, s2, F * twoT, k);
-    skip = fmaxf((float)(m1 - 62.0), skip0);
+    skip = fmaxf((float)(m1 - far), skip0);
   }
   __device__ __forceinline__ void cell(bool data, const double W[7], bool t1, float F32) {
     if (!data) {
@@ -618,10 +625,10 @@ struct DiffLse {
 // the window's magnitude, against FP64 recurrences at GB300's 1/70 FP64
 // rate), F of the weighted cells in FP64 from them (the reference's formula
 // and conditioning test, fstat64) into FP64 log-sum-exps.  A cell whose
-// tier-1 F lies more than 62 below a lower bound of the template's maximum
-// carries exp(F - max) < e^-60 in both sums (the soft-max's 2F/T - max is 2/T
-// times lower still) and is skipped -- the tier-1 F is good to ~1.5e-6
-// relative and passes only for cond < 32, where the FP64 test passes too.
+// tier-1 F lies more than 62 max(1, T/2) below a lower bound of the template's
+// maximum carries less than e^-60 in both sums (no_weight_below) and is skipped
+// -- the tier-1 F is good to ~1.5e-6 relative and passes only for cond < 32,
+// where the FP64 test passes too.
 __global__ void __launch_bounds__(kDiffBlock, 5)
     diff_fwd_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
                     const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
@@ -636,7 +643,7 @@ __global__ void __launch_bounds__(kDiffBlock, 5)
   const uint32_t cg = tile / L.t.n_chunk, mb = tile % L.t.n_chunk * L.t.chunk_rows;
   if (cg >= L.t.n_cg) return;
   DiffPartial *out = parts + L.t.part_off + tile;
-  const FwdBounds bd(est[k]);
+  const FwdBounds bd(est[k], temp);
   const float skip0 = bd.skip, nd = need[L.t.part_off + tile];
   if (nd < skip0) {
     if (lane == 0) *out = DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
@@ -966,7 +973,7 @@ __global__ void __launch_bounds__(kHotThreads, 1)
     skip = w.skip;
     grad = DiffGrad(w, temp);
   } else {
-    const FwdBounds bd(est[k]);
+    const FwdBounds bd(est[k], temp);
     hot = bd.hot;
     skip = bd.skip;
   }
@@ -1588,7 +1595,7 @@ __global__ void __launch_bounds__(kDiffBlock)
   double z1 = 0.0, z2 = 0.0, gb = 0.0, gs = 0.0;
   float skip0;
   if (kPass == 0) {
-    skip0 = FwdBounds(est[k]).skip;
+    skip0 = FwdBounds(est[k], temp).skip;
   } else {  // a cell whose weights are below e^-62 in both sums has no gradient
     z1 = lnZ1[k] - log(70.0 / ((double)t.N_t0 * (double)t.N_tau));
     z2 = lnZ2[k] / temp;
