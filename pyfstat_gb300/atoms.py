@@ -128,8 +128,8 @@ def atoms_matrix(a2, b2, ab, Fa, Fb):
     Fa = np.asarray(Fa)
     Fb = np.asarray(Fb)
     cols = (np.asarray(a2), np.asarray(b2), np.asarray(ab), Fa.real, Fa.imag, Fb.real, Fb.imag)
-    n = cols[0].shape[:1]
-    if any(c.shape != n for c in cols):
+    n = cols[0].shape
+    if len(n) != 1 or any(c.shape != n for c in cols):
         # other forms (scalars, 2-D blocks, mismatched lengths) as column_stack takes them
         return np.ascontiguousarray(np.column_stack([c.astype(np.float32) for c in cols]))
     mat = np.empty(n + (7,), np.float32)

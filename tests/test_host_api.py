@@ -187,3 +187,34 @@ def test_merge_adds_the_same_bits_whatever_the_bins_look_like(order):
     assert M.shape == (40, 7)
     assert np.array_equal(M, expect, equal_nan=True)
     assert np.array_equal(np.signbit(M), np.signbit(expect))
+
+
+@pytest.mark.parametrize("form", ["arrays", "lists", "scalars", "columns", "blocks", "empty",
+                                  "mismatched", "mixed"])
+def test_atoms_matrix_takes_every_form_that_column_stack_takes(form):
+    """The matrix (or the exception) of np.column_stack, whatever the inputs' shapes."""
+    rng = np.random.default_rng(3)
+    shape = {"scalars": (), "columns": (4, 1), "blocks": (4, 2), "empty": (0,)}.get(form, (4,))
+    x = [rng.normal(size=shape) for _ in range(3)]
+    z = [rng.normal(size=shape) + 1j * rng.normal(size=shape) for _ in range(2)]
+    if form == "lists":
+        x, z = [v.tolist() for v in x], [v.tolist() for v in z]
+    if form == "mismatched":
+        x[1] = x[1][:3]
+    if form == "mixed":
+        x = [v[:, None] for v in x]
+
+    def stacked():
+        Fa, Fb = np.asarray(z[0]), np.asarray(z[1])
+        return np.column_stack([np.asarray(v).astype(np.float32) for v in
+                                (*x, Fa.real, Fa.imag, Fb.real, Fb.imag)])
+
+    try:
+        expect = stacked()
+    except ValueError:
+        with pytest.raises(ValueError):
+            A.atoms_matrix(*x, *z)
+        return
+    M = A.atoms_matrix(*x, *z)
+    assert M.dtype == np.float32 and M.flags.c_contiguous
+    assert np.array_equal(M, expect)
