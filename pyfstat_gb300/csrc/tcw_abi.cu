@@ -1215,10 +1215,24 @@ struct DiffSetup {
   std::vector<DiffGroup> groups;
 };
 
-// Workspace of one group of exponential templates (adjoint sources, segment
-// sums, recurrence ends) and the most templates of one (grid y dimension).
+// Backward workspace of one group of exponential templates (adjoint sources
+// and recurrence ends; the segment sums of a pass have as much again) and the
+// most templates of one (grid y dimension).  A template that needs more is a
+// group by itself, in slices of column groups within kDiffSliceBytes for the
+// sources and for the ends; of the sources at least one column group per SM,
+// the width at which diff_hot_kernel fills the GPU.
 constexpr uint64_t kDiffGroupBytes = 1ull << 30;
+constexpr uint64_t kDiffSliceBytes = 4ull << 30;
 constexpr uint32_t kDiffGroupMax = 65535u;
+
+// Adjoint sources (unpadded row chunks) and recurrence ends of one column group.
+static uint64_t diff_source_bytes(const DiffTemplate &t) {
+  return (uint64_t)t.N_t0 * TCW_DIFF_SLOTS * 32u * sizeof(float);
+}
+static uint64_t diff_end_bytes(const DiffTemplate &t) {
+  return ((uint64_t)t.g.numAtoms + kDiffAtomSeg - 1u) / kDiffAtomSeg * kDiffSegFloats *
+         sizeof(float);
+}
 
 // Tiles of the exponential templates elist[y0, y1): as many row chunks per
 // column as give every resident warp (32 per SM) four tiles, at least 16 rows
@@ -1238,6 +1252,13 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
   g = DiffGroup{};
   g.y0 = y0;
   g.ny = y1 - y0;
+  g.cg_slice = 0xFFFFFFFFu;
+  if (pass && g.ny == 1u) {
+    const DiffTemplate &t = T[elist[y0]];
+    const uint64_t src = std::max<uint64_t>(h->n_sms, kDiffSliceBytes / diff_source_bytes(t));
+    const uint64_t end = std::max<uint64_t>(1, kDiffSliceBytes / diff_end_bytes(t));
+    g.cg_slice = (uint32_t)std::min<uint64_t>(g.cg_slice, std::min(src, end));
+  }
   for (uint32_t y = y0; y < y1; y++) {
     DiffTemplate &t = T[elist[y]];
     t.n_cg = (t.N_tau + 31u) / 32u;
@@ -1256,14 +1277,16 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     t.scr_off = scr;
     t.cend_off = cend;
     seg += (uint64_t)t.n_cg * t.g_nseg;
-    scr += (uint64_t)t.n_cg * t.n_chunk * t.chunk_rows * TCW_DIFF_SLOTS * 32u;
-    cend += (uint64_t)t.n_cg * t.n_aseg;
+    const uint32_t cgs = std::min(t.n_cg, g.cg_slice);
+    scr += (uint64_t)cgs * t.n_chunk * t.chunk_rows * TCW_DIFF_SLOTS * 32u;
+    cend += (uint64_t)cgs * t.n_aseg;
     g.max_cg = std::max(g.max_cg, t.n_cg);
     g.max_atoms = std::max(g.max_atoms, t.g.numAtoms);
     g.max_tiles = std::max(g.max_tiles, t.n_cg * t.n_chunk);
     if (t.g_nseg)
       g.max_segs = std::max(g.max_segs, t.n_cg * t.g_nseg);
-    g.max_aseg = std::max(g.max_aseg, t.n_cg * t.n_aseg);
+    g.slice_tiles = std::max(g.slice_tiles, cgs * t.n_chunk);
+    g.slice_aseg = std::max(g.slice_aseg, cgs * t.n_aseg);
   }
   g.seg_per = segs_per_warp(seg, h->n_sms);
   g.seg_floats = seg * seg_floats;
@@ -1335,17 +1358,17 @@ static int diff_prepare(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n,
       }
       T[k] = t;
     }
-    // groups of exponential templates within the workspace bound (the
-    // backward pass keeps 36 bytes per cell of a group), one template at least
+    // groups of exponential templates within the workspace bound, one template
+    // at least
     for (uint32_t y0 = 0; y0 < elist.size();) {
       uint32_t y1 = y0;
-      uint64_t cells = 0;
+      uint64_t bytes = 0;
       while (y1 < elist.size() && y1 - y0 < kDiffGroupMax) {
         const DiffTemplate &t = T[elist[y1]];
-        const uint64_t c = (uint64_t)((t.N_tau + 31u) / 32u * 32u) * t.N_t0;
-        if (pass && y1 > y0 && (cells + c) * TCW_DIFF_SLOTS * sizeof(float) > kDiffGroupBytes)
-          break;
-        cells += c;
+        const uint64_t b =
+            ((uint64_t)t.N_tau + 31u) / 32u * (diff_source_bytes(t) + diff_end_bytes(t));
+        if (pass && y1 > y0 && bytes + b > kDiffGroupBytes) break;
+        bytes += b;
         y1++;
       }
       DiffGroup g;

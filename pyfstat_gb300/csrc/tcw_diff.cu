@@ -849,16 +849,18 @@ __global__ void __launch_bounds__(kDiffBlock)
                     const ColConsts *__restrict__ cols, const float *__restrict__ seg,
                     const float *__restrict__ need, double temp, const double *__restrict__ lnZ1,
                     const double *__restrict__ lnZ2, const double *__restrict__ gB,
-                    const double *__restrict__ gS, float *__restrict__ scratch,
-                    double *__restrict__ grad_tau) {
+                    const double *__restrict__ gS, uint32_t cg0, uint32_t cgs,
+                    float *__restrict__ scratch, double *__restrict__ grad_tau) {
   __shared__ __align__(16) ExpRow s_tab[kDiffBlock / 32][kDiffRowTab];
   DiffLane L;
   const uint32_t k = list[blockIdx.y];
   L.t = T[k];
   const DiffTemplate &t = L.t;
-  const uint32_t tile = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
-  const uint32_t cg = tile / t.n_chunk, mb = tile % t.n_chunk * t.chunk_rows;
-  if (cg >= t.n_cg) return;
+  // the slice's tiles; scratch holds those of column groups [cg0, cg0 + cgs)
+  const uint32_t stile = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+  const uint32_t scg = stile / t.n_chunk, cg = cg0 + scg, tile = cg0 * t.n_chunk + stile;
+  const uint32_t mb = stile % t.n_chunk * t.chunk_rows;
+  if (scg >= cgs || cg >= t.n_cg) return;
   const DiffWeights w(t, k, temp, lnZ1, lnZ2, gB, gS);
   const float nd = need[t.part_off + tile];
   if (nd < w.skip) return;    // diff_atoms_kernel skips its rows
@@ -873,7 +875,7 @@ __global__ void __launch_bounds__(kDiffBlock)
   CV.reset_v();
   const float *sg =
       t.g_nseg ? seg + (t.seg_off + (size_t)cg * t.g_nseg) * kDiffSegFloatsV + lane : nullptr;
-  float *my = scratch + t.scr_off + (size_t)tile * t.chunk_rows * (TCW_DIFF_SLOTS * 32u) + lane;
+  float *my = scratch + t.scr_off + (size_t)stile * t.chunk_rows * (TCW_DIFF_SLOTS * 32u) + lane;
   diff_rows(L, mb, me, CV, sg, kDiffSegFloatsV, s_tab[threadIdx.x >> 5],
             [&](uint32_t m, uint32_t lo, uint32_t top, bool data) {
               float Gf[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -941,7 +943,7 @@ __global__ void __launch_bounds__(kHotThreads, 1)
                     const ColConsts *__restrict__ cols, const float *__restrict__ need,
                     const uint32_t *__restrict__ est, double temp,
                     const double *__restrict__ lnZ1, const double *__restrict__ lnZ2,
-                    const double *__restrict__ gB, const double *__restrict__ gS,
+                    const double *__restrict__ gB, const double *__restrict__ gS, uint32_t cg0,
                     float *__restrict__ scratch, double *__restrict__ grad_tau,
                     DiffPartial *__restrict__ parts, uint32_t smem_atoms) {
   extern __shared__ float s_x[];  // channel-major atoms, where a template's fit
@@ -958,7 +960,7 @@ __global__ void __launch_bounds__(kHotThreads, 1)
   __shared__ DiffPartial s_part[kHotEval];
   __shared__ uint8_t s_hot[kDiffRowTab];
   DiffLane L;
-  const uint32_t k = list[blockIdx.y], cg = blockIdx.x;
+  const uint32_t k = list[blockIdx.y], cg = cg0 + blockIdx.x;  // (grid x: a slice's groups)
   L.t = T[k];
   const DiffTemplate &t = L.t;
   if (cg >= t.n_cg) return;
@@ -1113,7 +1115,8 @@ __global__ void __launch_bounds__(kHotThreads, 1)
       }
       const uint32_t c = row.m / t.chunk_rows;
       float *scr = scratch + t.scr_off +
-                   ((size_t)(cg * t.n_chunk + c) * t.chunk_rows + (row.m - c * t.chunk_rows)) *
+                   ((size_t)((cg - cg0) * t.n_chunk + c) * t.chunk_rows +
+                    (row.m - c * t.chunk_rows)) *
                        (TCW_DIFF_SLOTS * 32u) +
                    lane;
 #pragma unroll
@@ -1245,15 +1248,16 @@ __global__ void __launch_bounds__(kDiffBlock)
                       const ColConsts *__restrict__ cols, const float *__restrict__ need,
                       double temp, const double *__restrict__ lnZ1,
                       const double *__restrict__ lnZ2, const double *__restrict__ gB,
-                      const double *__restrict__ gS, const float *__restrict__ scratch,
-                      float *__restrict__ cend, double *__restrict__ grad_atoms) {
+                      const double *__restrict__ gS, uint32_t cg0, uint32_t cgs,
+                      const float *__restrict__ scratch, float *__restrict__ cend,
+                      double *__restrict__ grad_atoms) {
   DiffLane L;
   const uint32_t k = list[blockIdx.y];
   L.t = T[k];
   const DiffTemplate &t = L.t;
   const uint32_t wi = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
-  const uint32_t cg = wi / t.n_aseg, as = wi % t.n_aseg;
-  if (cg >= t.n_cg) return;
+  const uint32_t scg = wi / t.n_aseg, cg = cg0 + scg, as = wi % t.n_aseg;
+  if (scg >= cgs || cg >= t.n_cg) return;
   // the group's weighted chunks: first and last
   uint32_t c0 = 0xFFFFFFFFu, c1 = 0;
   {
@@ -1300,7 +1304,7 @@ __global__ void __launch_bounds__(kDiffBlock)
     const F2 zp{0.0f, 0.0f};
     FF2 H01{zp, zp}, H34{zp, zp}, H56{zp, zp};
     FF H2{0.0f, 0.0f};
-    float *ends = cend + (t.cend_off + (size_t)cg * t.n_aseg) * kDiffSegFloats + lane;
+    float *ends = cend + (t.cend_off + (size_t)scg * t.n_aseg) * kDiffSegFloats + lane;
     if (!kEnds) {  // H = r^len H + end, segment by segment from the first
       const uint32_t s0 = i_begin / kDiffAtomSeg;
       FF R = kc.r1;  // r^64
@@ -1340,7 +1344,7 @@ __global__ void __launch_bounds__(kDiffBlock)
     auto sources = [&](uint32_t m) -> const float * {  // NULL: the row carries no weight
       const uint32_t c = m / t.chunk_rows;
       if (nd[c] < w.skip) return nullptr;
-      return scr0 + ((size_t)(cg * t.n_chunk + c) * t.chunk_rows + (m - c * t.chunk_rows)) *
+      return scr0 + ((size_t)(scg * t.n_chunk + c) * t.chunk_rows + (m - c * t.chunk_rows)) *
                         (TCW_DIFF_SLOTS * 32u);
     };
     for (uint32_t i = a; i < b; i++) {
@@ -1801,7 +1805,6 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
       const DiffGroup &g = groups[q];
       const uint32_t *list = L.exp_list + g.y0;
       const dim3 tiles((g.max_tiles + 3u) / 4u, g.ny), segs((g.max_segs + 3u) / 4u, g.ny);
-      const dim3 aseg((g.max_aseg + 3u) / 4u, g.ny), hot(g.max_cg, g.ny);
       // atoms that diff_hot_kernel stages in shared memory (28 bytes each)
       const uint32_t smem_atoms = g.max_atoms < kHotAtoms ? g.max_atoms : kHotAtoms;
       const uint32_t atom_blocks = (g.max_atoms + 255u) / 256u;
@@ -1813,40 +1816,46 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
             nullptr, g.seg_per, L.seg);
       diff_est_kernel<<<tiles, kDiffBlock, 0, stream>>>(L.T, list, L.atoms8, L.t0s, L.cols, L.seg,
                                                         L.need, L.est);
-      if ((e = cudaEventRecord(fork, stream)) != cudaSuccess ||
-          (e = cudaStreamWaitEvent(side, fork, 0)) != cudaSuccess)
-        return e;
-      if (pass == 0) {
-        diff_hot_kernel<false><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
-            L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, nullptr, nullptr, nullptr,
-            nullptr, nullptr, nullptr, L.parts, smem_atoms);
-        diff_fwd_kernel<<<tiles, kDiffBlock, 0, stream>>>(L.T, list, L.atoms8, L.t0s, L.cols,
-                                                          L.seg, L.need, L.est, L.temp, L.parts);
-      } else {
-        diff_hot_kernel<true><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
-            L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
-            L.scratch, L.grad_tau, nullptr, smem_atoms);
-        if (g.max_segs)  // (over the window sums, which nothing reads any more)
-          diff_seg_kernel<true><<<segs, kDiffBlock, 0, stream>>>(
-              L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
-              g.seg_per, L.seg);
-        diff_src_kernel<<<tiles, kDiffBlock, 0, stream>>>(
-            L.T, list, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
-            L.scratch, L.grad_tau);
+      // (one slice unless the group is one large template in its backward pass)
+      for (uint32_t cg0 = 0; cg0 < g.max_cg; cg0 += g.cg_slice) {
+        const uint32_t cgs = g.max_cg - cg0 < g.cg_slice ? g.max_cg - cg0 : g.cg_slice;
+        const dim3 hot(cgs, g.ny), stiles((g.slice_tiles + 3u) / 4u, g.ny);
+        const dim3 aseg((g.slice_aseg + 3u) / 4u, g.ny);
+        if ((e = cudaEventRecord(fork, stream)) != cudaSuccess ||
+            (e = cudaStreamWaitEvent(side, fork, 0)) != cudaSuccess)
+          return e;
+        if (pass == 0) {
+          diff_hot_kernel<false><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
+              L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, nullptr, nullptr, nullptr,
+              nullptr, cg0, nullptr, nullptr, L.parts, smem_atoms);
+          diff_fwd_kernel<<<tiles, kDiffBlock, 0, stream>>>(
+              L.T, list, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.est, L.temp, L.parts);
+        } else {
+          diff_hot_kernel<true><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
+              L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1, L.lnZ2, L.gB,
+              L.gS, cg0, L.scratch, L.grad_tau, nullptr, smem_atoms);
+          if (g.max_segs && cg0 == 0)  // (over the window sums, which nothing reads any more)
+            diff_seg_kernel<true><<<segs, kDiffBlock, 0, stream>>>(
+                L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
+                g.seg_per, L.seg);
+          diff_src_kernel<<<stiles, kDiffBlock, 0, stream>>>(
+              L.T, list, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB,
+              L.gS, cg0, cgs, L.scratch, L.grad_tau);
+        }
+        if ((e = cudaEventRecord(join, side)) != cudaSuccess ||
+            (e = cudaStreamWaitEvent(stream, join, 0)) != cudaSuccess)
+          return e;
+        if (pass == 1) {
+          diff_atoms_kernel<true><<<aseg, kDiffBlock, 0, stream>>>(
+              L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS, cg0,
+              cgs, L.scratch, L.cend, L.grad_atoms);
+          diff_atoms_kernel<false><<<aseg, kDiffBlock, 0, stream>>>(
+              L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS, cg0,
+              cgs, L.scratch, L.cend, L.grad_atoms);
+        }
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
       }
-      if ((e = cudaEventRecord(join, side)) != cudaSuccess ||
-          (e = cudaStreamWaitEvent(stream, join, 0)) != cudaSuccess)
-        return e;
-      if (pass == 1) {
-        diff_atoms_kernel<true><<<aseg, kDiffBlock, 0, stream>>>(
-            L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
-            L.scratch, L.cend, L.grad_atoms);
-        diff_atoms_kernel<false><<<aseg, kDiffBlock, 0, stream>>>(
-            L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
-            L.scratch, L.cend, L.grad_atoms);
-      }
-      e = cudaGetLastError();
-      if (e != cudaSuccess) return e;
     }
   }
   for (uint32_t y0 = 0; y0 < L.n_rect; y0 += 65535u) {

@@ -349,11 +349,14 @@ struct DiffPartial {
   double m1, s1, m2, s2;
 };
 // Exponential templates [y0, y0 + ny) of exp_list with workspaces of their
-// own: a backward pass runs in groups that bound the scratch.
+// own: a backward pass runs in groups that bound the scratch, a group of one
+// large template in slices of cg_slice column groups.
 struct DiffGroup {
   uint32_t y0, ny;
-  // most column groups / tiles / segments / atom segments / atoms of one template
-  uint32_t max_cg, max_tiles, max_segs, max_aseg, max_atoms;
+  // most column groups / tiles / segments / atoms of one template
+  uint32_t max_cg, max_tiles, max_segs, max_atoms;
+  // column groups of a slice, most tiles / atom segments of one template in it
+  uint32_t cg_slice, slice_tiles, slice_aseg;
   uint32_t seg_per;  // segments per warp
   uint64_t seg_floats, scr_floats, cend_floats;
 };
