@@ -554,7 +554,7 @@ struct PlainLayout {
 
 static int plain_layout(tcw_handle *h, uint32_t numAtoms, uint32_t TAtom, uint32_t t0_data,
                         int window, uint32_t N_t0, uint32_t N_tau, int flags, size_t off,
-                        PlainLayout &P) {
+                        bool cut, PlainLayout &P) {
   TemplateDev &t = P.t;
   t = make_tdev(numAtoms, TAtom, t0_data, window, N_t0, N_tau);
   uint64_t seg_floats = 0;
@@ -562,7 +562,7 @@ static int plain_layout(tcw_handle *h, uint32_t numAtoms, uint32_t TAtom, uint32
   P.seg_per = 1;
   if (window == TCW_WINDOW_EXP) {
     const ExpSplit sp =
-        plain_exp_split(numAtoms, N_t0, N_tau, h->n_sms, prec_of(flags) != kPrecPlain32);
+        plain_exp_split(numAtoms, N_t0, N_tau, h->n_sms, cut && prec_of(flags) != kPrecPlain32);
     set_split(t, sp);
     seg_floats = sp.seg_floats(N_tau);
     const uint32_t groups = (N_tau + 31u) / 32u;
@@ -591,21 +591,31 @@ static int plain_layout(tcw_handle *h, uint32_t numAtoms, uint32_t TAtom, uint32
   return TCW_OK;
 }
 
+// Layout and workspace of one map.  Where the memory for the segment sums of
+// exp columns (up to 1 GiB) is not to be had, the columns stay whole histories.
+static int plain_fit(tcw_handle *h, uint32_t numAtoms, uint32_t TAtom, uint32_t t0_data,
+                     int window, uint32_t N_t0, uint32_t N_tau, int flags, size_t off,
+                     PlainLayout &P) {
+  for (bool cut : {true, false}) {
+    int rc =
+        plain_layout(h, numAtoms, TAtom, t0_data, window, N_t0, N_tau, flags, off, cut, P);
+    if (rc) return rc;
+    rc = ensure_ws(h, P.total);
+    if (rc != TCW_ERR_ALLOC || P.n_seg_items == 0) return rc;
+  }
+  return TCW_ERR_ALLOC;
+}
+
 // One map: prepare (prefix or repacked rows, the descriptor), exp segment sums,
 // map tiles, finalize, posteriors -- a chain of programmatic dependent
-// launches that needs nothing from the host but their arguments.  `ws_off`:
-// the workspace's first bytes are the caller's.
-static int plain_enqueue(tcw_handle *h, const float *d_atoms, uint32_t numAtoms, uint32_t TAtom,
-                         uint32_t t0_data, int window, const uint32_t *d_t0s, uint32_t N_t0,
-                         const uint32_t *d_taus, uint32_t N_tau, float *d_Fmn,
-                         tcw_result *d_result, int flags, size_t ws_off) {
-  PlainLayout L;
-  int rc = plain_layout(h, numAtoms, TAtom, t0_data, window, N_t0, N_tau, flags, ws_off, L);
-  if (rc) return rc;
-  rc = ensure_ws(h, L.total);
-  if (rc) return rc;
+// launches that needs nothing from the host but their arguments (and the
+// workspace that L was fitted into).
+static int plain_enqueue(tcw_handle *h, const PlainLayout &L, const float *d_atoms,
+                         const uint32_t *d_t0s, const uint32_t *d_taus, float *d_Fmn,
+                         tcw_result *d_result, int flags) {
   char *ws = h->d_ws;
-  const int prec = prec_of(flags);
+  const int prec = prec_of(flags), window = (int)L.t.window;
+  const uint32_t numAtoms = L.t.g.numAtoms;
   const bool rect = window == TCW_WINDOW_RECT;
   TemplateDev *dT = reinterpret_cast<TemplateDev *>(ws + L.o_T);
   float *drows = reinterpret_cast<float *>(ws + L.o_rows);
@@ -660,8 +670,10 @@ int tcw_map_plain(tcw_handle *h, const float *d_atoms, uint32_t numAtoms, uint32
     return set_err(h, TCW_ERR_INVALID_ARG, "posteriors need a map (d_Fmn is NULL)");
   rc = set_device(h);
   if (rc) return rc;
-  return plain_enqueue(h, d_atoms, numAtoms, TAtom, t0_data, window, d_t0s, N_t0, d_taus, N_tau,
-                       d_Fmn, d_result, flags, 0);
+  PlainLayout P;
+  rc = plain_fit(h, numAtoms, TAtom, t0_data, window, N_t0, N_tau, flags, 0, P);
+  if (rc) return rc;
+  return plain_enqueue(h, P, d_atoms, d_t0s, d_taus, d_Fmn, d_result, flags);
 }
 
 int tcw_map_plain_host(tcw_handle *h, const float *atoms, uint32_t numAtoms, uint32_t TAtom,
@@ -706,9 +718,7 @@ int tcw_map_plain_host(tcw_handle *h, const float *atoms, uint32_t numAtoms, uin
   const size_t o_res = L.add(sizeof(tcw_result));
   const size_t o_map = want_map ? L.add(sizeof(float) * (size_t)N_t0 * N_tau) : 0;
   PlainLayout P;
-  rc = plain_layout(h, numAtoms, TAtom, t0_data, window, N_t0, N_tau, flags, L.total, P);
-  if (rc) return rc;
-  rc = ensure_ws(h, P.total);
+  rc = plain_fit(h, numAtoms, TAtom, t0_data, window, N_t0, N_tau, flags, L.total, P);
   if (rc) return rc;
   const bool staged = in_bytes <= kStagedInputs;
   const size_t s_res = align_up(staged ? in_bytes : 0, 64);
@@ -727,10 +737,9 @@ int tcw_map_plain_host(tcw_handle *h, const float *atoms, uint32_t numAtoms, uin
   }
   float *dmap = want_map ? reinterpret_cast<float *>(ws + o_map) : nullptr;
   tcw_result *dres = reinterpret_cast<tcw_result *>(ws + o_res);
-  rc = plain_enqueue(h, reinterpret_cast<const float *>(ws + o_atoms), numAtoms, TAtom, t0_data,
-                     window, reinterpret_cast<const uint32_t *>(ws + o_t0), N_t0,
-                     reinterpret_cast<const uint32_t *>(ws + o_tau), N_tau, dmap, dres, flags,
-                     L.total);
+  rc = plain_enqueue(h, P, reinterpret_cast<const float *>(ws + o_atoms),
+                     reinterpret_cast<const uint32_t *>(ws + o_t0),
+                     reinterpret_cast<const uint32_t *>(ws + o_tau), dmap, dres, flags);
   // on any error below the stream is drained first: the staging and the
   // caller's buffers must not be in use when this returns
   if (rc == TCW_OK) {
@@ -750,11 +759,12 @@ int tcw_map_plain_host(tcw_handle *h, const float *atoms, uint32_t numAtoms, uin
 
 // ---------------------------------------------------------------- batched plans
 
-int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_templates,
-                    const uint32_t *t0s, uint64_t n_t0s, const uint32_t *taus, uint64_t n_taus,
-                    const tcw_tile_config *cfg_in, int flags, tcw_plan **out) {
-  if (!h || !out) return TCW_ERR_INVALID_ARG;
-  *out = nullptr;
+// `cut`: exp columns may be cut into row chunks; *segments: some were, and the
+// plan's buffer has their sums.
+static int plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_templates,
+                       const uint32_t *t0s, uint64_t n_t0s, const uint32_t *taus, uint64_t n_taus,
+                       const tcw_tile_config *cfg_in, int flags, bool cut, bool *segments,
+                       tcw_plan **out) {
   if (!desc || n_templates == 0 || !t0s || !taus)
     return set_err(h, TCW_ERR_INVALID_ARG, "empty or null template list / grids");
   int rc = set_device(h);
@@ -791,7 +801,7 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   // 1.85.  6 or 12 warps are no faster (96 templates 1.66 and 1.64 ms).
   uint64_t seg_blocks = 0;
   double chunk_steps = 0.0;  // 0: whole columns
-  if (cfg.exp_rows == 0 && p->prec != kPrecPlain32) {
+  if (cut && cfg.exp_rows == 0 && p->prec != kPrecPlain32) {
     uint64_t tiles = 0;
     double steps = 0.0;
     for (uint32_t k = 0; k < n_templates; k++) {
@@ -879,10 +889,10 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
       if (d.window == TCW_WINDOW_EXP) {
         const uint32_t hist = exp_hist(cfg.exp_rows, d.N_t0), groups = (d.N_tau + 31u) / 32u;
         // cut where the shortest windows' columns hold more than a chunk
-        const bool cut = chunk_steps > 0.0 &&
-                         ExpGroupSteps(d.numAtoms, d.TAtom, d.N_t0, taus[d.tau_offset])
-                                 .rows(0, d.N_t0) > chunk_steps;
-        ExpSplit sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, hist, cut ? 2 : 1);
+        const bool more = chunk_steps > 0.0 &&
+                          ExpGroupSteps(d.numAtoms, d.TAtom, d.N_t0, taus[d.tau_offset])
+                                  .rows(0, d.N_t0) > chunk_steps;
+        ExpSplit sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, hist, more ? 2 : 1);
         if ((seg_blocks + (uint64_t)groups * sp.nseg) * kSegFloats * sizeof(float) > kSegBytesMax)
           sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, hist, 1);
         set_split(t, sp);
@@ -939,6 +949,7 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   p->n_rect = (uint32_t)rect_list.size();
   p->n_exp = (uint32_t)exp_list.size();
   p->n_segs = (uint32_t)segs.size();
+  *segments = p->n_segs != 0;
   p->n_cells = cells;
   p->n_atom_rows = atom_rows;
   p->p_rows = p_rows;
@@ -1022,6 +1033,21 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
   }
   *out = p;
   return TCW_OK;
+}
+
+int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_templates,
+                    const uint32_t *t0s, uint64_t n_t0s, const uint32_t *taus, uint64_t n_taus,
+                    const tcw_tile_config *cfg, int flags, tcw_plan **out) {
+  if (!h || !out) return TCW_ERR_INVALID_ARG;
+  *out = nullptr;
+  bool segments = false;
+  int rc = plan_create(h, desc, n_templates, t0s, n_t0s, taus, n_taus, cfg, flags, true,
+                       &segments, out);
+  // without the memory for segment sums (up to 1 GiB): whole columns
+  if (rc == TCW_ERR_ALLOC && segments)
+    rc = plan_create(h, desc, n_templates, t0s, n_t0s, taus, n_taus, cfg, flags, false,
+                     &segments, out);
+  return rc;
 }
 
 int tcw_plan_destroy(tcw_plan *p) {
@@ -1211,7 +1237,7 @@ struct DiffSetup {
   size_t o_T, o_parts, o_t0, o_est, o_rlist, o_ident, o_RT, o_P, o_B64, o_D64, o_elist, o_A8;
   size_t o_cols, o_seg, o_need, o_scratch, o_cend, total;
   uint32_t n_rect, max_rect_tiles, max_rect_atoms, n_exp, max_cols;
-  uint64_t p_rows;
+  uint64_t p_rows, seg_floats;
   std::vector<DiffGroup> groups;
 };
 
@@ -1243,7 +1269,7 @@ static uint64_t diff_end_bytes(const DiffTemplate &t) {
 // estimate starts too many chunks).
 static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
                                 const std::vector<uint32_t> &elist, uint32_t y0, uint32_t y1,
-                                int pass, DiffGroup &g) {
+                                int pass, bool cut, DiffGroup &g) {
   uint64_t total_cg = 0;
   for (uint32_t y = y0; y < y1; y++) total_cg += (T[elist[y]].N_tau + 31u) / 32u;
   const uint64_t chunks = ((uint64_t)h->n_sms * 128u + total_cg - 1u) / total_cg;
@@ -1263,7 +1289,7 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     DiffTemplate &t = T[elist[y]];
     t.n_cg = (t.N_tau + 31u) / 32u;
     const uint64_t most = (t.N_t0 + 15u) / 16u;
-    uint64_t nc = std::max<uint64_t>(1, std::min(chunks, most));
+    uint64_t nc = cut ? std::max<uint64_t>(1, std::min(chunks, most)) : 1;
     t.g_shift = 5;
     while ((4ull << (2u * t.g_shift)) <= t.g.numAtoms) t.g_shift++;
     t.g_nseg = (uint32_t)(((uint64_t)t.g.numAtoms + (1u << t.g_shift) - 1u) >> t.g_shift);
@@ -1294,8 +1320,9 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
   g.cend_floats = pass ? cend * kDiffSegFloats : 0;
 }
 
-static int diff_prepare(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n,
-                        const uint32_t *t0s, uint64_t n_t0s, int pass, DiffSetup &S) {
+static int diff_setup(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n, const uint32_t *t0s,
+                      uint64_t n_t0s, int pass, bool cut, DiffSetup &S) {
+  S = DiffSetup{};
   if (!desc || n == 0 || !t0s) return set_err(h, TCW_ERR_INVALID_ARG, "empty template list");
   std::vector<DiffTemplate> T;
   std::vector<TemplateDev> RT;
@@ -1372,7 +1399,7 @@ static int diff_prepare(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n,
         y1++;
       }
       DiffGroup g;
-      diff_tile_group(h, T, elist, y0, y1, pass, g);
+      diff_tile_group(h, T, elist, y0, y1, pass, cut, g);
       S.groups.push_back(g);
       seg_floats = std::max(seg_floats, g.seg_floats);
       scr_floats = std::max(scr_floats, g.scr_floats);
@@ -1416,6 +1443,7 @@ static int diff_prepare(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n,
   S.o_parts = L.add(sizeof(DiffPartial) * n_tiles);
   S.o_need = L.add(sizeof(float) * n_tiles);
   S.o_cols = L.add(sizeof(ColConsts) * n_cols);
+  S.seg_floats = seg_floats;
   S.o_seg = L.add(sizeof(float) * seg_floats);
   S.o_scratch = L.add(sizeof(float) * scr_floats);
   S.o_cend = L.add(sizeof(float) * cend_floats);
@@ -1442,6 +1470,14 @@ static int diff_prepare(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n,
   TCW_CUDA(h, cudaEventRecord(h->stage_ev, h->stream));
   h->stage_pending = true;
   return TCW_OK;
+}
+
+static int diff_prepare(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n,
+                        const uint32_t *t0s, uint64_t n_t0s, int pass, DiffSetup &S) {
+  int rc = diff_setup(h, desc, n, t0s, n_t0s, pass, true, S);
+  // without the memory for segment sums (up to 1 GiB): whole columns
+  if (rc == TCW_ERR_ALLOC && S.seg_floats) rc = diff_setup(h, desc, n, t0s, n_t0s, pass, false, S);
+  return rc;
 }
 
 static DiffLaunch diff_launch(tcw_handle *h, const DiffSetup &S, const float *d_atoms,
