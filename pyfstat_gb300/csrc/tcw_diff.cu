@@ -281,7 +281,7 @@ struct ExpColumnV {
       C.power(ex);
       F2 x[4];
       TCW_DCHECK(C.wtop < g.numAtoms);
-      load_row8(atoms8 + (size_t)C.wtop * 8u, x);
+      load_row8<true>(atoms8 + (size_t)C.wtop * 8u, x);
       const F2 ph0{C.p2.h, C.p2.h}, pl0{C.p2.l, C.p2.l}, nph0{-C.p2.h, -C.p2.h};
       const F2 ph1{C.pw.h, C.pw.h}, pl1{C.pw.l, C.pw.l}, nph1{-C.pw.h, -C.pw.h};
       C.W0 = ff2_sub_scaled_x(C.W0, ph0, nph0, pl0, x[0]);
@@ -301,7 +301,7 @@ struct ExpColumnV {
       C.wlo--;
       F2 x[4];
       TCW_DCHECK(C.wlo < g.numAtoms);
-      load_row8(atoms8 + (size_t)C.wlo * 8u, x);
+      load_row8<true>(atoms8 + (size_t)C.wlo * 8u, x);
       V0 = ff2_scale_dw(C.k2.rh[0], C.k2.nrh[0], C.k2.rl[0], ff2_add_dw(V0, C.W0));
       Vc = ff_scale_dw(C.k.r2, ff_add_dw(Vc, C.Wc));
       V2 = ff2_scale_dw(C.k2.rh[1], C.k2.nrh[1], C.k2.rl[1], ff2_add_dw(V2, C.W2));

@@ -68,7 +68,8 @@ __device__ __forceinline__ void exp_rows(Column &C, const Geom &g, uint32_t shif
       t0min = min(t0min, t0);
       ExpRow e;
       e.lo = exp_lo(t0, g);
-      e.nz = e.lo < g.numAtoms ? __ldg(a8u + (size_t)e.lo * 8u + 3u) : 0xFFFFFFFFu;
+      const uint32_t *nz = a8u + (size_t)e.lo * 8u + 3u;
+      e.nz = e.lo < g.numAtoms ? (Column::kReadOnly ? __ldg(nz) : *nz) : 0xFFFFFFFFu;
       const uint32_t d = t0 - g.t0_data;
       e.a = fdiv(d, g.div);
       e.b = d - e.a * g.TAtom;

@@ -48,22 +48,31 @@ __device__ __forceinline__ FF shfl_up_ff(FF v, int d) {
 // Programmatic dependent launch (the chain of small kernels of one map): a
 // kernel's blocks may start while the kernel before it still runs and wait
 // here until it has finished and its writes are visible; both are no-ops in
-// launches without the attribute.
+// launches without the attribute.  What the chain's own kernels write
+// (descriptor, prefix and atom rows, segment sums, partials, results, maps,
+// posterior sums) changes while the next kernel is resident, so it is read by
+// plain loads: no __restrict__ parameter, no __ldg, no ld.global.nc, which
+// promise read-only data and may move above the wait.  Kernels that plans
+// launch as well, without the attribute, keep read-only loads there.
 __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // One 64-byte prefix row as two 256-bit loads (each lane's request covers
-// whole 32-byte sectors).
+// whole 32-byte sectors); kReadOnly as in load_row8.
+template <bool kReadOnly>
 __device__ __forceinline__ void ld_row16(const float *p, float r[16]) {
 #pragma unroll
-  for (int k = 0; k < 2; k++)
-    asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=f"(r[8 * k + 0]), "=f"(r[8 * k + 1]), "=f"(r[8 * k + 2]),
-                   "=f"(r[8 * k + 3]), "=f"(r[8 * k + 4]), "=f"(r[8 * k + 5]),
-                   "=f"(r[8 * k + 6]), "=f"(r[8 * k + 7])
-                 : "l"(p + 8 * k));
+  for (int k = 0; k < 2; k++) {
+    F2 x[4];
+    load_row8<kReadOnly>(p + 8 * k, x);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      r[8 * k + 2 * j] = x[j].x;
+      r[8 * k + 2 * j + 1] = x[j].y;
+    }
+  }
 }
 
 // ------------------------------------------------------------------ repack
@@ -465,7 +474,7 @@ __device__ void block_reduce_store(const Red &red, Partial *out) {
 // cell's end-index chain).  With a map to write, each warp transposes
 // 32 x 32 blocks through shared memory so that global stores are
 // row-contiguous.
-template <bool kWrite, int kPrec>
+template <bool kWrite, int kPrec, bool kReadOnly>
 __device__ void rect_tile(const TemplateDev &t, const WorkItem &w,
                           const uint32_t *__restrict__ t0s_all,
                           const uint32_t *__restrict__ taus_all, const float *__restrict__ P_all,
@@ -491,7 +500,7 @@ __device__ void rect_tile(const TemplateDev &t, const WorkItem &w,
     wr = rect_row_wrapped(t0, tau_first, t.g);
     ef = wr ? idx_end(t0 + tau_first, t.g) : 0u;
     TCW_DCHECK(j0 <= t.g.numAtoms);
-    ld_row16(P + (size_t)j0 * kPrefixStride, row0);
+    ld_row16<kReadOnly>(P + (size_t)j0 * kPrefixStride, row0);
   }
   auto end_of = [&](uint32_t tau) {
     uint32_t e = idx_end(t0 + tau, t.g);
@@ -504,7 +513,7 @@ __device__ void rect_tile(const TemplateDev &t, const WorkItem &w,
   if (row_ok && nb < ne) {
     e_cur = end_of(__ldg(taus + nb));
     TCW_DCHECK(e_cur + 1u <= t.g.numAtoms);
-    ld_row16(P + (size_t)(e_cur + 1u) * kPrefixStride, cur);
+    ld_row16<kReadOnly>(P + (size_t)(e_cur + 1u) * kPrefixStride, cur);
   }
   // One cell: F of column n from prefix row `a` (end ea); the next column's
   // prefix row is loaded into `b` (end eb) while this one is computed.  A
@@ -519,7 +528,7 @@ __device__ void rect_tile(const TemplateDev &t, const WorkItem &w,
     if (row_ok && n + 1u < ne) {
       eb = end_of(n + 1u < cb + 32u ? stau[n + 1u - cb] : __ldg(taus + n + 1u));
       TCW_DCHECK(eb + 1u <= t.g.numAtoms);
-      if (eb != ea) ld_row16(P + (size_t)(eb + 1u) * kPrefixStride, b);
+      if (eb != ea) ld_row16<kReadOnly>(P + (size_t)(eb + 1u) * kPrefixStride, b);
     }
     float F = F_prev;
     if (row_ok) {
@@ -688,14 +697,14 @@ __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *_
     reg = reg && exp_row_regular(__ldg(t0s + m), taumax, t.g);
   if (!__all_sync(0xffffffffu, reg)) {
     if (active) {
-      exp_column2<kPrec == kPrecFF_F64Det>(a8, t.g, t0s, mb, me, tau, sink, nullptr);
+      exp_column2<kPrec == kPrecFF_F64Det, kWarp>(a8, t.g, t0s, mb, me, tau, sink, nullptr);
       red.row_to_index(t.N_tau, n);
     }
     return;
   }
   const float *seg =
       t.g_nseg ? G + (t.g_off + (size_t)(n >> 5) * t.g_nseg) * kSegFloats + lane : nullptr;
-  ExpColumn<kPrec == kPrecFF_F64Det, true> C;
+  ExpColumn<kPrec == kPrecFF_F64Det, true, false, kWarp> C;
   C.init(t.g, tau);
   exp_rows<kChunks, kChunks>(C, t.g, t.g_shift, t.g_nseg, a8, t0s, mb, me, ms, active, sink, tab, seg);
   if (active) red.row_to_index(t.N_tau, n);
@@ -715,8 +724,8 @@ __device__ void exp_tile(const TemplateDev &t, const WorkItem &w, const float *_
 // 32) to 188 us for 12 templates of up to 1500 atoms and 600 x 600 cells.
 template <bool kList>
 __global__ void __launch_bounds__(128, 8)
-    exp_seg_kernel(const TemplateDev *__restrict__ T, const SegItem *__restrict__ items,
-                   uint32_t n_items, uint32_t per, const float *__restrict__ atoms8,
+    exp_seg_kernel(const TemplateDev *T, const SegItem *__restrict__ items,
+                   uint32_t n_items, uint32_t per, const float *atoms8,
                    const uint32_t *__restrict__ taus_all, float *__restrict__ G) {
   const uint32_t wi = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
   pdl_begin();
@@ -739,7 +748,7 @@ __global__ void __launch_bounds__(128, 8)
   if (3ull * taumax + 2ull * t.g.TAtom < ((uint64_t)t.g.TAtom << (t.g_shift + 1u))) return;
   if (n >= t.N_tau) tau = taumax;
   const float *a8 = atoms8 + t.a8_off * 8u;
-  ExpColumn<false, true> C;
+  ExpColumn<false, true, false, kList> C;
   C.init(t.g, tau);
   for (uint32_t j = w.j0; j < w.j1; j++) {
     C.reset_window(min(t.g.numAtoms, (j + 1u) << t.g_shift));
@@ -784,11 +793,10 @@ constexpr int map_min_blocks() {
 // history (TemplateDev::e_sub > 1).
 template <int kWin, bool kPersist, bool kWrite, int kPrec, bool kChunks>
 __global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kChunks>()))
-    map_kernel(const TemplateDev *__restrict__ T, const WorkItem *__restrict__ items,
+    map_kernel(const TemplateDev *T, const WorkItem *__restrict__ items,
                uint32_t n_items, uint32_t *__restrict__ counter, const float *__restrict__ atoms,
-               const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s,
-               const uint32_t *__restrict__ taus,
-               const float *__restrict__ P, const float *__restrict__ G,
+               const float *atoms8, const uint32_t *__restrict__ t0s,
+               const uint32_t *__restrict__ taus, const float *P, const float *G,
                float *__restrict__ Fmn, Partial *__restrict__ parts) {
   constexpr uint32_t kSmem = kWin == TCW_WINDOW_RECT ? (kWrite ? (kBlock / 32) * 32 * 33 : 1)
                                                      : (kBlock / 32) * kExpRowTab * 4;
@@ -812,8 +820,8 @@ __global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kChunk
       for (uint32_t g = 0; g < w.tn; g++) {
         Red red;
         red.init();
-        rect_tile<kWrite, kPrec>(t, w, t0s, taus, P, Fmn, red, smw, g, 1u, 0u,
-                                 s_tau + (threadIdx.x >> 5) * 32u);
+        rect_tile<kWrite, kPrec, true>(t, w, t0s, taus, P, Fmn, red, smw, g, 1u, 0u,
+                                       s_tau + (threadIdx.x >> 5) * 32u);
         acc = red_combine(acc, RedVal{red.mx, red.bidx, fsub(red.s, red.c)});
       }
 #pragma unroll
@@ -878,9 +886,9 @@ __global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kChunk
     w.m1 = min(t.N_t0, w.m0 + t.tile_tm);
     w.tn = (uint16_t)(t.tile_tm / 32u);  // row groups of 32 rows (one per warp)
     const uint32_t warp = threadIdx.x >> 5, rg = w.tn;
-    rect_tile<kWrite, kPrec>(t, w, t0s, taus, P, Fmn, red,
-                             reinterpret_cast<float *>(sm) + warp * (32 * 33), warp % rg, 4u / rg,
-                             warp / rg, s_tau + warp * 32u);
+    rect_tile<kWrite, kPrec, false>(t, w, t0s, taus, P, Fmn, red,
+                                    reinterpret_cast<float *>(sm) + warp * (32 * 33), warp % rg,
+                                    4u / rg, warp / rg, s_tau + warp * 32u);
   } else {
     w.m1 = w.m0 + t.tile_tm;
     w.tn = (uint16_t)t.tile_tn;
@@ -894,9 +902,9 @@ __global__ void __launch_bounds__(kBlock, (map_min_blocks<kWin, kPersist, kChunk
 // ------------------------------------------------------------------ finalize
 
 // One warp per template: merge its partials in index order.
-__global__ void __launch_bounds__(128) finalize_kernel(const TemplateDev *__restrict__ T,
+__global__ void __launch_bounds__(128) finalize_kernel(const TemplateDev *T,
                                                        uint32_t n_templates,
-                                                       const Partial *__restrict__ parts,
+                                                       const Partial *parts,
                                                        tcw_result *__restrict__ results) {
   const uint32_t tmpl = blockIdx.x * 4u + (threadIdx.x >> 5);
   const uint32_t lane = threadIdx.x & 31u;
@@ -1124,8 +1132,8 @@ int map_blocks_per_sm(int window, int prec, bool chunks) {
 // One block per template where there are few (up to thousands of tiles
 // each): its partials merged by 256 threads, warps' results combined in warp
 // order.
-__global__ void __launch_bounds__(256) finalize_block_kernel(const TemplateDev *__restrict__ T,
-                                                             const Partial *__restrict__ parts,
+__global__ void __launch_bounds__(256) finalize_block_kernel(const TemplateDev *T,
+                                                             const Partial *parts,
                                                              tcw_result *__restrict__ results) {
   __shared__ float s_best[8];
   __shared__ int64_t s_bidx[8];
@@ -1215,9 +1223,12 @@ constexpr uint32_t kPostThreads = 256;
 constexpr uint32_t kPostCols = 1024;
 constexpr uint32_t kPostMaxRows = 256;
 
+// kChained (both kernels): launched as a dependent in a single map's chain
+// (pdl_begin); a plan's launches take read-only loads.
+template <bool kChained>
 __global__ void __launch_bounds__(kPostThreads) post_sums_kernel(
-    const TemplateDev *__restrict__ T, const uint2 *__restrict__ chunks, uint32_t rows,
-    uint32_t cols, const float *__restrict__ maps, const tcw_result *__restrict__ results,
+    const TemplateDev *T, const uint2 *__restrict__ chunks, uint32_t rows,
+    uint32_t cols, const float *maps, const tcw_result *results,
     double *__restrict__ rowsum, double *__restrict__ colsum, uint32_t *__restrict__ ticket) {
   __shared__ float2 srow[kPostThreads / 32][kPostMaxRows];
   pdl_begin();
@@ -1235,6 +1246,7 @@ __global__ void __launch_bounds__(kPostThreads) post_sums_kernel(
   if (ch.y == 0u && tid == 0u) ticket[ch.x] = 0u;
   const float maxF = results[ch.x].maxF;
   const float *F = maps + t.map_off;
+  auto load = [](const float *p) { return kChained ? *p : __ldg(p); };
   for (uint32_t k = lane; k < m1 - m0; k += 32u) srow[wid][k] = make_float2(0.0f, 0.0f);
   __syncwarp();
   for (uint32_t n0 = nb + tid; n0 - tid < ne; n0 += kPostCols) {
@@ -1248,7 +1260,7 @@ __global__ void __launch_bounds__(kPostThreads) post_sums_kernel(
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           const uint32_t n = n0 + 256u * j;
-          e[j] = (m + q < m1 && n < ne) ? ex2_approx((__ldg(row + n) - maxF) * kLog2e) : 0.0f;
+          e[j] = (m + q < m1 && n < ne) ? ex2_approx((load(row + n) - maxF) * kLog2e) : 0.0f;
         }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -1322,9 +1334,10 @@ __device__ __forceinline__ PostBest post_block_best(PostBest best, PostBest *sh)
   return best;
 }
 
+template <bool kChained>
 __global__ void __launch_bounds__(kPostThreads) post_argmax_kernel(
-    const TemplateDev *__restrict__ T, uint32_t rows, uint32_t cols,
-    const double *__restrict__ rowsum, const double *__restrict__ colsum,
+    const TemplateDev *T, uint32_t rows, uint32_t cols, const double *rowsum,
+    const double *colsum,
     PostPart *__restrict__ parts, uint32_t *__restrict__ ticket,
     tcw_result *__restrict__ results) {
   __shared__ PostBest sh[kPostThreads / 32];
@@ -1341,14 +1354,15 @@ __global__ void __launch_bounds__(kPostThreads) post_argmax_kernel(
   const uint32_t i0 = (is_row ? part : part - p_row) * e, i1 = min(N, i0 + e);
   const uint32_t n_sum = is_row ? (t.N_tau + cols - 1u) / cols : (t.N_t0 + rows - 1u) / rows;
   const double *S = is_row ? rowsum + t.row_off : colsum + t.col_off;
+  auto load = [](const double *p) { return kChained ? *p : __ldg(p); };
   PostBest best{-1, INT64_MAX};
   for (uint32_t i = i0 + threadIdx.x; i < i1; i += kPostThreads) {
     double v[4] = {0.0, 0.0, 0.0, 0.0};  // four chains: FP64 additions are slow to return
     uint32_t c = 0;
     for (; c + 4u <= n_sum; c += 4u)
 #pragma unroll
-      for (uint32_t q = 0; q < 4u; q++) v[q] += S[(size_t)(c + q) * N + i];
-    for (; c < n_sum; c++) v[0] += S[(size_t)c * N + i];
+      for (uint32_t q = 0; q < 4u; q++) v[q] += load(S + (size_t)(c + q) * N + i);
+    for (; c < n_sum; c++) v[0] += load(S + (size_t)c * N + i);
     const int64_t key = post_key((v[0] + v[1]) + (v[2] + v[3]));
     if (key > best.v) best = PostBest{key, (int64_t)i};  // i increases: keeps the first
   }
@@ -1378,14 +1392,16 @@ cudaError_t launch_posteriors(const TemplateDev *d_T, uint32_t n_templates, cons
                               const float *d_maps, tcw_result *d_results, bool chained,
                               cudaStream_t stream) {
   if (L.n_chunks == 0 || n_templates == 0) return cudaSuccess;
-  cudaError_t e = launch_kernel(post_sums_kernel, L.n_chunks, kPostThreads, stream, chained, d_T,
-                                L.chunks, L.rows, L.cols, d_maps, d_results, L.rowsum, L.colsum,
+  cudaError_t e = launch_kernel(chained ? post_sums_kernel<true> : post_sums_kernel<false>,
+                                L.n_chunks, kPostThreads, stream, chained, d_T, L.chunks, L.rows,
+                                L.cols, d_maps, (const tcw_result *)d_results, L.rowsum, L.colsum,
                                 L.ticket);
   if (e != cudaSuccess) return e;
   for (uint32_t y0 = 0; y0 < n_templates; y0 += 65535u) {
     const uint32_t ny = n_templates - y0 < 65535u ? n_templates - y0 : 65535u;
-    e = launch_kernel(post_argmax_kernel, dim3(2u * kPostParts, ny), kPostThreads, stream,
-                      chained && y0 == 0, d_T + y0, L.rows, L.cols, L.rowsum, L.colsum,
+    e = launch_kernel(chained ? post_argmax_kernel<true> : post_argmax_kernel<false>,
+                      dim3(2u * kPostParts, ny), kPostThreads, stream, chained && y0 == 0,
+                      d_T + y0, L.rows, L.cols, (const double *)L.rowsum, (const double *)L.colsum,
                       L.parts + (size_t)y0 * 2u * kPostParts, L.ticket + y0, d_results + y0);
     if (e != cudaSuccess) return e;
   }
