@@ -109,7 +109,9 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
   t.N_tau = N_tau;
   t.ln_prior = log(70.0 / ((double)N_t0 * (double)N_tau));
   ExpSplit sp{};
-  const uint32_t n_chunks = (N_t0 + 63u) / 64u;
+  // posterior sums by blocks of p_rows x p_cols cells; documented: 64 rows of
+  // all columns
+  uint32_t p_rows = 64u, p_cols = 0xFFFFFC00u, n_rc = 0, n_cc = 0;
   size_t o_T = 0, o_parts = 0, o_rows = 0, o_row = 0, o_col = 0, o_G = 0;
   auto layout = [&](bool cut, bool documented) {
     if (window == TCW_WINDOW_EXP) {
@@ -130,9 +132,11 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
                               ? sizeof(float) * kPrefixStride * ((size_t)numAtoms + 1u)
                               : sizeof(float) * 8u * (size_t)numAtoms));
     o_row = off;
-    if (post) off = align256(off + sizeof(double) * N_t0);
+    n_rc = (uint32_t)(((uint64_t)N_t0 + p_rows - 1u) / p_rows);
+    n_cc = (uint32_t)(((uint64_t)N_tau + p_cols - 1u) / p_cols);
+    if (post) off = align256(off + sizeof(double) * (size_t)N_t0 * n_cc);
     o_col = off;
-    if (post) off = align256(off + sizeof(double) * (size_t)n_chunks * N_tau);
+    if (post) off = align256(off + sizeof(double) * (size_t)n_rc * N_tau);
     o_G = off;
     if (sp.nseg) off = align256(off + sizeof(float) * sp.seg_floats(N_tau));
     return off <= kNoallocScratchBytes;
@@ -141,7 +145,23 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
   // they admit fits without the list
   if (!layout(false, true)) return TCW_ERR_OVERFLOW;
   const bool cut = window == TCW_WINDOW_EXP && prec != kPrecPlain32;
-  if (!layout(cut, false)) layout(false, false);
+  // the handle's posterior blocks (post_rows x 1024 columns), larger ones where
+  // their sums do not fit (64 x 60000 cells: one block for all of them 1781 us
+  // a call, 236 blocks 64 us)
+  auto fit = [&](bool c) {
+    p_rows = post_rows((uint64_t)N_t0 * N_tau, sms);
+    p_cols = 1024u;
+    while (!layout(c, false)) {
+      if (p_rows < 64u)
+        p_rows *= 2u;
+      else if (n_cc > 1u)
+        p_cols *= 2u;
+      else
+        return false;
+    }
+    return true;
+  };
+  if (!fit(cut)) fit(false);
 
   unsigned char *base = nullptr;
   PostPart *pp = nullptr;
@@ -177,8 +197,7 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
   if (launch_map(window, ml, s) != cudaSuccess) return TCW_ERR_CUDA;
   if (launch_finalize(dT, 1, dparts, d_result, true, s) != cudaSuccess) return TCW_ERR_CUDA;
   if (post) {
-    // one column chunk per row chunk of 64 rows: the documented scratch
-    const PostLayout pl{64u, (N_tau + 1023u) / 1024u * 1024u, n_chunks, nullptr,
+    const PostLayout pl{p_rows, p_cols, n_rc * n_cc, nullptr,
                         reinterpret_cast<double *>(base + o_row),
                         reinterpret_cast<double *>(base + o_col), pp,
                         reinterpret_cast<uint32_t *>(pp + 2u * kPostParts)};

@@ -173,3 +173,72 @@ def test_noalloc_rejects_problems_beyond_its_scratch():
     with pytest.raises(_lib.TcwError) as e:
         _lib.map_plain_noalloc(None, A, n, 1800, 700000000, 1, grid, 4, grid, 4, None, r)
     assert e.value.code == _lib.TCW_ERR_OVERFLOW
+
+
+def _post_call(torch, lib, window, nsft, n_t0, n_tau, alloc):
+    """One map with posteriors (a closure that enqueues it, its map and record)."""
+    from pyfstat_gb300 import _lib
+
+    t0_data, A = synth.merged_atoms(3, nsft, 1)
+    span = nsft * 1800
+    t0s = (t0_data + max(1, span // n_t0) * np.arange(n_t0)).astype(np.uint32)
+    taus = (1800 + max(1, span // n_tau) * np.arange(n_tau)).astype(np.uint32)
+    dev = [torch.from_numpy(x).cuda() for x in (A, t0s.view(np.int32), taus.view(np.int32))]
+    F = torch.empty((n_t0, n_tau), dtype=torch.float32, device="cuda")
+    r = torch.zeros(5, dtype=torch.float64, device="cuda")
+    args = (dev[0], nsft, 1800, t0_data, window, dev[1], n_t0, dev[2], n_tau, F, r, FLAGS)
+    if alloc:
+        h = _lib.Handle(0)
+        h.set_stream(0x1)
+        return lambda: h.map_plain(*args), F, r, h
+    return lambda: _lib.map_plain_noalloc(0x1, *args), F, r, None
+
+
+@pytest.mark.parametrize("shape", [(1, 480, 64, 60000), (2, 480, 16, 33000), (1, 480, 9000, 65),
+                                   (1, 250000, 63, 1500), (1, 1, 1, 1)])
+def test_posteriors_of_wide_and_tall_maps(shape):
+    """Column and row sums in the blocks that fit the scratch (all of them, few
+    of them beside 250000 prefix rows): the handle's record."""
+    torch = pytest.importorskip("torch")
+    from pyfstat_gb300 import _lib
+
+    lib = _lib.load()
+    recs, maps = [], []
+    for alloc in (True, False):
+        call, F, r, h = _post_call(torch, lib, *shape, alloc)
+        call()
+        torch.cuda.synchronize()
+        recs.append(r.cpu().numpy().view(_lib.RESULT_DTYPE)[0])
+        maps.append(F.cpu().numpy())
+        if h:
+            h.close()
+    np.testing.assert_allclose(maps[1], maps[0], rtol=1e-6, atol=0)
+    e = np.exp(maps[1].astype(np.float64) - maps[1].max())
+    for field, sums in (("t0_mp_idx", e.sum(1)), ("tau_mp_idx", e.sum(0))):
+        assert sums[recs[1][field]] >= sums.max() * (1.0 - 1e-6), field
+        top = np.sort(sums)[-2:]
+        if top[-1] - top[0] > 1e-5 * top[-1]:  # a clear maximum
+            assert recs[1][field] == recs[0][field], field
+
+
+def test_wide_posteriors_take_about_as_long_as_the_handles():
+    """64 x 60000 cells: within three times the handle's call (ten times while
+    one block added all of them)."""
+    torch = pytest.importorskip("torch")
+    from pyfstat_gb300 import _lib
+
+    times = []
+    for alloc in (True, False):
+        call, _, _, h = _post_call(torch, _lib.load(), 1, 480, 64, 60000, alloc)
+        best = np.inf
+        for _ in range(12):
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record()
+            call()
+            ev[1].record()
+            torch.cuda.synchronize()
+            best = min(best, ev[0].elapsed_time(ev[1]))
+        times.append(best)
+        if h:
+            h.close()
+    assert times[1] <= 3.0 * times[0], times
