@@ -649,7 +649,7 @@ __global__ void __launch_bounds__(kDiffBlock, 5)
     if (lane == 0) *out = DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
     return;
   }
-  if (!(nd < bd.hot)) return;  // diff_hot_kernel
+  if (!(nd < bd.hot) && !L.t.whole) return;  // diff_hot_kernel
   const uint32_t me = min(L.t.N_t0, mb + L.t.chunk_rows);
   L.columns(atoms8, t0s_all, cg);
   ExpColumn<false> C;
@@ -864,7 +864,7 @@ __global__ void __launch_bounds__(kDiffBlock)
   const DiffWeights w(t, k, temp, lnZ1, lnZ2, gB, gS);
   const float nd = need[t.part_off + tile];
   if (nd < w.skip) return;    // diff_atoms_kernel skips its rows
-  if (!(nd < w.hot)) return;  // diff_hot_kernel
+  if (!(nd < w.hot) && !t.whole) return;  // diff_hot_kernel
   const uint32_t me = min(t.N_t0, mb + t.chunk_rows);
   L.columns(atoms8, t0s_all, cg);
   const DiffGrad grad(w, temp);
@@ -963,7 +963,7 @@ __global__ void __launch_bounds__(kHotThreads, 1)
   const uint32_t k = list[blockIdx.y], cg = cg0 + blockIdx.x;  // (grid x: a slice's groups)
   L.t = T[k];
   const DiffTemplate &t = L.t;
-  if (cg >= t.n_cg) return;
+  if (cg >= t.n_cg || t.whole) return;
   const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
   const float *nd = need + t.part_off + (size_t)cg * t.n_chunk;
   // the first and last hot chunk
@@ -1821,19 +1821,21 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
         const uint32_t cgs = g.max_cg - cg0 < g.cg_slice ? g.max_cg - cg0 : g.cg_slice;
         const dim3 hot(cgs, g.ny), stiles((g.slice_tiles + 3u) / 4u, g.ny);
         const dim3 aseg((g.slice_aseg + 3u) / 4u, g.ny);
-        if ((e = cudaEventRecord(fork, stream)) != cudaSuccess ||
-            (e = cudaStreamWaitEvent(side, fork, 0)) != cudaSuccess)
+        if (g.hot && ((e = cudaEventRecord(fork, stream)) != cudaSuccess ||
+                      (e = cudaStreamWaitEvent(side, fork, 0)) != cudaSuccess))
           return e;
         if (pass == 0) {
-          diff_hot_kernel<false><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
-              L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, nullptr, nullptr, nullptr,
-              nullptr, cg0, nullptr, nullptr, L.parts, smem_atoms);
+          if (g.hot)
+            diff_hot_kernel<false><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
+                L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, nullptr, nullptr,
+                nullptr, nullptr, cg0, nullptr, nullptr, L.parts, smem_atoms);
           diff_fwd_kernel<<<tiles, kDiffBlock, 0, stream>>>(
               L.T, list, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.est, L.temp, L.parts);
         } else {
-          diff_hot_kernel<true><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
-              L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1, L.lnZ2, L.gB,
-              L.gS, cg0, L.scratch, L.grad_tau, nullptr, smem_atoms);
+          if (g.hot)
+            diff_hot_kernel<true><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
+                L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1, L.lnZ2, L.gB,
+                L.gS, cg0, L.scratch, L.grad_tau, nullptr, smem_atoms);
           if (g.max_segs && cg0 == 0)  // (over the window sums, which nothing reads any more)
             diff_seg_kernel<true><<<segs, kDiffBlock, 0, stream>>>(
                 L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
@@ -1842,8 +1844,8 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
               L.T, list, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB,
               L.gS, cg0, cgs, L.scratch, L.grad_tau);
         }
-        if ((e = cudaEventRecord(join, side)) != cudaSuccess ||
-            (e = cudaStreamWaitEvent(stream, join, 0)) != cudaSuccess)
+        if (g.hot && ((e = cudaEventRecord(join, side)) != cudaSuccess ||
+                      (e = cudaStreamWaitEvent(stream, join, 0)) != cudaSuccess))
           return e;
         if (pass == 1) {
           diff_atoms_kernel<true><<<aseg, kDiffBlock, 0, stream>>>(

@@ -327,7 +327,8 @@ struct DiffTemplate {
   uint32_t N_t0, N_tau;
   double tau_min, tau_max;
   uint32_t part_off, n_parts;  // this template's tiles (need, partials)
-  uint32_t window, pad;
+  uint32_t window;
+  uint32_t whole;  // its tiles are whole columns and none is left to diff_hot_kernel
   uint64_t p_off;
   uint32_t n_cg, n_chunk, chunk_rows;
   uint32_t g_shift, g_nseg, n_aseg;  // segment sums; atom segments of the transposed recurrence
@@ -357,6 +358,7 @@ struct DiffGroup {
   uint32_t max_cg, max_tiles, max_segs, max_atoms;
   // column groups of a slice, most tiles / atom segments of one template in it
   uint32_t cg_slice, slice_tiles, slice_aseg;
+  bool hot;  // some template's hot tiles are diff_hot_kernel's
   uint32_t seg_per;  // segments per warp
   uint64_t seg_floats, scr_floats, cend_floats;
 };
