@@ -1267,13 +1267,15 @@ static uint64_t diff_end_bytes(const DiffTemplate &t) {
 // walk them last as long as their longest tile (24 templates 3.19 -> 2.99 ms,
 // 100 5.4 -> 5.0, 600 17.8 -> 12.9; two 2.98 / 5.1 / 14.3, eight 3.1: the
 // estimate starts too many chunks).
-// Where whole columns give every scheduler a warp, templates of few rows keep
-// whole columns: their hot tiles are most of them, the walk that diff_hot_kernel
-// would repeat is then the tile's own, bit for bit, and a warp per column group
-// shares the SM with others where that kernel's nine take it alone (forward /
+// Where whole columns give every scheduler a warp, templates of few rows and
+// atoms keep whole columns: their hot tiles are most of them, the walk that
+// diff_hot_kernel would repeat is then the tile's own, bit for bit, and a warp
+// per column group shares the SM with others where that kernel's nine take it
+// alone.  More atoms make the walk the longest chain (64 rows of 17532 atoms
+// among 300 templates: 12.5 + 14.7 -> 26 + 34 ms, so they are cut; forward /
 // backward of 3000 templates of 47 x 47 cells 1.72 / 1.28 -> 1.21 / 0.83 ms, 1000 of
 // 32 x 32 0.55 / 0.52 -> 0.41 / 0.41).
-constexpr uint32_t kDiffFewRows = 64;
+constexpr uint32_t kDiffFewRows = 64, kDiffFewAtoms = 256;
 static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
                                 const std::vector<uint32_t> &elist, uint32_t y0, uint32_t y1,
                                 int pass, bool cut, DiffGroup &g) {
@@ -1297,7 +1299,7 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     DiffTemplate &t = T[elist[y]];
     t.n_cg = (t.N_tau + 31u) / 32u;
     const uint64_t most = (t.N_t0 + 15u) / 16u;
-    uint64_t nc = cut && !(filled && t.N_t0 <= kDiffFewRows)
+    uint64_t nc = cut && !(filled && t.N_t0 <= kDiffFewRows && t.g.numAtoms <= kDiffFewAtoms)
                       ? std::max<uint64_t>(1, std::min(chunks, most))
                       : 1;
     t.g_shift = 5;
@@ -1308,7 +1310,7 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     t.chunk_rows = (uint32_t)((t.N_t0 + nc - 1) / nc);
     t.n_chunk = (t.N_t0 + t.chunk_rows - 1u) / t.chunk_rows;
     if (t.n_chunk == 1u || t.g.numAtoms < 64u) t.g_nseg = 0;
-    t.whole = filled && t.n_chunk == 1u ? 1u : 0u;
+    t.whole = filled && t.n_chunk == 1u && t.g.numAtoms <= kDiffFewAtoms ? 1u : 0u;
     g.hot = g.hot || !t.whole;
     t.n_aseg = (t.g.numAtoms + kDiffAtomSeg - 1u) / kDiffAtomSeg;
     t.seg_off = seg;
