@@ -1236,9 +1236,10 @@ int tcw_plan_run_timed(tcw_handle *h, tcw_plan *p, const float *d_atoms, tcw_res
 struct DiffSetup {
   size_t o_T, o_parts, o_t0, o_est, o_rlist, o_ident, o_RT, o_P, o_B64, o_D64, o_elist, o_A8;
   size_t o_cols, o_seg, o_need, o_scratch, o_cend, total;
-  uint32_t n_rect, max_rect_tiles, max_rect_atoms, n_exp, max_cols;
+  uint32_t n_rect, max_rect_tiles, max_rect_atoms, n_exp;
   uint64_t p_rows, seg_floats;
   std::vector<DiffGroup> groups;
+  std::vector<DiffClass> classes;
 };
 
 // Backward workspace of one group of exponential templates (adjoint sources
@@ -1276,9 +1277,16 @@ static uint64_t diff_end_bytes(const DiffTemplate &t) {
 // backward of 3000 templates of 47 x 47 cells 1.72 / 1.28 -> 1.21 / 0.83 ms, 1000 of
 // 32 x 32 0.55 / 0.52 -> 0.41 / 0.41).
 constexpr uint32_t kDiffFewRows = 64, kDiffFewAtoms = 256;
+// Warps of a class's grid that have no tile: above this, half a millisecond of
+// empty blocks, the templates of unequal size go in launches of their own,
+// each of which lasts as long as its longest tile (gradients of 2000 templates
+// of 32 x 32 cells beside one of 17532 atoms and 1024 x 2048: one grid for all
+// 8.3 + 21.1 ms, two classes 5.2 + 8.8; 300 templates of log-uniform sizes: one
+// 12.1 + 14.3, three 13.1 + 17.0).
+constexpr uint64_t kDiffEmptyWarps = 1ull << 22;
 static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
-                                const std::vector<uint32_t> &elist, uint32_t y0, uint32_t y1,
-                                int pass, bool cut, DiffGroup &g) {
+                            const std::vector<uint32_t> &elist, uint32_t y0, uint32_t y1,
+                            int pass, bool cut, DiffGroup &g, std::vector<DiffClass> &classes) {
   uint64_t total_cg = 0;
   for (uint32_t y = y0; y < y1; y++) total_cg += (T[elist[y]].N_tau + 31u) / 32u;
   const uint64_t chunks = ((uint64_t)h->n_sms * 128u + total_cg - 1u) / total_cg;
@@ -1288,6 +1296,8 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
   g = DiffGroup{};
   g.y0 = y0;
   g.ny = y1 - y0;
+  g.c0 = (uint32_t)classes.size();
+  uint64_t most_warps = 0, class_warps = 0;  // of one template, of all of the class
   g.cg_slice = 0xFFFFFFFFu;
   if (pass && g.ny == 1u) {
     const DiffTemplate &t = T[elist[y0]];
@@ -1322,12 +1332,27 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     cend += (uint64_t)cgs * t.n_aseg;
     g.max_cg = std::max(g.max_cg, t.n_cg);
     g.max_atoms = std::max(g.max_atoms, t.g.numAtoms);
-    g.max_tiles = std::max(g.max_tiles, t.n_cg * t.n_chunk);
-    if (t.g_nseg)
-      g.max_segs = std::max(g.max_segs, t.n_cg * t.g_nseg);
-    g.slice_tiles = std::max(g.slice_tiles, cgs * t.n_chunk);
-    g.slice_aseg = std::max(g.slice_aseg, cgs * t.n_aseg);
+    const uint64_t warps =
+        (uint64_t)cgs * std::max(std::max(t.n_chunk, t.g_nseg), pass ? t.n_aseg : 0u);
+    const uint64_t most_now = std::max(most_warps, warps);
+    if (y == y0 || (classes.back().ny + 1u) * most_now > class_warps + warps + kDiffEmptyWarps) {
+      classes.push_back(DiffClass{y, 0, 0, 0, 0, 0, 0, 0});
+      most_warps = warps;
+      class_warps = 0;
+    } else {
+      most_warps = most_now;
+    }
+    class_warps += warps;
+    DiffClass &c = classes.back();
+    c.ny++;
+    c.max_tiles = std::max(c.max_tiles, t.n_cg * t.n_chunk);
+    c.max_segs = std::max(c.max_segs, t.n_cg * t.g_nseg);
+    c.max_atoms = std::max(c.max_atoms, t.g.numAtoms);
+    c.max_cols = std::max(c.max_cols, t.N_tau);
+    c.slice_tiles = std::max(c.slice_tiles, cgs * t.n_chunk);
+    c.slice_aseg = std::max(c.slice_aseg, cgs * t.n_aseg);
   }
+  g.n_classes = (uint32_t)classes.size() - g.c0;
   g.seg_per = segs_per_warp(seg, h->n_sms);
   g.seg_floats = seg * seg_floats;
   g.scr_floats = pass ? scr : 0;
@@ -1344,7 +1369,6 @@ static int diff_setup(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n, cons
   uint64_t p_rows = 0, atom_rows = 0, n_cols = 0, n_tiles = 0, b_rows = 0, row_groups = 0;
   S.max_rect_tiles = S.max_rect_atoms = 0;
   uint64_t seg_floats = 0, scr_floats = 0, cend_floats = 0;
-  uint32_t max_cols = 0;
   try {
     T.resize(n);
     for (uint32_t k = 0; k < n; k++) {
@@ -1393,12 +1417,19 @@ static int diff_setup(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n, cons
       } else {
         t.col_off = n_cols;
         n_cols += d.N_tau;
-        max_cols = std::max(max_cols, d.N_tau);
         elist.push_back(k);
         atom_rows = std::max<uint64_t>(atom_rows, d.atom_offset + d.numAtoms);
       }
       T[k] = t;
     }
+    // largest templates first, so that those of a launch are of like size
+    auto size_of = [&](uint32_t k) {
+      const DiffTemplate &t = T[k];
+      return ((uint64_t)t.N_tau + 31u) / 32u *
+             (t.N_t0 / 16u + (uint64_t)t.g.numAtoms / kDiffAtomSeg + 1u);
+    };
+    std::stable_sort(elist.begin(), elist.end(),
+                     [&](uint32_t a, uint32_t b) { return size_of(a) > size_of(b); });
     // groups of exponential templates within the workspace bound, one template
     // at least
     for (uint32_t y0 = 0; y0 < elist.size();) {
@@ -1413,7 +1444,7 @@ static int diff_setup(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n, cons
         y1++;
       }
       DiffGroup g;
-      diff_tile_group(h, T, elist, y0, y1, pass, cut, g);
+      diff_tile_group(h, T, elist, y0, y1, pass, cut, g, S.classes);
       S.groups.push_back(g);
       seg_floats = std::max(seg_floats, g.seg_floats);
       scr_floats = std::max(scr_floats, g.scr_floats);
@@ -1443,7 +1474,6 @@ static int diff_setup(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n, cons
   }
   S.n_rect = (uint32_t)rlist.size();
   S.n_exp = (uint32_t)elist.size();
-  S.max_cols = max_cols;
   S.p_rows = p_rows;
   Layout L;
   S.o_T = L.add(sizeof(DiffTemplate) * n);
@@ -1520,7 +1550,6 @@ static DiffLaunch diff_launch(tcw_handle *h, const DiffSetup &S, const float *d_
   L.atoms8 = S.o_A8 ? reinterpret_cast<float *>(h->d_ws + S.o_A8) : nullptr;
   L.exp_list = reinterpret_cast<const uint32_t *>(h->d_ws + S.o_elist);
   L.n_exp = S.n_exp;
-  L.max_cols = S.max_cols;
   return L;
 }
 
@@ -1537,8 +1566,8 @@ int tcw_map_forward(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n_templat
   rc = diff_prepare(h, desc, n_templates, t0s, n_t0s, 0, S);
   if (rc) return rc;
   DiffLaunch L = diff_launch(h, S, d_atoms, temperature);
-  TCW_CUDA(h, launch_diff(0, L, S.groups.data(), (uint32_t)S.groups.size(), h->stream,
-                          h->side_stream, h->fork_ev, h->join_ev));
+  TCW_CUDA(h, launch_diff(0, L, S.groups.data(), (uint32_t)S.groups.size(), S.classes.data(),
+                          h->stream, h->side_stream, h->fork_ev, h->join_ev));
   TCW_CUDA(h, launch_diff_finalize(L.T, n_templates, L.parts, temperature, d_lnBtSG, d_softmax2F,
                                    h->stream));
   return TCW_OK;
@@ -1573,8 +1602,8 @@ int tcw_map_backward(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n_templa
   TCW_CUDA(h, cudaMemsetAsync(d_grad_tau, 0, sizeof(double) * 2u * n_templates, h->stream));
   if (S.n_rect)
     TCW_CUDA(h, cudaMemsetAsync(L.D64, 0, sizeof(double) * 8u * S.p_rows, h->stream));
-  TCW_CUDA(h, launch_diff(1, L, S.groups.data(), (uint32_t)S.groups.size(), h->stream,
-                          h->side_stream, h->fork_ev, h->join_ev));
+  TCW_CUDA(h, launch_diff(1, L, S.groups.data(), (uint32_t)S.groups.size(), S.classes.data(),
+                          h->stream, h->side_stream, h->fork_ev, h->join_ev));
   return TCW_OK;
 }
 

@@ -1793,8 +1793,8 @@ __global__ void __launch_bounds__(256)
 // `side`: a second stream for diff_hot_kernel, whose few long blocks run beside
 // the tiles that need no whole walk; fork and join are the caller's events.
 cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, uint32_t n_groups,
-                        cudaStream_t stream, cudaStream_t side, cudaEvent_t fork,
-                        cudaEvent_t join) {
+                        const DiffClass *classes, cudaStream_t stream, cudaStream_t side,
+                        cudaEvent_t fork, cudaEvent_t join) {
   cudaError_t e = cudaSuccess;
   if (L.n_exp) {
     e = cudaFuncSetAttribute(pass == 0 ? (const void *)diff_hot_kernel<false>
@@ -1803,57 +1803,69 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
     if (e != cudaSuccess) return e;
     for (uint32_t q = 0; q < n_groups; q++) {
       const DiffGroup &g = groups[q];
-      const uint32_t *list = L.exp_list + g.y0;
-      const dim3 tiles((g.max_tiles + 3u) / 4u, g.ny), segs((g.max_segs + 3u) / 4u, g.ny);
+      const DiffClass *c0 = classes + g.c0, *c1 = c0 + g.n_classes;
       // atoms that diff_hot_kernel stages in shared memory (28 bytes each)
       const uint32_t smem_atoms = g.max_atoms < kHotAtoms ? g.max_atoms : kHotAtoms;
-      const uint32_t atom_blocks = (g.max_atoms + 255u) / 256u;
-      diff_prep_kernel<<<dim3(atom_blocks + (L.max_cols + 255u) / 256u, g.ny), 256, 0, stream>>>(
-          L.T, list, atom_blocks, L.atoms, L.atoms8, L.cols);
-      if (g.max_segs)
-        diff_seg_kernel<false><<<segs, kDiffBlock, 0, stream>>>(
-            L.T, list, L.atoms8, L.t0s, L.cols, nullptr, L.temp, nullptr, nullptr, nullptr,
-            nullptr, g.seg_per, L.seg);
-      diff_est_kernel<<<tiles, kDiffBlock, 0, stream>>>(L.T, list, L.atoms8, L.t0s, L.cols, L.seg,
-                                                        L.need, L.est);
+      auto warps = [](const DiffClass *c, uint32_t n) { return dim3((n + 3u) / 4u, c->ny); };
+      for (const DiffClass *c = c0; c < c1; c++) {
+        const uint32_t atom_blocks = (c->max_atoms + 255u) / 256u;
+        diff_prep_kernel<<<dim3(atom_blocks + (c->max_cols + 255u) / 256u, c->ny), 256, 0,
+                           stream>>>(L.T, L.exp_list + c->y0, atom_blocks, L.atoms, L.atoms8,
+                                     L.cols);
+      }
+      for (const DiffClass *c = c0; c < c1; c++)
+        if (c->max_segs)
+          diff_seg_kernel<false><<<warps(c, c->max_segs), kDiffBlock, 0, stream>>>(
+              L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, nullptr, L.temp, nullptr, nullptr,
+              nullptr, nullptr, g.seg_per, L.seg);
+      for (const DiffClass *c = c0; c < c1; c++)
+        diff_est_kernel<<<warps(c, c->max_tiles), kDiffBlock, 0, stream>>>(
+            L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.est);
       // (one slice unless the group is one large template in its backward pass)
       for (uint32_t cg0 = 0; cg0 < g.max_cg; cg0 += g.cg_slice) {
         const uint32_t cgs = g.max_cg - cg0 < g.cg_slice ? g.max_cg - cg0 : g.cg_slice;
-        const dim3 hot(cgs, g.ny), stiles((g.slice_tiles + 3u) / 4u, g.ny);
-        const dim3 aseg((g.slice_aseg + 3u) / 4u, g.ny);
-        if (g.hot && ((e = cudaEventRecord(fork, stream)) != cudaSuccess ||
-                      (e = cudaStreamWaitEvent(side, fork, 0)) != cudaSuccess))
-          return e;
-        if (pass == 0) {
-          if (g.hot)
+        const dim3 hot(cgs, g.ny);
+        if (g.hot) {
+          if ((e = cudaEventRecord(fork, stream)) != cudaSuccess ||
+              (e = cudaStreamWaitEvent(side, fork, 0)) != cudaSuccess)
+            return e;
+          if (pass == 0)
             diff_hot_kernel<false><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
-                L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, nullptr, nullptr,
-                nullptr, nullptr, cg0, nullptr, nullptr, L.parts, smem_atoms);
-          diff_fwd_kernel<<<tiles, kDiffBlock, 0, stream>>>(
-              L.T, list, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.est, L.temp, L.parts);
-        } else {
-          if (g.hot)
+                L.T, L.exp_list + g.y0, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, nullptr,
+                nullptr, nullptr, nullptr, cg0, nullptr, nullptr, L.parts, smem_atoms);
+          else
             diff_hot_kernel<true><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
-                L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1, L.lnZ2, L.gB,
-                L.gS, cg0, L.scratch, L.grad_tau, nullptr, smem_atoms);
-          if (g.max_segs && cg0 == 0)  // (over the window sums, which nothing reads any more)
-            diff_seg_kernel<true><<<segs, kDiffBlock, 0, stream>>>(
-                L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
-                g.seg_per, L.seg);
-          diff_src_kernel<<<stiles, kDiffBlock, 0, stream>>>(
-              L.T, list, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB,
-              L.gS, cg0, cgs, L.scratch, L.grad_tau);
+                L.T, L.exp_list + g.y0, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1,
+                L.lnZ2, L.gB, L.gS, cg0, L.scratch, L.grad_tau, nullptr, smem_atoms);
+        }
+        if (pass == 0) {
+          for (const DiffClass *c = c0; c < c1; c++)
+            diff_fwd_kernel<<<warps(c, c->max_tiles), kDiffBlock, 0, stream>>>(
+                L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.est, L.temp,
+                L.parts);
+        } else {
+          for (const DiffClass *c = c0; c < c1; c++)
+            if (c->max_segs && cg0 == 0)  // (over the window sums, which nothing reads any more)
+              diff_seg_kernel<true><<<warps(c, c->max_segs), kDiffBlock, 0, stream>>>(
+                  L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1,
+                  L.lnZ2, L.gB, L.gS, g.seg_per, L.seg);
+          for (const DiffClass *c = c0; c < c1; c++)
+            diff_src_kernel<<<warps(c, c->slice_tiles), kDiffBlock, 0, stream>>>(
+                L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.temp, L.lnZ1,
+                L.lnZ2, L.gB, L.gS, cg0, cgs, L.scratch, L.grad_tau);
         }
         if (g.hot && ((e = cudaEventRecord(join, side)) != cudaSuccess ||
                       (e = cudaStreamWaitEvent(stream, join, 0)) != cudaSuccess))
           return e;
         if (pass == 1) {
-          diff_atoms_kernel<true><<<aseg, kDiffBlock, 0, stream>>>(
-              L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS, cg0,
-              cgs, L.scratch, L.cend, L.grad_atoms);
-          diff_atoms_kernel<false><<<aseg, kDiffBlock, 0, stream>>>(
-              L.T, list, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS, cg0,
-              cgs, L.scratch, L.cend, L.grad_atoms);
+          for (const DiffClass *c = c0; c < c1; c++)
+            diff_atoms_kernel<true><<<warps(c, c->slice_aseg), kDiffBlock, 0, stream>>>(
+                L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2,
+                L.gB, L.gS, cg0, cgs, L.scratch, L.cend, L.grad_atoms);
+          for (const DiffClass *c = c0; c < c1; c++)
+            diff_atoms_kernel<false><<<warps(c, c->slice_aseg), kDiffBlock, 0, stream>>>(
+                L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2,
+                L.gB, L.gS, cg0, cgs, L.scratch, L.cend, L.grad_atoms);
         }
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;

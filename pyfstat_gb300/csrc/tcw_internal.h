@@ -349,15 +349,22 @@ constexpr uint32_t kDiffSegFloatsV = 28u * 32u;
 struct DiffPartial {
   double m1, s1, m2, s2;
 };
+// Exponential templates [y0, y0 + ny) of exp_list (largest first) whose tiles
+// one launch takes, as a grid of the most that one of them has x ny.
+struct DiffClass {
+  uint32_t y0, ny;
+  // most tiles / segments / atoms / columns of one template
+  uint32_t max_tiles, max_segs, max_atoms, max_cols;
+  uint32_t slice_tiles, slice_aseg;  // most tiles / atom segments in a slice
+};
 // Exponential templates [y0, y0 + ny) of exp_list with workspaces of their
 // own: a backward pass runs in groups that bound the scratch, a group of one
-// large template in slices of cg_slice column groups.
+// large template in slices of cg_slice column groups.  Its launches go by
+// classes [c0, c0 + n_classes).
 struct DiffGroup {
-  uint32_t y0, ny;
-  // most column groups / tiles / segments / atoms of one template
-  uint32_t max_cg, max_tiles, max_segs, max_atoms;
-  // column groups of a slice, most tiles / atom segments of one template in it
-  uint32_t cg_slice, slice_tiles, slice_aseg;
+  uint32_t y0, ny, c0, n_classes;
+  uint32_t max_cg, max_atoms;  // most column groups / atoms of one template
+  uint32_t cg_slice;
   bool hot;  // some template's hot tiles are diff_hot_kernel's
   uint32_t seg_per;  // segments per warp
   uint64_t seg_floats, scr_floats, cend_floats;
@@ -368,7 +375,7 @@ struct DiffLaunch {
   float *atoms8;                     // exponential templates' atoms in 32-byte rows
                                      // (same row index as `atoms`), written by the launch
   const uint32_t *exp_list;          // the exponential templates' indices
-  uint32_t n_exp, max_cols;          // their number and the largest N_tau
+  uint32_t n_exp;                    // their number
   ColConsts *cols;                   // per exponential column, written by the launch
   float *seg;                        // segment sums
   float *need;                       // per exp tile: an upper bound of its F
@@ -392,7 +399,7 @@ struct DiffLaunch {
   double *B64, *D64;
 };
 cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, uint32_t n_groups,
-                        cudaStream_t stream, cudaStream_t side, cudaEvent_t fork,
+                        const DiffClass *classes, cudaStream_t stream, cudaStream_t side, cudaEvent_t fork,
                         cudaEvent_t join);
 // Failed device-side debug checks per translation unit (TCW_DEBUG_CHECKS).
 unsigned int dcheck_failures_kernels();

@@ -82,3 +82,22 @@ def test_few_rows_in_a_full_batch_match_torch_autograd():
         assert gt[k, 0] == pytest.approx(float(a.grad), rel=1.3e-5, abs=1e-15)
         if t["N_tau"] > 1:
             assert gt[k, 1] == pytest.approx(float(b.grad), rel=1.3e-5, abs=1e-15)
+
+
+def test_templates_of_unequal_size_match_those_alone():
+    """2000 small templates around one of 17532 atoms and 400 x 256 cells: launches
+    of their own for the large one, each template's result as by itself."""
+    pytest.importorskip("torch")
+    big = template(77, 17532, 400, 256, dt0=72000, gap=0.05)
+    small = [template(k, 90 + k, 30, 33) for k in range(4)]
+    tl = small * 300 + [big] + small * 200
+    lnB, soft, ga, gt = run(tl, 0.1)
+    first = np.cumsum([0] + [t["atoms"].shape[0] for t in tl])
+    for k in (0, 1, 2, 3, 1200, 1201, len(tl) - 1):
+        l1, s1, ga1, gt1 = run([tl[k]], 0.1)
+        assert lnB[k] == pytest.approx(l1[0], rel=1e-11)
+        assert soft[k] == pytest.approx(s1[0], rel=1e-11)
+        # other chunks and sums: F to 1e-13, 2F/T to 1e-9; FP32 weights 1.2e-5
+        np.testing.assert_allclose(ga[first[k]:first[k + 1]], ga1, rtol=1.3e-5,
+                                   atol=1e-9 * np.abs(ga1).max())
+        np.testing.assert_allclose(gt[k], gt1[0], rtol=1.3e-5, atol=1e-15)
