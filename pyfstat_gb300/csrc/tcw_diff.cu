@@ -583,17 +583,15 @@ struct FwdBounds {
 };
 
 // FP64 log-sum-exps of F and 2F/T over the cells of one lane, then over the
-// warp.
+// warp; cells below `skip` carry no weight.
 struct DiffLse {
-  double m1, s1, m2, s2, twoT, far;
-  float skip, skip0;
+  double m1, s1, m2, s2, twoT;
+  float skip;
   __device__ __forceinline__ DiffLse(double temp, float bound)
-      : m1(-INFINITY), s1(0.0), m2(-INFINITY), s2(0.0), twoT(2.0 / temp),
-        far(no_weight_below(temp)), skip(bound), skip0(bound) {}
+      : m1(-INFINITY), s1(0.0), m2(-INFINITY), s2(0.0), twoT(2.0 / temp), skip(bound) {}
   __device__ __forceinline__ void add(double F, double k = 1.0) {
     lse_add(m1, s1, F, k);
     lse_add(m2, s2, F * twoT, k);
-    skip = fmaxf((float)(m1 - far), skip0);
   }
   __device__ __forceinline__ void cell(bool data, const double W[7], bool t1, float F32) {
     if (!data) {
