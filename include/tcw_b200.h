@@ -199,8 +199,9 @@ int tcw_map_batched(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
                     int64_t *argmax, double *lnBtSG);
 /* One run without a graph and with the two map kernels one after the other,
  * CUDA events between the kernels on the handle's stream; synchronises and
- * writes the durations (ms) of the prefix, rectangular-map, exponential-map
- * and finalize kernels to ms[0..3].  For measurement. */
+ * writes the durations (ms) of the prefix (and repack), rectangular-map,
+ * exponential-map (with its segment sums) and finalize kernels to ms[0..3].
+ * For measurement. */
 int tcw_plan_run_timed(tcw_handle *h, tcw_plan *plan, const float *d_atoms, tcw_result *d_results,
                        float *ms);
 

@@ -409,7 +409,8 @@ class Plan:
                                        _p(d_maps), int(bool(use_graph))), self.handle.ptr)
 
     def run_timed(self, d_atoms, d_results):
-        """One run with per-kernel CUDA events: (prefix, rect map, exp map, finalize) ms."""
+        """One run with per-kernel CUDA events: (prefix, rect map, exp map with its
+        segment sums, finalize) ms."""
         ms = (ctypes.c_float * 4)()
         check(load().tcw_plan_run_timed(self.handle.ptr, self._p, _p(d_atoms), _p(d_results), ms),
               self.handle.ptr)

@@ -3,7 +3,9 @@
 The two map kernels of a plan are tuned independently (the timed run
 launches them one after the other): the rectangular kernel over
 (rows per tile, columns per tile) and the exponential kernel over (columns
-per block, rows per thread chunk).  Timing uses ``tcw_plan_run_timed`` (CUDA
+per block, rows per thread chunk), the library's own choice (0) among them.
+The exponential time includes the segment sums from which the library starts
+the row chunks that it cuts itself.  Timing uses ``tcw_plan_run_timed`` (CUDA
 events between the kernels) on a seeded sample of the batch's templates of
 about ``budget_cells`` cells per window type, best of ``repeats`` runs.  The
 default budget (4e9 cells, some 15 ms of kernel time per window type) takes
@@ -13,8 +15,9 @@ on a small sample far more than on the full batch (a 4e8-cell sample of the
 short row chunks look better than they are (19.5 ms with whole columns
 against 21.3 ms with 1024-row chunks on the full batch).
 
-Choices are cached per device name and workload signature (window mix and
-log2-bucketed mean grid sizes and atom counts) in a JSON file:
+Choices are cached per device name, version of the library's tile rules and
+workload signature (window mix and log2-bucketed mean grid sizes and atom
+counts) in a JSON file:
 ``$PYFSTAT_GB300_TUNE_CACHE`` or ``~/.cache/pyfstat_gb300/tiles.json``.
 """
 
@@ -25,7 +28,13 @@ import numpy as np
 
 from . import _lib
 
-RECT_CANDIDATES = [(tm, tn) for tm in (32, 64, 128) for tn in (32, 64, 128, 256)]
+# Version of what the library does with tile sizes that are 0 and with given
+# ones: a choice that was measured under other rules is measured again.
+# 2: small plans take small rectangular tiles, exponential columns are cut into
+# row chunks that start from segment sums.
+TILE_RULES = 2
+
+RECT_CANDIDATES = [(0, 0)] + [(tm, tn) for tm in (32, 64, 128) for tn in (32, 64, 128, 256)]
 # batched plans run exponential tiles as 32-column warp tiles: only the rows
 # per tile (0 = whole columns) are tuned
 EXP_CANDIDATES = [(32, rows) for rows in (0, 64, 256, 1024)]
@@ -52,6 +61,10 @@ def signature(desc):
         nb = int(np.round(np.log2(sel.shape[0])))
         parts.append(f"w{w}:{nb}:{b[0]}:{b[1]}:{b[2]}")
     return "|".join(parts)
+
+
+def cache_key(device_name, flags, desc):
+    return f"{device_name}|rules{TILE_RULES}|flags{int(flags)}|{signature(desc)}"
 
 
 def _load_cache(path):
@@ -129,7 +142,7 @@ def tune(desc, t0s, taus, atoms, handle, flags=_lib.TCW_FLAG_LNBTSG, budget_cell
 
     desc = np.ascontiguousarray(desc, dtype=_lib.DESC_DTYPE)
     name = _lib.device_info(handle.device)["name"]
-    key = f"{name}|flags{int(flags)}|{signature(desc)}"
+    key = cache_key(name, flags, desc)
     path = cache_path()
     if use_cache:
         hit = _load_cache(path).get(key)

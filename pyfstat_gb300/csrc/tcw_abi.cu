@@ -1211,12 +1211,12 @@ int tcw_plan_run_timed(tcw_handle *h, tcw_plan *p, const float *d_atoms, tcw_res
                             h->stream));
   TCW_CUDA(h, launch_repack(p->d_T, p->d_exp_list, p->n_exp, p->max_exp_atoms, d_atoms, p->d_A8,
                             h->stream));
-  TCW_CUDA(h, launch_exp_segments(p->d_T, p->d_segs, p->n_segs, 0, p->d_A8, p->d_taus, p->d_G,
-                                  h->stream));
   TCW_CUDA(h, cudaEventRecord(ev[1], h->stream));
   TCW_CUDA(h, launch_map(TCW_WINDOW_RECT, plan_launch(h, p, TCW_WINDOW_RECT, d_atoms, nullptr),
                          h->stream));
   TCW_CUDA(h, cudaEventRecord(ev[2], h->stream));
+  TCW_CUDA(h, launch_exp_segments(p->d_T, p->d_segs, p->n_segs, 0, p->d_A8, p->d_taus, p->d_G,
+                                  h->stream));
   TCW_CUDA(h, launch_map(TCW_WINDOW_EXP, plan_launch(h, p, TCW_WINDOW_EXP, d_atoms, nullptr),
                          h->stream));
   TCW_CUDA(h, cudaEventRecord(ev[3], h->stream));
