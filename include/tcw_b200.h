@@ -88,9 +88,9 @@ typedef struct {
 /* Tile shapes of a batched plan (0 = library default / autotuned). */
 typedef struct {
   uint32_t rect_tn;       /* columns per rect tile (any >= 1) */
-  uint32_t rect_tm;       /* rows per rect tile: 32, 64 or 128 (one thread per row) */
-  uint32_t exp_tn;        /* columns per exp block: 32, 64 or 128 (single-template
-                             calls; batched plans run 32-column warp tiles) */
+  uint32_t rect_tm;       /* rows per rect tile: 32, 64 or 128 (one thread per row);
+                             with both 0, small plans take 32 rows x 32..128 columns */
+  uint32_t exp_tn;        /* accepted and ignored: exp tiles are 32 columns, one warp */
   uint32_t exp_rows;      /* rows per exp thread chunk (0: whole columns, or the chunks
                              that the library starts from segment sums) */
   uint32_t blocks_per_sm; /* cap on persistent blocks per SM (occupancy limits it too) */
@@ -155,6 +155,7 @@ int tcw_plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_tem
                     const uint32_t *t0s, uint64_t n_t0s, const uint32_t *taus, uint64_t n_taus,
                     const tcw_tile_config *cfg, int flags, tcw_plan **plan);
 int tcw_plan_destroy(tcw_plan *plan);
+/* Cells, tiles and atom rows of a plan, and the tile shapes in use. */
 int tcw_plan_info(const tcw_plan *plan, uint64_t *n_cells, uint32_t *n_items,
                   uint64_t *n_atom_rows, tcw_tile_config *cfg);
 /* use_graph != 0: the first run captures the launch sequence into a CUDA

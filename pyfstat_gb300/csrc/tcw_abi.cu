@@ -309,7 +309,7 @@ uint32_t exp_hist(uint32_t exp_rows, uint32_t N_t0) {
 void fill_cfg_defaults(tcw_tile_config &c) {
   if (c.rect_tm != 32 && c.rect_tm != 64 && c.rect_tm != 128) c.rect_tm = 128;
   if (c.rect_tn == 0) c.rect_tn = 128;
-  if (c.exp_tn != 32 && c.exp_tn != 64 && c.exp_tn != 128) c.exp_tn = 128;
+  c.exp_tn = 32;  // exp tiles are 32 columns (tile_template)
   if (c.blocks_per_sm == 0) c.blocks_per_sm = 32;  // cap; occupancy decides below it
 }
 
@@ -772,7 +772,6 @@ static int plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_
   tcw_tile_config cfg{};
   if (cfg_in) cfg = *cfg_in;
   fill_cfg_defaults(cfg);
-  cfg.exp_tn = 32;  // plans run 32-column warp tiles (tile_template)
 
   tcw_plan *p = new (std::nothrow) tcw_plan();
   if (!p) return TCW_ERR_ALLOC;
@@ -780,7 +779,6 @@ static int plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_
   p->prec = prec_of(flags);
   p->flags = flags;
   p->n_templates = n_templates;
-  p->cfg = cfg;
   std::vector<uint2> post_chunks;
   uint64_t post_row_sums = 0, post_col_sums = 0;
   std::vector<TemplateDev> T(n_templates);
@@ -830,6 +828,7 @@ static int plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_
           (uint32_t)std::max<uint64_t>(32, std::min<uint64_t>(128, per / 32u / 32u * 32u));
     }
   }
+  p->cfg = rcfg;
   std::vector<SegItem> segs;
   {
     uint64_t all = 0;

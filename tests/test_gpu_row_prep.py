@@ -45,3 +45,23 @@ def test_windows_in_gaps_longer_than_a_repack_block(oracle, zeros):
     rel, _ = rel_err(F, F64, cond)
     assert rel.max() <= REL_TOL
     h.close()
+
+
+@pytest.mark.parametrize("n", [1, 3, 400])
+@pytest.mark.parametrize("cfg", [None, dict(rect_tm=64, rect_tn=48)])
+def test_plan_info_reports_the_rect_tiles_in_use(n, cfg):
+    """Small plans take small rectangular tiles: the reported shape gives the
+    reported number of tiles."""
+    from pyfstat_gb300.batched import TransientMapBatch
+
+    t0_data, A = synth.merged_atoms(3, 300, 1)
+    t = dict(window=1, atoms=A, TAtom=1800, t0_data=t0_data,
+             t0s=(t0_data + 1800 * np.arange(290)).astype(np.uint32),
+             taus=(1800 + 1800 * np.arange(270)).astype(np.uint32))
+    batch = TransientMapBatch([t] * n, tile_config=cfg)
+    c = batch.tile_config
+    assert batch.plan.n_items == n * -(-290 // c["rect_tm"]) * -(-270 // c["rect_tn"]), c
+    assert c["exp_tn"] == 32
+    if cfg:
+        assert (c["rect_tm"], c["rect_tn"]) == (64, 48)
+    batch.close()
