@@ -569,11 +569,14 @@ __device__ __forceinline__ double no_weight_below(double temp) {
 // From the key of a template's estimated maximum: cells below `skip` carry no
 // weight in either sum, tiles that reach `hot` may hold a cell whose last bits
 // show (lnBtSG: e^-8 of the largest; the soft-max multiplies them by 2/T,
-// where this is large its weights fall as much faster).
+// where this is large its weights fall as much faster).  Without an estimate
+// (key 0: no cell surely passes the conditioning test, F is 2 almost
+// everywhere) nothing is skipped and only NaN tiles are hot.
 struct FwdBounds {
   float skip, hot;
   __device__ __forceinline__ FwdBounds(uint32_t key, double temp) {
-    skip = hot = -INFINITY;
+    skip = -INFINITY;
+    hot = INFINITY;
     if (key) {
       const double top = (double)key_float(key);
       skip = (float)(top - 1e-5 * fabs(top) - no_weight_below(temp) - 1.0);
@@ -681,12 +684,13 @@ __global__ void __launch_bounds__(kDiffBlock, 5)
 // tier-1 F (good to ~1e-5 of F) lies more than 42 below Z1 (the lnBtSG term,
 // gB != 0) and more than 40 T + 1 below (T/2) Z2 (the soft-max term, gS != 0:
 // its exponent is then below -80).
-// `hot`: above it a single cell may carry more than e^-6 of either gradient.
+// `hot`: above it a single cell may carry more than e^-6 of either gradient
+// (without an estimate, key 0, only NaN tiles are, as in the forward).
 struct DiffWeights {
   double z1, z2, gb, gs;
   float skip, hot;
-  __device__ __forceinline__ DiffWeights(const DiffTemplate &t, uint32_t k, double temp,
-                                         const double *lnZ1, const double *lnZ2,
+  __device__ __forceinline__ DiffWeights(const DiffTemplate &t, uint32_t k, uint32_t key,
+                                         double temp, const double *lnZ1, const double *lnZ2,
                                          const double *gB, const double *gS) {
     z1 = lnZ1[k] - log(70.0 / ((double)t.N_t0 * (double)t.N_tau));
     z2 = lnZ2[k] / temp;
@@ -697,6 +701,7 @@ struct DiffWeights {
     skip = (float)fmin(sk1, sk2);
     hot = (float)fmin(gb != 0.0 ? z1 - 1e-5 * fabs(z1) - 7.0 : INFINITY,
                       gs != 0.0 ? 0.5 * temp * (z2 - 1e-5 * fabs(z2) - 25.0) - 0.1 : INFINITY);
+    if (!key) hot = INFINITY;
   }
 };
 
@@ -707,9 +712,10 @@ __global__ void __launch_bounds__(kDiffBlock)
     diff_seg_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
                     const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
                     const ColConsts *__restrict__ cols, const float *__restrict__ need,
-                    double temp, const double *__restrict__ lnZ1,
-                    const double *__restrict__ lnZ2, const double *__restrict__ gB,
-                    const double *__restrict__ gS, uint32_t per, float *__restrict__ seg) {
+                    const uint32_t *__restrict__ est, double temp,
+                    const double *__restrict__ lnZ1, const double *__restrict__ lnZ2,
+                    const double *__restrict__ gB, const double *__restrict__ gS, uint32_t per,
+                    float *__restrict__ seg) {
   DiffLane L;
   const uint32_t k = list[blockIdx.y];
   L.t = T[k];
@@ -717,7 +723,7 @@ __global__ void __launch_bounds__(kDiffBlock)
   const uint32_t cg = w % L.t.n_cg, j0 = w / L.t.n_cg * per;
   if (j0 >= L.t.g_nseg) return;
   if (kV) {
-    const DiffWeights w(L.t, k, temp, lnZ1, lnZ2, gB, gS);
+    const DiffWeights w(L.t, k, est[k], temp, lnZ1, lnZ2, gB, gS);
     const float *nd = need + L.t.part_off + (size_t)cg * L.t.n_chunk;
     bool any = false;
     for (uint32_t c = threadIdx.x & 31u; c < L.t.n_chunk; c += 32u)
@@ -845,10 +851,10 @@ __global__ void __launch_bounds__(kDiffBlock)
     diff_src_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
                     const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
                     const ColConsts *__restrict__ cols, const float *__restrict__ seg,
-                    const float *__restrict__ need, double temp, const double *__restrict__ lnZ1,
-                    const double *__restrict__ lnZ2, const double *__restrict__ gB,
-                    const double *__restrict__ gS, uint32_t cg0, uint32_t cgs,
-                    float *__restrict__ scratch, double *__restrict__ grad_tau) {
+                    const float *__restrict__ need, const uint32_t *__restrict__ est, double temp,
+                    const double *__restrict__ lnZ1, const double *__restrict__ lnZ2,
+                    const double *__restrict__ gB, const double *__restrict__ gS, uint32_t cg0,
+                    uint32_t cgs, float *__restrict__ scratch, double *__restrict__ grad_tau) {
   __shared__ __align__(16) ExpRow s_tab[kDiffBlock / 32][kDiffRowTab];
   DiffLane L;
   const uint32_t k = list[blockIdx.y];
@@ -859,7 +865,7 @@ __global__ void __launch_bounds__(kDiffBlock)
   const uint32_t scg = stile / t.n_chunk, cg = cg0 + scg, tile = cg0 * t.n_chunk + stile;
   const uint32_t mb = stile % t.n_chunk * t.chunk_rows;
   if (scg >= cgs || cg >= t.n_cg) return;
-  const DiffWeights w(t, k, temp, lnZ1, lnZ2, gB, gS);
+  const DiffWeights w(t, k, est[k], temp, lnZ1, lnZ2, gB, gS);
   const float nd = need[t.part_off + tile];
   if (nd < w.skip) return;    // diff_atoms_kernel skips its rows
   if (!(nd < w.hot) && !t.whole) return;  // diff_hot_kernel
@@ -968,7 +974,7 @@ __global__ void __launch_bounds__(kHotThreads, 1)
   float hot, skip;
   DiffGrad grad;
   if (kBack) {
-    const DiffWeights w(t, k, temp, lnZ1, lnZ2, gB, gS);
+    const DiffWeights w(t, k, est[k], temp, lnZ1, lnZ2, gB, gS);
     hot = w.hot;
     skip = w.skip;
     grad = DiffGrad(w, temp);
@@ -1244,10 +1250,10 @@ __global__ void __launch_bounds__(kDiffBlock)
     diff_atoms_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
                       const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
                       const ColConsts *__restrict__ cols, const float *__restrict__ need,
-                      double temp, const double *__restrict__ lnZ1,
-                      const double *__restrict__ lnZ2, const double *__restrict__ gB,
-                      const double *__restrict__ gS, uint32_t cg0, uint32_t cgs,
-                      const float *__restrict__ scratch, float *__restrict__ cend,
+                      const uint32_t *__restrict__ est, double temp,
+                      const double *__restrict__ lnZ1, const double *__restrict__ lnZ2,
+                      const double *__restrict__ gB, const double *__restrict__ gS, uint32_t cg0,
+                      uint32_t cgs, const float *__restrict__ scratch, float *__restrict__ cend,
                       double *__restrict__ grad_atoms) {
   DiffLane L;
   const uint32_t k = list[blockIdx.y];
@@ -1259,7 +1265,7 @@ __global__ void __launch_bounds__(kDiffBlock)
   // the group's weighted chunks: first and last
   uint32_t c0 = 0xFFFFFFFFu, c1 = 0;
   {
-    const DiffWeights w(t, k, temp, lnZ1, lnZ2, gB, gS);
+    const DiffWeights w(t, k, est[k], temp, lnZ1, lnZ2, gB, gS);
     const float *nd = need + t.part_off + (size_t)cg * t.n_chunk;
     for (uint32_t c = lane; c < t.n_chunk; c += 32u)
       if (!(nd[c] < w.skip)) {
@@ -1814,8 +1820,8 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
       for (const DiffClass *c = c0; c < c1; c++)
         if (c->max_segs)
           diff_seg_kernel<false><<<warps(c, c->max_segs), kDiffBlock, 0, stream>>>(
-              L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, nullptr, L.temp, nullptr, nullptr,
-              nullptr, nullptr, g.seg_per, L.seg);
+              L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, nullptr, nullptr, L.temp, nullptr,
+              nullptr, nullptr, nullptr, g.seg_per, L.seg);
       for (const DiffClass *c = c0; c < c1; c++)
         diff_est_kernel<<<warps(c, c->max_tiles), kDiffBlock, 0, stream>>>(
             L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.est);
@@ -1845,12 +1851,12 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
           for (const DiffClass *c = c0; c < c1; c++)
             if (c->max_segs && cg0 == 0)  // (over the window sums, which nothing reads any more)
               diff_seg_kernel<true><<<warps(c, c->max_segs), kDiffBlock, 0, stream>>>(
-                  L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1,
+                  L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1,
                   L.lnZ2, L.gB, L.gS, g.seg_per, L.seg);
           for (const DiffClass *c = c0; c < c1; c++)
             diff_src_kernel<<<warps(c, c->slice_tiles), kDiffBlock, 0, stream>>>(
-                L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.temp, L.lnZ1,
-                L.lnZ2, L.gB, L.gS, cg0, cgs, L.scratch, L.grad_tau);
+                L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.est, L.temp,
+                L.lnZ1, L.lnZ2, L.gB, L.gS, cg0, cgs, L.scratch, L.grad_tau);
         }
         if (g.hot && ((e = cudaEventRecord(join, side)) != cudaSuccess ||
                       (e = cudaStreamWaitEvent(stream, join, 0)) != cudaSuccess))
@@ -1858,12 +1864,12 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
         if (pass == 1) {
           for (const DiffClass *c = c0; c < c1; c++)
             diff_atoms_kernel<true><<<warps(c, c->slice_aseg), kDiffBlock, 0, stream>>>(
-                L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2,
-                L.gB, L.gS, cg0, cgs, L.scratch, L.cend, L.grad_atoms);
+                L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1,
+                L.lnZ2, L.gB, L.gS, cg0, cgs, L.scratch, L.cend, L.grad_atoms);
           for (const DiffClass *c = c0; c < c1; c++)
             diff_atoms_kernel<false><<<warps(c, c->slice_aseg), kDiffBlock, 0, stream>>>(
-                L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.need, L.temp, L.lnZ1, L.lnZ2,
-                L.gB, L.gS, cg0, cgs, L.scratch, L.cend, L.grad_atoms);
+                L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1,
+                L.lnZ2, L.gB, L.gS, cg0, cgs, L.scratch, L.cend, L.grad_atoms);
         }
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;

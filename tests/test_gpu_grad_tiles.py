@@ -65,3 +65,47 @@ def test_tiles_match_torch_autograd(case, weights):
             assert float(tmax.grad[k]) == pytest.approx(float(b.grad), rel=1e-5, abs=1e-15)
         assert float(tmin.grad[k]) == pytest.approx(float(a.grad), rel=1e-5, abs=1e-15)
         row += n
+
+
+@pytest.mark.parametrize("kind", ["one antenna pattern", "zero atoms"])
+def test_templates_whose_cells_all_fail_the_conditioning_test(kind):
+    """F = 2 in every cell (no lower bound of the maximum to sort tiles by):
+    the closed forms of both statistics, no gradient, and the template beside
+    them as by itself."""
+    torch = pytest.importorskip("torch")
+    from pyfstat_gb300.autograd import DiffBatch
+
+    def template(k, nsft, n_t0, n_tau, flat):
+        t0_data, A = synth.merged_atoms(40 + k, nsft, 2, amp=3.0)
+        if flat:
+            A = np.zeros_like(A) if kind == "zero atoms" else A * np.float32([1, 0, 0, 1, 1, 0, 0])
+        return dict(atoms=A, TAtom=1800, t0_data=t0_data, N_tau=n_tau, tau_min=9075.0,
+                    tau_max=9075.0 + 900.0 * (n_tau - 1),
+                    t0s=(t0_data + 450 + 3600 * np.arange(n_t0)).astype(np.uint32))
+
+    tl = [template(0, 200, 90, 70, True), template(1, 120, 17, 33, False),
+          template(2, 65, 16, 1, True), template(3, 30, 1, 40, True)]
+
+    def run(tl):
+        b = DiffBatch(tl)
+        atoms = torch.from_numpy(b.atoms).cuda()
+        lim = [np.array([t[k] for t in tl]) for k in ("tau_min", "tau_max")]
+        lnB, soft = b.forward_raw(atoms, *lim)
+        g = torch.ones_like(lnB)
+        out = [x.cpu().numpy() for x in (lnB, soft, *b.backward_raw(atoms, *lim, lnB, soft, g, g))]
+        b.handle.close()
+        return out
+
+    lnB, soft, ga, gt = run(tl)
+    first = np.cumsum([0] + [t["atoms"].shape[0] for t in tl])
+    for k in (0, 2, 3):
+        n = len(tl[k]["t0s"]) * tl[k]["N_tau"]
+        assert lnB[k] == pytest.approx(np.log(70.0) + 2.0, rel=1e-12)
+        assert soft[k] == pytest.approx(4.0 + 0.1 * np.log(n), rel=1e-12)
+        assert not ga[first[k]:first[k + 1]].any() and not gt[k].any()
+    one = run([tl[1]])
+    assert lnB[1] == pytest.approx(one[0][0], rel=1e-11)
+    assert soft[1] == pytest.approx(one[1][0], rel=1e-11)
+    # FP32 weights, exponents down to -80
+    np.testing.assert_allclose(ga[first[1]:first[2]], one[2], rtol=1.3e-5,
+                               atol=1e-9 * np.abs(one[2]).max())
