@@ -221,10 +221,20 @@ constexpr double kExpRowSteps = 3.0, kExpShortRowSteps = 10.0;
 
 // The columns of one 32-column group, whose first duration is tau.
 struct ExpGroupSteps {
-  double atoms, window, per_row, row;
+  double atoms, window, per_row, row, t_atom;
   ExpGroupSteps(double n_atoms, uint32_t TAtom, uint32_t N_t0, uint32_t tau)
       : atoms(n_atoms), window(3.0 * tau / TAtom), per_row(n_atoms / N_t0),
-        row(window < kShortWindow ? kExpShortRowSteps : kExpRowSteps) {}
+        row(window < kShortWindow ? kExpShortRowSteps : kExpRowSteps), t_atom(TAtom) {}
+  // Most steps of a chunk's first window.
+  double start(const ExpSplit &sp) const {
+    return std::min(window, 2.0 * ((1u << sp.shift) + (double)sp.nseg));
+  }
+  // Atoms of a chunk's run-up (kRunUp); last_tau: the group's longest duration.
+  double run_up_atoms(uint32_t last_tau) const {
+    return window < kShortWindow
+               ? std::min(atoms, kRunUp * std::min(last_tau / t_atom, kShortWindow / 3.0))
+               : 0.0;
+  }
   // Steps of `rows` rows from row m0 on (starts spread over the data): the
   // atoms that enter, those that leave while the window ends before the data
   // do, and the rows.
@@ -263,11 +273,9 @@ void tile_template(uint32_t tmpl, const TemplateDev &t, const tcw_tile_config &c
       const ExpGroupSteps steps(atoms, t.g.TAtom, N_t0, taus[n0]);
       double start = 0.0;  // most steps of a chunk's first window
       if (t.g_nseg) {
-        start = std::min(steps.window, 2.0 * ((1u << t.g_shift) + (double)t.g_nseg));
+        start = steps.start(ExpSplit{t.e_hist, t.e_rows, t.e_sub, t.g_shift, t.g_nseg});
         const double n = steps.rows(0, N_t0) / chunk_steps;
-        const double tau = taus[std::min(N_tau, n0 + 32u) - 1u] / (double)t.g.TAtom;
-        if (3.0 * taus[n0] < (double)kShortWindow * t.g.TAtom)
-          run_up = kRunUp * std::min(tau, kShortWindow / 3.0) * N_t0 / atoms;
+        run_up = steps.run_up_atoms(taus[std::min(N_tau, n0 + 32u) - 1u]) / steps.per_row;
         rows = std::min(rows, (uint32_t)std::max(8.0, ceil(N_t0 / std::max(1.0, ceil(n)))));
       }
       for (uint32_t h0 = 0; h0 < N_t0; h0 += t.e_hist)
@@ -787,30 +795,49 @@ static int plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_
   std::vector<uint32_t> rect_list, exp_list;
   uint64_t p_rows = 0, a8_rows = 0, atom_rows = 0, cells = 0;
   // Row chunks of exp columns when the caller leaves them to the library
-  // (exp_rows 0): whole columns where these give TCW_PLAN_EXP_WARPS warps per
-  // scheduler a tile and a third more (a lone warp is bound by its own latency,
-  // eight share the issue slots, and one wave of whole columns lasts as long
-  // as its longest), else cut into chunks of equal steps that bring the warp
-  // tiles there, started from segment sums.  Whole / cut, per run: 96 templates
-  // with maps and posteriors 3.55 / 1.55 ms, 24 templates 0.67 / 0.18, 298 of
-  // up to 2985 atoms and 1292 x 1292 cells (3300 column tiles) 2.33 / 1.44, 840
-  // of up to 2500 and 700 x 700 (5200) 1.90 / 1.70, 330 of up to 3500 and 2000
-  // x 2000 (5900) 3.05 / 2.99; 678 of up to 1132 and 1322 x 1322 (7900) 1.62 /
-  // 1.85.  6 or 12 warps are no faster (96 templates 1.66 and 1.64 ms).
+  // (exp_rows 0).  A lone warp is bound by its own latency, eight share a
+  // scheduler's issue slots, and one wave of whole columns lasts as long as its
+  // longest: plans with fewer column tiles than `limit` times `want` (eight
+  // warps per scheduler) are cut into chunks of equal steps that bring the warp
+  // tiles there, started from segment sums.  Equal columns are cut up to about
+  // `want` tiles, columns of unequal length up to 1.3 of it (`most`); a start
+  // and its run-up cost up to two and a half times their steps (they run beside
+  // fewer warps, behind the segment sums), less where rect tiles keep the SMs
+  // busy meanwhile.  Per run, cut / whole: 96 templates with maps and posteriors
+  // 1.55 / 3.55 ms, 24 templates 0.18 / 0.67; exp templates of up to 2500 atoms
+  // and 700 x 700 cells at 0.6, 0.95 and 1.3 `want` 1.01 / 1.40, 1.48 / 1.73,
+  // 1.90 / 1.77; 500 atoms, 60 x 60 cells at 0.25, 0.8, 1.0 0.34 / 0.41, 0.65 /
+  // 0.63, 0.77 / 0.64; 100 atoms, 20 x 20 at 0.1, 0.8 0.116 / 0.073, 0.220 /
+  // 0.154; of each pair the rule takes the smaller (to within 5 % but for a few
+  // sizes at its line).  6 or 12 warps are no faster (96 templates 1.66 and
+  // 1.64 ms).
   uint64_t seg_blocks = 0;
   double chunk_steps = 0.0;  // 0: whole columns
   if (cut && cfg.exp_rows == 0 && p->prec != kPrecPlain32) {
-    uint64_t tiles = 0;
-    double steps = 0.0;
+    double tiles = 0.0, steps = 0.0, most = 0.0, starts = 0.0;
+    bool rect = false;
     for (uint32_t k = 0; k < n_templates; k++) {
       const tcw_template_desc &d = desc[k];
-      if (d.window != TCW_WINDOW_EXP || d.tau_offset + d.N_tau > n_taus) continue;
-      tiles += ((uint64_t)d.N_tau + 31u) / 32u;
-      for (uint32_t n0 = 0; n0 < d.N_tau; n0 += 32u)
-        steps += ExpGroupSteps(d.numAtoms, d.TAtom, d.N_t0, taus[d.tau_offset + n0]).rows(0, d.N_t0);
+      rect = rect || d.window == TCW_WINDOW_RECT;
+      if (d.window != TCW_WINDOW_EXP || d.tau_offset + d.N_tau > n_taus || d.numAtoms == 0 ||
+          d.N_t0 == 0)
+        continue;
+      const ExpSplit sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, d.N_t0, 2);
+      for (uint32_t n0 = 0; n0 < d.N_tau; n0 += 32u) {
+        const uint32_t *tau = taus + d.tau_offset;
+        const ExpGroupSteps g(d.numAtoms, d.TAtom, d.N_t0, tau[n0]);
+        const double s = g.rows(0, d.N_t0);
+        tiles += 1.0;
+        steps += s;
+        most = std::max(most, s);
+        starts += g.start(sp) + 3.0 * g.run_up_atoms(tau[std::min(d.N_tau, n0 + 32u) - 1u]);
+      }
     }
-    const uint64_t want = (uint64_t)h->n_sms * 4u * TCW_PLAN_EXP_WARPS;
-    if (tiles && 3u * tiles <= 4u * want) chunk_steps = steps / (double)want;
+    const double want = (double)h->n_sms * 4.0 * TCW_PLAN_EXP_WARPS;
+    const double limit =
+        std::min(1.3, 0.75 + 0.3 * most * tiles / steps) *
+        (1.0 - (rect ? 1.5 * starts : 2.5 * starts + 100.0 * tiles) / steps);
+    if (tiles > 0.0 && tiles <= limit * want) chunk_steps = steps / want;
   }
   // Rect tiles when the caller leaves them to the library: 128 x 128 while
   // these give every scheduler TCW_PLAN_RECT_WARPS warps' worth of tiles, else
