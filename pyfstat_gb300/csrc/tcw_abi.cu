@@ -651,7 +651,8 @@ static int plain_enqueue(tcw_handle *h, const PlainLayout &L, const float *d_ato
   TCW_CUDA(h, launch_finalize(dT, 1, dparts, d_result, true, h->stream));
   if (flags & TCW_FLAG_POSTERIORS) {
     PostPart *pp = reinterpret_cast<PostPart *>(ws + L.o_pp);
-    const PostLayout pl{L.post_rows, 1024u, L.post_chunks, nullptr,
+    const PostLayout pl{L.post_rows, 1024u, L.post_chunks, post_parts(L.t.N_t0, L.t.N_tau),
+                        nullptr,
                         reinterpret_cast<double *>(ws + L.o_row),
                         reinterpret_cast<double *>(ws + L.o_col), pp,
                         reinterpret_cast<uint32_t *>(pp + 2u * kPostParts)};
@@ -860,8 +861,18 @@ static int plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_
   {
     uint64_t all = 0;
     for (uint32_t k = 0; k < n_templates; k++) all += (uint64_t)desc[k].N_t0 * desc[k].N_tau;
-    p->post.rows = post_rows(all, h->n_sms);
+    // post_rows, but no more blocks than 12 per SM where small maps give them
+    // (2000 maps of 20 x 20 cells: 2 blocks of 16 rows each 54 us, one block each
+    // 30; a block for both directions of a template's argmax 18 -> 14)
+    const uint32_t least = post_rows(all, h->n_sms);
     p->post.cols = 1024u;
+    for (p->post.rows = 256u; p->post.rows > least; p->post.rows >>= 1) {
+      uint64_t blocks = 0;
+      for (uint32_t k = 0; k < n_templates; k++)
+        blocks += ((uint64_t)desc[k].N_t0 + p->post.rows - 1u) / p->post.rows *
+                  (((uint64_t)desc[k].N_tau + 1023u) / 1024u);
+      if (blocks >= (uint64_t)h->n_sms * 12u) break;
+    }
   }
   try {
     for (uint32_t k = 0; k < n_templates; k++) {
@@ -895,6 +906,7 @@ static int plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_
       if (flags & TCW_FLAG_POSTERIORS) {
         const uint32_t n_cc = (d.N_tau + 1023u) / 1024u;
         const uint32_t n_rc = (d.N_t0 + p->post.rows - 1u) / p->post.rows;
+        p->post.argmax_blocks = std::max(p->post.argmax_blocks, post_parts(d.N_t0, d.N_tau));
         post_row_sums += (uint64_t)d.N_t0 * n_cc;
         post_col_sums += (uint64_t)d.N_tau * n_rc;
         for (uint32_t c = 0; c < n_cc * n_rc; c++) post_chunks.push_back(make_uint2(k, c));
@@ -932,6 +944,8 @@ static int plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_
       for (size_t i = first; i < items.size(); i++) items[i].part = (uint32_t)i;
       T[k] = t;
     }
+    p->post.argmax_blocks = std::min(p->post.argmax_blocks,
+                                     std::max(1u, (uint32_t)h->n_sms * 12u / n_templates));
     const uint32_t per = segs_per_warp(seg_blocks, h->n_sms);
     size_t n_segs = 0;
     for (uint32_t k : exp_list)

@@ -291,6 +291,7 @@ struct PostPart {
 };
 struct PostLayout {
   uint32_t rows, cols, n_chunks;
+  uint32_t argmax_blocks;  // blocks per template, up to the most parts of one (post_parts)
   const uint2 *chunks;  // (template, chunk); NULL: template 0's chunks
   double *rowsum, *colsum;
   PostPart *parts;      // 2 kPostParts per template
@@ -302,6 +303,11 @@ __host__ __device__
 inline uint32_t post_part_entries(uint32_t n) {
   const uint32_t e = (n + kPostParts - 1u) / kPostParts;
   return e < 256u ? 256u : e;
+}
+// Parts of one template: those of its rows, then those of its columns.
+inline uint32_t post_parts(uint32_t N_t0, uint32_t N_tau) {
+  const uint32_t r = post_part_entries(N_t0), c = post_part_entries(N_tau);
+  return (uint32_t)(((uint64_t)N_t0 + r - 1u) / r + ((uint64_t)N_tau + c - 1u) / c);
 }
 // Rows per block for maps of `cells` cells in all: 256, fewer where that
 // leaves fewer than 8 blocks per SM, 16 at least.

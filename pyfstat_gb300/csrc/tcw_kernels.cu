@@ -1218,7 +1218,10 @@ cudaError_t launch_finalize(const TemplateDev *d_T, uint32_t n_templates, const 
 // post_argmax_kernel: per template up to kPostParts blocks each for rows and
 // columns add the chunks' sums in FP64 and leave their first maximum; the
 // template's last block picks among them in index order (same maps: 68 ->
-// 33 us with one warp per template before).
+// 33 us with one warp per template before).  The grid is that of the template
+// with most parts, fewer blocks (down to one) where there are thousands of
+// templates: with 64 for each a run of 2000 templates of 20 x 20 cells took 255
+// us for 113.
 constexpr uint32_t kPostThreads = 256;
 constexpr uint32_t kPostCols = 1024;
 constexpr uint32_t kPostMaxRows = 256;
@@ -1249,7 +1252,8 @@ __global__ void __launch_bounds__(kPostThreads) post_sums_kernel(
   auto load = [](const float *p) { return kChained ? *p : __ldg(p); };
   for (uint32_t k = lane; k < m1 - m0; k += 32u) srow[wid][k] = make_float2(0.0f, 0.0f);
   __syncwarp();
-  for (uint32_t n0 = nb + tid; n0 - tid < ne; n0 += kPostCols) {
+  // (warps behind the last column leave their zeros)
+  for (uint32_t n0 = nb + tid; n0 - lane < ne; n0 += kPostCols) {
     float cs[4] = {0, 0, 0, 0}, cc4[4] = {0, 0, 0, 0};
     for (uint32_t m = m0; m < m1; m += 4u) {
       FF w[4];
@@ -1347,34 +1351,41 @@ __global__ void __launch_bounds__(kPostThreads) post_argmax_kernel(
   const TemplateDev t = T[k];
   const uint32_t e_row = post_part_entries(t.N_t0), e_col = post_part_entries(t.N_tau);
   const uint32_t p_row = (t.N_t0 + e_row - 1u) / e_row, p_col = (t.N_tau + e_col - 1u) / e_col;
-  const uint32_t n_parts = p_row + p_col, part = blockIdx.x;
-  if (part >= n_parts) return;
-  const bool is_row = part < p_row;
-  const uint32_t N = is_row ? t.N_t0 : t.N_tau, e = is_row ? e_row : e_col;
-  const uint32_t i0 = (is_row ? part : part - p_row) * e, i1 = min(N, i0 + e);
-  const uint32_t n_sum = is_row ? (t.N_tau + cols - 1u) / cols : (t.N_t0 + rows - 1u) / rows;
-  const double *S = is_row ? rowsum + t.row_off : colsum + t.col_off;
-  auto load = [](const double *p) { return kChained ? *p : __ldg(p); };
-  PostBest best{-1, INT64_MAX};
-  for (uint32_t i = i0 + threadIdx.x; i < i1; i += kPostThreads) {
-    double v[4] = {0.0, 0.0, 0.0, 0.0};  // four chains: FP64 additions are slow to return
-    uint32_t c = 0;
-    for (; c + 4u <= n_sum; c += 4u)
-#pragma unroll
-      for (uint32_t q = 0; q < 4u; q++) v[q] += load(S + (size_t)(c + q) * N + i);
-    for (; c < n_sum; c++) v[0] += load(S + (size_t)c * N + i);
-    const int64_t key = post_key((v[0] + v[1]) + (v[2] + v[3]));
-    if (key > best.v) best = PostBest{key, (int64_t)i};  // i increases: keeps the first
-  }
-  best = post_block_best(best, sh);
+  const uint32_t n_parts = p_row + p_col;
   PostPart *mine = parts + (size_t)k * (2u * kPostParts);
-  if (threadIdx.x == 0) {
-    mine[is_row ? part : kPostParts + part - p_row] = PostPart{best.v, best.i};
-    __threadfence();
-    s_last = atomicAdd(ticket + k, 1u) == n_parts - 1u ? 1u : 0u;
+  bool last = false;
+  for (uint32_t part = blockIdx.x; part < n_parts; part += gridDim.x) {
+    const bool is_row = part < p_row;
+    const uint32_t N = is_row ? t.N_t0 : t.N_tau, e = is_row ? e_row : e_col;
+    const uint32_t i0 = (is_row ? part : part - p_row) * e, i1 = min(N, i0 + e);
+    const uint32_t n_sum = is_row ? (t.N_tau + cols - 1u) / cols : (t.N_t0 + rows - 1u) / rows;
+    const double *S = is_row ? rowsum + t.row_off : colsum + t.col_off;
+    auto load = [](const double *p) { return kChained ? *p : __ldg(p); };
+    PostBest best{-1, INT64_MAX};
+    for (uint32_t i = i0 + threadIdx.x; i < i1; i += kPostThreads) {
+      double v[4] = {0.0, 0.0, 0.0, 0.0};  // four chains: FP64 additions are slow to return
+      uint32_t c = 0;
+      for (; c + 4u <= n_sum; c += 4u)
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; q++) v[q] += load(S + (size_t)(c + q) * N + i);
+      for (; c < n_sum; c++) v[0] += load(S + (size_t)c * N + i);
+      const int64_t key = post_key((v[0] + v[1]) + (v[2] + v[3]));
+      if (key > best.v) best = PostBest{key, (int64_t)i};  // i increases: keeps the first
+    }
+    best = post_block_best(best, sh);
+    if (threadIdx.x == 0) {
+      mine[is_row ? part : kPostParts + part - p_row] = PostPart{best.v, best.i};
+      if (gridDim.x > 1u) {
+        __threadfence();
+        s_last = atomicAdd(ticket + k, 1u) == n_parts - 1u ? 1u : 0u;
+      } else {
+        s_last = 1u;
+      }
+    }
+    __syncthreads();
+    last = s_last != 0u;
   }
-  __syncthreads();
-  if (!s_last || threadIdx.x >= 2u) return;
+  if (!last || threadIdx.x >= 2u) return;
   __threadfence();
   // thread 0 the rows' parts, thread 1 the columns'
   const uint32_t n = threadIdx.x == 0 ? p_row : p_col;
@@ -1400,7 +1411,7 @@ cudaError_t launch_posteriors(const TemplateDev *d_T, uint32_t n_templates, cons
   for (uint32_t y0 = 0; y0 < n_templates; y0 += 65535u) {
     const uint32_t ny = n_templates - y0 < 65535u ? n_templates - y0 : 65535u;
     e = launch_kernel(chained ? post_argmax_kernel<true> : post_argmax_kernel<false>,
-                      dim3(2u * kPostParts, ny), kPostThreads, stream, chained && y0 == 0,
+                      dim3(L.argmax_blocks, ny), kPostThreads, stream, chained && y0 == 0,
                       d_T + y0, L.rows, L.cols, (const double *)L.rowsum, (const double *)L.colsum,
                       L.parts + (size_t)y0 * 2u * kPostParts, L.ticket + y0, d_results + y0);
     if (e != cudaSuccess) return e;

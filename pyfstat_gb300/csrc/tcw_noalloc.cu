@@ -197,7 +197,7 @@ extern "C" int tcw_map_plain_noalloc(void *stream, const float *d_atoms, uint32_
   if (launch_map(window, ml, s) != cudaSuccess) return TCW_ERR_CUDA;
   if (launch_finalize(dT, 1, dparts, d_result, true, s) != cudaSuccess) return TCW_ERR_CUDA;
   if (post) {
-    const PostLayout pl{p_rows, p_cols, n_rc * n_cc, nullptr,
+    const PostLayout pl{p_rows, p_cols, n_rc * n_cc, post_parts(N_t0, N_tau), nullptr,
                         reinterpret_cast<double *>(base + o_row),
                         reinterpret_cast<double *>(base + o_col), pp,
                         reinterpret_cast<uint32_t *>(pp + 2u * kPostParts)};
