@@ -1372,8 +1372,9 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     cend += (uint64_t)cgs * t.n_aseg;
     g.max_cg = std::max(g.max_cg, t.n_cg);
     g.max_atoms = std::max(g.max_atoms, t.g.numAtoms);
-    const uint64_t warps =
-        (uint64_t)cgs * std::max(std::max(t.n_chunk, t.g_nseg), pass ? t.n_aseg : 0u);
+    const uint64_t warps = std::max<uint64_t>(
+        t.n_aseg,  // (diff_prep_kernel)
+        (uint64_t)cgs * std::max(std::max(t.n_chunk, t.g_nseg), pass ? t.n_aseg : 0u));
     const uint64_t most_now = std::max(most_warps, warps);
     if (y == y0 || (classes.back().ny + 1u) * most_now > class_warps + warps + kDiffEmptyWarps) {
       classes.push_back(DiffClass{y, 0, 0, 0, 0, 0, 0, 0});

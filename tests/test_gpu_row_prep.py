@@ -65,3 +65,29 @@ def test_plan_info_reports_the_rect_tiles_in_use(n, cfg):
     if cfg:
         assert (c["rect_tm"], c["rect_tn"]) == (64, 48)
     batch.close()
+
+
+@pytest.mark.parametrize("n", [0, 70, 9000])
+def test_long_template_among_many_short_ones(n):
+    """A template of 17532 atoms (gaps across blocks of 256) has the same map by
+    itself and behind n templates of 40 atoms, whose launch gives it a few
+    blocks only."""
+    from pyfstat_gb300.batched import TransientMapBatch
+
+    def template(nsft, n_t0, n_tau):
+        t0_data, A = synth.merged_atoms(nsft, nsft, 1, gap_frac=0.1)
+        A[nsft // 3:nsft // 2] = 0.0
+        span = nsft * 1800
+        return dict(window=2, atoms=A, TAtom=1800, t0_data=t0_data,
+                    t0s=(t0_data + span // n_t0 * np.arange(n_t0)).astype(np.uint32),
+                    taus=(1800 + span // n_tau * np.arange(n_tau)).astype(np.uint32))
+
+    cfg = dict(exp_rows=1 << 16)  # whole columns in both plans
+    big, small = template(17532, 21, 33), template(40, 3, 2)
+    one = TransientMapBatch([big], tile_config=cfg)
+    _, F = one.plan.run_maps_host(one.atoms)
+    many = TransientMapBatch([small] * n + [big, small], tile_config=cfg, handle=one.handle)
+    _, M = many.plan.run_maps_host(many.atoms)
+    assert np.array_equal(M[6 * n:6 * n + F.size].view(np.uint32), F.view(np.uint32))
+    many.close()
+    one.close()
