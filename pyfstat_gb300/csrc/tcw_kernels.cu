@@ -1236,6 +1236,11 @@ constexpr uint32_t kPostMaxRows = 256;
 
 // kChained (both kernels): launched as a dependent in a single map's chain
 // (pdl_begin); a plan's launches take read-only loads.
+template <bool kChained, class V>
+__device__ __forceinline__ V post_load(const V *p) {
+  return kChained ? *p : __ldg(p);
+}
+
 template <bool kChained>
 __global__ void __launch_bounds__(kPostThreads) post_sums_kernel(
     const TemplateDev *T, const uint2 *__restrict__ chunks, uint32_t rows,
@@ -1257,11 +1262,11 @@ __global__ void __launch_bounds__(kPostThreads) post_sums_kernel(
   if (ch.y == 0u && tid == 0u) ticket[ch.x] = 0u;
   const float maxF = results[ch.x].maxF;
   const float *F = maps + t.map_off;
-  auto load = [](const float *p) { return kChained ? *p : __ldg(p); };
   for (uint32_t k = lane; k < m1 - m0; k += 32u) srow[wid][k] = make_float2(0.0f, 0.0f);
   __syncwarp();
-  // (warps behind the last column leave their zeros)
-  for (uint32_t n0 = nb + tid; n0 - lane < ne; n0 += kPostCols) {
+  // (warps behind a narrow map's last column leave their zeros; tested once, not
+  // per strip: that made 1024 x 1024 exponential calls 127 -> 137 us)
+  for (uint32_t n0 = nb + wid * 32u < ne ? nb + tid : ne + tid; n0 - tid < ne; n0 += kPostCols) {
     float cs[4] = {0, 0, 0, 0}, cc4[4] = {0, 0, 0, 0};
     for (uint32_t m = m0; m < m1; m += 4u) {
       FF w[4];
@@ -1272,7 +1277,7 @@ __global__ void __launch_bounds__(kPostThreads) post_sums_kernel(
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           const uint32_t n = n0 + 256u * j;
-          e[j] = (m + q < m1 && n < ne) ? ex2_approx((load(row + n) - maxF) * kLog2e) : 0.0f;
+          e[j] = (m + q < m1 && n < ne) ? ex2_approx((post_load<kChained>(row + n) - maxF) * kLog2e) : 0.0f;
         }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -1368,17 +1373,37 @@ __global__ void __launch_bounds__(kPostThreads) post_argmax_kernel(
     const uint32_t i0 = (is_row ? part : part - p_row) * e, i1 = min(N, i0 + e);
     const uint32_t n_sum = is_row ? (t.N_tau + cols - 1u) / cols : (t.N_t0 + rows - 1u) / rows;
     const double *S = is_row ? rowsum + t.row_off : colsum + t.col_off;
-    auto load = [](const double *p) { return kChained ? *p : __ldg(p); };
     PostBest best{-1, INT64_MAX};
-    for (uint32_t i = i0 + threadIdx.x; i < i1; i += kPostThreads) {
-      double v[4] = {0.0, 0.0, 0.0, 0.0};  // four chains: FP64 additions are slow to return
-      uint32_t c = 0;
-      for (; c + 4u <= n_sum; c += 4u)
+    if (n_sum >= 64u && i1 - i0 <= kPostThreads / 8u) {
+      // few entries of many sums (a map of many rows and few columns): eight
+      // lanes share an entry (100000 x 3 cells: 3 threads adding 6250 sums each
+      // 700 us a call, 180 now)
+      const uint32_t i = i0 + threadIdx.x / 8u;
+      double s = 0.0;
+      if (i < i1) {
+        const double *col = S + i;
+        double v[4] = {0.0, 0.0, 0.0, 0.0};
+        uint32_t c = threadIdx.x & 7u;
+        for (; c + 24u < n_sum; c += 32u)
 #pragma unroll
-        for (uint32_t q = 0; q < 4u; q++) v[q] += load(S + (size_t)(c + q) * N + i);
-      for (; c < n_sum; c++) v[0] += load(S + (size_t)c * N + i);
-      const int64_t key = post_key((v[0] + v[1]) + (v[2] + v[3]));
-      if (key > best.v) best = PostBest{key, (int64_t)i};  // i increases: keeps the first
+          for (uint32_t q = 0; q < 4u; q++) v[q] += post_load<kChained>(col + (size_t)(c + 8u * q) * N);
+        for (; c < n_sum; c += 8u) v[0] += post_load<kChained>(col + (size_t)c * N);
+        s = (v[0] + v[1]) + (v[2] + v[3]);
+      }
+#pragma unroll
+      for (int d = 4; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+      if (i < i1) best = PostBest{post_key(s), (int64_t)i};
+    } else {
+      for (uint32_t i = i0 + threadIdx.x; i < i1; i += kPostThreads) {
+        double v[4] = {0.0, 0.0, 0.0, 0.0};  // four chains: FP64 additions are slow to return
+        uint32_t c = 0;
+        for (; c + 4u <= n_sum; c += 4u)
+#pragma unroll
+          for (uint32_t q = 0; q < 4u; q++) v[q] += post_load<kChained>(S + (size_t)(c + q) * N + i);
+        for (; c < n_sum; c++) v[0] += post_load<kChained>(S + (size_t)c * N + i);
+        const int64_t key = post_key((v[0] + v[1]) + (v[2] + v[3]));
+        if (key > best.v) best = PostBest{key, (int64_t)i};  // i increases: keeps the first
+      }
     }
     best = post_block_best(best, sh);
     if (threadIdx.x == 0) {

@@ -46,3 +46,23 @@ def test_posteriors_of_many_maps(n):
             # FP32 terms of 1e-7: the index of the largest sum, or of one as large
             assert sums[rec[field][k]] >= sums.max() * (1.0 - 1e-6), (k, field)
     b.close()
+
+
+# 63, 64 and 65 sums of 16 rows per column, up to 32 columns (eight lanes each)
+# and more, and many sums
+@pytest.mark.parametrize("shape", [(1008, 32), (1009, 32), (1024, 33), (1025, 1), (1040, 31),
+                                   (30000, 3), (30011, 32)])
+def test_posteriors_of_tall_maps(shape):
+    from pyfstat_gb300 import _lib
+
+    n_t0, n_tau = shape
+    t0_data, A = synth.merged_atoms(2, 90, 1)
+    t0s = (t0_data + 5 * np.arange(n_t0)).astype(np.uint32)
+    taus = (1800 + 3600 * np.arange(n_tau)).astype(np.uint32)
+    h = _lib.Handle(0)
+    F, r = h.map_plain_host(A, 1800, t0_data, 1, t0s, taus,
+                            flags=_lib.TCW_FLAG_LNBTSG | _lib.TCW_FLAG_POSTERIORS)
+    e = np.exp(F.astype(np.float64) - F.max())
+    for idx, sums in ((r["t0_mp_idx"], e.sum(1)), (r["tau_mp_idx"], e.sum(0))):
+        assert sums[idx] >= sums.max() * (1.0 - 1e-6)
+    h.close()
