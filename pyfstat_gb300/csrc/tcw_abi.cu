@@ -1312,10 +1312,13 @@ static uint64_t diff_end_bytes(const DiffTemplate &t) {
 // atoms keep whole columns: their hot tiles are most of them, the walk that
 // diff_hot_kernel would repeat is then the tile's own, bit for bit, and a warp
 // per column group shares the SM with others where that kernel's nine take it
-// alone.  More atoms make the walk the longest chain (64 rows of 17532 atoms
-// among 300 templates: 12.5 + 14.7 -> 26 + 34 ms, so they are cut; forward /
-// backward of 3000 templates of 47 x 47 cells 1.72 / 1.28 -> 1.21 / 0.83 ms, 1000 of
-// 32 x 32 0.55 / 0.52 -> 0.41 / 0.41).
+// alone (forward / backward of 3000 templates of 47 x 47 cells 1.72 / 1.28 ->
+// 1.21 / 0.83 ms, 1000 of 32 x 32 0.55 / 0.52 -> 0.41 / 0.41).  So do, with up to
+// 2048 atoms, the columns of 16 rows that are not cut anyway (200 templates of
+// 1000 atoms, 16 x 500 cells 1.85 / 3.13 -> 1.36 / 2.75 ms) and the shortest
+// columns of any batch (10 x 10 cells of 48 atoms 235 -> 223 us without the second
+// stream).  More atoms make the walk the longest chain (64 rows of 17532 atoms
+// among 300 templates: 12.5 + 14.7 -> 26 + 34 ms), so they are cut.
 constexpr uint32_t kDiffFewRows = 64, kDiffFewAtoms = 256;
 // Warps of a class's grid that have no tile: above this, half a millisecond of
 // empty blocks, the templates of unequal size go in launches of their own,
@@ -1360,7 +1363,9 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     t.chunk_rows = (uint32_t)((t.N_t0 + nc - 1) / nc);
     t.n_chunk = (t.N_t0 + t.chunk_rows - 1u) / t.chunk_rows;
     if (t.n_chunk == 1u || t.g.numAtoms < 64u) t.g_nseg = 0;
-    t.whole = filled && t.n_chunk == 1u && t.g.numAtoms <= kDiffFewAtoms ? 1u : 0u;
+    const bool few = t.g.numAtoms <= (t.N_t0 <= 16u ? 8u : 1u) * kDiffFewAtoms;
+    const bool tiny = 2u * (uint64_t)t.g.numAtoms + 10u * (uint64_t)t.N_t0 <= 512u;
+    t.whole = t.n_chunk == 1u && ((filled && few) || tiny) ? 1u : 0u;
     g.hot = g.hot || !t.whole;
     t.n_aseg = (t.g.numAtoms + kDiffAtomSeg - 1u) / kDiffAtomSeg;
     t.seg_off = seg;

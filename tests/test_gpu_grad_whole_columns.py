@@ -56,11 +56,11 @@ def test_whole_columns_have_the_bits_of_the_channel_split_walk(nsft):
 
 
 def test_few_rows_in_a_full_batch_match_torch_autograd():
-    """Rows around the limit of 64 and atoms around that of 256, one and two
-    column groups, beside templates that are cut."""
+    """Rows around the limits of 64 and 16 and atoms around that of 256, one and
+    two column groups, beside templates that are cut."""
     torch = pytest.importorskip("torch")
     shapes = [(40, 1, 1), (50, 63, 33), (63, 64, 32), (64, 65, 31), (65, 64, 9), (90, 17, 64),
-              (70, 150, 20), (256, 40, 9), (257, 40, 9)]
+              (70, 150, 20), (256, 40, 9), (257, 40, 9), (330, 16, 10), (330, 17, 10)]
     tl = [template(k, n, rows, cols, dt0=max(450, n * 1800 // rows // 450 * 450),
                    amp=[0.0, 1.0, 6.0][k % 3])
           for k, (n, rows, cols) in enumerate(shapes * (MANY // len(shapes)))]
