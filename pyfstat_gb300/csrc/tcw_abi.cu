@@ -804,7 +804,10 @@ static int plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_
   // `want` tiles, columns of unequal length up to 1.3 of it (`most`); a start
   // and its run-up cost up to two and a half times their steps (they run beside
   // fewer warps, behind the segment sums), less where rect tiles keep the SMs
-  // busy meanwhile.  Per run, cut / whole: 96 templates with maps and posteriors
+  // busy meanwhile.  Short columns (the longest of few starts' length) stay whole
+  // where their chunks would crowd schedulers that whole columns leave free
+  // (`crowded`: 97 templates of 200 atoms, 64 x 32 cells: 776 chunks 0.150 ms a
+  // run, 97 columns 0.102; 9 templates 0.091 / 0.099).  Per run, cut / whole: 96 templates with maps and posteriors
   // 1.55 / 3.55 ms, 24 templates 0.18 / 0.67; exp templates of up to 2500 atoms
   // and 700 x 700 cells at 0.6, 0.95 and 1.3 `want` 1.01 / 1.40, 1.48 / 1.73,
   // 1.90 / 1.77; 500 atoms, 60 x 60 cells at 0.25, 0.8, 1.0 0.34 / 0.41, 0.65 /
@@ -815,7 +818,7 @@ static int plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_
   uint64_t seg_blocks = 0;
   double chunk_steps = 0.0;  // 0: whole columns
   if (cut && cfg.exp_rows == 0 && p->prec != kPrecPlain32) {
-    double tiles = 0.0, steps = 0.0, most = 0.0, starts = 0.0;
+    double tiles = 0.0, steps = 0.0, most = 0.0, most_mean = 0.0, starts = 0.0, pieces = 0.0;
     bool rect = false;
     for (uint32_t k = 0; k < n_templates; k++) {
       const tcw_template_desc &d = desc[k];
@@ -824,6 +827,7 @@ static int plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_
           d.N_t0 == 0)
         continue;
       const ExpSplit sp = exp_split(d.numAtoms, d.N_t0, d.N_tau, d.N_t0, 2);
+      const double before = steps;
       for (uint32_t n0 = 0; n0 < d.N_tau; n0 += 32u) {
         const uint32_t *tau = taus + d.tau_offset;
         const ExpGroupSteps g(d.numAtoms, d.TAtom, d.N_t0, tau[n0]);
@@ -831,14 +835,19 @@ static int plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_
         tiles += 1.0;
         steps += s;
         most = std::max(most, s);
+        pieces += ceil(d.N_t0 / 8.0);
         starts += g.start(sp) + 3.0 * g.run_up_atoms(tau[std::min(d.N_tau, n0 + 32u) - 1u]);
       }
+      most_mean = std::max(most_mean, (steps - before) / ceil(d.N_tau / 32.0));
     }
     const double want = (double)h->n_sms * 4.0 * TCW_PLAN_EXP_WARPS;
     const double limit =
         std::min(1.3, 0.75 + 0.3 * most * tiles / steps) *
         (1.0 - (rect ? 1.5 * starts : 2.5 * starts + 100.0 * tiles) / steps);
-    if (tiles > 0.0 && tiles <= limit * want) chunk_steps = steps / want;
+    const double scheds = (double)h->n_sms * 4.0;
+    const bool crowded =
+        most_mean * tiles < 6.0 * starts && pieces > scheds && tiles < (rect ? 0.5 : 1.0) * scheds;
+    if (tiles > 0.0 && tiles <= limit * want && !crowded) chunk_steps = steps / want;
   }
   // Rect tiles when the caller leaves them to the library: 128 x 128 while
   // these give every scheduler TCW_PLAN_RECT_WARPS warps' worth of tiles, else
