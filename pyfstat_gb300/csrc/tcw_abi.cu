@@ -973,16 +973,25 @@ static int plan_create(tcw_handle *h, const tcw_template_desc *desc, uint32_t n_
       memcpy(&bits, &c, sizeof bits);
       return (T[items[i].tmpl].window == TCW_WINDOW_RECT ? 0u : 0x8000u) + 0x7FFFu - (bits >> 16);
     };
-    std::vector<uint32_t> at(0x10001u, 0u);
     std::vector<uint16_t> key(items.size());
+    uint32_t nr = 0;
     for (size_t i = 0; i < items.size(); i++) {
       key[i] = (uint16_t)bucket(i);
-      at[key[i] + 1u]++;
+      nr += key[i] < 0x8000u ? 1u : 0u;
     }
-    for (uint32_t b = 0; b < 0x10000u; b++) at[b + 1u] += at[b];
-    const uint32_t nr = at[0x8000u];
     std::vector<WorkItem> sorted(items.size());
-    for (size_t i = 0; i < items.size(); i++) sorted[at[key[i]]++] = items[i];
+    if (items.size() < 4096u) {  // (40 us for the counts alone)
+      std::vector<uint32_t> order(items.size());
+      for (size_t i = 0; i < order.size(); i++) order[i] = (uint32_t)i;
+      std::stable_sort(order.begin(), order.end(),
+                       [&](uint32_t a, uint32_t b) { return key[a] < key[b]; });
+      for (size_t i = 0; i < order.size(); i++) sorted[i] = items[order[i]];
+    } else {
+      std::vector<uint32_t> at(0x10001u, 0u);
+      for (uint16_t k : key) at[k + 1u]++;
+      for (uint32_t b = 0; b < 0x10000u; b++) at[b + 1u] += at[b];
+      for (size_t i = 0; i < items.size(); i++) sorted[at[key[i]]++] = items[i];
+    }
     items.swap(sorted);
     p->n_items_rect = nr;
     p->n_items_exp = (uint32_t)items.size() - nr;
