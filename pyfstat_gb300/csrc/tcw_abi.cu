@@ -1292,7 +1292,7 @@ int tcw_plan_run_timed(tcw_handle *h, tcw_plan *p, const float *d_atoms, tcw_res
 // Validates descriptors, uploads descriptors, tiles and grids into the
 // handle's workspace; returns the layout of what follows them.
 struct DiffSetup {
-  size_t o_T, o_parts, o_t0, o_est, o_rlist, o_ident, o_RT, o_P, o_B64, o_D64, o_elist, o_A8;
+  size_t o_T, o_parts, o_t0, o_est, o_hot, o_rlist, o_ident, o_RT, o_P, o_B64, o_D64, o_elist, o_A8;
   size_t o_cols, o_seg, o_need, o_scratch, o_cend, total;
   uint32_t n_rect, max_rect_tiles, max_rect_atoms, n_exp;
   uint64_t p_rows, seg_floats;
@@ -1384,7 +1384,7 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     const bool few = t.g.numAtoms <= (t.N_t0 <= 16u ? 8u : 1u) * kDiffFewAtoms;
     const bool tiny = 2u * (uint64_t)t.g.numAtoms + 10u * (uint64_t)t.N_t0 <= 512u;
     t.whole = t.n_chunk == 1u && ((filled && few) || tiny) ? 1u : 0u;
-    g.hot = g.hot || !t.whole;
+    if (!t.whole) g.hot += t.n_cg;
     t.n_aseg = (t.g.numAtoms + kDiffAtomSeg - 1u) / kDiffAtomSeg;
     t.seg_off = seg;
     t.scr_off = scr;
@@ -1400,7 +1400,8 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
         (uint64_t)cgs * std::max(std::max(t.n_chunk, t.g_nseg), pass ? t.n_aseg : 0u));
     const uint64_t most_now = std::max(most_warps, warps);
     if (y == y0 || (classes.back().ny + 1u) * most_now > class_warps + warps + kDiffEmptyWarps) {
-      classes.push_back(DiffClass{y, 0, 0, 0, 0, 0, 0, 0});
+      classes.push_back(DiffClass{});
+      classes.back().y0 = y;
       most_warps = warps;
       class_warps = 0;
     } else {
@@ -1415,6 +1416,7 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     c.max_cols = std::max(c.max_cols, t.N_tau);
     c.slice_tiles = std::max(c.slice_tiles, cgs * t.n_chunk);
     c.slice_aseg = std::max(c.slice_aseg, cgs * t.n_aseg);
+    c.slice_cg = std::max(c.slice_cg, cgs);
   }
   g.n_classes = (uint32_t)classes.size() - g.c0;
   g.seg_per = segs_per_warp(seg, h->n_sms);
@@ -1543,6 +1545,7 @@ static int diff_setup(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n, cons
   S.o_T = L.add(sizeof(DiffTemplate) * n);
   S.o_t0 = L.add(sizeof(uint32_t) * n_t0s);
   S.o_est = L.add(sizeof(uint32_t) * n);
+  S.o_hot = L.add(sizeof(uint32_t) * S.groups.size());
   S.o_rlist = L.add(sizeof(uint32_t) * std::max<size_t>(1, rlist.size()));
   S.o_elist = L.add(sizeof(uint32_t) * std::max<size_t>(1, elist.size()));
   S.o_ident = L.add(sizeof(uint32_t) * ident.size());
@@ -1568,6 +1571,7 @@ static int diff_setup(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n, cons
   memcpy(h->h_stage + S.o_T, T.data(), sizeof(DiffTemplate) * n);
   memcpy(h->h_stage + S.o_t0, t0s, sizeof(uint32_t) * n_t0s);
   memset(h->h_stage + S.o_est, 0, sizeof(uint32_t) * n);
+  memset(h->h_stage + S.o_hot, 0, sizeof(uint32_t) * S.groups.size());
   if (!rlist.empty()) {
     memcpy(h->h_stage + S.o_rlist, rlist.data(), sizeof(uint32_t) * rlist.size());
     memcpy(h->h_stage + S.o_ident, ident.data(), sizeof(uint32_t) * ident.size());
@@ -1600,6 +1604,8 @@ static DiffLaunch diff_launch(tcw_handle *h, const DiffSetup &S, const float *d_
   L.seg = reinterpret_cast<float *>(h->d_ws + S.o_seg);
   L.need = reinterpret_cast<float *>(h->d_ws + S.o_need);
   L.est = reinterpret_cast<uint32_t *>(h->d_ws + S.o_est);
+  L.hot_groups = reinterpret_cast<uint32_t *>(h->d_ws + S.o_hot);
+  L.n_sms = (uint32_t)h->n_sms;
   L.scratch = reinterpret_cast<float *>(h->d_ws + S.o_scratch);
   L.cend = reinterpret_cast<float *>(h->d_ws + S.o_cend);
   L.rect_list = reinterpret_cast<const uint32_t *>(h->d_ws + S.o_rlist);

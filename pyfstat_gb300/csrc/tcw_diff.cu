@@ -116,10 +116,12 @@ __device__ __forceinline__ F64Cell fstat64(const double W[7], bool passes = fals
     passes = denom > 0.0 && sumAB + disc < 1e4 * denom;
   }
   if (passes) {
-    const double D = A * B - C * C;
+    // (explicit roundings: every kernel forms the same bits)
+    const double D = fma(A, B, -(C * C));
     if (D > 0.0) {
-      const double N = B * (W[3] * W[3] + W[4] * W[4]) + A * (W[5] * W[5] + W[6] * W[6]) -
-                       2.0 * C * (W[3] * W[5] + W[4] * W[6]);
+      const double Fa2 = fma(W[3], W[3], W[4] * W[4]), Fb2 = fma(W[5], W[5], W[6] * W[6]);
+      const double re = fma(W[3], W[5], W[4] * W[6]);
+      const double N = fma(B, Fa2, fma(A, Fb2, -2.0 * C * re));
       r.iD = 1.0 / D;
       r.F = N * r.iD;
       r.ok = true;
@@ -621,6 +623,54 @@ struct DiffLse {
   }
 };
 
+// Which kernel walks a group's hot tiles: diff_hot_kernel, a block per column
+// group, where few column groups have any; else the kHot tile kernels, a warp per
+// column group with the same steps -- the block's walk is a third as long, but
+// an SM holds one block and four warps of the other on each scheduler.
+// `groups` (NULL: blocks) counts the column groups with hot tiles
+// (diff_route_kernel), `few` is two blocks per SM.  Forward / backward by blocks
+// and by warps, noise: 2000 templates of 1500 atoms, 600 x 4 cells 18.0 / 16.2 ->
+// 9.1 / 11.1 ms; of 400 atoms, 32 x 128 cells 5.7 / 7.4 -> 2.6 / 5.2; 256 of 2000
+// atoms, 1024 x 1024 cells and a signal 11.8 / 17.2 -> 7.8 / 17.3; 24 of those
+// have few hot groups and keep the blocks (1.46 / 1.82 ms).
+struct HotRoute {
+  const uint32_t *groups;
+  uint32_t few;
+  __device__ __forceinline__ bool warps() const { return groups && __ldg(groups) > few; }
+};
+
+// One column group's hot tiles (at or above `hot` and not below `skip`), for a
+// warp that walks its rows from the last one down.
+struct HotGroup {
+  const float *nd;
+  uint32_t n_chunk, chunk_rows, first, row0;
+  float skip, hot;
+  bool on;
+  __device__ __forceinline__ HotGroup(const float *need, const DiffTemplate &t, float skip_,
+                                      float hot_)
+      : nd(need), n_chunk(t.n_chunk), chunk_rows(t.chunk_rows), first(0xFFFFFFFFu),
+        row0(0xFFFFFFFFu), skip(skip_), hot(hot_), on(false) {}
+  __device__ __forceinline__ bool is_hot(uint32_t c) const {
+    return !(nd[c] < skip) && !(nd[c] < hot);
+  }
+  // all lanes: finds the first hot tile
+  __device__ __forceinline__ bool any() {
+    for (uint32_t c = threadIdx.x & 31u; c < n_chunk; c += 32u)
+      if (is_hot(c)) first = min(first, c);
+    first = __reduce_min_sync(0xffffffffu, first);
+    return first != 0xFFFFFFFFu;
+  }
+  // whether row m, below those asked for before, is in a hot tile
+  __device__ __forceinline__ bool row(uint32_t m) {
+    if (m < row0) {
+      const uint32_t c = m / chunk_rows;
+      row0 = c * chunk_rows;
+      on = is_hot(c);
+    }
+    return on;
+  }
+};
+
 // Forward pass of the tiles that may carry weight (lnBtSG and the soft-max
 // 2F): the window sums in double-word FP32 (ExpColumn; sums good to ~1e-14 of
 // the window's magnitude, against FP64 recurrences at GB300's 1/70 FP64
@@ -630,36 +680,51 @@ struct DiffLse {
 // maximum carries less than e^-60 in both sums (no_weight_below) and is skipped
 // -- the tier-1 F is good to ~1.5e-6 relative and passes only for cond < 32,
 // where the FP64 test passes too.
+// kHot: the hot tiles of one column group per warp, their columns walked whole
+// (HotGroup), where diff_hot_kernel leaves them to it.
+template <bool kHot>
 __global__ void __launch_bounds__(kDiffBlock, 5)
     diff_fwd_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
                     const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
                     const ColConsts *__restrict__ cols, const float *__restrict__ seg,
                     const float *__restrict__ need, const uint32_t *__restrict__ est, double temp,
-                    DiffPartial *__restrict__ parts) {
+                    DiffPartial *__restrict__ parts, HotRoute route) {
   __shared__ __align__(16) ExpRow s_tab[kDiffBlock / 32][kDiffRowTab];
+  if (kHot && !route.warps()) return;
   DiffLane L;
   const uint32_t k = list[blockIdx.y];
   L.t = T[k];
-  const uint32_t tile = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
-  const uint32_t cg = tile / L.t.n_chunk, mb = tile % L.t.n_chunk * L.t.chunk_rows;
-  if (cg >= L.t.n_cg) return;
-  DiffPartial *out = parts + L.t.part_off + tile;
+  const uint32_t warp = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+  const uint32_t cg = kHot ? warp : warp / L.t.n_chunk;
+  if (cg >= L.t.n_cg || (kHot && L.t.whole)) return;
   const FwdBounds bd(est[k], temp);
-  const float skip0 = bd.skip, nd = need[L.t.part_off + tile];
-  if (nd < skip0) {
-    if (lane == 0) *out = DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
-    return;
+  const float skip0 = bd.skip;
+  DiffPartial *out = parts + L.t.part_off + (kHot ? (size_t)cg * L.t.n_chunk : warp);
+  uint32_t mb, me = L.t.N_t0;
+  HotGroup hot(need + L.t.part_off + (size_t)cg * L.t.n_chunk, L.t, skip0, bd.hot);
+  if (kHot) {
+    if (!hot.any()) return;
+    mb = hot.first * L.t.chunk_rows;
+  } else {
+    const float nd = need[L.t.part_off + warp];
+    if (nd < skip0) {
+      if (lane == 0) *out = DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
+      return;
+    }
+    if (!(nd < bd.hot) && !L.t.whole) return;  // a hot tile
+    mb = warp % L.t.n_chunk * L.t.chunk_rows;
+    me = min(me, mb + L.t.chunk_rows);
   }
-  if (!(nd < bd.hot) && !L.t.whole) return;  // diff_hot_kernel
-  const uint32_t me = min(L.t.N_t0, mb + L.t.chunk_rows);
   L.columns(atoms8, t0s_all, cg);
   ExpColumn<false> C;
   C.init_consts(L.consts(cols));
-  const float *sg =
-      L.t.g_nseg ? seg + (L.t.seg_off + (size_t)cg * L.t.g_nseg) * kDiffSegFloats + lane : nullptr;
+  const float *sg = !kHot && L.t.g_nseg
+                        ? seg + (L.t.seg_off + (size_t)cg * L.t.g_nseg) * kDiffSegFloats + lane
+                        : nullptr;
   DiffLse lse(temp, skip0);
   diff_rows(L, mb, me, C, sg, kDiffSegFloats, s_tab[threadIdx.x >> 5],
-            [&](uint32_t, uint32_t, uint32_t, bool data) {
+            [&](uint32_t m, uint32_t, uint32_t, bool data) {
+              if (kHot && !hot.row(m)) return;
               float F32 = 0.0f;
               const bool t1 = data && diff_tier1(C, F32);
               double W[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -675,7 +740,13 @@ __global__ void __launch_bounds__(kDiffBlock, 5)
               lse.cell(data, W, t1, F32);
             });
   const DiffPartial p = lse.merge();
-  if (lane == 0) *out = p;
+  if (!kHot) {
+    if (lane == 0) *out = p;
+    return;
+  }
+  // the group's hot cells are one partial, its other hot tiles' are empty
+  for (uint32_t c = lane; c < L.t.n_chunk; c += 32u)
+    if (hot.is_hot(c)) out[c] = c == hot.first ? p : DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
 }
 
 // Whether a template's cells below `skip` carry no weight in the gradient: a
@@ -846,7 +917,8 @@ __device__ __forceinline__ void add_grad_tau(const DiffLane &L, FF dtw, double *
 // Adjoint sources of the tiles that may carry weight: W and V slide down each
 // tau column in double-word FP32 (ExpColumnV); a cell gets F, dF/dW and its
 // sources (in double-word arithmetic, dw_fstat) only when it carries weight
-// (DiffWeights).
+// (DiffWeights).  kHot: as in diff_fwd_kernel.
+template <bool kHot>
 __global__ void __launch_bounds__(kDiffBlock)
     diff_src_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
                     const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
@@ -854,22 +926,31 @@ __global__ void __launch_bounds__(kDiffBlock)
                     const float *__restrict__ need, const uint32_t *__restrict__ est, double temp,
                     const double *__restrict__ lnZ1, const double *__restrict__ lnZ2,
                     const double *__restrict__ gB, const double *__restrict__ gS, uint32_t cg0,
-                    uint32_t cgs, float *__restrict__ scratch, double *__restrict__ grad_tau) {
+                    uint32_t cgs, float *__restrict__ scratch, double *__restrict__ grad_tau,
+                    HotRoute route) {
   __shared__ __align__(16) ExpRow s_tab[kDiffBlock / 32][kDiffRowTab];
+  if (kHot && !route.warps()) return;
   DiffLane L;
   const uint32_t k = list[blockIdx.y];
   L.t = T[k];
   const DiffTemplate &t = L.t;
   // the slice's tiles; scratch holds those of column groups [cg0, cg0 + cgs)
-  const uint32_t stile = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
-  const uint32_t scg = stile / t.n_chunk, cg = cg0 + scg, tile = cg0 * t.n_chunk + stile;
-  const uint32_t mb = stile % t.n_chunk * t.chunk_rows;
-  if (scg >= cgs || cg >= t.n_cg) return;
+  const uint32_t warp = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+  const uint32_t scg = kHot ? warp : warp / t.n_chunk, cg = cg0 + scg;
+  if (scg >= cgs || cg >= t.n_cg || (kHot && t.whole)) return;
   const DiffWeights w(t, k, est[k], temp, lnZ1, lnZ2, gB, gS);
-  const float nd = need[t.part_off + tile];
-  if (nd < w.skip) return;    // diff_atoms_kernel skips its rows
-  if (!(nd < w.hot) && !t.whole) return;  // diff_hot_kernel
-  const uint32_t me = min(t.N_t0, mb + t.chunk_rows);
+  uint32_t mb, me = t.N_t0;
+  HotGroup hot(need + t.part_off + (size_t)cg * t.n_chunk, t, w.skip, w.hot);
+  if (kHot) {
+    if (!hot.any()) return;
+    mb = hot.first * t.chunk_rows;
+  } else {
+    const float nd = need[t.part_off + cg0 * t.n_chunk + warp];
+    if (nd < w.skip) return;                // diff_atoms_kernel skips its rows
+    if (!(nd < w.hot) && !t.whole) return;  // a hot tile
+    mb = warp % t.n_chunk * t.chunk_rows;
+    me = min(me, mb + t.chunk_rows);
+  }
   L.columns(atoms8, t0s_all, cg);
   const DiffGrad grad(w, temp);
   DiffPower power;
@@ -877,11 +958,15 @@ __global__ void __launch_bounds__(kDiffBlock)
   ExpColumnV CV;
   CV.C.init_consts(L.consts(cols));
   CV.reset_v();
-  const float *sg =
-      t.g_nseg ? seg + (t.seg_off + (size_t)cg * t.g_nseg) * kDiffSegFloatsV + lane : nullptr;
-  float *my = scratch + t.scr_off + (size_t)stile * t.chunk_rows * (TCW_DIFF_SLOTS * 32u) + lane;
+  const float *sg = !kHot && t.g_nseg
+                        ? seg + (t.seg_off + (size_t)cg * t.g_nseg) * kDiffSegFloatsV + lane
+                        : nullptr;
+  // (a column group's rows in order: its tiles are chunk_rows each but for the last)
+  float *my = scratch + t.scr_off +
+              (size_t)scg * t.n_chunk * t.chunk_rows * (TCW_DIFF_SLOTS * 32u) + lane;
   diff_rows(L, mb, me, CV, sg, kDiffSegFloatsV, s_tab[threadIdx.x >> 5],
             [&](uint32_t m, uint32_t lo, uint32_t top, bool data) {
+              if (kHot && !hot.row(m)) return;
               float Gf[7] = {0, 0, 0, 0, 0, 0, 0};
               FF p1{0.0f, 0.0f};
               if (data) {
@@ -898,8 +983,8 @@ __global__ void __launch_bounds__(kDiffBlock)
                   if (grad.cell(W, V, Gf, dtw)) p1 = power.at(L, top - lo);
                 }
               }
-              TCW_DCHECK(m - mb < t.chunk_rows);
-              float *scr = my + (size_t)(m - mb) * (TCW_DIFF_SLOTS * 32u);
+              TCW_DCHECK(m < t.N_t0);
+              float *scr = my + (size_t)m * (TCW_DIFF_SLOTS * 32u);
 #pragma unroll
               for (int c = 0; c < 7; c++) scr[32 * c] = Gf[c];
               scr[32 * 7] = p1.h;
@@ -931,7 +1016,8 @@ __device__ __forceinline__ void hot_walk_sync() {
 // channels: 2.4 ms for 1024 rows); here a block takes 32 columns with one
 // warp per channel, whose steps are the packed pairs' bit for bit, and two
 // more warps evaluate the hot rows from shared memory while the others walk
-// on.  Column groups without a hot tile leave at once.
+// on.  Column groups without a hot tile leave at once, and so do all of them
+// where more have one than blocks are good for (HotRoute).
 // Bound by the latency of each walking warp's own dependent instructions
 // (~1000 cycles per row of 2 atoms), so: the loops hold no evaluation code,
 // the next removal power is prepared beside the present sums, and a block may
@@ -949,7 +1035,7 @@ __global__ void __launch_bounds__(kHotThreads, 1)
                     const double *__restrict__ lnZ1, const double *__restrict__ lnZ2,
                     const double *__restrict__ gB, const double *__restrict__ gS, uint32_t cg0,
                     float *__restrict__ scratch, double *__restrict__ grad_tau,
-                    DiffPartial *__restrict__ parts, uint32_t smem_atoms) {
+                    DiffPartial *__restrict__ parts, uint32_t smem_atoms, HotRoute route) {
   extern __shared__ float s_x[];  // channel-major atoms, where a template's fit
   __shared__ float2 s_pow[32][32];  // r^(2^b) of the lanes' columns
   constexpr int kWords = kBack ? 4 : 2;
@@ -963,6 +1049,7 @@ __global__ void __launch_bounds__(kHotThreads, 1)
   __shared__ HotRow s_row[2][kHotEval];
   __shared__ DiffPartial s_part[kHotEval];
   __shared__ uint8_t s_hot[kDiffRowTab];
+  if (route.warps()) return;
   DiffLane L;
   const uint32_t k = list[blockIdx.y], cg = cg0 + blockIdx.x;  // (grid x: a slice's groups)
   L.t = T[k];
@@ -1238,6 +1325,35 @@ __global__ void __launch_bounds__(kHotThreads, 1)
     if (is_hot(c))
       parts[t.part_off + (size_t)cg * t.n_chunk + c] =
           c == c0 ? sum : DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
+}
+
+// Counts the column groups that have a hot tile (HotRoute), a thread each.
+template <bool kBack>
+__global__ void __launch_bounds__(kDiffBlock)
+    diff_route_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
+                      const float *__restrict__ need, const uint32_t *__restrict__ est,
+                      double temp, const double *__restrict__ lnZ1,
+                      const double *__restrict__ lnZ2, const double *__restrict__ gB,
+                      const double *__restrict__ gS, uint32_t *__restrict__ groups) {
+  const uint32_t k = list[blockIdx.y], cg = blockIdx.x * kDiffBlock + threadIdx.x;
+  const DiffTemplate t = T[k];
+  bool any = false;
+  if (cg < t.n_cg && !t.whole) {
+    float skip, hot;
+    if (kBack) {
+      const DiffWeights w(t, k, est[k], temp, lnZ1, lnZ2, gB, gS);
+      skip = w.skip;
+      hot = w.hot;
+    } else {
+      const FwdBounds bd(est[k], temp);
+      skip = bd.skip;
+      hot = bd.hot;
+    }
+    const HotGroup g(need + t.part_off + (size_t)cg * t.n_chunk, t, skip, hot);
+    for (uint32_t c = 0; c < t.n_chunk && !any; c++) any = g.is_hot(c);
+  }
+  const uint32_t n = __syncthreads_count(any);
+  if (threadIdx.x == 0 && n) atomicAdd(groups, n);
 }
 
 // The transposed recurrence over one 64-atom segment of one column group, in
@@ -1829,24 +1945,46 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
       for (uint32_t cg0 = 0; cg0 < g.max_cg; cg0 += g.cg_slice) {
         const uint32_t cgs = g.max_cg - cg0 < g.cg_slice ? g.max_cg - cg0 : g.cg_slice;
         const dim3 hot(cgs, g.ny);
+        const HotRoute route{g.hot > 2u * L.n_sms ? L.hot_groups + q : nullptr, 2u * L.n_sms};
         if (g.hot) {
+          if (route.groups && cg0 == 0) {
+            const dim3 all((g.max_cg + kDiffBlock - 1u) / kDiffBlock, g.ny);
+            if (pass == 0)
+              diff_route_kernel<false><<<all, kDiffBlock, 0, stream>>>(
+                  L.T, L.exp_list + g.y0, L.need, L.est, L.temp, nullptr, nullptr, nullptr,
+                  nullptr, L.hot_groups + q);
+            else
+              diff_route_kernel<true><<<all, kDiffBlock, 0, stream>>>(
+                  L.T, L.exp_list + g.y0, L.need, L.est, L.temp, L.lnZ1, L.lnZ2, L.gB, L.gS,
+                  L.hot_groups + q);
+          }
           if ((e = cudaEventRecord(fork, stream)) != cudaSuccess ||
               (e = cudaStreamWaitEvent(side, fork, 0)) != cudaSuccess)
             return e;
           if (pass == 0)
             diff_hot_kernel<false><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
                 L.T, L.exp_list + g.y0, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, nullptr,
-                nullptr, nullptr, nullptr, cg0, nullptr, nullptr, L.parts, smem_atoms);
+                nullptr, nullptr, nullptr, cg0, nullptr, nullptr, L.parts, smem_atoms, route);
           else
             diff_hot_kernel<true><<<hot, kHotThreads, (size_t)smem_atoms * 28u, side>>>(
                 L.T, L.exp_list + g.y0, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1,
-                L.lnZ2, L.gB, L.gS, cg0, L.scratch, L.grad_tau, nullptr, smem_atoms);
+                L.lnZ2, L.gB, L.gS, cg0, L.scratch, L.grad_tau, nullptr, smem_atoms, route);
+          for (const DiffClass *c = c0; route.groups && c < c1; c++) {
+            if (pass == 0)
+              diff_fwd_kernel<true><<<warps(c, c->slice_cg), kDiffBlock, 0, side>>>(
+                  L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.est, L.temp,
+                  L.parts, route);
+            else
+              diff_src_kernel<true><<<warps(c, c->slice_cg), kDiffBlock, 0, side>>>(
+                  L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.est, L.temp,
+                  L.lnZ1, L.lnZ2, L.gB, L.gS, cg0, cgs, L.scratch, L.grad_tau, route);
+          }
         }
         if (pass == 0) {
           for (const DiffClass *c = c0; c < c1; c++)
-            diff_fwd_kernel<<<warps(c, c->max_tiles), kDiffBlock, 0, stream>>>(
+            diff_fwd_kernel<false><<<warps(c, c->max_tiles), kDiffBlock, 0, stream>>>(
                 L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.est, L.temp,
-                L.parts);
+                L.parts, route);
         } else {
           for (const DiffClass *c = c0; c < c1; c++)
             if (c->max_segs && cg0 == 0)  // (over the window sums, which nothing reads any more)
@@ -1854,9 +1992,9 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
                   L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1,
                   L.lnZ2, L.gB, L.gS, g.seg_per, L.seg);
           for (const DiffClass *c = c0; c < c1; c++)
-            diff_src_kernel<<<warps(c, c->slice_tiles), kDiffBlock, 0, stream>>>(
+            diff_src_kernel<false><<<warps(c, c->slice_tiles), kDiffBlock, 0, stream>>>(
                 L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.est, L.temp,
-                L.lnZ1, L.lnZ2, L.gB, L.gS, cg0, cgs, L.scratch, L.grad_tau);
+                L.lnZ1, L.lnZ2, L.gB, L.gS, cg0, cgs, L.scratch, L.grad_tau, route);
         }
         if (g.hot && ((e = cudaEventRecord(join, side)) != cudaSuccess ||
                       (e = cudaStreamWaitEvent(stream, join, 0)) != cudaSuccess))

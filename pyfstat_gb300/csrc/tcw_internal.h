@@ -334,7 +334,7 @@ struct DiffTemplate {
   double tau_min, tau_max;
   uint32_t part_off, n_parts;  // this template's tiles (need, partials)
   uint32_t window;
-  uint32_t whole;  // its tiles are whole columns and none is left to diff_hot_kernel
+  uint32_t whole;  // its tiles are whole columns and none is walked apart
   uint64_t p_off;
   uint32_t n_cg, n_chunk, chunk_rows;
   uint32_t g_shift, g_nseg, n_aseg;  // segment sums; atom segments of the transposed recurrence
@@ -362,6 +362,7 @@ struct DiffClass {
   // most tiles / segments / atoms / columns of one template
   uint32_t max_tiles, max_segs, max_atoms, max_cols;
   uint32_t slice_tiles, slice_aseg;  // most tiles / atom segments in a slice
+  uint32_t slice_cg;                 // most column groups in a slice
 };
 // Exponential templates [y0, y0 + ny) of exp_list with workspaces of their
 // own: a backward pass runs in groups that bound the scratch, a group of one
@@ -371,7 +372,7 @@ struct DiffGroup {
   uint32_t y0, ny, c0, n_classes;
   uint32_t max_cg, max_atoms;  // most column groups / atoms of one template
   uint32_t cg_slice;
-  bool hot;  // some template's hot tiles are diff_hot_kernel's
+  uint32_t hot;  // column groups of templates whose hot tiles are walked apart
   uint32_t seg_per;  // segments per warp
   uint64_t seg_floats, scr_floats, cend_floats;
 };
@@ -386,6 +387,8 @@ struct DiffLaunch {
   float *seg;                        // segment sums
   float *need;                       // per exp tile: an upper bound of its F
   uint32_t *est;                     // per template: key of a lower bound of max F (zeroed)
+  uint32_t *hot_groups;              // per group: column groups with hot tiles (zeroed)
+  uint32_t n_sms;
   const uint32_t *t0s;
   double temp;
   DiffPartial *parts;                // pass A output
