@@ -1327,17 +1327,16 @@ static uint64_t diff_end_bytes(const DiffTemplate &t) {
 // 100 5.4 -> 5.0, 600 17.8 -> 12.9; two 2.98 / 5.1 / 14.3, eight 3.1: the
 // estimate starts too many chunks).
 // Where whole columns give every scheduler a warp, templates of few rows and
-// atoms keep whole columns: their hot tiles are most of them, the walk that
-// diff_hot_kernel would repeat is then the tile's own, bit for bit, and a warp
-// per column group shares the SM with others where that kernel's nine take it
-// alone (forward / backward of 3000 templates of 47 x 47 cells 1.72 / 1.28 ->
-// 1.21 / 0.83 ms, 1000 of 32 x 32 0.55 / 0.52 -> 0.41 / 0.41).  So do, with up to
-// 2048 atoms, the columns of 16 rows that are not cut anyway (200 templates of
-// 1000 atoms, 16 x 500 cells 1.85 / 3.13 -> 1.36 / 2.75 ms) and the shortest
-// columns of any batch (10 x 10 cells of 48 atoms 235 -> 223 us without the second
-// stream).  More atoms make the walk the longest chain (64 rows of 17532 atoms
-// among 300 templates: 12.5 + 14.7 -> 26 + 34 ms), so they are cut.
-constexpr uint32_t kDiffFewRows = 64, kDiffFewAtoms = 256;
+// atoms keep whole columns (so do the shortest columns of any batch, 10 x 10
+// cells of 48 atoms 235 -> 223 us): a handful of chunks per column buys little,
+// most of them hold a cell that matters by itself, and the walk that
+// diff_hot_kernel would repeat is then the tile's own, bit for bit.  Whole columns
+// go without the estimate, a walk as long as their own that skips nothing where
+// signals are weak, and, from four warps per scheduler on, without the segments
+// of the transposed recurrence (one pass in place of two).  More atoms make the
+// walk the longest chain (64 rows of 17532 atoms among 300 templates: 12.5 + 14.7
+// -> 26 + 34 ms), so they are cut.
+constexpr uint32_t kDiffFewRows = 64, kDiffFewAtoms = 2048;
 // Warps of a class's grid that have no tile: above this, half a millisecond of
 // empty blocks, the templates of unequal size go in launches of their own,
 // each of which lasts as long as its longest tile (gradients of 2000 templates
@@ -1352,6 +1351,7 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
   for (uint32_t y = y0; y < y1; y++) total_cg += (T[elist[y]].N_tau + 31u) / 32u;
   const uint64_t chunks = ((uint64_t)h->n_sms * 128u + total_cg - 1u) / total_cg;
   const bool filled = total_cg >= (uint64_t)h->n_sms * 4u;
+  const bool full = total_cg >= (uint64_t)h->n_sms * 16u;
   const uint64_t seg_floats = pass ? kDiffSegFloatsV : kDiffSegFloats;
   uint64_t seg = 0, scr = 0, cend = 0;
   g = DiffGroup{};
@@ -1381,11 +1381,12 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     t.chunk_rows = (uint32_t)((t.N_t0 + nc - 1) / nc);
     t.n_chunk = (t.N_t0 + t.chunk_rows - 1u) / t.chunk_rows;
     if (t.n_chunk == 1u || t.g.numAtoms < 64u) t.g_nseg = 0;
-    const bool few = t.g.numAtoms <= (t.N_t0 <= 16u ? 8u : 1u) * kDiffFewAtoms;
     const bool tiny = 2u * (uint64_t)t.g.numAtoms + 10u * (uint64_t)t.N_t0 <= 512u;
-    t.whole = t.n_chunk == 1u && ((filled && few) || tiny) ? 1u : 0u;
+    t.whole = t.n_chunk == 1u && ((filled && t.g.numAtoms <= kDiffFewAtoms) || tiny) ? 1u : 0u;
     if (!t.whole) g.hot += t.n_cg;
-    t.n_aseg = (t.g.numAtoms + kDiffAtomSeg - 1u) / kDiffAtomSeg;
+    t.a_shift = kDiffAtomShift;
+    while (((t.g.numAtoms - 1u) >> t.a_shift) >= (t.whole && full ? 1u : kDiffMaxAseg)) t.a_shift++;
+    t.n_aseg = ((t.g.numAtoms - 1u) >> t.a_shift) + 1u;
     t.seg_off = seg;
     t.scr_off = scr;
     t.cend_off = cend;
@@ -1396,7 +1397,7 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     g.max_cg = std::max(g.max_cg, t.n_cg);
     g.max_atoms = std::max(g.max_atoms, t.g.numAtoms);
     const uint64_t warps = std::max<uint64_t>(
-        t.n_aseg,  // (diff_prep_kernel)
+        (t.g.numAtoms + kDiffAtomSeg - 1u) / kDiffAtomSeg,  // (diff_prep_kernel)
         (uint64_t)cgs * std::max(std::max(t.n_chunk, t.g_nseg), pass ? t.n_aseg : 0u));
     const uint64_t most_now = std::max(most_warps, warps);
     if (y == y0 || (classes.back().ny + 1u) * most_now > class_warps + warps + kDiffEmptyWarps) {
@@ -1417,6 +1418,8 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     c.slice_tiles = std::max(c.slice_tiles, cgs * t.n_chunk);
     c.slice_aseg = std::max(c.slice_aseg, cgs * t.n_aseg);
     c.slice_cg = std::max(c.slice_cg, cgs);
+    if (!t.whole) c.est_tiles = std::max(c.est_tiles, t.n_cg * t.n_chunk);
+    if (t.n_aseg > 1u) c.slice_ends = std::max(c.slice_ends, cgs * t.n_aseg);
   }
   g.n_classes = (uint32_t)classes.size() - g.c0;
   g.seg_per = segs_per_warp(seg, h->n_sms);

@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(kDiffBlock, 8)
   L.t = T[k];
   const uint32_t tile = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
   const uint32_t cg = tile / L.t.n_chunk, mb = tile % L.t.n_chunk * L.t.chunk_rows;
-  if (cg >= L.t.n_cg) return;
+  if (cg >= L.t.n_cg || L.t.whole) return;
   const uint32_t me = min(L.t.N_t0, mb + L.t.chunk_rows);
   L.columns(atoms8, t0s_all, cg);
   ExpColumn<false, true, true> C;
@@ -604,6 +604,11 @@ struct DiffLse {
     } else if (!(t1 && F32 < skip)) {
       add(fstat64(W, t1).F);
     }
+  }
+  // without an estimate: the bound of this lane's own largest F so far
+  __device__ __forceinline__ void follow(double below) {
+    const float bound = (float)(m1 - 1e-5 * fabs(m1) - below - 1.0);
+    if (bound > skip) skip = bound;
   }
   // every lane's sums brought to the warp's maximum (one exp per sum), added
   __device__ __forceinline__ DiffPartial merge() const {
@@ -706,12 +711,14 @@ __global__ void __launch_bounds__(kDiffBlock, 5)
     if (!hot.any()) return;
     mb = hot.first * L.t.chunk_rows;
   } else {
-    const float nd = need[L.t.part_off + warp];
-    if (nd < skip0) {
-      if (lane == 0) *out = DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
-      return;
+    if (!L.t.whole) {
+      const float nd = need[L.t.part_off + warp];
+      if (nd < skip0) {
+        if (lane == 0) *out = DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
+        return;
+      }
+      if (!(nd < bd.hot)) return;  // a hot tile
     }
-    if (!(nd < bd.hot) && !L.t.whole) return;  // a hot tile
     mb = warp % L.t.n_chunk * L.t.chunk_rows;
     me = min(me, mb + L.t.chunk_rows);
   }
@@ -722,6 +729,8 @@ __global__ void __launch_bounds__(kDiffBlock, 5)
                         ? seg + (L.t.seg_off + (size_t)cg * L.t.g_nseg) * kDiffSegFloats + lane
                         : nullptr;
   DiffLse lse(temp, skip0);
+  const bool whole = L.t.whole != 0u;
+  const double below = no_weight_below(temp);
   diff_rows(L, mb, me, C, sg, kDiffSegFloats, s_tab[threadIdx.x >> 5],
             [&](uint32_t m, uint32_t, uint32_t, bool data) {
               if (kHot && !hot.row(m)) return;
@@ -738,6 +747,7 @@ __global__ void __launch_bounds__(kDiffBlock, 5)
                 W[6] = (double)C.W3.h.y + (double)C.W3.l.y;
               }
               lse.cell(data, W, t1, F32);
+              if (!kHot && whole) lse.follow(below);
             });
   const DiffPartial p = lse.merge();
   if (!kHot) {
@@ -923,7 +933,7 @@ __global__ void __launch_bounds__(kDiffBlock)
     diff_src_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
                     const float *__restrict__ atoms8, const uint32_t *__restrict__ t0s_all,
                     const ColConsts *__restrict__ cols, const float *__restrict__ seg,
-                    const float *__restrict__ need, const uint32_t *__restrict__ est, double temp,
+                    float *__restrict__ need, const uint32_t *__restrict__ est, double temp,
                     const double *__restrict__ lnZ1, const double *__restrict__ lnZ2,
                     const double *__restrict__ gB, const double *__restrict__ gS, uint32_t cg0,
                     uint32_t cgs, float *__restrict__ scratch, double *__restrict__ grad_tau,
@@ -945,9 +955,11 @@ __global__ void __launch_bounds__(kDiffBlock)
     if (!hot.any()) return;
     mb = hot.first * t.chunk_rows;
   } else {
-    const float nd = need[t.part_off + cg0 * t.n_chunk + warp];
-    if (nd < w.skip) return;                // diff_atoms_kernel skips its rows
-    if (!(nd < w.hot) && !t.whole) return;  // a hot tile
+    if (!t.whole) {
+      const float nd = need[t.part_off + cg0 * t.n_chunk + warp];
+      if (nd < w.skip) return;     // diff_atoms_kernel skips its rows
+      if (!(nd < w.hot)) return;  // a hot tile
+    }
     mb = warp % t.n_chunk * t.chunk_rows;
     me = min(me, mb + t.chunk_rows);
   }
@@ -955,6 +967,7 @@ __global__ void __launch_bounds__(kDiffBlock)
   const DiffGrad grad(w, temp);
   DiffPower power;
   FF dtw{0.0f, 0.0f};
+  bool some = false;
   ExpColumnV CV;
   CV.C.init_consts(L.consts(cols));
   CV.reset_v();
@@ -980,7 +993,10 @@ __global__ void __launch_bounds__(kDiffBlock)
                   const FF V[7] = {FF{CV.V0.h.x, CV.V0.l.x}, FF{CV.V0.h.y, CV.V0.l.y}, CV.Vc,
                                    FF{CV.V2.h.x, CV.V2.l.x}, FF{CV.V2.h.y, CV.V2.l.y},
                                    FF{CV.V3.h.x, CV.V3.l.x}, FF{CV.V3.h.y, CV.V3.l.y}};
-                  if (grad.cell(W, V, Gf, dtw)) p1 = power.at(L, top - lo);
+                  if (grad.cell(W, V, Gf, dtw)) {
+                    p1 = power.at(L, top - lo);
+                    some = true;
+                  }
                 }
               }
               TCW_DCHECK(m < t.N_t0);
@@ -991,6 +1007,10 @@ __global__ void __launch_bounds__(kDiffBlock)
               scr[32 * 8] = p1.l;
             });
   add_grad_tau(L, dtw, grad_tau + 2u * k);
+  if (!kHot && t.whole) {  // (no estimate: for diff_atoms_kernel)
+    some = __any_sync(0xffffffffu, some);
+    if (lane == 0) need[t.part_off + cg] = some ? INFINITY : -INFINITY;
+  }
 }
 
 // Most atoms of a template that diff_hot_kernel keeps in shared memory.
@@ -1356,11 +1376,12 @@ __global__ void __launch_bounds__(kDiffBlock)
   if (threadIdx.x == 0 && n) atomicAdd(groups, n);
 }
 
-// The transposed recurrence over one 64-atom segment of one column group, in
-// double-word FP32, from the adjoint sources of the rows in the group's
-// weighted chunks.  kEnds: leaves H at the segment's end, started from zero,
-// in `cend`; else starts from the ends below and adds every atom's sum over
-// the warp's columns to the gradient.
+// The transposed recurrence over one segment of 2^a_shift atoms of one column
+// group, in double-word FP32, from the adjoint sources of the rows in the
+// group's weighted chunks.  kEnds: leaves H at the segment's end, started from
+// zero, in `cend` (but for the last segment, whose end nothing reads); else
+// starts from the ends below and adds every atom's sum over the warp's columns
+// to the gradient.
 template <bool kEnds>
 __global__ void __launch_bounds__(kDiffBlock)
     diff_atoms_kernel(const DiffTemplate *__restrict__ T, const uint32_t *__restrict__ list,
@@ -1377,7 +1398,7 @@ __global__ void __launch_bounds__(kDiffBlock)
   const DiffTemplate &t = L.t;
   const uint32_t wi = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
   const uint32_t scg = wi / t.n_aseg, cg = cg0 + scg, as = wi % t.n_aseg;
-  if (scg >= cgs || cg >= t.n_cg) return;
+  if (scg >= cgs || cg >= t.n_cg || (kEnds && as + 1u >= t.n_aseg)) return;
   // the group's weighted chunks: first and last
   uint32_t c0 = 0xFFFFFFFFu, c1 = 0;
   {
@@ -1416,7 +1437,8 @@ __global__ void __launch_bounds__(kDiffBlock)
     const uint32_t i_begin = exp_lo(__ldg(t0s + rb), t.g);
     const uint32_t i_end =
         __reduce_max_sync(0xffffffffu, L.active ? row_end(re - 1u) : i_begin);
-    const uint32_t a = max(i_begin, as * kDiffAtomSeg), b = min(i_end, (as + 1u) * kDiffAtomSeg);
+    const uint32_t a = max(i_begin, as << t.a_shift);
+    const uint32_t b = as + 1u < t.n_aseg ? min(i_end, (as + 1u) << t.a_shift) : i_end;
     if (a >= b) return;
     const ExpConsts kc = cc.consts();
     const ExpConsts2 kp = exp_consts2(kc);
@@ -1426,10 +1448,10 @@ __global__ void __launch_bounds__(kDiffBlock)
     FF H2{0.0f, 0.0f};
     float *ends = cend + (t.cend_off + (size_t)scg * t.n_aseg) * kDiffSegFloats + lane;
     if (!kEnds) {  // H = r^len H + end, segment by segment from the first
-      const uint32_t s0 = i_begin / kDiffAtomSeg;
-      FF R = kc.r1;  // r^64
+      const uint32_t s0 = i_begin >> t.a_shift;
+      FF R = kc.r1;  // r^(2^a_shift)
 #pragma unroll 1
-      for (int q = 0; q < 6; q++) R = ff_mul(R, R);
+      for (uint32_t q = 0; q < t.a_shift; q++) R = ff_mul(R, R);
       const FF R2 = ff_mul(R, R);
       const F2 rh0{R2.h, R2.h}, nrh0{-R2.h, -R2.h}, rl0{R2.l, R2.l};
       const F2 rh1{R.h, R.h}, nrh1{-R.h, -R.h}, rl1{R.l, R.l};
@@ -1536,8 +1558,8 @@ __global__ void __launch_bounds__(kDiffBlock)
       }
     }
     if (kEnds) {
-      // a first segment that starts inside its 64 atoms ends at the same
-      // atom as a whole one: joins decay by r^64 from end to end
+      // a first segment that starts inside its atoms ends at the same atom as
+      // a whole one: joins decay by r^(2^a_shift) from end to end
       float *o = ends + (size_t)as * kDiffSegFloats;
       const float v[14] = {H01.h.x, H01.h.y, H01.l.x, H01.l.y, H2.h,    H2.l,    H34.h.x,
                            H34.h.y, H34.l.x, H34.l.y, H56.h.x, H56.h.y, H56.l.x, H56.l.y};
@@ -1939,8 +1961,9 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
               L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, nullptr, nullptr, L.temp, nullptr,
               nullptr, nullptr, nullptr, g.seg_per, L.seg);
       for (const DiffClass *c = c0; c < c1; c++)
-        diff_est_kernel<<<warps(c, c->max_tiles), kDiffBlock, 0, stream>>>(
-            L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.est);
+        if (c->est_tiles)
+          diff_est_kernel<<<warps(c, c->est_tiles), kDiffBlock, 0, stream>>>(
+              L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.seg, L.need, L.est);
       // (one slice unless the group is one large template in its backward pass)
       for (uint32_t cg0 = 0; cg0 < g.max_cg; cg0 += g.cg_slice) {
         const uint32_t cgs = g.max_cg - cg0 < g.cg_slice ? g.max_cg - cg0 : g.cg_slice;
@@ -2001,9 +2024,10 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
           return e;
         if (pass == 1) {
           for (const DiffClass *c = c0; c < c1; c++)
-            diff_atoms_kernel<true><<<warps(c, c->slice_aseg), kDiffBlock, 0, stream>>>(
-                L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1,
-                L.lnZ2, L.gB, L.gS, cg0, cgs, L.scratch, L.cend, L.grad_atoms);
+            if (c->slice_ends)
+              diff_atoms_kernel<true><<<warps(c, c->slice_ends), kDiffBlock, 0, stream>>>(
+                  L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1,
+                  L.lnZ2, L.gB, L.gS, cg0, cgs, L.scratch, L.cend, L.grad_atoms);
           for (const DiffClass *c = c0; c < c1; c++)
             diff_atoms_kernel<false><<<warps(c, c->slice_aseg), kDiffBlock, 0, stream>>>(
                 L.T, L.exp_list + c->y0, L.atoms8, L.t0s, L.cols, L.need, L.est, L.temp, L.lnZ1,

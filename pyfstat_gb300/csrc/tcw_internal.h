@@ -334,19 +334,22 @@ struct DiffTemplate {
   double tau_min, tau_max;
   uint32_t part_off, n_parts;  // this template's tiles (need, partials)
   uint32_t window;
-  uint32_t whole;  // its tiles are whole columns and none is walked apart
+  uint32_t whole;  // its tiles are whole columns, without an estimate; none is walked apart
   uint64_t p_off;
   uint32_t n_cg, n_chunk, chunk_rows;
-  uint32_t g_shift, g_nseg, n_aseg;  // segment sums; atom segments of the transposed recurrence
+  uint32_t g_shift, g_nseg;          // segment sums
+  uint32_t n_aseg, a_shift;          // segments of 2^a_shift atoms of the transposed recurrence
   uint64_t col_off;   // column constants
   uint64_t seg_off;   // segment sums, in 32-lane blocks of one segment
   uint64_t scr_off;   // backward: adjoint sources, in floats
   uint64_t cend_off;  // backward: recurrence ends, in 32-lane blocks
 };
 // Adjoint sources of one cell in the backward pass's scratch (7 channels and
-// r^L as a float pair) and atoms per segment of the transposed recurrence.
+// r^L as a float pair), least atoms per segment of the transposed recurrence and
+// most segments (a segment joins the ends of all below it).
 #define TCW_DIFF_SLOTS 9u
-constexpr uint32_t kDiffAtomSeg = 64u;
+constexpr uint32_t kDiffAtomShift = 6u, kDiffAtomSeg = 1u << kDiffAtomShift;
+constexpr uint32_t kDiffMaxAseg = 4096u;
 // Floats of one 32-column segment: window sums (forward), with their
 // tau derivatives (backward).
 constexpr uint32_t kDiffSegFloats = 14u * 32u;
@@ -363,6 +366,8 @@ struct DiffClass {
   uint32_t max_tiles, max_segs, max_atoms, max_cols;
   uint32_t slice_tiles, slice_aseg;  // most tiles / atom segments in a slice
   uint32_t slice_cg;                 // most column groups in a slice
+  // most tiles that are estimated, most atom segments that leave their ends
+  uint32_t est_tiles, slice_ends;
 };
 // Exponential templates [y0, y0 + ny) of exp_list with workspaces of their
 // own: a backward pass runs in groups that bound the scratch, a group of one
