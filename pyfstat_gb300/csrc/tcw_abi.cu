@@ -1332,11 +1332,14 @@ static uint64_t diff_end_bytes(const DiffTemplate &t) {
 // most of them hold a cell that matters by itself, and the walk that
 // diff_hot_kernel would repeat is then the tile's own, bit for bit.  Whole columns
 // go without the estimate, a walk as long as their own that skips nothing where
-// signals are weak, and, from four warps per scheduler on, without the segments
-// of the transposed recurrence (one pass in place of two).  More atoms make the
+// signals are weak -- but for the forward pass of few atoms per row, whose FP64 F
+// is most of the work (kDiffEstAtoms; with / without it, noise and a loud signal:
+// 500 templates of 400 atoms, 32 x 600 cells 2.6, 1.3 / 1.9, 1.7 ms, 2000 of 1500,
+// 32 x 128 6.0, 4.4 / 2.7, 2.7) -- and, from four warps per scheduler on, without
+// the segments of the transposed recurrence (one pass in place of two).  More atoms make the
 // walk the longest chain (64 rows of 17532 atoms among 300 templates: 12.5 + 14.7
 // -> 26 + 34 ms), so they are cut.
-constexpr uint32_t kDiffFewRows = 64, kDiffFewAtoms = 2048;
+constexpr uint32_t kDiffFewRows = 64, kDiffFewAtoms = 2048, kDiffEstAtoms = 14;
 // Warps of a class's grid that have no tile: above this, half a millisecond of
 // empty blocks, the templates of unequal size go in launches of their own,
 // each of which lasts as long as its longest tile (gradients of 2000 templates
@@ -1382,7 +1385,9 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     t.n_chunk = (t.N_t0 + t.chunk_rows - 1u) / t.chunk_rows;
     if (t.n_chunk == 1u || t.g.numAtoms < 64u) t.g_nseg = 0;
     const bool tiny = 2u * (uint64_t)t.g.numAtoms + 10u * (uint64_t)t.N_t0 <= 512u;
-    t.whole = t.n_chunk == 1u && ((filled && t.g.numAtoms <= kDiffFewAtoms) || tiny) ? 1u : 0u;
+    if (t.n_chunk == 1u && ((filled && t.g.numAtoms <= kDiffFewAtoms) || tiny))
+      t.whole = !pass && filled && t.g.numAtoms / kDiffEstAtoms < t.N_t0 ? kDiffWhole
+                                                                       : kDiffWholeBlind;
     if (!t.whole) g.hot += t.n_cg;
     t.a_shift = kDiffAtomShift;
     while (((t.g.numAtoms - 1u) >> t.a_shift) >= (t.whole && full ? 1u : kDiffMaxAseg)) t.a_shift++;
@@ -1418,7 +1423,7 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
     c.slice_tiles = std::max(c.slice_tiles, cgs * t.n_chunk);
     c.slice_aseg = std::max(c.slice_aseg, cgs * t.n_aseg);
     c.slice_cg = std::max(c.slice_cg, cgs);
-    if (!t.whole) c.est_tiles = std::max(c.est_tiles, t.n_cg * t.n_chunk);
+    if (t.whole != kDiffWholeBlind) c.est_tiles = std::max(c.est_tiles, t.n_cg * t.n_chunk);
     if (t.n_aseg > 1u) c.slice_ends = std::max(c.slice_ends, cgs * t.n_aseg);
   }
   g.n_classes = (uint32_t)classes.size() - g.c0;

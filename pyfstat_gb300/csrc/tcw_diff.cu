@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(kDiffBlock, 8)
   L.t = T[k];
   const uint32_t tile = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
   const uint32_t cg = tile / L.t.n_chunk, mb = tile % L.t.n_chunk * L.t.chunk_rows;
-  if (cg >= L.t.n_cg || L.t.whole) return;
+  if (cg >= L.t.n_cg || L.t.whole == kDiffWholeBlind) return;
   const uint32_t me = min(L.t.N_t0, mb + L.t.chunk_rows);
   L.columns(atoms8, t0s_all, cg);
   ExpColumn<false, true, true> C;
@@ -711,13 +711,13 @@ __global__ void __launch_bounds__(kDiffBlock, 5)
     if (!hot.any()) return;
     mb = hot.first * L.t.chunk_rows;
   } else {
-    if (!L.t.whole) {
+    if (L.t.whole != kDiffWholeBlind) {
       const float nd = need[L.t.part_off + warp];
       if (nd < skip0) {
         if (lane == 0) *out = DiffPartial{-INFINITY, 0.0, -INFINITY, 0.0};
         return;
       }
-      if (!(nd < bd.hot)) return;  // a hot tile
+      if (!(nd < bd.hot) && !L.t.whole) return;  // a hot tile
     }
     mb = warp % L.t.n_chunk * L.t.chunk_rows;
     me = min(me, mb + L.t.chunk_rows);
@@ -729,7 +729,7 @@ __global__ void __launch_bounds__(kDiffBlock, 5)
                         ? seg + (L.t.seg_off + (size_t)cg * L.t.g_nseg) * kDiffSegFloats + lane
                         : nullptr;
   DiffLse lse(temp, skip0);
-  const bool whole = L.t.whole != 0u;
+  const bool blind = L.t.whole == kDiffWholeBlind;
   const double below = no_weight_below(temp);
   diff_rows(L, mb, me, C, sg, kDiffSegFloats, s_tab[threadIdx.x >> 5],
             [&](uint32_t m, uint32_t, uint32_t, bool data) {
@@ -747,7 +747,7 @@ __global__ void __launch_bounds__(kDiffBlock, 5)
                 W[6] = (double)C.W3.h.y + (double)C.W3.l.y;
               }
               lse.cell(data, W, t1, F32);
-              if (!kHot && whole) lse.follow(below);
+              if (!kHot && blind) lse.follow(below);
             });
   const DiffPartial p = lse.merge();
   if (!kHot) {

@@ -334,7 +334,7 @@ struct DiffTemplate {
   double tau_min, tau_max;
   uint32_t part_off, n_parts;  // this template's tiles (need, partials)
   uint32_t window;
-  uint32_t whole;  // its tiles are whole columns, without an estimate; none is walked apart
+  uint32_t whole;  // its tiles are whole columns, none walked apart: kDiffWhole, kDiffWholeBlind
   uint64_t p_off;
   uint32_t n_cg, n_chunk, chunk_rows;
   uint32_t g_shift, g_nseg;          // segment sums
@@ -350,6 +350,8 @@ struct DiffTemplate {
 #define TCW_DIFF_SLOTS 9u
 constexpr uint32_t kDiffAtomShift = 6u, kDiffAtomSeg = 1u << kDiffAtomShift;
 constexpr uint32_t kDiffMaxAseg = 4096u;
+// DiffTemplate::whole: with an estimate, without one.
+constexpr uint32_t kDiffWhole = 1u, kDiffWholeBlind = 2u;
 // Floats of one 32-column segment: window sums (forward), with their
 // tau derivatives (backward).
 constexpr uint32_t kDiffSegFloats = 14u * 32u;
