@@ -1326,7 +1326,7 @@ static uint64_t diff_end_bytes(const DiffTemplate &t) {
 // walk them last as long as their longest tile (24 templates 3.19 -> 2.99 ms,
 // 100 5.4 -> 5.0, 600 17.8 -> 12.9; two 2.98 / 5.1 / 14.3, eight 3.1: the
 // estimate starts too many chunks).
-// Where whole columns give every scheduler a warp, templates of few rows and
+// Where whole columns give most schedulers a warp, templates of few rows and
 // atoms keep whole columns (so do the shortest columns of any batch, 10 x 10
 // cells of 48 atoms 235 -> 223 us): a handful of chunks per column buys little,
 // most of them hold a cell that matters by itself, and the walk that
@@ -1353,7 +1353,7 @@ static void diff_tile_group(const tcw_handle *h, std::vector<DiffTemplate> &T,
   uint64_t total_cg = 0;
   for (uint32_t y = y0; y < y1; y++) total_cg += (T[elist[y]].N_tau + 31u) / 32u;
   const uint64_t chunks = ((uint64_t)h->n_sms * 128u + total_cg - 1u) / total_cg;
-  const bool filled = total_cg >= (uint64_t)h->n_sms * 4u;
+  const bool filled = total_cg >= (uint64_t)h->n_sms * 3u;
   const bool full = total_cg >= (uint64_t)h->n_sms * 16u;
   const uint64_t seg_floats = pass ? kDiffSegFloatsV : kDiffSegFloats;
   uint64_t seg = 0, scr = 0, cend = 0;
