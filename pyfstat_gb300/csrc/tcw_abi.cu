@@ -1295,6 +1295,7 @@ struct DiffSetup {
   size_t o_T, o_parts, o_t0, o_est, o_hot, o_rlist, o_ident, o_RT, o_P, o_B64, o_D64, o_elist, o_A8;
   size_t o_cols, o_seg, o_need, o_scratch, o_cend, total;
   uint32_t n_rect, max_rect_tiles, max_rect_atoms, n_exp;
+  uint32_t max_parts;  // most tiles of one template
   uint64_t p_rows, seg_floats;
   std::vector<DiffGroup> groups;
   std::vector<DiffClass> classes;
@@ -1540,6 +1541,7 @@ static int diff_setup(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n, cons
       for (uint32_t k : *l) {
         T[k].part_off = (uint32_t)n_tiles;
         T[k].n_parts = T[k].n_cg * T[k].n_chunk;
+        S.max_parts = std::max(S.max_parts, T[k].n_parts);
         n_tiles += T[k].n_parts;
         if (n_tiles > 0xFFFFFFF0ull) return set_err(h, TCW_ERR_OVERFLOW, "too many tiles");
       }
@@ -1646,8 +1648,8 @@ int tcw_map_forward(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n_templat
   DiffLaunch L = diff_launch(h, S, d_atoms, temperature);
   TCW_CUDA(h, launch_diff(0, L, S.groups.data(), (uint32_t)S.groups.size(), S.classes.data(),
                           h->stream, h->side_stream, h->fork_ev, h->join_ev));
-  TCW_CUDA(h, launch_diff_finalize(L.T, n_templates, L.parts, temperature, d_lnBtSG, d_softmax2F,
-                                   h->stream));
+  TCW_CUDA(h, launch_diff_finalize(L.T, n_templates, S.max_parts, L.parts, temperature, d_lnBtSG,
+                                   d_softmax2F, h->stream));
   return TCW_OK;
 }
 

@@ -1883,15 +1883,18 @@ __global__ void __launch_bounds__(kScanBlock)
 }
 
 // One block per template: its partials brought to their maximum and added
-// (one warp: 33 us for the 2048 partials of a lone template, now 8).
+// (one warp: 33 us for the 2048 partials of a lone template, now 8), one warp
+// where there are few, as the FP64 maxima and sums of idle warps cost as much as
+// theirs (2000 templates of 4 x 4 cells 73 us by eight warps each).
 __global__ void __launch_bounds__(256)
     diff_finalize_kernel(const DiffTemplate *__restrict__ T, const DiffPartial *__restrict__ parts,
                          double temp, double *__restrict__ lnB, double *__restrict__ soft) {
   __shared__ DiffPartial sh[8];
   const uint32_t k = blockIdx.x, lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  const uint32_t warps = blockDim.x >> 5;
   const DiffTemplate t = T[k];
   DiffPartial a{-INFINITY, 0.0, -INFINITY, 0.0};
-  for (uint32_t p = threadIdx.x; p < t.n_parts; p += 256u) {
+  for (uint32_t p = threadIdx.x; p < t.n_parts; p += blockDim.x) {
     a.m1 = fmax(a.m1, parts[t.part_off + p].m1);
     a.m2 = fmax(a.m2, parts[t.part_off + p].m2);
   }
@@ -1902,11 +1905,11 @@ __global__ void __launch_bounds__(256)
   }
   if (lane == 0) sh[wid] = a;
   __syncthreads();
-  for (int w = 0; w < 8; w++) {
+  for (uint32_t w = 0; w < warps; w++) {
     a.m1 = fmax(a.m1, sh[w].m1);
     a.m2 = fmax(a.m2, sh[w].m2);
   }
-  for (uint32_t p = threadIdx.x; p < t.n_parts; p += 256u) {
+  for (uint32_t p = threadIdx.x; p < t.n_parts; p += blockDim.x) {
     const DiffPartial q = parts[t.part_off + p];
     if (q.s1 != 0.0) a.s1 += q.s1 * exp(q.m1 - a.m1);
     if (q.s2 != 0.0) a.s2 += q.s2 * exp(q.m2 - a.m2);
@@ -1921,7 +1924,7 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   if (threadIdx.x == 0) {
     double s1 = 0.0, s2 = 0.0;
-    for (int w = 0; w < 8; w++) {
+    for (uint32_t w = 0; w < warps; w++) {
       s1 += sh[w].s1;
       s2 += sh[w].s2;
     }
@@ -2066,11 +2069,12 @@ cudaError_t launch_diff(int pass, const DiffLaunch &L, const DiffGroup *groups, 
   return cudaSuccess;
 }
 
-cudaError_t launch_diff_finalize(const DiffTemplate *T, uint32_t n_templates,
+cudaError_t launch_diff_finalize(const DiffTemplate *T, uint32_t n_templates, uint32_t max_parts,
                                  const DiffPartial *parts, double temp, double *lnB, double *soft,
                                  cudaStream_t stream) {
   if (n_templates == 0) return cudaSuccess;
-  diff_finalize_kernel<<<n_templates, 256, 0, stream>>>(T, parts, temp, lnB, soft);
+  const uint32_t threads = max_parts <= 64u ? 32u : 256u;
+  diff_finalize_kernel<<<n_templates, threads, 0, stream>>>(T, parts, temp, lnB, soft);
   return cudaGetLastError();
 }
 

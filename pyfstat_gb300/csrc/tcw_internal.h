@@ -427,7 +427,8 @@ unsigned int dcheck_failures_noalloc();
 cudaError_t launch_map_f64(int window, const float *atoms, const Geom &g, const uint32_t *t0s,
                            const uint32_t *taus, uint32_t N_tau, const uint32_t *rows,
                            uint32_t n_rows, double *F, double *cond, cudaStream_t stream);
-cudaError_t launch_diff_finalize(const DiffTemplate *T, uint32_t n_templates,
+// max_parts: the most tiles of one template.
+cudaError_t launch_diff_finalize(const DiffTemplate *T, uint32_t n_templates, uint32_t max_parts,
                                  const DiffPartial *parts, double temp, double *lnB, double *soft,
                                  cudaStream_t stream);
 
