@@ -20,12 +20,15 @@
 //
 // Exponential templates are tiled by 32 tau columns x a chunk of t0 rows, one
 // warp per tile; a chunk's first window is joined from segment sums
-// (ExpColumn::warm_start), so that a single template fills the GPU.
+// (ExpColumn::warm_start), so that a single template fills the GPU.  Batches of
+// templates of few rows keep whole columns (DiffTemplate::whole).
 //
 //   diff_est_kernel  FP32 only: the tile's largest tier-1 F (`need`, infinite
 //            where a cell has none) and a lower bound of the template's
 //            maximum.  With a signal almost no tile holds a cell that carries
 //            weight, and the FP64 and adjoint work below skips whole tiles.
+//   diff_hot_kernel  the tiles whose cells matter by themselves, their columns
+//            walked whole (many of them: by the kHot forms of the next two);
 //   diff_fwd_kernel  the tiles that may carry weight: double-word window
 //            sums, FP64 log-sum-exps of F and 2F/T -> partials -> finalize
 //            per template.
@@ -37,14 +40,15 @@
 //   diff_atoms_kernel  per column, atoms ascending, the transposed recurrence
 //            H(i) = r H(i-1) + sum_{lo(m)=i} G(m) - sum_{hi(m)+1=i} G(m)
 //            r^(L(m)) in double-word FP32 gives dL/dx(i) = H(i).  It is linear
-//            in H, so it runs in segments of 64 atoms side by side: a first
-//            pass leaves each segment's end from H = 0, a second one joins the
-//            ends below its segment, walks it again and adds each warp's 32
+//            in H, so it runs in segments of 64 atoms and more side by side: a
+//            first pass leaves each segment's end from H = 0, a second one joins
+//            the ends below its segment, walks it again and adds each warp's 32
 //            columns per atom (recursive halving over the 7 channels) to the
 //            FP64 atom gradient.
 // Measured (forward + backward, 2000 atoms, 1024 x 1024 cells, signal): one
 // template 7.7-9.6 -> 1.6 ms (one block per 128 columns and all rows before),
-// 24 templates 16.5 -> 3.0 ms, 256 templates 53 -> 24 ms.
+// 24 templates 16.5 -> 3.0 ms, 256 templates 53 -> 22 ms; noise alone: 6.9 -> 0.9,
+// 17.6 -> 7.9, 101 -> 85 ms.
 // The window-sum factor e^(-k (t_lo - t0)/tau) is left out everywhere: F does
 // not depend on it, so neither do g, dF/dW (in this frame) or dF/dtau.
 //

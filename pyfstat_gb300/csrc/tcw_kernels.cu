@@ -1,8 +1,9 @@
 // CUDA kernels of the transient-CW F-statistic map for GB300 (sm_103a).
 //
-//   prefix_kernel    compensated exclusive prefix sums of the 7 atom channels of
-//                    each rectangular template (one block per template), stored
-//                    as quantised double-word rows (see tcw_cell.h)
+//   prefix kernels   compensated exclusive prefix sums of the 7 atom channels of
+//                    each rectangular template (a cluster of blocks per template,
+//                    one block each where there are many), stored as quantised
+//                    double-word rows (see tcw_cell.h)
 //   map_kernel       the (t0, tau) cells of a list of tiles; a block owns one tile
 //                    (grid launch) or pulls tiles from an atomic counter
 //                    (persistent launch).  Rectangular tiles difference two prefix
