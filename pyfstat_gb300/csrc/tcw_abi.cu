@@ -1529,10 +1529,9 @@ static int diff_setup(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n, cons
     // rectangular tiles: as many column chunks per row group as give every
     // resident warp a tile, at least 16 columns each; where the row groups alone
     // keep the FP64 pipe busy (two warps per SM) 64 columns, as each chunk sums
-    // its first window anew, but for what fills a block of four tiles (forward /
-    // backward, noise: 500 templates of 1500 atoms, 4 x 128 cells 1.45 / 1.58 ->
-    // 1.16 / 1.46 ms; of 100 atoms, 128 x 32 0.84 / 1.32 -> 0.67 / 1.08; 24 of 1024
-    // x 1024 6.05 / 6.22, as before)
+    // its first window anew (forward / backward, noise: 500 templates of 1500
+    // atoms, 4 x 128 cells 1.45 / 1.58 -> 1.07 / 1.40 ms; of 100 atoms, 128 x 32
+    // 0.84 / 1.32 -> 0.67 / 1.07; 2000 of 480, 32 x 32 1.49 / 1.53 -> 1.29 / 1.42)
     const bool busy = row_groups >= (uint64_t)h->n_sms * 2u;
     const uint64_t rchunks =
         row_groups ? ((uint64_t)h->n_sms * 32u + row_groups - 1u) / row_groups : 1u;
@@ -1540,7 +1539,7 @@ static int diff_setup(tcw_handle *h, const tcw_diff_desc *desc, uint32_t n, cons
       DiffTemplate &t = T[k];
       uint64_t nc = std::max<uint64_t>(1, std::min<uint64_t>(rchunks, (t.N_tau + 15u) / 16u));
       if (busy)
-        nc = std::min<uint64_t>(nc, std::max((t.N_tau + 63u) / 64u, (t.n_cg + 3u) / t.n_cg));
+        nc = std::min<uint64_t>(nc, (t.N_tau + 63u) / 64u);
       t.chunk_rows = (uint32_t)((t.N_tau + nc - 1) / nc);
       t.n_chunk = (t.N_tau + t.chunk_rows - 1u) / t.chunk_rows;
       S.max_rect_tiles = std::max(S.max_rect_tiles, t.n_cg * t.n_chunk);
